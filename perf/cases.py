@@ -49,9 +49,9 @@ def listed():
         # a batch of padded sentences through two encoder layers of the usual base size
         {"name": "encode_padded", "kind": "encode", "batch": 32, "seq": 384, "d": 768, "heads": 12, "ffn": 3072, "vocab": 30522, "layers": 2},
         # the 28x28 stage of ResNet-50 at the benchmark's batch, entered with a stride
-        {"name": "residual_28", "kind": "residual", "batch": 256, "size": 56, "cin": 256, "width": 128, "stride": 2, "stride_in": "1x1", "classes": 64},
-        # a small batch of odd-sized images, the stride on the 3x3 convolution
-        {"name": "residual_odd", "kind": "residual", "batch": 24, "size": 35, "cin": 192, "width": 96, "stride": 2, "stride_in": "3x3", "classes": 37},
+        {"name": "residual_28", "kind": "residual", "batch": 256, "size": 56, "cin": 256, "width": 128, "stride": 2, "classes": 64},
+        # a small batch of odd-sized images, channels that are no power of two
+        {"name": "residual_odd", "kind": "residual", "batch": 24, "size": 35, "cin": 192, "width": 96, "stride": 2, "classes": 37},
         # the 28x28 stage of a MobileNet-style network
         {"name": "mobile_28", "kind": "mobile", "batch": 128, "size": 56, "cin": 24, "cout": 32, "expand": 6, "k": 3, "stride": 2, "classes": 21},
         # a forecaster over windows of a multivariate series
@@ -83,8 +83,7 @@ def draw(rng):
     if kind == "residual":
         size, cin, width = rng.choice([(56, 64, 64), (56, 256, 128), (28, 512, 256), (14, 1024, 512)])
         size = max(7, size + rng.randint(-3, 3))
-        return {"kind": kind, "batch": _log(rng, 8, 192), "size": size, "cin": cin, "width": width, "stride": rng.choice([1, 2]),
-                "stride_in": rng.choice(["1x1", "3x3"]), "classes": _log(rng, 2, 150)}
+        return {"kind": kind, "batch": _log(rng, 8, 192), "size": size, "cin": cin, "width": width, "stride": rng.choice([1, 2]), "classes": _log(rng, 2, 150)}
     if kind == "mobile":
         size, cin, cout = rng.choice([(112, 16, 24), (56, 24, 32), (28, 32, 64), (14, 96, 160)])
         size = max(7, size + rng.randint(-3, 3))
@@ -148,9 +147,8 @@ def _residual(c):
     def conv(t, filters, k, stride=1):
         return L.BatchNormalization(epsilon=1.001e-5)(L.Conv2D(filters, k, strides=stride, padding="same", use_bias=False)(t))
 
-    first, second = (s, 1) if c["stride_in"] == "1x1" else (1, s)
-    t = L.ReLU()(conv(x, w, 1, first))
-    t = L.ReLU()(conv(t, w, 3, second))
+    t = L.ReLU()(conv(x, w, 1, s))
+    t = L.ReLU()(conv(t, w, 3))
     t = conv(t, 4 * w, 1)
     h = L.ReLU()(L.Add()([conv(x, 4 * w, 1, s), t]))
     t = L.ReLU()(conv(h, w, 1))
@@ -242,11 +240,12 @@ def _weights(c, seed):
     # In the convolutional cases the weights are whole 16-bit numbers and the shifts keep most rectifiers open: each rectifier
     # that rounding turns over costs its whole gradient, and the comparison with 64 bits would see little else
     exactly = c["kind"] not in ("residual", "mobile")
+    open_at = 1.0 if c["kind"] == "residual" else 1.5  # wider open, and the gradients of the shifts in front of a normalised convolution cancel
     g = _generator(seed, 1)
     out = []
     for shape, fan in _shapes(c):
         t = torch.randn(shape, generator=g, device="cuda")
-        t = 1.0 + 0.1 * t if fan == 0 else 0.05 * t if fan == -1 else 0.6 + 0.4 * t if fan == -2 else t * fan ** -0.5
+        t = 1.0 + 0.1 * t if fan == 0 else 0.05 * t if fan == -1 else open_at + 0.5 * t if fan == -2 else t * fan ** -0.5
         out.append(t if exactly else t.bfloat16().float())
     return out
 
@@ -294,7 +293,7 @@ def prepare(case, seed):
     elif float32:
         optimizer = keras.optimizers.Adam(learning_rate=1e-3)
     else:
-        optimizer = keras.optimizers.SGD(learning_rate=0.1, momentum=0.9)
+        optimizer = keras.optimizers.SGD(learning_rate=0.01, momentum=0.9)
     loss = keras.losses.MeanSquaredError() if case["kind"] == "lstm" else keras.losses.SparseCategoricalCrossentropy(from_logits=True)
     model.compile(optimizer=optimizer, loss=loss)
     optimizer.build(model.trainable_variables)
@@ -415,10 +414,9 @@ def _exact_residual(c, w, x):
     w = list(w)
     x = x.permute(0, 3, 1, 2)
     s = c["stride"]
-    first, second = (s, 1) if c["stride_in"] == "1x1" else (1, s)
     eps, relu = 1.001e-5, torch.relu
-    t = relu(_bn64(_conv64(x, w[0], first), w[1], w[2], eps))
-    t = relu(_bn64(_conv64(t, w[3], second), w[4], w[5], eps))
+    t = relu(_bn64(_conv64(x, w[0], s), w[1], w[2], eps))
+    t = relu(_bn64(_conv64(t, w[3], 1), w[4], w[5], eps))
     short, t = _conv64(x, w[6], s), _conv64(t, w[7], 1)
     h = relu(_bn64(short, w[8], w[9], eps) + _bn64(t, w[10], w[11], eps))
     t = relu(_bn64(_conv64(h, w[12], 1), w[13], w[14], eps))
@@ -479,7 +477,7 @@ def exact(case, seed):
     for t, g in zip(w, grads):
         t = t.detach()
         if k in ("residual", "mobile"):
-            m = -0.1 * g
+            m = -0.01 * g
             new = t + m
         else:
             lr = 3e-4 if k == "lm" else 1e-3
@@ -521,23 +519,21 @@ def work(case):
         s, n, o, stride = case["size"], 0, -(-case["size"] // case["stride"]), case["stride"]
         if k == "residual":
             ci, w = case["cin"], case["width"]
-            mid = o if case["stride_in"] == "1x1" else s
-            convs = [(mid, ci, w, 1, s if mid == s else o), (o, w, w, 9, mid), (o, w, 4 * w, 1, o), (o, ci, 4 * w, 1, o), (o, 4 * w, w, 1, o), (o, w, w, 9, o),
-                     (o, w, 4 * w, 1, o)]
+            convs = [(o, ci, w, 1), (o, w, w, 9), (o, w, 4 * w, 1), (o, ci, 4 * w, 1), (o, 4 * w, w, 1), (o, w, w, 9), (o, w, 4 * w, 1)]
         else:
             convs = []
             for ci, si, so in ((case["cin"], s, o), (case["cout"], o, o)):
                 e = case["expand"] * ci
-                convs += [(si, ci, e, 1, si), (so, 1, e, case["k"] ** 2, si), (so, e, case["cout"], 1, so)]
-        macs = sum(b * so * so * ci * co * taps for so, ci, co, taps, _ in convs) + b * o * o * convs[-1][2] * case["classes"]
+                convs += [(si, ci, e, 1), (so, 1, e, case["k"] ** 2), (so, e, case["cout"], 1)]
+        macs = sum(b * so * so * ci * co * taps for so, ci, co, taps in convs) + b * o * o * convs[-1][2] * case["classes"]
         size += 4 * b * s * s * case["cin"]
         # each activation written, normalised and read on the way there, and its gradient twice on the way back, in 16 bits
-        size += sum(2 * b * so * so * co * 5 for so, _, co, _, _ in convs)
+        size += sum(2 * b * so * so * co * 5 for so, _, co, _ in convs)
     return {"bytes": int(size), "flops": int(2 * macs * (3 if training else 1))}
 
 
 def tolerance(case):
     # about four times the largest error against 64 bits over listed and drawn cases: 5e-7 in float32, 0.007 of logits and
-    # states, 0.01 of a decoder's gradients; a convolutional step's first gradients are 0.03 to 0.08 off, because each rectifier
-    # that rounding turns over adds its whole gradient, and two implementations differ by about as much
-    return {"rel": {"mlp": 1e-5, "lstm": 1e-5, "infer": 0.03, "encode": 0.03, "lm": 0.05}.get(case["kind"], 0.15)}
+    # states, 0.01 of a decoder's gradients; a convolutional step's first gradients are 0.02 to 0.04 off, because each rectifier
+    # that rounding turns over adds its whole gradient: two implementations round most of them alike
+    return {"rel": {"mlp": 1e-5, "lstm": 1e-5}.get(case["kind"], 0.03)}
