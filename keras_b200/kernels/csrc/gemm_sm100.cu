@@ -325,6 +325,247 @@ gemm_bf16_tcgen05_persistent(const __grid_constant__ CUtensorMap map_a, const __
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(v2::TMEM_COLS) : "memory");
   }
 }
+
+// ---------------------------------------------------------------------------------------------
+// CTA-pair variant (cta_group::2): two CTAs of a cluster compute one 256 x 256 tile.  Each holds its own 128 rows of A, half of
+// the B tile and the accumulator of its 128 rows; the even CTA issues the MMAs for both.
+//
+// What bounds the one-CTA kernel is operand traffic: a 128 x 256 tile moves 48 KB from L2 into shared memory for every 512
+// tensor-pipe cycles (96 B/clk/SM), more than L2 delivers.  A pair shares B, so the same tile costs 32 KB a CTA (64 B/clk/SM),
+// and the smaller stages leave room for eight epilogue warps.
+namespace v3 {
+constexpr int BM = 128, BN = 256, BK = 64, STAGES = 5;  // BM: rows of one CTA; BN: columns of the pair
+constexpr int EPI_WARPS = 8, PAIR_THREADS = 64 + 32 * EPI_WARPS;
+constexpr int A_BYTES = BM * BK * 2;
+constexpr int OUT_BYTES = EPI_WARPS * 2 * 4096;
+constexpr int STAGE_BYTES = A_BYTES + (BN / 2) * BK * 2;
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + OUT_BYTES + 1024 + 256;
+constexpr uint32_t TMEM_COLS = 2 * BN;  // two accumulators: the epilogue of a tile overlaps the main loop of the next
+constexpr int GROUP_M = 8;  // row tiles of 256 side by side: 74 pairs then work on a square patch of the output (4 and 16 measure the same or up to 8 % slower)
+}  // namespace v3
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// `bar` may be the peer's barrier (a shared::cluster address); the data always lands in this CTA
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+               ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
+               : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrives on the barrier at this offset in both CTAs once the MMAs issued so far are done
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  for (uint32_t it = 0; it < SPIN_LIMIT; ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if ((it & 1023u) == 1023u && *abort_flag) return false;
+  }
+  return false;
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(v3::PAIR_THREADS, 1)
+gemm_bf16_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                       const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
+  constexpr int BM = v3::BM, BN = v3::BN, BK = v3::BK, STAGES = v3::STAGES, A_BYTES = v3::A_BYTES, STAGE_BYTES = v3::STAGE_BYTES;
+  constexpr uint32_t TMEM_COLS = v3::TMEM_COLS;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
+  const uint32_t stage_out = base + STAGES * STAGE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base_ptr + STAGES * STAGE_BYTES + v3::OUT_BYTES);
+  const uint32_t bar_base = stage_out + v3::OUT_BYTES;
+  auto full_bar = [&](int s) { return bar_base + 8u * s; };              // even CTA's is used: bytes of both CTAs
+  auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };  // each CTA its own, signalled by the MMA commit
+  auto acc_full_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + a); };
+  auto acc_empty_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + 2 + a); };  // even CTA's is used
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * STAGES + 4);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * STAGES + 5);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_rank();
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int m_tiles = (p.M + 2 * BM - 1) / (2 * BM), n_tiles = (p.N + BN - 1) / BN;
+  const int split = p.split_k > 1 ? p.split_k : 1;
+  const int total_tiles = m_tiles * n_tiles * split;
+  const int k_blocks_all = (p.K + BK - 1) / BK;
+  const int kb_per = split > 1 ? p.kb_per_split : k_blocks_all;
+  auto coords = [&](int t, int& m0, int& n0) {
+    const int per_group = v3::GROUP_M * n_tiles;
+    const int g = t / per_group, first_m = g * v3::GROUP_M;
+    const int rows = min(v3::GROUP_M, m_tiles - first_m);
+    const int r = t - g * per_group;
+    m0 = (first_m + r % rows) * (2 * BM);
+    n0 = (r / rows) * BN;
+  };
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(acc_full_bar(a), 1);
+      mbar_init(acc_empty_bar(a), 2 * v3::EPI_WARPS);  // one arrival per epilogue warp of both CTAs
+    }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  __syncwarp();
+  cluster_sync_all();  // the peer signals this CTA's barriers: they must be initialised first
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer (each CTA loads its half of the stage)
+    if (elect_one()) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int t = pair; t < total_tiles && ok; t += pairs) {
+        int m0, n0;
+        coords(t / split, m0, n0);
+        m0 += rank * BM;
+        n0 += rank * (BN / 2);
+        const int kb0 = (t % split) * kb_per, kb1 = min(kb0 + kb_per, k_blocks_all);
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+          const int s = it % STAGES;
+          ok = mbar_wait(empty_bar(s), ((it / STAGES) & 1) ^ 1, abort_flag);
+          if (!ok) break;
+          const uint32_t sa = base + s * STAGE_BYTES, sb = sa + A_BYTES;
+          // The even CTA announces the bytes of both halves.  The odd CTA's copies may complete first: the phase cannot end
+          // before the announcement, which is its only arrival.
+          if (rank == 0) mbar_expect_tx(full_bar(s), 2 * STAGE_BYTES);
+          const uint32_t bar = map_to_rank(full_bar(s), 0);
+          const int k0 = kb * BK;
+          if (p.a_mn_major) {
+            tma_load_2d_pair(sa, &map_a, bar, m0, k0);
+            tma_load_2d_pair(sa + 8192, &map_a, bar, m0 + 64, k0);
+          } else {
+            tma_load_2d_pair(sa, &map_a, bar, k0, m0);
+          }
+          if (p.b_mn_major) {
+#pragma unroll
+            for (int j = 0; j < BN / 128; ++j) tma_load_2d_pair(sb + j * 8192, &map_b, bar, n0 + j * 64, k0);
+          } else {
+            tma_load_2d_pair(sb, &map_b, bar, k0, n0);
+          }
+        }
+      }
+      // Every stage this CTA filled has to be released before it may leave: the releases are remote arrivals on its barriers, and
+      // they say that its copies have landed.
+      const uint32_t first = it > (uint32_t)STAGES ? it - STAGES : 0;
+      for (uint32_t i = first; i < it && ok; ++i) ok = mbar_wait(empty_bar(i % STAGES), (i / STAGES) & 1, abort_flag);
+      if (!ok) {
+        if (p.err) atomicExch(p.err, 21);
+        *abort_flag = 1;
+        for (int i = 0; i < 1024; ++i) __nanosleep(1000);  // about a millisecond for the copies in flight
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer (even CTA, for both)
+    if (rank == 0 && elect_one()) {
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)p.a_mn_major << 15) | ((uint32_t)p.b_mn_major << 16) |
+                             ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
+      const uint32_t a_step = p.a_mn_major ? (2048u >> 4) : (32u >> 4);
+      const uint32_t b_step = p.b_mn_major ? (2048u >> 4) : (32u >> 4);
+      uint32_t it = 0, local = 0;
+      bool ok = true;
+      for (int t = pair; t < total_tiles && ok; t += pairs, ++local) {
+        const uint32_t acc = local & 1;
+        ok = mbar_wait_cluster(acc_empty_bar(acc), ((local >> 1) & 1) ^ 1, abort_flag);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t tmem_d = tmem_base + acc * (uint32_t)BN;
+        const int kb0 = (t % split) * kb_per, kb1 = min(kb0 + kb_per, k_blocks_all);
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+          const int s = it % STAGES;
+          ok = mbar_wait_cluster(full_bar(s), (it / STAGES) & 1, abort_flag);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t sa = base + s * STAGE_BYTES, sb = sa + A_BYTES;
+          const uint64_t adesc = make_smem_desc(sa, p.a_mn_major), bdesc = make_smem_desc(sb, p.b_mn_major);
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            umma_bf16_pair(tmem_d, adesc + (uint64_t)(a_step * k), bdesc + (uint64_t)(b_step * k), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+          umma_commit_pair(empty_bar(s));
+        }
+        if (ok) umma_commit_pair(acc_full_bar(acc));
+      }
+      if (!ok) {
+        if (p.err) atomicExch(p.err, 22);
+        *abort_flag = 1;
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue (warps 2..9): lane quarter and column half
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    const uint32_t my_stage = stage_out + (uint32_t)(warp - 2) * 8192u;
+    uint32_t local = 0, stores = 0;
+    bool ok = true;
+    for (int t = pair; t < total_tiles && ok; t += pairs, ++local) {
+      int m0, n0;
+      coords(t / split, m0, n0);
+      const uint32_t acc = local & 1;
+      ok = mbar_wait_cluster(acc_full_bar(acc), (local >> 1) & 1, abort_flag);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t tmem_row = tmem_base + acc * (uint32_t)BN + (uint32_t)(half * (BN / 2)) + ((uint32_t)(q * 32) << 16);
+      store_rows_tma(tmem_row, BN / 2, n0 + half * (BN / 2), m0 + rank * BM + q * 32, my_stage, stores, &map_c, p, lane);
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive_remote(map_to_rank(acc_empty_bar(acc), 0));
+    }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    if (!ok) {
+      if (lane == 0 && p.err) atomicExch(p.err, 23);
+      *abort_flag = 1;
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  __syncwarp();
+  cluster_sync_all();  // the peer's MMAs read this CTA's shared memory and write its TMEM; its epilogue arrives on these barriers
+  if (warp == 1) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+  }
+}
 }  // namespace
 
 
@@ -338,9 +579,27 @@ gemm_bf16_tcgen05_persistent(const __grid_constant__ CUtensorMap map_a, const __
 // split_k > 1 (persistent kernel only): the K range is cut into `split_k` slices that run as separate work units and
 // add their fp32 partial tiles into C with TMA reduce stores; C must be fp32 and zero on entry, bias/act must be off.
 // split_k < 0: |split_k| slices and the product is ADDED to what C holds (fp32 gradient accumulation in place).
-KB_API int kb200_gemm_bf16_splitk(const void* a, const void* b, void* c, const float* bias, int M, int N, int K, long long lda, long long ldb,
-                                  long long ldc, int a_mn_major, int b_mn_major, int act, int out_fp32, int split_k, int* err,
-                                  cudaStream_t stream) {
+//
+// `variant`: 0 picks one (gemm_variant below); 1: one 128x128 tile a CTA; 2: persistent 128x256 tiles; 3: CTA pairs
+// with 256x256 tiles.
+enum { GV_AUTO = 0, GV_TILE = 1, GV_PERSISTENT = 2, GV_PAIR256 = 3 };
+
+// Which kernel: work units (output tiles x K slices) against the slots that run at once.  A pair's tile is two SMs' worth of the
+// one-CTA kernel's, so both take the same number of waves unless M ends in half a pair, and a wave of pairs is the quicker one
+// wherever it was measured: [16384, 50264, 768] 1357 -> 1117 us, [16384, 768, 50264] 1467 -> 1104, weight gradient
+// [768, 50264, 16384] 1132 -> 904, [8192, 14336, 4096] 698 -> 636, [768, 3072, 16384] in two slices 70 -> 64.  Below nine tenths of
+// a wave of pairs the smaller tiles fill the chip better ([512, 2048, 2664] in four slices: 17.5 us against 19.4).
+static int gemm_variant(int M, int N, int split_k, int sms) {
+  const long long t1 = (long long)((M + 127) / 128) * ((N + 255) / 256) * split_k, t2 = (long long)((M + 255) / 256) * ((N + 255) / 256) * split_k;
+  const long long pairs = sms / 2;
+  if (M > 128 && N > 128 && t2 * 10 >= pairs * 9 && (t2 + pairs - 1) / pairs <= (t1 + sms - 1) / sms) return GV_PAIR256;
+  if (split_k > 1) return GV_PERSISTENT;
+  return N > 128 && t1 >= sms / 2 ? GV_PERSISTENT : GV_TILE;
+}
+
+KB_API int kb200_gemm_bf16_run(const void* a, const void* b, void* c, const float* bias, int M, int N, int K, long long lda, long long ldb,
+                               long long ldc, int a_mn_major, int b_mn_major, int act, int out_fp32, int split_k, int variant, int* err,
+                               cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const int accumulate = split_k < 0 ? 1 : 0;
   if (split_k < 0) split_k = -split_k;
@@ -353,23 +612,19 @@ KB_API int kb200_gemm_bf16_splitk(const void* a, const void* b, void* c, const f
     return -2;
   }
   CUtensorMap map_a, map_b, map_c;
-  static int force_v1 = -1;
-  if (force_v1 < 0) {
-    const char* e = getenv("KB200_GEMM_V1");
-    force_v1 = (e != nullptr && e[0] == '1') ? 1 : 0;
-  }
   const int sm_count = kb_sm_count();
-  const long long tiles_v2 = (long long)((M + v2::BM - 1) / v2::BM) * ((N + v2::BN - 1) / v2::BN);
   int kb_per_split = 0;
   if (split_k > 1) {
-    const int k_blocks = (K + v2::BK - 1) / v2::BK;
+    const int k_blocks = (K + BK - 1) / BK;
     if (split_k > k_blocks) split_k = k_blocks;
     kb_per_split = (k_blocks + split_k - 1) / split_k;
     split_k = (k_blocks + kb_per_split - 1) / kb_per_split;  // every slice holds at least one K block
   }
   if (split_k < 1) split_k = 1;
-  const bool use_v2 = split_k > 1 || (!force_v1 && N > 128 && tiles_v2 >= sm_count / 2);
-  const int bn = use_v2 ? v2::BN : BN;
+  if (variant == GV_AUTO) variant = gemm_variant(M, N, split_k, sm_count);
+  if (split_k > 1 && variant == GV_TILE) variant = GV_PERSISTENT;
+  // rows of B's box: the N range one CTA loads
+  const int bn = variant == GV_PERSISTENT ? 256 : 128;
   bool ok = a_mn_major ? make_map(&map_a, a, M, K, lda, 64, BK) : make_map(&map_a, a, K, M, lda, BK, BM);
   ok = ok && (b_mn_major ? make_map(&map_b, b, N, K, ldb, 64, BK) : make_map(&map_b, b, K, N, ldb, BK, bn));
   ok = ok && make_map(&map_c, c, N, M, ldc, out_fp32 ? 32 : 64, 32, out_fp32 != 0);
@@ -377,23 +632,34 @@ KB_API int kb200_gemm_bf16_splitk(const void* a, const void* b, void* c, const f
     kb200_set_error("gemm_bf16: cuTensorMapEncodeTiled failed");
     return -3;
   }
-  static bool attr_v1[KB_MAX_DEVICES] = {false}, attr_v2[KB_MAX_DEVICES] = {false};
-  if (!kb_allow_smem(gemm_bf16_tcgen05_kernel, SMEM_BYTES, attr_v1) || !kb_allow_smem(gemm_bf16_tcgen05_persistent, v2::SMEM_BYTES, attr_v2)) {
-    kb200_set_error("gemm_bf16: cannot raise the shared-memory limit of the kernels on this device");
+  static bool attr_v1[KB_MAX_DEVICES] = {false}, attr_v2[KB_MAX_DEVICES] = {false}, attr_v3[KB_MAX_DEVICES] = {false};
+  const bool allowed = variant == GV_TILE         ? kb_allow_smem(gemm_bf16_tcgen05_kernel, SMEM_BYTES, attr_v1)
+                       : variant == GV_PERSISTENT ? kb_allow_smem(gemm_bf16_tcgen05_persistent, v2::SMEM_BYTES, attr_v2)
+                                                  : kb_allow_smem(gemm_bf16_tcgen05_pair, v3::SMEM_BYTES, attr_v3);
+  if (!allowed) {
+    kb200_set_error("gemm_bf16: cannot raise the shared-memory limit of the kernel on this device");
     return -3;
   }
   GemmParams p{c, bias, M, N, K, ldc, a_mn_major, b_mn_major, act, out_fp32, err, split_k, kb_per_split};
   p.accumulate = accumulate;
-  if (use_v2) {
-    const long long units = tiles_v2 * split_k;
-    const unsigned grid = (unsigned)(units < sm_count ? units : sm_count);
-    gemm_bf16_tcgen05_persistent<<<grid, THREADS, v2::SMEM_BYTES, stream>>>(map_a, map_b, map_c, p);
+  const int tile_m = variant == GV_PAIR256 ? 256 : 128, tile_n = variant == GV_TILE ? 128 : 256;
+  const long long units = (long long)((M + tile_m - 1) / tile_m) * ((N + tile_n - 1) / tile_n) * split_k;
+  if (variant == GV_TILE) {
+    gemm_bf16_tcgen05_kernel<<<(unsigned)units, THREADS, SMEM_BYTES, stream>>>(map_a, map_b, map_c, p);
+  } else if (variant == GV_PERSISTENT) {
+    gemm_bf16_tcgen05_persistent<<<(unsigned)(units < sm_count ? units : sm_count), THREADS, v2::SMEM_BYTES, stream>>>(map_a, map_b, map_c, p);
   } else {
-    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-    gemm_bf16_tcgen05_kernel<<<(unsigned)tiles, THREADS, SMEM_BYTES, stream>>>(map_a, map_b, map_c, p);
+    const int pairs = (int)(units < sm_count / 2 ? units : sm_count / 2);
+    gemm_bf16_tcgen05_pair<<<(unsigned)(2 * pairs), v3::PAIR_THREADS, v3::SMEM_BYTES, stream>>>(map_a, map_b, map_c, p);
   }
   KB_CHECK_LAUNCH("gemm_bf16");
   return 0;
+}
+
+KB_API int kb200_gemm_bf16_splitk(const void* a, const void* b, void* c, const float* bias, int M, int N, int K, long long lda, long long ldb,
+                                  long long ldc, int a_mn_major, int b_mn_major, int act, int out_fp32, int split_k, int* err,
+                                  cudaStream_t stream) {
+  return kb200_gemm_bf16_run(a, b, c, bias, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, act, out_fp32, split_k, GV_AUTO, err, stream);
 }
 
 KB_API int kb200_gemm_bf16(const void* a, const void* b, void* c, const float* bias, int M, int N, int K, long long lda, long long ldb,
