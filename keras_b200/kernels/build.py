@@ -25,6 +25,13 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-Xptxas", "-v",
 ]
 
+# Sources whose float32 results stand next to the library's own float32 math: exact division and full-accuracy functions.
+PRECISE = {"lstm.cu"}
+
+
+def _flags(src):
+    return [f for f in NVCC_FLAGS if not (f == "--use_fast_math" and os.path.basename(src) in PRECISE)]
+
 
 def _nvcc():
     for cand in (os.environ.get("NVCC"), shutil.which("nvcc"), "/usr/local/cuda/bin/nvcc"):
@@ -39,7 +46,7 @@ def sources():
 
 def _digest():
     h = hashlib.sha256()
-    h.update(" ".join(NVCC_FLAGS).encode())
+    h.update(" ".join(NVCC_FLAGS + sorted(PRECISE)).encode())
     for path in sorted(os.listdir(CSRC)):
         if path.endswith((".cu", ".cuh", ".h")):
             with open(os.path.join(CSRC, path), "rb") as f:
@@ -65,7 +72,7 @@ def build(force=False, verbose=False):
 
     def compile_one(src):
         obj = os.path.join(BUILD_DIR, os.path.basename(src)[:-3] + ".o")
-        cmd = [nvcc, "-c", src, "-o", obj, "-I", CSRC] + NVCC_FLAGS
+        cmd = [nvcc, "-c", src, "-o", obj, "-I", CSRC] + _flags(src)
         r = subprocess.run(cmd, capture_output=True, text=True)
         logs[src] = r.stdout + r.stderr
         if r.returncode != 0:

@@ -328,6 +328,22 @@ def flash_attention(q, k, v, mask, scale, is_causal):
     return attention.flash_attention(q, k, v, mask, scale, is_causal)
 
 
+# ---------------------------------------------------------------------------- recurrent layers
+def lstm_takes(sequences, initial_state, cell):
+    """Whether the whole-sequence kernel runs this LSTM layer: float32 CUDA tensors, unsharded weights, a size it takes."""
+    if not enabled(sequences):
+        return False
+    from keras_b200.kernels import lstm as klstm
+
+    return klstm.takes(sequences, initial_state, cell)
+
+
+def lstm(xz, bias, h0, c0, recurrent_kernel, reverse, want_sequence):
+    from keras_b200.kernels import lstm as klstm
+
+    return klstm.run(xz, bias, h0, c0, recurrent_kernel, reverse, want_sequence)
+
+
 # ---------------------------------------------------------------------------- optimizers
 def _plan_for(opt, grads, variables, slot_lists):
     if not variables:

@@ -653,6 +653,9 @@ class LSTM(_CellRNN):
         cell = self.cell
         if mask is not None or (training and (cell.dropout > 0 or cell.recurrent_dropout > 0)) or not isinstance(sequences, torch.Tensor):
             return None
+        fused = self._whole_sequence(sequences, initial_state)
+        if fused is not None:
+            return fused
         xz = _time_major_projection(cell, sequences, cell.bias.value if cell.bias is not None else None)
         h, c = initial_state[0], initial_state[1]
         rk = cell.recurrent_kernel.value
@@ -664,6 +667,20 @@ class LSTM(_CellRNN):
                 outs.append(h)
         outputs = torch.stack(outs, dim=1) if self.return_sequences else h.unsqueeze(1)
         return h, outputs, [h, c]
+
+    def _whole_sequence(self, sequences, initial_state):
+        """All time steps in one kernel launch a direction (float32 on the GPU, the stock cell), or ``None``."""
+        from keras_b200.kernels import dispatch
+
+        cell = self.cell
+        if type(cell) is not LSTMCell or cell.activation is not activations.tanh or cell.recurrent_activation is not activations.sigmoid:
+            return None
+        if not dispatch.lstm_takes(sequences, initial_state, cell):
+            return None
+        bias = cell.bias.value if cell.bias is not None else None
+        outputs, h, c = dispatch.lstm(ops.matmul(sequences, cell.kernel), bias, initial_state[0], initial_state[1], cell.recurrent_kernel.value,
+                                      self.go_backwards, self.return_sequences)
+        return h, outputs if self.return_sequences else h.unsqueeze(1), [h, c]
 
     def call(self, sequences, initial_state=None, mask=None, training=False):
         return super().call(sequences, mask=mask, training=training, initial_state=initial_state)

@@ -63,3 +63,56 @@ def test_gemm_variants_agree_with_the_product_in_64_bits(M, N, K, variant):
             # fp32 sums of K exact products (2^-24 each), one rounding to bf16 (2^-9)
             assert rel < (2.0 ** -17 if fp32 else 2.0 ** -8), (a_mn, b_mn, split, fp32, rel)
             assert int(err.item()) == 0
+
+
+@pytest.mark.parametrize("B,T,U,F", [(1, 1, 4, 3), (3, 7, 20, 5), (64, 5, 256, 16), (37, 9, 72, 8), (200, 3, 512, 8), (300, 2, 640, 4)])
+@pytest.mark.parametrize("reverse,sequence", [(False, True), (True, True), (False, False)])
+def test_lstm_sequence_against_the_steps_in_64_bits(B, T, U, F, reverse, sequence):
+    from keras_b200.kernels import gemm, lstm
+
+    g = torch.Generator(device="cuda").manual_seed(B + U)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")  # noqa: E731
+    args = [rnd(B, T, 4 * U), rnd(4 * U), 0.5 * rnd(B, U), rnd(B, U), rnd(U, 4 * U) * U ** -0.5]
+    mine = [a.clone().requires_grad_(True) for a in args]
+    exact = [a.double().requires_grad_(True) for a in args]
+    out, h, c = lstm.run(*mine, reverse, sequence)
+    want, hw, cw = lstm._composed(*exact, reverse)
+    up = [rnd(B, T, U), rnd(B, U), rnd(B, U)]
+    loss = (h * up[1]).sum() + (c * up[2]).sum() + ((out * up[0]).sum() if sequence else 0)
+    ref = (hw * up[1]).sum() + (cw * up[2]).sum() + ((want * up[0]).sum() if sequence else 0)
+    loss.backward()
+    ref.backward()
+    gemm.check_errors()
+    # fp32 sums over U terms a step and up to B * T in the weight gradient, a few steps deep
+    rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()  # noqa: E731
+    assert rel(h, hw) < 3e-6 and rel(c, cw) < 3e-6 and (not sequence or rel(out, want) < 3e-6)
+    for a, b in zip(mine, exact):
+        assert rel(a.grad, b.grad) < 1e-5
+    with torch.no_grad():
+        out2, h2, c2 = lstm.run(*mine, reverse, sequence)
+    assert torch.equal(h2, h) and torch.equal(c2, c)
+
+
+def test_lstm_layer_routes_and_second_derivatives():
+    import keras_b200 as keras
+    from keras_b200.kernels import lstm
+
+    keras.utils.set_random_seed(0)
+    layer = keras.layers.LSTM(24, return_sequences=True)
+    x = torch.randn(5, 6, 8, device="cuda", requires_grad=True)
+    y = layer(x)
+    assert "LstmSequence" in str(type(y.grad_fn)) or any("LstmSequence" in str(type(f[0])) for f in y.grad_fn.next_functions)
+    weights = [v.value for v in layer.trainable_variables]
+    z = torch.matmul(x, weights[0])
+    zero = torch.zeros(5, 24, device="cuda")
+    want = lstm._composed(z, weights[2], zero, zero, weights[1], False)[0]
+    assert torch.allclose(y, want, atol=2e-6)
+    second = []
+    for out in (y, want):
+        (g,) = torch.autograd.grad((out ** 2).sum(), x, create_graph=True)
+        second.append(torch.autograd.grad((g ** 2).sum(), weights[1])[0])
+    assert torch.allclose(second[0], second[1], rtol=1e-4, atol=1e-5 * second[1].abs().max().item())
+    # function transforms keep to the composed operations
+    frozen = x.detach()
+    batched = torch.func.vmap(lambda s: layer(s.unsqueeze(0)).squeeze(0))(frozen)
+    assert torch.allclose(batched, want, atol=2e-6)
