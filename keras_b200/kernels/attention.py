@@ -36,8 +36,9 @@ def _ok(t):
             and all(s % 8 == 0 for s in t.stride()[:3]))
 
 
-def forward(q, k, v, scale, is_causal):
-    """Raw kernel launch: returns ``(out [B, Tq, H, D] bf16, lse [B, H, Tq] fp32)``."""
+def forward(q, k, v, scale, is_causal, mask=None, row_mask=None):
+    """Raw kernel launch: returns ``(out [B, Tq, H, D] bf16, lse [B, H, Tq] fp32)``.  ``mask``: bool ``[B, H, Tq, Tk]``, unit stride over
+    the keys, any (also zero) strides over the rest; ``row_mask`` (with ``mask``): bool ``[B, Tq]``, unit stride over the rows."""
     lib = kops._lib()
     B, Tq, H, D = q.shape
     Tk, Hkv = k.shape[1], k.shape[2]
@@ -46,7 +47,10 @@ def forward(q, k, v, scale, is_causal):
     args = [kops._p(q), kops._p(k), kops._p(v), kops._p(out), kops._p(lse), kops._i(B), kops._i(Tq), kops._i(Tk), kops._i(H), kops._i(Hkv), kops._i(D)]
     for t in (q, k, v, out):
         args += [kops._ll(t.stride(1)), kops._ll(t.stride(2)), kops._ll(t.stride(0))]
-    args += [kops._f(float(scale)), kops._i(1 if is_causal else 0), kops._p(_err_flag(q.device)), kops._stream()]
+    # a dimension of one element may carry any stride: rows that are all the same are read once
+    ms = [0 if mask is None or mask.shape[i] == 1 else mask.stride(i) for i in range(3)]
+    args += [kops._f(float(scale)), kops._i(1 if is_causal else 0), kops._p(mask), kops._ll(ms[0]), kops._ll(ms[1]), kops._ll(ms[2]),
+             kops._p(row_mask), kops._ll(row_mask.stride(0) if row_mask is not None else 0), kops._p(_err_flag(q.device)), kops._stream()]
     kops._check(lib.kb200_flash_attention_fwd(*args), "flash_attention_fwd")
     return out, lse
 
@@ -70,20 +74,42 @@ class FlashAttentionFn(torch.autograd.Function):
         return dq, dk, dv, None, None
 
 
+def _kernel_mask(mask, q, k, is_causal):
+    """``mask`` (anything that broadcasts against ``[B, H, Tq, Tk]``) as the kernel reads it, the causal one included."""
+    if mask.device != q.device or mask.ndim > 4 or mask.ndim == 0:
+        return None
+    mask = mask if mask.dtype == torch.bool else mask != 0
+    if is_causal:
+        mask = mask & torch.ones((q.shape[1], k.shape[1]), dtype=torch.bool, device=q.device).tril()
+    try:
+        if mask.shape[-1] != k.shape[1] or (mask.shape[-1] > 1 and mask.stride(-1) != 1):
+            mask = mask.expand(tuple(mask.shape[:-1]) + (k.shape[1],)).contiguous()
+        return mask.expand(q.shape[0], q.shape[2], q.shape[1], k.shape[1])
+    except RuntimeError:
+        return None
+
+
 def flash_attention(q, k, v, mask, scale, is_causal):
-    """Attention on this package's kernel, or ``None`` when the call does not fit it (mask tensors, other head sizes,
-    unaligned layouts) or the kernel is not selected for training."""
-    if mask is not None or not (_ok(q) and _ok(k) and _ok(v)):
+    """Attention on this package's kernel, or ``None`` when the call does not fit it (other head sizes, unaligned layouts, a scale
+    that is not positive) or the kernel is not selected for training."""
+    if not (_ok(q) and _ok(k) and _ok(v)):
         return None
     D = q.shape[-1]
     if D not in (64, 128) or k.shape[-1] != D or v.shape[-1] != D or q.shape[2] % k.shape[2] or k.shape[1] != v.shape[1]:
         return None
     needs_grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
     mode = os.environ.get("KERAS_B200_FLASH_ATTENTION", "inference")
-    if mode == "0" or (needs_grad and mode != "1"):
+    if mode == "0" or (needs_grad and (mode != "1" or mask is not None)):
         return None
     if scale is None:
         scale = D ** -0.5
+    if not scale > 0 or 0 in q.shape or 0 in k.shape:
+        return None
     if needs_grad:
         return FlashAttentionFn.apply(q, k, v, float(scale), bool(is_causal))
-    return forward(q, k, v, float(scale), bool(is_causal))[0]
+    if mask is not None:
+        mask = _kernel_mask(mask, q, k, is_causal)
+        if mask is None:
+            return None
+        is_causal = False
+    return forward(q, k, v, float(scale), bool(is_causal), mask)[0]

@@ -679,7 +679,7 @@ def dot_product_attention(query, key, value, bias=None, mask=None, scale=None, i
     if scale is None:
         scale = 1.0 / math.sqrt(q.shape[-1])
     if bias is None and attn_logits_soft_cap is None and flash_attention is not False:
-        fused = dispatch.flash_attention(q, k, v, mask, scale, is_causal)
+        fused = dispatch.flash_attention(q, k, v, _t(mask) if mask is not None else None, scale, is_causal)
         if fused is not None:
             return fused
     if flash_attention and (bias is not None or attn_logits_soft_cap is not None):

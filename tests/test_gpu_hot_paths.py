@@ -116,3 +116,86 @@ def test_lstm_layer_routes_and_second_derivatives():
     frozen = x.detach()
     batched = torch.func.vmap(lambda s: layer(s.unsqueeze(0)).squeeze(0))(frozen)
     assert torch.allclose(batched, want, atol=2e-6)
+
+
+def _attention_in_64_bits(q, k, v, scale, causal, mask):
+    """[B, T, heads, head size]; masked scores are a finite negative, as the layers define them."""
+    q, k, v = (t.double().transpose(1, 2) for t in (q, k, v))
+    k, v = (t.repeat_interleave(q.shape[1] // t.shape[1], dim=1) for t in (k, v))
+    s = torch.matmul(q, k.transpose(-1, -2)) * scale
+    if causal:
+        s = s.masked_fill(torch.ones(s.shape[-2:], dtype=torch.bool, device=s.device).triu(1), float("-inf"))
+    if mask is not None:
+        s = s.masked_fill(~mask, -1e30)
+    return torch.matmul(torch.softmax(s, dim=-1), v).transpose(1, 2)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,Tq,Tk,H,Hkv", [(2, 1, 1, 2, 2), (3, 77, 77, 4, 2), (1, 128, 129, 2, 1), (2, 129, 300, 2, 2), (1, 256, 256, 6, 2), (2, 333, 333, 3, 3),
+                                           (1, 700, 65, 2, 2), (1, 1024, 1024, 2, 1)])
+@pytest.mark.parametrize("kind", ["none", "causal", "rows", "keys", "causal+keys"])
+def test_attention_against_64_bits(B, Tq, Tk, H, Hkv, D, kind):
+    from keras_b200.kernels import attention
+
+    g = torch.Generator(device="cuda").manual_seed(Tq + Tk)
+    q, k, v = (torch.randn(s, generator=g, device="cuda").bfloat16() for s in ((B, Tq, H, D), (B, Tk, Hkv, D), (B, Tk, Hkv, D)))
+    q = q * 4  # peaked rows: the maximum moves from block to block
+    mask = None
+    if kind == "rows":
+        mask = torch.rand((B, 1, Tq, Tk), generator=g, device="cuda") < 0.7
+        mask[:, :, Tq // 2:Tq // 2 + 3] = False  # rows without any key attend uniformly
+        mask[:, :, :, : min(130, Tk // 2)] &= torch.rand((B, 1, Tq, 1), generator=g, device="cuda") < 0.5  # whole blocks without a key
+    elif "keys" in kind:
+        mask = (torch.arange(Tk, device="cuda") < torch.randint(1, Tk + 1, (B, 1), generator=g, device="cuda"))[:, None, None, :]
+    causal = "causal" in kind
+    out = attention.flash_attention(q, k, v, mask, D ** -0.5, causal)
+    assert out is not None
+    attention.check_errors()
+    if causal and mask is not None:
+        mask, causal = mask & torch.ones((Tq, Tk), dtype=torch.bool, device="cuda").tril(), False
+    want = _attention_in_64_bits(q, k, v, D ** -0.5, causal, mask)
+    # probabilities and result are rounded to bf16 once each (2^-9), the sums are fp32
+    rel = ((out.double() - want).norm() / want.norm()).item()
+    assert rel < 2.0 ** -8, rel
+    assert (out.double() - want).abs().max().item() < 0.03 * v.abs().max().item()
+
+
+@pytest.mark.parametrize("D,T", [(64, 77), (128, 300), (64, 512)])
+def test_attention_with_masked_rows_and_keys(D, T):
+    from keras_b200.kernels import attention
+
+    g = torch.Generator(device="cuda").manual_seed(T)
+    q, k, v = (torch.randn((3, T, 4, D), generator=g, device="cuda").bfloat16() for _ in range(3))
+    lengths = torch.tensor([[T], [1], [T // 2]], device="cuda")
+    real = torch.arange(T, device="cuda") < lengths
+    out = attention.forward(q, k, v, D ** -0.5, False, real[:, None, None, :].expand(3, 4, T, T), real)[0]
+    attention.check_errors()
+    want = _attention_in_64_bits(q, k, v, D ** -0.5, False, real[:, None, :, None] & real[:, None, None, :])
+    assert ((out.double() - want).norm() / want.norm()).item() < 2.0 ** -8
+
+
+def test_attention_keeps_a_nan_to_the_rows_that_see_it():
+    from keras_b200.kernels import attention
+
+    for bad in (0, 7, 70, 129):  # exponentials on either pipe, both halves of a block, the second block
+        q, k, v = (torch.randn((1, 200, 2, 64), device="cuda").bfloat16() for _ in range(3))
+        k[0, bad, 0, 3] = float("nan")
+        out = attention.forward(q, k, v, 0.125, True)[0]
+        assert torch.equal(out.isnan().any(-1)[0, :, 0], torch.arange(200, device="cuda") >= bad) and not out[:, :, 1].isnan().any()
+
+
+def test_attention_strides_and_refusals():
+    from keras_b200.kernels import attention
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    qkv = torch.randn((2, 200, 3, 4, 64), generator=g, device="cuda").bfloat16()
+    q, k, v = qkv.unbind(2)  # rows of another pitch
+    wide = torch.rand((2, 4, 200, 512), generator=g, device="cuda") < 0.6
+    for mask in (wide[..., 7:207], wide[..., ::2][..., :200], wide[:1, :1, :, :1], wide[0, 0, :, 3:203].to(torch.int32)):
+        out = attention.flash_attention(q, k, v, mask, 0.125, False)
+        want = _attention_in_64_bits(q, k, v, 0.125, False, torch.broadcast_to(mask != 0, (2, 4, 200, 200)))
+        assert ((out.double() - want).norm() / want.norm()).item() < 2.0 ** -8
+    assert attention.flash_attention(q, k, v, None, -0.125, False) is None  # a negative scale turns the maximum around
+    assert attention.flash_attention(q[..., :40], k[..., :40], v[..., :40], None, 0.125, False) is None
+    assert attention.flash_attention(q.float(), k.float(), v.float(), None, 0.125, False) is None
+    assert attention.flash_attention(q.detach().requires_grad_(True), k, v, wide[..., :200], 0.125, False) is None
