@@ -199,3 +199,104 @@ def test_attention_strides_and_refusals():
     assert attention.flash_attention(q[..., :40], k[..., :40], v[..., :40], None, 0.125, False) is None
     assert attention.flash_attention(q.float(), k.float(), v.float(), None, 0.125, False) is None
     assert attention.flash_attention(q.detach().requires_grad_(True), k, v, wide[..., :200], 0.125, False) is None
+
+
+def _bf16_model(vocab=300, d=64):
+    import keras_b200 as keras
+
+    old = keras.config.dtype_policy()
+    keras.config.set_dtype_policy("mixed_bfloat16")
+    try:
+        x = keras.Input((16, d))
+        return keras.Model(x, keras.layers.Dense(vocab)(keras.layers.Dense(d, activation="relu")(x)))
+    finally:
+        keras.config.set_dtype_policy(old)
+
+
+def _plain(model, x):
+    h = x.bfloat16()
+    for i, layer in enumerate(model.layers[1:]):
+        h = torch.matmul(h, layer.kernel.value.bfloat16()) + layer.bias.value.bfloat16()
+        h = torch.relu(h) if i == 0 else h
+    return h
+
+
+@pytest.mark.parametrize("vocab", [300, 301, 304])
+def test_inference_copies_of_weights_follow_every_change(vocab):
+    import keras_b200 as keras
+
+    keras.utils.set_random_seed(0)
+    model = _bf16_model(vocab)
+    x = torch.randn(8, 16, 64, device="cuda")
+    kernels = [layer.kernel for layer in model.layers[1:]]
+
+    def check(times=3):
+        for _ in range(times):
+            with torch.no_grad():
+                out = model(x, training=False)
+                want = _plain(model, x)
+            assert torch.allclose(out.float(), want.float(), atol=0.05, rtol=0.02)
+
+    check()
+    assert all(k._copy is not None and k._copy[1] is not None for k in kernels)  # kept from the second call on
+    assert kernels[1]._copy[1].shape == (64, -(-vocab // 8) * 8)
+    kernels[0].assign(torch.randn(64, 64, device="cuda") * 0.1)  # a variable update
+    check()
+    with torch.no_grad():
+        kernels[1].value.mul_(2.0)  # in place on the parameter
+    check()
+    with torch.no_grad():
+        kernels[0]._copy[1].zero_()  # somebody wrote into what was read
+    check()
+    weights = [w * 0.5 for w in model.get_weights()]
+    model.set_weights(weights)
+    check()
+    # updates by the fused optimizer write through raw pointers
+    model.compile(optimizer=keras.optimizers.SGD(0.5, momentum=0.9), loss="mse")
+    y = torch.randn(8, 16, vocab, device="cuda")
+    for _ in range(6):
+        model.train_on_batch(x, y)
+        check(2)
+    assert all(k._copy is None for k in kernels)
+
+
+def test_inference_copies_stay_out_of_recordings_and_transforms():
+    import keras_b200 as keras
+
+    keras.utils.set_random_seed(1)
+    model = _bf16_model(301)
+    x = torch.randn(8, 16, 64, device="cuda")
+    with torch.no_grad():
+        for _ in range(3):
+            model(x, training=False)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = model(x, training=False)
+        for layer in model.layers[1:]:
+            layer.kernel.value.mul_(-1.5)
+        graph.replay()
+        assert torch.allclose(out.float(), _plain(model, x).float(), atol=0.05, rtol=0.02)
+        with torch.inference_mode():
+            assert torch.allclose(model(x, training=False).float(), _plain(model, x).float(), atol=0.05, rtol=0.02)
+    # with gradients on, the variable itself is read
+    loss = model(x, training=True).float().square().mean()
+    loss.backward()
+    assert all(v.value.grad is not None for v in model.trainable_variables)
+
+
+def test_inference_copies_across_streams():
+    import keras_b200 as keras
+
+    keras.utils.set_random_seed(2)
+    model = _bf16_model(301)
+    x = torch.randn(8, 16, 64, device="cuda")
+    side = torch.cuda.Stream()
+    with torch.no_grad():
+        want = _plain(model, x).float()
+        side.wait_stream(torch.cuda.current_stream())
+        for _ in range(2):
+            with torch.cuda.stream(side):
+                model(x, training=False)  # the copies are made on this stream
+        out = model(x, training=False)
+        assert torch.allclose(out.float(), want, atol=0.05, rtol=0.02)
+        assert model.layers[2].kernel._copy[3] == side.cuda_stream
