@@ -164,6 +164,14 @@ def conv(x, kernel, strides, padding, data_format, dilation):
     return conv_mod.conv(x, kernel, strides, padding, data_format, dilation)
 
 
+def depthwise(x, kernel, strides, padding, data_format, dilation, variable=None):
+    if not (enabled(x) and enabled(kernel)):
+        return None
+    from keras_b200.kernels import depthwise as dw
+
+    return dw.depthwise(x, kernel, strides, padding, data_format, dilation, variable)
+
+
 # ------------------------------------------------------------------------- normalisation
 def layer_norm(x, gamma, beta, eps):
     if not enabled(x) or x.dtype not in _FLOAT_IO or x.shape[-1] > 8192 or x.numel() == 0:

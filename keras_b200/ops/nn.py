@@ -392,6 +392,12 @@ def conv(inputs, kernel, strides=1, padding="valid", data_format=None, dilation_
 def depthwise_conv(inputs, kernel, strides=1, padding="valid", data_format=None, dilation_rate=1):
     k = _t(kernel)
     sp = tuple(k.shape[:-2])
+    if len(sp) == 2:
+        x = _t(inputs)
+        fused = dispatch.depthwise(x, k, _tuple(strides, 2), padding, config.standardize_data_format(data_format), _tuple(dilation_rate, 2),
+                                   kernel if hasattr(kernel, "_value") else None)
+        if fused is not None:
+            return fused
     k2 = k.reshape(sp + (1, k.shape[-2] * k.shape[-1]))
     return conv(inputs, k2, strides, padding, data_format, dilation_rate)
 

@@ -300,3 +300,51 @@ def test_inference_copies_across_streams():
         out = model(x, training=False)
         assert torch.allclose(out.float(), want, atol=0.05, rtol=0.02)
         assert model.layers[2].kernel._copy[3] == side.cuda_stream
+
+
+@pytest.mark.parametrize("K", [3, 5, 7])
+@pytest.mark.parametrize("S", [1, 2])
+@pytest.mark.parametrize("padding", ["same", "valid"])
+@pytest.mark.parametrize("N,H,W,C", [(1, 7, 7, 8), (3, 9, 14, 40), (2, 15, 10, 144), (5, 8, 33, 264), (2, 29, 28, 320)])
+def test_depthwise_convolution_and_gradients_against_64_bits(K, S, padding, N, H, W, C):
+    from keras_b200.kernels import depthwise as dw
+
+    g = torch.Generator(device="cuda").manual_seed(H * W + K)
+    x = torch.randn((N, H, W, C), generator=g, device="cuda").bfloat16().requires_grad_(True)
+    w = (torch.randn((K, K, C, 1), generator=g, device="cuda") / K).bfloat16().requires_grad_(True)
+    y = dw.depthwise(x * 1, w, (S, S), padding, "channels_last", (1, 1))
+    geometry = y.grad_fn.g
+    xe, we = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    want = dw._composed(xe, we, geometry)
+    assert y.shape == want.shape
+    dy = torch.randn(y.shape, generator=g, device="cuda").bfloat16()
+    y.backward(dy)
+    want.backward(dy.double())
+    rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()  # noqa: E731
+    # one rounding to bf16 each (2^-9); the weight gradient sums N*OH*OW products in fp32 first
+    assert rel(y, want) < 2.0 ** -8 and rel(x.grad, xe.grad) < 2.0 ** -8 and rel(w.grad, we.grad) < 2.0 ** -8
+
+
+def test_depthwise_routes():
+    import keras_b200 as keras
+    from keras_b200.kernels import depthwise as dw
+
+    x = torch.randn(2, 9, 9, 16, device="cuda").bfloat16()
+    w = torch.randn(3, 3, 16, 1, device="cuda").bfloat16()
+    assert dw.depthwise(x, w, (1, 1), "same", "channels_first", (1, 1)) is None
+    assert dw.depthwise(x, w, (1, 2), "same", "channels_last", (1, 1)) is None
+    assert dw.depthwise(x, w, (1, 1), "same", "channels_last", (2, 2)) is None
+    assert dw.depthwise(x, w.expand(3, 3, 16, 2).contiguous(), (1, 1), "same", "channels_last", (1, 1)) is None
+    assert dw.depthwise(x.float(), w.float(), (1, 1), "same", "channels_last", (1, 1)) is None
+    assert dw.depthwise(x[:, :2], w, (1, 1), "valid", "channels_last", (1, 1)) is None
+    odd = torch.randn(2 * 9 * 9 * 16 + 1, device="cuda").bfloat16()[1:].reshape(2, 9, 9, 16)  # not 16-byte aligned
+    flipped = x.transpose(1, 2)
+    for t in (odd, flipped, x[:, ::2]):
+        y = keras.ops.depthwise_conv(t, w, strides=2, padding="same", data_format="channels_last")
+        want = keras.ops.depthwise_conv(t.float(), w.float(), strides=2, padding="same", data_format="channels_last")
+        assert ((y.float() - want).norm() / want.norm()).item() < 2.0 ** -8
+    # second derivatives
+    xg = x.clone().requires_grad_(True)
+    y = dw.depthwise(xg * 1, w, (1, 1), "same", "channels_last", (1, 1))
+    (g,) = torch.autograd.grad((y.float() ** 2).sum(), xg, create_graph=True)
+    assert torch.autograd.grad(g.float().square().sum(), xg)[0].isfinite().all()
