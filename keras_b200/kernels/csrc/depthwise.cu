@@ -7,12 +7,14 @@
 // strip of 4 pixels of a row: a row of input vectors is loaded once, all loads in flight together, unpacked once and used for every
 // pixel of the strip; the rows above and below come from L1 / L2, where the neighbouring strips left them.  Sums are fp32 in a fixed
 // order; the weight gradient sums strips per thread, then per CTA, then with one fp32 atomic add per CTA and weight.
-// MEASURED
+// us, this / the library (which pads and re-lays in passes of its own at stride 2), 128 images:
+//   56x56x144 3x3 /2   forward 64 / 208   both gradients 160 / 394      28x28x192 5x5   forward 67 / 66   gradients 153 / 230
+//   28x28x192 3x3      forward 38 / 32    both gradients  84 / 120      56x56x96 7x7 (64 images)   119 / 115   287 / 673
 #include "common.cuh"
 
 namespace {
 
-constexpr int TW = 4, THREADS = 256;
+constexpr int TW = 4, TW2 = 2, THREADS = 256;  // pixels of a strip; TW2: data gradient at stride 2
 
 struct DwArgs {
   const __nv_bfloat16* x;   // forward, weight gradient: input;  data gradient: dy
@@ -40,18 +42,19 @@ __device__ __forceinline__ void stage_weights(const DwArgs& a, float* sw, int cv
 
 // FLIP = false: forward.  FLIP = true (stride 1): data gradient, the same sum with mirrored taps; the launcher mirrors the padding.
 template <int K, int S, bool FLIP>
-__global__ void __launch_bounds__(THREADS) depthwise_kernel(const DwArgs a) {
+__global__ void __launch_bounds__(THREADS, K == 3 ? 1 : 2) depthwise_kernel(const DwArgs a) {
   extern __shared__ float sw[];
   const int cx = 1 << a.cx_log2, cvecs = a.C / 8, ch = cx * 8;
   const int tx = threadIdx.x & (cx - 1), cv = blockIdx.y * cx + tx;
   stage_weights<K, FLIP>(a, sw, blockIdx.y * cx, cx);
   if (cv >= cvecs) return;
-  const int strips = (a.OW + TW - 1) / TW;
-  const long long total = (long long)a.N * a.OH * strips, step = (long long)gridDim.x * (THREADS >> a.cx_log2);
+  const unsigned strips = (a.OW + TW - 1) / TW;
+  const unsigned total = (unsigned)(a.N * a.OH * strips), step = gridDim.x * (THREADS >> a.cx_log2);
   constexpr int IN = (TW - 1) * S + K;
-  for (long long t = (long long)blockIdx.x * (THREADS >> a.cx_log2) + (threadIdx.x >> a.cx_log2); t < total; t += step) {
-    const int ow0 = (int)(t % strips) * TW, oh = (int)((t / strips) % a.OH);
-    const long long n = t / strips / a.OH;
+  for (unsigned t = blockIdx.x * (THREADS >> a.cx_log2) + (threadIdx.x >> a.cx_log2); t < total; t += step) {
+    const unsigned line = t / strips;  // 32-bit divisions: the launcher keeps the pixels below 2^30
+    const int ow0 = (int)(t - line * strips) * TW, oh = (int)(line % a.OH);
+    const long long n = line / a.OH;
     const int iw0 = ow0 * S - a.pl, ih0 = oh * S - a.pt;
     float acc[TW][8] = {};
 #pragma unroll
@@ -89,22 +92,26 @@ __global__ void __launch_bounds__(THREADS) depthwise_kernel(const DwArgs a) {
   }
 }
 
+// Strips of 2 with 64 registers (four CTAs an SM) hide the latency of the few loads a strip has better than strips of 4: [128, 56, 56,
+// 144] 3x3 116 -> 81 us, 5x5 152 -> 126.
 // Data gradient at stride 2: dx[ih, iw] = sum dy[oh, ow] w[ih + pt - 2 oh, iw + pl - 2 ow].  Strips start where iw + pl is even, so that the
 // taps of each pixel are known at compile time.
 template <int K>
-__global__ void __launch_bounds__(THREADS) depthwise_dgrad2_kernel(const DwArgs a) {
+__global__ void __launch_bounds__(THREADS, 4) depthwise_dgrad2_kernel(const DwArgs a) {
   extern __shared__ float sw[];
-  constexpr int S = 2;
+  constexpr int S = 2, TW = TW2;
   const int cx = 1 << a.cx_log2, cvecs = a.C / 8, ch = cx * 8;
   const int tx = threadIdx.x & (cx - 1), cv = blockIdx.y * cx + tx;
   stage_weights<K, false>(a, sw, blockIdx.y * cx, cx);
   if (cv >= cvecs) return;
-  const int off = a.pl & 1, strips = (a.W + off + TW - 1) / TW;
-  const long long total = (long long)a.N * a.H * strips, step = (long long)gridDim.x * (THREADS >> a.cx_log2);
+  const int off = a.pl & 1;
+  const unsigned strips = (a.W + off + TW - 1) / TW;
+  const unsigned total = (unsigned)(a.N * a.H * strips), step = gridDim.x * (THREADS >> a.cx_log2);
   constexpr int BACK = (K - 1) / S, COLS = BACK + (TW - 1) / S + 1;  // output columns base/2 - BACK ... base/2 + (TW - 1)/2
-  for (long long t = (long long)blockIdx.x * (THREADS >> a.cx_log2) + (threadIdx.x >> a.cx_log2); t < total; t += step) {
-    const int iw0 = (int)(t % strips) * TW - off, ih = (int)((t / strips) % a.H);
-    const long long n = t / strips / a.H;
+  for (unsigned t = blockIdx.x * (THREADS >> a.cx_log2) + (threadIdx.x >> a.cx_log2); t < total; t += step) {
+    const unsigned line = t / strips;
+    const int iw0 = (int)(t - line * strips) * TW - off, ih = (int)(line % a.H);
+    const long long n = line / a.H;
     const int ow0 = (iw0 + a.pl) / S - BACK;
     float acc[TW][8] = {};
 #pragma unroll
@@ -146,19 +153,20 @@ __global__ void __launch_bounds__(THREADS) depthwise_dgrad2_kernel(const DwArgs 
 
 // R rows of taps a thread (all of them for 3x3, whose 72 sums fit the registers; else one, blockIdx.z): dw[r, s] += x[oh*S - pt + r, ow*S - pl + s] dy[oh, ow]
 template <int K, int S, int R>
-__global__ void __launch_bounds__(THREADS) depthwise_wgrad_kernel(const DwArgs a) {
+__global__ void __launch_bounds__(THREADS, K == 3 ? 1 : 2) depthwise_wgrad_kernel(const DwArgs a) {
   extern __shared__ float red[];  // [THREADS / cx strips] folded to warps: [8 warps][cx * 8]
   const int cx = 1 << a.cx_log2, cvecs = a.C / 8;
   const int tx = threadIdx.x & (cx - 1), cv = blockIdx.y * cx + tx;
   const int r_first = blockIdx.z * R;
   const bool active = cv < cvecs;
-  const int strips = (a.OW + TW - 1) / TW;
-  const long long total = active ? (long long)a.N * a.OH * strips : 0, step = (long long)gridDim.x * (THREADS >> a.cx_log2);
+  const unsigned strips = (a.OW + TW - 1) / TW;
+  const unsigned total = active ? (unsigned)(a.N * a.OH * strips) : 0u, step = gridDim.x * (THREADS >> a.cx_log2);
   constexpr int IN = (TW - 1) * S + K;
   float acc[R][K][8] = {};
-  for (long long t = (long long)blockIdx.x * (THREADS >> a.cx_log2) + (threadIdx.x >> a.cx_log2); t < total; t += step) {
-    const int ow0 = (int)(t % strips) * TW, oh = (int)((t / strips) % a.OH);
-    const long long n = t / strips / a.OH;
+  for (unsigned t = blockIdx.x * (THREADS >> a.cx_log2) + (threadIdx.x >> a.cx_log2); t < total; t += step) {
+    const unsigned line = t / strips;
+    const int ow0 = (int)(t - line * strips) * TW, oh = (int)(line % a.OH);
+    const long long n = line / a.OH;
     const int iw0 = ow0 * S - a.pl;
     const __nv_bfloat16* grow = a.dy + ((n * a.OH + oh) * a.OW + ow0) * a.C + cv * 8;
     float g[TW][8];
@@ -243,7 +251,7 @@ DwGrid dw_grid(int C, long long strips, int ctas_per_sm, int z) {
 
 template <int K>
 int dw_launch(int mode, DwArgs a, int S, cudaStream_t st) {
-  const long long out_strips = (long long)a.N * a.OH * ((a.OW + TW - 1) / TW), in_strips = (long long)a.N * a.H * ((a.W + 1 + TW - 1) / TW);
+  const long long out_strips = (long long)a.N * a.OH * ((a.OW + TW - 1) / TW), in_strips = (long long)a.N * a.H * ((a.W + 1 + TW2 - 1) / TW2);
   const DwGrid g = mode == 0 ? dw_grid(a.C, out_strips, 16, 1) : mode == 1 ? dw_grid(a.C, in_strips, 16, 1) : dw_grid(a.C, out_strips, 2, K == 3 ? 1 : K);
   a.cx_log2 = g.cx_log2;
   const int smem = mode == 2 ? (THREADS / 32) * (1 << a.cx_log2) * 8 * 4 : K * K * (1 << a.cx_log2) * 8 * 4;
@@ -281,6 +289,10 @@ int dw_launch(int mode, DwArgs a, int S, cudaStream_t st) {
 KB_API int kb200_depthwise(int mode, const void* x, const void* w, void* y, const void* dy, float* dw, int N, int H, int W, int C, int OH, int OW, int K, int S,
                            int pt, int pl, cudaStream_t stream) {
   if (N <= 0 || H <= 0 || W <= 0 || C <= 0 || OH <= 0 || OW <= 0) return 0;
+  if ((long long)N * H * W >= (1ll << 30) || (long long)N * OH * OW >= (1ll << 30)) {
+    kb200_set_error("depthwise: more than 2^30 pixels");
+    return -2;
+  }
   if (C % 8 || (S != 1 && S != 2) || (K != 3 && K != 5 && K != 7) || pt < 0 || pl < 0 || pt >= K || pl >= K ||
       (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y | (uintptr_t)dy) & 15)) {
     kb200_set_error("depthwise: 3, 5 or 7 taps, stride 1 or 2, channels a multiple of 8, 16-byte aligned tensors");

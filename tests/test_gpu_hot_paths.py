@@ -337,6 +337,7 @@ def test_depthwise_routes():
     assert dw.depthwise(x, w.expand(3, 3, 16, 2).contiguous(), (1, 1), "same", "channels_last", (1, 1)) is None
     assert dw.depthwise(x.float(), w.float(), (1, 1), "same", "channels_last", (1, 1)) is None
     assert dw.depthwise(x[:, :2], w, (1, 1), "valid", "channels_last", (1, 1)) is None
+    assert dw.depthwise(x, w, (1, 1), "same", "channels_last", (1, 1)) is None and dw.depthwise(x, w, (2, 2), "same", "channels_last", (1, 1)) is not None
     odd = torch.randn(2 * 9 * 9 * 16 + 1, device="cuda").bfloat16()[1:].reshape(2, 9, 9, 16)  # not 16-byte aligned
     flipped = x.transpose(1, 2)
     for t in (odd, flipped, x[:, ::2]):
