@@ -258,8 +258,10 @@ template <typename T, int MODE, int U = BN_U>
 __global__ void __launch_bounds__(BN_THREADS, 2) bn_apply_kernel(const T* __restrict__ in0, const T* __restrict__ in1, const T* __restrict__ ymask,
                                                              unsigned char* __restrict__ bits, T* __restrict__ out0, T* __restrict__ out1,
                                                              const float* __restrict__ p0, const float* __restrict__ p1,
-                                                             const float* __restrict__ p2, long long M, int C, int cx_log2, int relu) {
+                                                             const float* __restrict__ p2, long long M, int C, int cx_log2, int relu,
+                                                             float cap = INFINITY) {
   constexpr int V = Vec<T>::N;
+  const bool capped = cap < INFINITY;
   // the 8-row instance is the forward pass without a second input: known at compile time so that no registers are held for it
   const bool has1 = (U == 8) ? false : in1 != nullptr;
   const int cvecs = C / V;
@@ -306,8 +308,13 @@ __global__ void __launch_bounds__(BN_THREADS, 2) bn_apply_kernel(const T* __rest
         for (int k = 0; k < V; ++k) {
           float t = v0[k] * a[k] + b[k];
           if (has1) t += v1[k];
-          m |= (t > 0.f ? 1u : 0u) << k;
+          bool pass = t > 0.f;
           o[k] = relu ? fmaxf(t, 0.f) : t;
+          if (capped && to_f32<T>(from_f32<T>(t)) >= cap) {  // decided on the value that is stored, as a separate layer would
+            o[k] = cap;
+            pass = false;
+          }
+          m |= (pass ? 1u : 0u) << k;
         }
         Vec<T>::store(out0 + e, o);
         if (bits != nullptr) bits[r * cvecs + cv] = (unsigned char)m;
@@ -390,14 +397,15 @@ KB_API int kb200_bn_finalize_partials(const float* partials, int grid, int n_til
 
 template <typename T>
 static int bn_apply_launch(const void* x, const void* res, void* y, unsigned char* bits, const float* scale, const float* shift, long long M,
-                           int C, int relu, cudaStream_t stream) {
+                           int C, int relu, cudaStream_t stream, float cap = INFINITY) {
   constexpr int V = Vec<T>::N;
   if (C % V != 0) { kb200_set_error("bn: C must be a multiple of the vector width"); return -2; }
+  if (cap < INFINITY && (res != nullptr || !relu)) { kb200_set_error("bn: an upper bound needs the ReLU and no residual"); return -2; }
   if (res == nullptr) {
     static const int resident8 = bn_resident_blocks(bn_apply_kernel<T, 0, 8>);
     const BnGeom g8 = bn_geom(M, C / V, resident8, 8);
     bn_apply_kernel<T, 0, 8><<<dim3(g8.gx, g8.gy), BN_THREADS, 0, stream>>>((const T*)x, nullptr, nullptr, bits, (T*)y, nullptr, scale, shift, nullptr,
-                                                                           M, C, ilog2(g8.cx), relu);
+                                                                           M, C, ilog2(g8.cx), relu, cap);
     KB_CHECK_LAUNCH("bn_apply");
     return 0;
   }
@@ -425,6 +433,14 @@ KB_API int kb200_bn_apply_mask(const void* x, const void* res, void* y, unsigned
                                int C, int relu, int dtype, cudaStream_t stream) {
   return dtype == 1 ? bn_apply_launch<__nv_bfloat16>(x, res, y, bits, scale, shift, M, C, relu, stream)
                     : bn_apply_launch<float>(x, res, y, bits, scale, shift, M, C, relu, stream);
+}
+
+// As kb200_bn_apply_mask without a residual, for a ReLU with an upper bound: y = min(max(., 0), cap), bit k = 0 < element k < cap
+// (`bits` may be null).
+KB_API int kb200_bn_apply_cap(const void* x, void* y, unsigned char* bits, const float* scale, const float* shift, long long M, int C, float cap, int dtype,
+                              cudaStream_t stream) {
+  return dtype == 1 ? bn_apply_launch<__nv_bfloat16>(x, nullptr, y, bits, scale, shift, M, C, 1, stream, cap)
+                    : bn_apply_launch<float>(x, nullptr, y, bits, scale, shift, M, C, 1, stream, cap);
 }
 
 KB_API int kb200_bn_bwd_reduce(const void* dy, const void* x, const void* y, const float* mean, const float* invstd, long long M, int C, int dtype,

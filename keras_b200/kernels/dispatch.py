@@ -185,11 +185,11 @@ def rms_norm(x, scale, eps):
     return _ops().FusedNorm.apply(x, scale, None, float(eps), True)
 
 
-def batch_norm(layer, inputs, training, residual=None, relu=False, pre_bias=None, conv_stats=None):
+def batch_norm(layer, inputs, training, residual=None, relu=False, pre_bias=None, conv_stats=None, cap=None):
     """Fused channels-last BatchNorm (+residual)(+ReLU).  Returns ``None`` when not applicable.
 
     ``conv_stats``: partial sums of ``inputs`` left by the producing convolution kernel (training mode only); the
-    statistics pass over ``inputs`` is then skipped."""
+    statistics pass over ``inputs`` is then skipped.  ``cap``: upper bound of the ReLU (no residual then)."""
     x = inputs
     if not enabled(x) or x.dtype not in _FLOAT_IO or x.ndim < 2:
         return None
@@ -214,7 +214,7 @@ def batch_norm(layer, inputs, training, residual=None, relu=False, pre_bias=None
         from keras_b200.kernels import grad_merge
 
         return ops.FusedBatchNormAct.apply(x, gamma, beta, residual, mm, mv, float(layer.momentum), float(layer.epsilon), bool(relu), pre_bias, conv_stats,
-                                           grad_merge.slot_of(residual))
+                                           grad_merge.slot_of(residual), cap)
     if torch.is_grad_enabled() and (x.requires_grad or (gamma is not None and gamma.requires_grad and layer.trainable)):
         return None
     with torch.no_grad():
@@ -223,7 +223,7 @@ def batch_norm(layer, inputs, training, residual=None, relu=False, pre_bias=None
         shift = -mm * scale if pre_bias is None else (pre_bias.float() - mm) * scale
         if beta is not None:
             shift = shift + beta
-    return ops.bn_inference(x, scale.contiguous(), shift.contiguous(), residual, relu)
+    return ops.bn_inference(x, scale.contiguous(), shift.contiguous(), residual, relu, cap)
 
 
 def max_pool2d(x, pool_size, strides, padding, zero_pad=None):

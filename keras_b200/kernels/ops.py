@@ -272,7 +272,7 @@ class FusedBatchNormAct(torch.autograd.Function):
     """y = relu?(batchnorm_train(x) (+ residual)) for channels-last x, with moving-stat update."""
 
     @staticmethod
-    def forward(ctx, x, gamma, beta, residual, moving_mean, moving_var, momentum, eps, relu, pre_bias=None, conv_stats=None, merge=None):
+    def forward(ctx, x, gamma, beta, residual, moving_mean, moving_var, momentum, eps, relu, pre_bias=None, conv_stats=None, merge=None, cap=None):
         lib = _lib()
         C = x.shape[-1]
         M = x.numel() // C
@@ -298,6 +298,9 @@ class FusedBatchNormAct(torch.autograd.Function):
         bits = None
         if relu:
             bits = torch.empty(M * (C // (8 if dt == 1 else 4)), dtype=torch.uint8, device=dev)
+        if relu and cap is not None:
+            _check(lib.kb200_bn_apply_cap(_p(x), _p(y), _p(bits), _p(scale), _p(shift), _ll(M), _i(C), _f(cap), _i(dt), st), "bn_apply")
+        elif relu:
             _check(lib.kb200_bn_apply_mask(_p(x), _p(res), _p(y), _p(bits), _p(scale), _p(shift), _ll(M), _i(C), _i(1), _i(dt), st), "bn_apply")
         else:
             _check(lib.kb200_bn_apply(_p(x), _p(res), _p(y), _p(scale), _p(shift), _ll(M), _i(C), _i(0), _i(dt), st), "bn_apply")
@@ -344,16 +347,19 @@ class FusedBatchNormAct(torch.autograd.Function):
                 dres = None
             else:
                 grad_merge.offer(ctx.merge, dres)
-        return dx, dgamma, dbeta, dres, None, None, None, None, None, None, None, None
+        return dx, dgamma, dbeta, dres, None, None, None, None, None, None, None, None, None
 
 
-def bn_inference(x, scale, shift, residual, relu):
-    """y = relu?(x*scale + shift (+ residual)) with per-channel fp32 scale/shift (no autograd)."""
+def bn_inference(x, scale, shift, residual, relu, cap=None):
+    """y = relu?(x*scale + shift (+ residual)) with per-channel fp32 scale/shift (no autograd); ``cap``: upper bound of the ReLU."""
     lib = _lib()
     C = x.shape[-1]
     M = x.numel() // C
     x = x.contiguous()
     y = torch.empty_like(x)
+    if cap is not None:
+        _check(lib.kb200_bn_apply_cap(_p(x), _p(y), _vp(0), _p(scale), _p(shift), _ll(M), _i(C), _f(cap), _i(_dt(x)), _stream()), "bn_apply")
+        return y
     res = residual.contiguous() if residual is not None else None
     _check(lib.kb200_bn_apply(_p(x), _p(res), _p(y), _p(scale), _p(shift), _ll(M), _i(C), _i(1 if relu else 0), _i(_dt(x)), _stream()), "bn_apply")
     return y

@@ -3,7 +3,7 @@
 The executor of a ``Functional`` walks its nodes in order; this module finds, once per model,
 the node patterns that a single sm_100a kernel can execute:
 
-* ``BatchNormalization → ReLU``                         → BN apply with fused ReLU
+* ``BatchNormalization → ReLU`` (or ReLU6)              → BN apply with fused ReLU
 * ``BatchNormalization → Add(other) [→ ReLU]``          → BN apply with fused residual add (and ReLU)
 
 (the residual bottleneck of keras/src/applications/resnet.py:219-273 is conv→BN→ReLU ×2, conv→BN,
@@ -14,6 +14,7 @@ with a channels-last BN; otherwise execution is node by node as written.
 
 import torch
 
+from keras_b200 import activations
 from keras_b200.layers.activations.activation_layers import Activation, ReLU
 from keras_b200.layers.merging.merging_layers import Add
 from keras_b200.layers.normalization.normalization_layers import BatchNormalization
@@ -53,6 +54,15 @@ def _is_relu(op):
     return False
 
 
+def _relu_cap(op):
+    """Upper bound of a ReLU layer with the sixes' strict derivative (the library's ``relu6``), or ``None``."""
+    if isinstance(op, ReLU):
+        six = op.max_value == 6.0 and op.negative_slope == 0.0 and op.threshold == 0.0
+    else:
+        six = isinstance(op, Activation) and op.activation is activations.relu6
+    return 6.0 if six else None
+
+
 def build_plan(function):
     """Return {id(node): role} with roles 'defer_bn', 'consume_add', 'consume_relu', 'maybe_identity'."""
     nodes = function._ordered_nodes()
@@ -81,7 +91,7 @@ def build_plan(function):
             continue
         if id(c) in plan:
             continue
-        if _is_relu(c.operation) and len(c.input_tensors) == 1:
+        if (_is_relu(c.operation) or _relu_cap(c.operation) is not None) and len(c.input_tensors) == 1:
             plan[id(n)] = "defer_bn"
             plan[id(c)] = "consume_relu"
         elif isinstance(c.operation, Add) and len(c.input_tensors) == 2 and len(c.outputs) == 1:
@@ -216,13 +226,13 @@ def applicable(x):
     return isinstance(x, torch.Tensor) and x.is_cuda
 
 
-def run_bn(layer, x, training, residual=None, relu=False, pre_bias=None, stats=None):
+def run_bn(layer, x, training, residual=None, relu=False, pre_bias=None, stats=None, cap=None):
     """Execute a (possibly fused) BatchNormalization outside of ``Layer.__call__``."""
     from keras_b200.kernels import dispatch
 
     train = bool(training) and layer.trainable
     bias_value = pre_bias._value if pre_bias is not None else None
-    out = dispatch.batch_norm(layer, x, train, residual=residual, relu=relu, pre_bias=bias_value, conv_stats=stats)
+    out = dispatch.batch_norm(layer, x, train, residual=residual, relu=relu, pre_bias=bias_value, conv_stats=stats, cap=cap)
     if out is not None:
         if pre_bias is not None and train:
             # A bias in front of a batch normalization in training mode is removed with the batch mean: its gradient is exactly
@@ -236,5 +246,5 @@ def run_bn(layer, x, training, residual=None, relu=False, pre_bias=None, stats=N
     if residual is not None:
         out = out + residual
     if relu:
-        out = torch.relu(out)
+        out = torch.relu(out) if cap is None else torch.nn.functional.hardtanh(out, 0.0, cap)
     return out

@@ -180,7 +180,8 @@ class Function(Operation):
                 continue
             if role == "consume_relu":
                 d = env[id(ins[0])]
-                env[id(outs[0])] = fusion.run_bn(d.layer, d.x, training, relu=True, pre_bias=d.pre_bias, stats=d.stats) if isinstance(d, fusion.Deferred) else node.operation(d)
+                env[id(outs[0])] = fusion.run_bn(d.layer, d.x, training, relu=True, pre_bias=d.pre_bias, stats=d.stats,
+                                                       cap=fusion.relu_cap(node.operation)) if isinstance(d, fusion.Deferred) else node.operation(d)
                 continue
             if role in ("consume_add", "consume_add_relu"):
                 a, b = env[id(ins[0])], env[id(ins[1])]

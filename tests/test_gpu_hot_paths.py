@@ -349,3 +349,56 @@ def test_depthwise_routes():
     y = dw.depthwise(xg * 1, w, (1, 1), "same", "channels_last", (1, 1))
     (g,) = torch.autograd.grad((y.float() ** 2).sum(), xg, create_graph=True)
     assert torch.autograd.grad(g.float().square().sum(), xg)[0].isfinite().all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,C", [(5, 8), (4097, 48), (30000, 144)])
+def test_batch_norm_with_relu6_is_the_two_layers(rows, C, dtype):
+    from keras_b200.kernels import ops as kops
+
+    torch.manual_seed(C)
+    x = (torch.randn(rows, C, device="cuda") * 2).to(dtype).requires_grad_(True)
+    gamma = (torch.rand(C, device="cuda") * 4 + 0.5).requires_grad_(True)
+    beta = (torch.randn(C, device="cuda") + 1.5).requires_grad_(True)
+    dy = torch.randn(rows, C, device="cuda").to(dtype)
+    results = []
+    for fused in (True, False):
+        mm, mv = torch.zeros(C, device="cuda"), torch.ones(C, device="cuda")
+        args = (x, gamma, beta, None, mm, mv, 0.9, 1e-3)
+        y = kops.FusedBatchNormAct.apply(*args, True, None, None, None, 6.0) if fused else torch.nn.functional.relu6(kops.FusedBatchNormAct.apply(*args, False))
+        results.append((y.detach(),) + torch.autograd.grad(y, (x, gamma, beta), dy))
+    # the statistics are fp32 atomic sums (a few 2^-24 apart from run to run), the output is rounded once
+    step = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-5
+    (y0, dx0, dg0, db0), (y1, dx1, dg1, db1) = results
+    assert torch.allclose(y0.float(), y1.float(), rtol=step, atol=step)
+    # an element that those sums move across a bound gains or loses its gradient: hardly any may
+    assert (~torch.isclose(dx0.float(), dx1.float(), rtol=4 * step, atol=4 * step * dx1.float().abs().max().item())).float().mean().item() < 1e-3
+    for a, b in ((dg0, dg1), (db0, db1)):
+        assert torch.allclose(a, b, rtol=1e-2, atol=1e-2 * b.abs().max().item())
+
+
+def test_model_with_relu6_folds_it_into_the_normalisation():
+    import keras_b200 as keras
+
+    L = keras.layers
+    keras.utils.set_random_seed(3)
+    x = keras.Input((8, 8, 16))
+    h = L.ReLU(6.0)(L.BatchNormalization()(L.Conv2D(32, 1)(x)))
+    h = L.Activation("relu6")(L.BatchNormalization()(L.DepthwiseConv2D(3, padding="same")(h)))
+    model = keras.Model(x, L.ReLU(4.0)(L.BatchNormalization()(L.Conv2D(16, 1)(h))))
+    data = torch.randn(4, 8, 8, 16, device="cuda") * 3
+    for training in (False, True):
+        state = [v.value.clone() for v in model.weights]
+        got = model(data, training=training)
+        for v, s in zip(model.weights, state):
+            v.assign(s)
+        want = data
+        for layer in model.layers[1:]:
+            want = layer(want, training=training)
+        for v, s in zip(model.weights, state):
+            v.assign(s)
+        assert torch.allclose(got, want, atol=1e-4, rtol=1e-4)
+    from keras_b200.models import fusion
+
+    plan = fusion.build_plan(model)
+    assert list(plan.values()).count("consume_relu") == 2  # the bound of four keeps its own layer
