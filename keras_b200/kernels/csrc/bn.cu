@@ -67,6 +67,32 @@ static BnGeom bn_geom(long long M, int cvecs, int resident, int rows_per_iter) {
   return g;
 }
 
+// Geometry of the apply kernels, which exchange nothing between lanes: as many channel vectors a block as the tensor has, up to 32
+// (or a divisor of a larger number), so that 144 channels (18 vectors) keep 252 of 256 threads busy where the next power of two
+// kept 144: the five forward passes of two inverted residual blocks (48 to 192 channels) 149 -> 106 us.
+static BnGeom bn_geom_apply(long long M, int cvecs, int resident, int rows_per_iter) {
+  BnGeom g;
+  g.cx = 1;
+  double best = 0.0;
+  for (int cx = 1; cx <= 64 && cx <= cvecs; ++cx) {
+    const int blocks = (cvecs + cx - 1) / cx;
+    double busy = (double)(BN_THREADS / cx * cx) / BN_THREADS * cvecs / ((double)blocks * cx);
+    if (cx < 8 && cx < cvecs) busy *= 0.8;  // rows of less than 128 bytes
+    if (busy >= best) {
+      best = busy;
+      g.cx = cx;
+    }
+  }
+  g.ry = BN_THREADS / g.cx;
+  g.gy = (cvecs + g.cx - 1) / g.cx;
+  long long want = ((long long)bn_sm_count() * resident) / g.gy;
+  if (want < 1) want = 1;
+  const long long maxb = (M + (long long)g.ry * rows_per_iter - 1) / ((long long)g.ry * rows_per_iter);
+  g.gx = (int)(want < maxb ? want : maxb);
+  if (g.gx < 1) g.gx = 1;
+  return g;
+}
+
 template <typename K>
 static int bn_resident_blocks(K kernel) {
   int n = 0;
@@ -258,17 +284,16 @@ template <typename T, int MODE, int U = BN_U>
 __global__ void __launch_bounds__(BN_THREADS, 2) bn_apply_kernel(const T* __restrict__ in0, const T* __restrict__ in1, const T* __restrict__ ymask,
                                                              unsigned char* __restrict__ bits, T* __restrict__ out0, T* __restrict__ out1,
                                                              const float* __restrict__ p0, const float* __restrict__ p1,
-                                                             const float* __restrict__ p2, long long M, int C, int cx_log2, int relu,
+                                                             const float* __restrict__ p2, long long M, int C, int cx, int relu,
                                                              float cap = INFINITY) {
   constexpr int V = Vec<T>::N;
   const bool capped = cap < INFINITY;
   // the 8-row instance is the forward pass without a second input: known at compile time so that no registers are held for it
   const bool has1 = (U == 8) ? false : in1 != nullptr;
   const int cvecs = C / V;
-  const int cx = 1 << cx_log2, ry = BN_THREADS >> cx_log2;
-  const int tx = threadIdx.x & (cx - 1), ty = threadIdx.x >> cx_log2;
+  const int ry = BN_THREADS / cx, tx = threadIdx.x % cx, ty = threadIdx.x / cx;
   const int cv = blockIdx.y * cx + tx;
-  if (cv >= C / V) return;
+  if (cv >= cvecs || ty >= ry) return;
   const int c0 = cv * V;
   float a[V], b[V], cc[V];
 #pragma unroll
@@ -403,9 +428,9 @@ static int bn_apply_launch(const void* x, const void* res, void* y, unsigned cha
   if (cap < INFINITY && (res != nullptr || !relu)) { kb200_set_error("bn: an upper bound needs the ReLU and no residual"); return -2; }
   if (res == nullptr) {
     static const int resident8 = bn_resident_blocks(bn_apply_kernel<T, 0, 8>);
-    const BnGeom g8 = bn_geom(M, C / V, resident8, 8);
+    const BnGeom g8 = bn_geom_apply(M, C / V, resident8, 8);
     bn_apply_kernel<T, 0, 8><<<dim3(g8.gx, g8.gy), BN_THREADS, 0, stream>>>((const T*)x, nullptr, nullptr, bits, (T*)y, nullptr, scale, shift, nullptr,
-                                                                           M, C, ilog2(g8.cx), relu, cap);
+                                                                           M, C, g8.cx, relu, cap);
     KB_CHECK_LAUNCH("bn_apply");
     return 0;
   }
@@ -414,9 +439,9 @@ static int bn_apply_launch(const void* x, const void* res, void* y, unsigned cha
     if (rc <= 0) return rc;
   }
   static const int resident = bn_resident_blocks(bn_apply_kernel<T, 0>);
-  const BnGeom g = bn_geom(M, C / V, resident, BN_U);
+  const BnGeom g = bn_geom_apply(M, C / V, resident, BN_U);
   bn_apply_kernel<T, 0><<<dim3(g.gx, g.gy), BN_THREADS, 0, stream>>>((const T*)x, (const T*)res, nullptr, bits, (T*)y, nullptr, scale, shift,
-                                                                    nullptr, M, C, ilog2(g.cx), relu);
+                                                                    nullptr, M, C, g.cx, relu);
   KB_CHECK_LAUNCH("bn_apply");
   return 0;
 }
@@ -458,9 +483,9 @@ static int bn_bwd_apply_launch(const void* dy, const void* x, const void* y, con
     if (rc <= 0) return rc;
   }
   static const int resident = bn_resident_blocks(bn_apply_kernel<T, 1>);
-  const BnGeom g = bn_geom(M, C / V, resident, BN_U);
+  const BnGeom g = bn_geom_apply(M, C / V, resident, BN_U);
   bn_apply_kernel<T, 1><<<dim3(g.gx, g.gy), BN_THREADS, 0, stream>>>((const T*)dy, (const T*)x, (const T*)y, const_cast<unsigned char*>(bits),
-                                                                    (T*)dx, (T*)dres, coef, coef + C, coef + 2 * C, M, C, ilog2(g.cx), 0);
+                                                                    (T*)dx, (T*)dres, coef, coef + C, coef + 2 * C, M, C, g.cx, 0);
   KB_CHECK_LAUNCH("bn_bwd_apply");
   return 0;
 }

@@ -36,9 +36,9 @@ struct BsParams {
   float* sums;
   long long M;
   long long tiles;
-  int C, cvecs, cv_log2;
+  int C, cvecs;
   int rows_per_pass;  // BS_CONSUMERS / cvecs
-  int tile_rows;      // multiple of rows_per_pass, tile_rows * C * 2 <= BS_TILE_BYTES
+  int tile_rows;      // tile_rows * C * 2 <= BS_TILE_BYTES, tile_rows * cvecs a multiple of 16
   int relu;
 };
 
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) bn_stream_kernel(const BsParams
   __shared__ int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool stage_bits = MODE != 0 && p.bits_in != nullptr;
-  const uint32_t bits_stage_bytes = (uint32_t)p.tile_rows * p.cvecs;  // a multiple of BS_CONSUMERS, hence of 16
+  const uint32_t bits_stage_bytes = (uint32_t)p.tile_rows * p.cvecs;  // a multiple of 16: size and offset of a bulk copy
   const uint32_t stage_bytes = 2u * BS_TILE_BYTES + (stage_bits ? bits_stage_bytes : 0u);
   if (tid == 0) {
     for (int s = 0; s < BS_STAGES; ++s) {
@@ -142,7 +142,8 @@ __global__ void __launch_bounds__(BS_THREADS, 1) bn_stream_kernel(const BsParams
   }
 
   // ---- consumers
-  const int cv = tid & (p.cvecs - 1), rl = tid >> p.cv_log2;
+  // any number of vectors up to the consumers: 18 (144 channels) leave 8 of the 512 threads without a row
+  const int cv = tid % p.cvecs, rl = tid / p.cvecs < p.rows_per_pass ? tid / p.cvecs : p.tile_rows;
   const int c0 = cv * 8;
   float a[8], b[8], cc[8], sa[8], sb[8];
 #pragma unroll
@@ -227,7 +228,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) bn_stream_kernel(const BsParams
     asm volatile("bar.sync 1, %0;" ::"n"(BS_CONSUMERS) : "memory");
     // 16 * cvecs sums, each over rows_per_pass threads: thread j handles (quantity q, vector v) pairs
     for (int j = tid; j < 16 * p.cvecs; j += BS_CONSUMERS) {
-      const int q = j >> p.cv_log2, v = j & (p.cvecs - 1);
+      const int q = j / p.cvecs, v = j % p.cvecs;
       float acc = 0.f;
       for (int r = 0; r < p.rows_per_pass; ++r) acc += red[q * BS_CONSUMERS + r * p.cvecs + v];
       const int c = v * 8 + (q & 7);
@@ -283,8 +284,10 @@ int kb200_bn_stream_launch(int mode, const void* in0, const void* in1, const uns
                            const float* p0, const float* p1, const float* p2, float* sums, long long M, int C, int relu, cudaStream_t stream) {
   if (!bs_enabled() || in0 == nullptr || in1 == nullptr || C % 8 != 0) return 1;
   const int cvecs = C / 8;
-  if (cvecs < 1 || cvecs > BS_CONSUMERS || (cvecs & (cvecs - 1)) != 0) return 1;
+  if (cvecs < 1 || cvecs > BS_CONSUMERS) return 1;
   if (M * (long long)C < (1ll << 21)) return 1;  // small tensors: the register kernels have less set-up
+  // the reduction hands each of its few blocks a handful of tiles there, [7776, 384] 12 us against 6 in registers
+  if (mode == 1 && (cvecs & (cvecs - 1)) != 0 && M * (long long)C < (1ll << 23)) return 1;
   const uintptr_t align = (uintptr_t)in0 | (uintptr_t)in1 | (uintptr_t)out0 | (uintptr_t)out1 | (uintptr_t)bits_in;
   if (align & 15) return 1;
   BsParams p;
@@ -301,28 +304,33 @@ int kb200_bn_stream_launch(int mode, const void* in0, const void* in1, const uns
   p.M = M;
   p.C = C;
   p.cvecs = cvecs;
-  p.cv_log2 = 0;
-  while ((1 << p.cv_log2) < cvecs) ++p.cv_log2;
   p.rows_per_pass = BS_CONSUMERS / cvecs;
-  int passes = BS_TILE_BYTES / (C * 2) / p.rows_per_pass;
-  if (passes < 1) return 1;
-  p.tile_rows = passes * p.rows_per_pass;
+  const int fit = BS_TILE_BYTES / (C * 2);
+  // whole passes where they keep the mask bytes of a tile a multiple of 16, else the most rows that do
+  p.tile_rows = fit / p.rows_per_pass * p.rows_per_pass;
+  if ((p.tile_rows * cvecs) % 16) {
+    int step = 16;
+    while (step > 1 && (step / 2 * cvecs) % 16 == 0) step /= 2;
+    p.tile_rows = fit / step * step;
+  }
+  if (p.tile_rows < 1) return 1;
   p.tiles = (M + p.tile_rows - 1) / p.tile_rows;
   p.relu = relu;
   const size_t bits_stage = (mode != 0 && bits_in != nullptr) ? (size_t)p.tile_rows * cvecs : 0;
   const size_t smem = (size_t)BS_STAGES * (2 * BS_TILE_BYTES + bits_stage);
+  const size_t most = (size_t)BS_STAGES * (2 * BS_TILE_BYTES + BS_TILE_BYTES / 16);  // with the mask bytes of any tile
   long long grid = bs_sm_count();
   if (grid > p.tiles) grid = p.tiles;
   if (mode == 1 && grid > p.tiles / 4) grid = p.tiles / 4 > 0 ? p.tiles / 4 : 1;  // fewer blocks, fewer atomics per channel
   int rc = 0;
   if (mode == 0) {
-    rc = bs_set_attr<0>(smem);
+    rc = bs_set_attr<0>(most);
     if (rc == 0) bn_stream_kernel<0><<<(int)grid, BS_THREADS, smem, stream>>>(p);
   } else if (mode == 1) {
-    rc = bs_set_attr<1>(smem);
+    rc = bs_set_attr<1>(most);
     if (rc == 0) bn_stream_kernel<1><<<(int)grid, BS_THREADS, smem, stream>>>(p);
   } else {
-    rc = bs_set_attr<2>(smem);
+    rc = bs_set_attr<2>(most);
     if (rc == 0) bn_stream_kernel<2><<<(int)grid, BS_THREADS, smem, stream>>>(p);
   }
   if (rc != 0) return 1;

@@ -402,3 +402,31 @@ def test_model_with_relu6_folds_it_into_the_normalisation():
 
     plan = fusion.build_plan(model)
     assert list(plan.values()).count("consume_relu") == 2  # the bound of four keeps its own layer
+
+
+@pytest.mark.parametrize("relu,res", [(True, True), (True, False), (False, False)])
+@pytest.mark.parametrize("rows,C", [(20011, 144), (15003, 192), (70001, 48), (3001, 960), (9001, 320), (2200, 1000), (600, 4096), (30, 24)])
+def test_batch_norm_at_channel_counts_that_are_no_power_of_two(rows, C, relu, res):
+    """The bulk-copy ring and the register kernels, with ragged last tiles; against the same mathematics in 64 bits."""
+    from keras_b200.kernels import ops as kops
+
+    torch.manual_seed(C)
+    x = (torch.randn(rows, C, device="cuda") * 1.5 + 0.25).bfloat16().requires_grad_(True)
+    r = torch.randn(rows, C, device="cuda").bfloat16().requires_grad_(True) if res else None
+    gamma, beta = (torch.rand(C, device="cuda") + 0.5).requires_grad_(True), torch.randn(C, device="cuda").requires_grad_(True)
+    mm, mv = torch.zeros(C, device="cuda"), torch.ones(C, device="cuda")
+    y = kops.FusedBatchNormAct.apply(x, gamma, beta, r, mm, mv, 0.9, 1e-3, relu)
+    dy = torch.randn_like(y)
+    got = torch.autograd.grad(y, [x, gamma, beta] + ([r] if res else []), dy)
+    kops.check_stream_kernels()
+    xe, ge, be = (t.detach().double().requires_grad_(True) for t in (x, gamma, beta))
+    re = r.detach().double().requires_grad_(True) if res else None
+    mean, var = xe.mean(0), xe.var(0, correction=0)
+    ref = (xe - mean) * torch.rsqrt(var + 1e-3) * ge + be + (re if res else 0)
+    # the mask that the kernel took: a value within rounding of zero may go either way
+    ref = ref * (y.double() > 0) if relu else ref
+    want = torch.autograd.grad(ref, [xe, ge, be] + ([re] if res else []), dy.double())
+    rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()  # noqa: E731
+    assert rel(y, ref) < 2.0 ** -8
+    for a, b, bound in zip(got, want, (2.0 ** -8, 2.0 ** -10, 2.0 ** -10, 2.0 ** -8)):  # dx and dres rounded to bf16; sums in fp32 of exact products
+        assert rel(a, b) < bound
