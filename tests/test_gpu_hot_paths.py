@@ -1,5 +1,7 @@
 """The variants a dispatch rule chooses between, each at the sizes where it can go wrong (needs a B200)."""
 
+import gc
+
 import pytest
 import torch
 
@@ -269,6 +271,7 @@ def test_inference_copies_stay_out_of_recordings_and_transforms():
     with torch.no_grad():
         for _ in range(3):
             model(x, training=False)
+        gc.collect()  # a recorded step of an earlier model, released during a capture, would invalidate it
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
             out = model(x, training=False)
@@ -430,3 +433,27 @@ def test_batch_norm_at_channel_counts_that_are_no_power_of_two(rows, C, relu, re
     assert rel(y, ref) < 2.0 ** -8
     for a, b, bound in zip(got, want, (2.0 ** -8, 2.0 ** -10, 2.0 ** -10, 2.0 ** -8)):  # dx and dres rounded to bf16; sums in fp32 of exact products
         assert rel(a, b) < bound
+
+
+@pytest.mark.parametrize("M,K,N", [(77, 64, 301), (129, 72, 136), (1001, 256, 512), (8446, 128, 1001), (2667, 512, 2048), (3, 768, 5001)])
+def test_dense_products_at_any_number_of_rows(M, K, N):
+    from keras_b200.kernels import gemm
+
+    torch.manual_seed(M)
+    x = torch.randn(M, K, device="cuda").bfloat16().requires_grad_(True)
+    w = (torch.randn(K, N, device="cuda") * K ** -0.5).bfloat16().requires_grad_(True)
+    b = torch.randn(N, device="cuda").requires_grad_(True)
+    assert gemm._qualifies(x, w) == (2 * M * N * K >= gemm._MIN_WORK)
+    y = gemm.GemmFn.apply(x, w, b, None, None)
+    dy = torch.randn(M, N, device="cuda").bfloat16()
+    y.backward(dy)
+    gemm.check_errors()
+    xe, we, be = (t.detach().double().requires_grad_(True) for t in (x, w, b))
+    ye = xe @ we + be
+    ye.backward(dy.double())
+    rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()  # noqa: E731
+    assert rel(y, ye) < 2.0 ** -8 and rel(x.grad, xe.grad) < 2.0 ** -8 and rel(w.grad, we.grad) < 2.0 ** -8 and rel(b.grad, be.grad) < 1e-5
+    with torch.no_grad():  # the fused form of inference
+        out, done = gemm.dense(x, w, b, "gelu") or (None, None)
+        if out is not None:
+            assert done and rel(out, torch.nn.functional.gelu(ye)) < 2.0 ** -8
