@@ -171,8 +171,10 @@ def _qualifies(x2, w, padded=False):
     # Rows may be any number: the copies clip them.  Below a tile of them the library's small-batch kernels are quicker (77 x 3072 x
     # 768: 4 us against 10) where it has aligned ones; a width that is no multiple of 8 sends it to kernels of three generations ago
     # (77 x 50257 x 768 100 us).
-    if K % 8 or (N % 8 and N < 256) or (M % 8 and M < 128 and N % 8 == 0):
+    if K % 8 or (M % 8 and M < 128 and N % 8 == 0):
         return False
+    if N % 8 and N < 256 and (N < 16 or M < 8192):
+        return False  # few classes: padding them pays where the rows are many
     return 2 * M * N * K >= _MIN_WORK
 
 

@@ -435,7 +435,7 @@ def test_batch_norm_at_channel_counts_that_are_no_power_of_two(rows, C, relu, re
         assert rel(a, b) < bound
 
 
-@pytest.mark.parametrize("M,K,N", [(77, 64, 301), (129, 72, 136), (1001, 256, 512), (8446, 128, 1001), (2667, 512, 2048), (3, 768, 5001)])
+@pytest.mark.parametrize("M,K,N", [(77, 64, 301), (129, 72, 136), (1001, 256, 512), (8446, 128, 1001), (2667, 512, 2048), (3, 768, 5001), (8193, 32, 21), (20000, 384, 37)])
 def test_dense_products_at_any_number_of_rows(M, K, N):
     from keras_b200.kernels import gemm
 
