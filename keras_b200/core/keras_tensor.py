@@ -3,6 +3,8 @@
 Reference behaviour: keras/src/backend/common/keras_tensor.py:7-425.
 """
 
+import torch
+
 from keras_b200.core.dtypes import standardize_dtype
 from keras_b200.core.export_registry import keras_export
 from keras_b200.core.naming import auto_name
@@ -134,17 +136,17 @@ KerasTensor.__round__ = lambda self, ndigits=None: __import__("keras_b200").ops.
 def any_symbolic_tensors(args=None, kwargs=None):
     """True when any leaf of (args, kwargs) is a KerasTensor."""
     for x in args or ():
-        if isinstance(x, KerasTensor):
-            return True
-        if isinstance(x, (list, tuple, dict)) and _has_symbolic(x):
+        if type(x) not in _NEVER_SYMBOLIC and (isinstance(x, KerasTensor) or (isinstance(x, (list, tuple, dict)) and _has_symbolic(x))):
             return True
     if kwargs:
         for x in kwargs.values():
-            if isinstance(x, KerasTensor):
-                return True
-            if isinstance(x, (list, tuple, dict)) and _has_symbolic(x):
+            if type(x) not in _NEVER_SYMBOLIC and (isinstance(x, KerasTensor) or (isinstance(x, (list, tuple, dict)) and _has_symbolic(x))):
                 return True
     return False
+
+
+# what most arguments of an eager call are, by exact type
+_NEVER_SYMBOLIC = frozenset((torch.Tensor, torch.nn.Parameter, type(None), bool, int, float, str))
 
 
 def _has_symbolic(x):

@@ -215,15 +215,15 @@ def _wide_weight(variable, x):
     return (value.to(torch.bfloat16), None) if wide is None else (wide[:, : shape[1]], wide)
 
 
-def dense(x, kernel, bias, activation_name, kernel_shape=None):
-    """Returns ``(output, activation_applied)`` or ``None``.  ``kernel`` may be a ``Variable`` (reshaped to the 2-D
+def dense(x, kernel, bias, activation_name, kernel_shape=None, value=None):
+    """``value``: what ``kernel`` (a ``Variable``) reads as, when the caller has already read it.  Returns ``(output, activation_applied)`` or ``None``.  ``kernel`` may be a ``Variable`` (reshaped to the 2-D
     ``kernel_shape`` when given) or a tensor."""
     from keras_b200.core.variables import Variable
 
     wide = None
     if isinstance(kernel, Variable):
         read = _wide_weight(kernel, x) if kernel_shape is None and isinstance(x, torch.Tensor) else None
-        w, wide = (kernel.value, None) if read is None else read
+        w, wide = (kernel.value if value is None else value, None) if read is None else read
     else:
         w = kernel
     if kernel_shape is not None:

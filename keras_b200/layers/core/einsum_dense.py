@@ -268,12 +268,16 @@ class EinsumDense(CalibratedKernel, Layer):
                 bv = bias.value if hasattr(bias, "value") else bias
                 if tuple(bv.shape) == out_dims:
                     bflat = bv.reshape(-1)
-            if bias is None or bflat is not None:
-                fused = dispatch.dense(x2, source, bflat, None, kernel_shape=(kdim, -1))
+            asked = bias is None or bflat is not None
+            if asked:
+                fused = dispatch.dense(x2, source, bflat, None, kernel_shape=(kdim, -1), value=kv)
                 if fused is not None:
                     out = fused[0].reshape(tuple(lead) + out_dims)
                     return out if bias is None else (out, True)
-            out = ops.matmul(x2, kv.reshape(kdim, -1)).reshape(tuple(lead) + out_dims)
+            k2 = kv.reshape(kdim, -1)
+            # the GEMM has just declined these operands: the op would only ask it again
+            product = torch.matmul if asked and type(x2) is torch.Tensor and x2.is_cuda and x2.dtype == k2.dtype == torch.bfloat16 else ops.matmul
+            out = product(x2, k2).reshape(tuple(lead) + out_dims)
             return out if bias is None else (out, False)
         out = ops.einsum(self.equation, inputs, kernel)
         return out if bias is None else (out, False)

@@ -118,6 +118,9 @@ class _CallPlan:
         self.build_by_name = len(self.build_names) > 0 and all(n.endswith("_shape") or n.endswith("_shapes") for n in self.build_names) and not (len(self.build_names) == 1 and self.build_names[0] in ("input_shape", "inputs_shape", "input_shapes"))
 
 
+# policies that stand for themselves (anything else may be a map from layer paths to policies)
+_SINGLE_POLICIES = (dtype_policies.DTypePolicy, dtype_policies.FloatDTypePolicy)
+
 _PLANS = {}
 
 
@@ -640,9 +643,11 @@ class Layer(Operation):
                 self.quantize(policy.quantization_mode)
 
     def _resolved_policy(self):
+        p = self._dtype_policy
+        if type(p) in _SINGLE_POLICIES:
+            return p
         from keras_b200.dtype_policies.dtype_policy_map import DTypePolicyMap
 
-        p = self._dtype_policy
         if isinstance(p, DTypePolicyMap):
             return p[self.path] if self.path else p.default_policy
         return p

@@ -26,6 +26,23 @@ class SymbolicArguments:
             and isinstance(self.args[0], KerasTensor)
             and len(self.keras_tensors) == 1
         )
+        # Nearly as fast: KerasTensors and plain lists of them among the positional arguments, none among the others.
+        self._template = self._make_template()
+
+    def _make_template(self):
+        if any(isinstance(x, KerasTensor) for x in tree.flatten(self.kwargs)):
+            return None
+        template = []
+        for a in self.args:
+            if isinstance(a, KerasTensor):
+                template.append((id(a), None, None))
+            elif type(a) is list and a and all(isinstance(x, KerasTensor) for x in a):
+                template.append((None, [id(x) for x in a], None))
+            elif any(isinstance(x, KerasTensor) for x in tree.flatten(a)):
+                return None
+            else:
+                template.append((None, None, a))
+        return template
 
     def convert(self, conversion_fn):
         return tree.map_structure(
@@ -37,6 +54,10 @@ class SymbolicArguments:
         if self._single:
             v = tensor_dict.get(id(self.args[0]), None)
             return (v,) + tuple(self.args[1:]), self.kwargs
+        if self._template is not None:
+            get = tensor_dict.get
+            return tuple(get(one) if one is not None else [get(i) for i in many] if many is not None else constant
+                         for one, many, constant in self._template), self.kwargs
         flat = list(self._flat)
         for i in self._slots:
             v = tensor_dict.get(id(flat[i]), None)

@@ -7,6 +7,8 @@ dict entries are visited in sorted-key order, ``None`` is a leaf, namedtuples ke
 import collections
 import collections.abc
 
+import torch
+
 from keras_b200.core.export_registry import keras_export
 
 
@@ -36,6 +38,10 @@ def register_tree_node(cls, flatten_func=None, unflatten_func=None):
     return cls
 
 
+# exact types that are leaves whatever is registered: the usual ones never reach the abstract-class checks below
+_LEAVES = frozenset((torch.Tensor, torch.nn.Parameter, type(None), bool, int, float, str))
+
+
 def _is_namedtuple(x):
     return isinstance(x, tuple) and hasattr(x, "_fields")
 
@@ -52,6 +58,8 @@ def _sorted_keys(d):
 def _children(x):
     """Return (keys, values, rebuild) or None for a leaf."""
     t = type(x)
+    if t in _LEAVES:
+        return None
     if t in _REGISTERED:
         fl, un = _REGISTERED[t]
         children, aux = fl(x)
