@@ -115,7 +115,7 @@ class GemmFn(torch.autograd.Function):
         Np = (N + 7) // 8 * 8
         b32 = bias.float().contiguous() if bias is not None else None
         if Np != N:
-            w = torch.nn.functional.pad(w, (0, Np - N))
+            w = kops.pad_columns(w, Np)
             if b32 is not None:
                 b32 = torch.nn.functional.pad(b32, (0, Np - N))
         out = gemm(x, w, 0, 1, M, Np, K, bias=b32)
@@ -243,7 +243,7 @@ def dense(x, kernel, bias, activation_name, kernel_shape=None, value=None):
         N = w.shape[1]
         b32 = b.float().contiguous() if b is not None else None
         if N % 8:
-            w = torch.nn.functional.pad(w, (0, 8 - N % 8)) if wide is None else wide
+            w = kops.pad_columns(w, N + 8 - N % 8) if wide is None else wide
             b32 = torch.nn.functional.pad(b32, (0, 8 - N % 8)) if b32 is not None else None
         out = gemm(x2, w, 0, 1, x2.shape[0], w.shape[1], x2.shape[1], bias=b32, act=act or 0)
         if N % 8:

@@ -559,6 +559,25 @@ class OptimizerPlan:
                                     _stream()), "fused_rule")
 
 
+def pad_columns(x, width):
+    """A 2-D tensor with zero columns appended up to ``width``; one kernel for a contiguous bf16 CUDA matrix."""
+    if not (type(x) in (torch.Tensor, torch.nn.Parameter) and x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and width % 8 == 0
+            and max(x.shape[0], width) < 1 << 31) or (torch.is_grad_enabled() and x.requires_grad) or torch._C._are_functorch_transforms_active():
+        return torch.nn.functional.pad(x, (0, width - x.shape[1]))
+    out = torch.empty((x.shape[0], width), dtype=x.dtype, device=x.device)
+    _check(_lib().kb200_pad_columns(_p(x), _p(out), _i(x.shape[0]), _i(x.shape[1]), _i(width), _stream()), "pad_columns")
+    return out
+
+
+def add_rows(dst, src):
+    """``dst += src`` for a contiguous fp32 matrix and a bf16 one whose rows may be the leading columns of wider ones."""
+    if (dst.ndim == 2 and src.dtype == torch.bfloat16 and dst.dtype == torch.float32 and dst.is_cuda and src.is_cuda and dst.is_contiguous()
+            and src.shape == dst.shape and src.stride(1) == 1 and src.shape[1] > 1 and not src.is_contiguous() and max(src.shape) < 1 << 31):
+        _check(_lib().kb200_add_rows(_p(src), _ll(src.stride(0)), _p(dst), _i(src.shape[0]), _i(src.shape[1]), _stream()), "add_rows")
+        return dst
+    return dst.add_(src)
+
+
 def cast_f32_to_bf16(src, dst):
     lib = _lib()
     _check(lib.kb200_cast_f32_bf16(_p(src), _p(dst), _ll(src.numel()), _stream()), "cast_f32_bf16")

@@ -91,7 +91,9 @@ class _ShadowRead(torch.autograd.Function):
             return None, None
         g = grad_slot(ctx.param, grad.shape)
         if g is not None:
-            g.view(grad.shape).add_(grad)
+            from keras_b200.kernels import ops
+
+            ops.add_rows(g.view(grad.shape), grad)
             return None, None
         return grad.float(), None
 

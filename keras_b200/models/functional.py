@@ -289,12 +289,12 @@ class Functional(Function, Model):
 
 
 class _FusionCtx:
-    __slots__ = ("mod", "training", "Deferred", "NoBias", "run_bn", "run_conv_nobias", "run_pool_padded", "Padded", "build_plan", "applicable", "relu_cap")
+    __slots__ = ("mod", "training", "Deferred", "NoBias", "run_bn", "run_conv_nobias", "run_pool_padded", "Padded", "build_plan", "applicable", "relu_cap", "shared_cast")
 
     def __init__(self, mod, training):
         self.mod, self.training = mod, training
         self.Deferred, self.NoBias, self.run_bn, self.build_plan, self.applicable = mod.Deferred, mod.NoBias, mod.run_bn, mod.build_plan, mod.applicable
-        self.relu_cap = mod._relu_cap
+        self.relu_cap, self.shared_cast = mod._relu_cap, mod.shared_cast
         self.run_conv_nobias, self.run_pool_padded, self.Padded = mod.run_conv_nobias, mod.run_pool_padded, mod.Padded
 
 

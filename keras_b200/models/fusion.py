@@ -187,6 +187,21 @@ def run_pool_padded(layer, x, pairs):
     return layer(ops.pad(x, pads))
 
 
+def shared_cast(layer, x, casts):
+    """``x`` in the layer's compute dtype, cast once for all the convolutions of a pass that read it (the input of a block with a
+    projected shortcut: [256, 56, 56, 256] in float32 is 185 us a cast).  Only where no gradient flows back, which would
+    otherwise be summed in the narrow type; ``casts`` lives for one pass."""
+    if not isinstance(x, torch.Tensor) or x.requires_grad or not x.dtype.is_floating_point:
+        return x
+    td = layer._compute_torch_dtype()
+    if x.dtype == td or not td.is_floating_point or (x.dtype == torch.float32 and x.shape[-1] % 8):
+        return x  # an fp32 input with few channels is cast inside the patch kernel
+    kept = casts.get((id(x), td))
+    if kept is None or kept[0] is not x:
+        kept = casts[(id(x), td)] = (x, x.to(td))
+    return kept[1]
+
+
 def run_conv_nobias(layer, x, pairs=None, want_stats=False):
     """The convolution of ``layer`` without its bias add (autocast applied as ``Layer.__call__`` would).
 

@@ -132,6 +132,7 @@ class Function(Operation):
         sp = global_state.get_global_attribute("tp_sequence_parallel")
         merge = plan.get("merge_tensors", ())
         marked = set()
+        casts = {}
         if merge:
             import torch
 
@@ -166,6 +167,7 @@ class Function(Operation):
                     x, pairs = x.x, x.pairs
                 elif isinstance(x, fusion.Deferred):
                     x = fusion.run_bn(x.layer, x.x, training, pre_bias=x.pre_bias, stats=x.stats)
+                x = fusion.shared_cast(node.operation, x, casts)
                 y, stats = fusion.run_conv_nobias(node.operation, x, pairs, want_stats=bool(training))
                 env[id(outs[0])] = fusion.NoBias(y, node.operation.bias if node.operation.use_bias else None, stats)
                 continue

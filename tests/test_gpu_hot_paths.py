@@ -457,3 +457,48 @@ def test_dense_products_at_any_number_of_rows(M, K, N):
         out, done = gemm.dense(x, w, b, "gelu") or (None, None)
         if out is not None:
             assert done and rel(out, torch.nn.functional.gelu(ye)) < 2.0 ** -8
+
+
+def test_shortcut_and_branch_share_the_cast_of_a_float32_input():
+    import keras_b200 as keras
+
+    L = keras.layers
+    old = keras.config.dtype_policy()
+    keras.config.set_dtype_policy("mixed_bfloat16")
+    try:
+        x = keras.Input((16, 16, 64))
+        a = L.BatchNormalization()(L.Conv2D(64, 1, use_bias=False)(x))
+        b = L.BatchNormalization()(L.Conv2D(64, 1, use_bias=False)(x))
+        model = keras.Model(x, L.ReLU()(L.Add()([a, b])))
+    finally:
+        keras.config.set_dtype_policy(old)
+    data = torch.randn(64, 16, 16, 64, device="cuda")
+    from keras_b200.models import fusion
+
+    casts = {}
+    convs = [layer for layer in model.layers if isinstance(layer, L.Conv2D)]
+    first, second = (fusion.shared_cast(layer, data, casts) for layer in convs)
+    assert first is second and first.dtype == torch.bfloat16 and len(casts) == 1
+    assert fusion.shared_cast(convs[0], data.clone(), casts) is not first
+    out = model(data, training=True)
+    assert out.dtype == torch.bfloat16 and torch.isfinite(out).all()
+    grown = data.clone().requires_grad_(True)  # with a gradient the casts stay apart: their gradients are summed in float32
+    model(grown, training=True).float().square().mean().backward()
+    assert grown.grad is not None and grown.grad.dtype == torch.float32
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (3, 9), (64, 301), (7, 2047), (70000, 5), (768, 50257)])
+def test_padded_matrices(rows, cols):
+    from keras_b200.kernels import ops as kops
+
+    torch.manual_seed(cols)
+    w = torch.randn(rows, cols, device="cuda").bfloat16()
+    wide = -(-cols // 8) * 8
+    padded = kops.pad_columns(w, wide)
+    assert torch.equal(padded, torch.nn.functional.pad(w, (0, wide - cols)))
+    odd = torch.randn(rows * cols + 1, device="cuda").bfloat16()[1:].reshape(rows, cols)  # not even 4-byte aligned
+    assert torch.equal(kops.pad_columns(odd, wide + 8)[:, :cols], odd)
+    total = torch.randn(rows, cols, device="cuda")
+    want = total + padded[:, :cols].float()
+    assert torch.equal(kops.add_rows(total, padded[:, :cols]), want)
+    assert torch.equal(kops.add_rows(total, w), want + w.float())
