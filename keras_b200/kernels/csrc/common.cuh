@@ -131,3 +131,22 @@ template <>
 __device__ __forceinline__ float from_f32<float>(float v) { return v; }
 template <>
 __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+
+// Cumulative distribution function of the normal distribution, Phi(v) = erfc(-v / sqrt(2)) / 2, for the exact GELU and its derivative.
+// With a = |v| and t = 1 / (1 + 0.35 a):  Phi(-a) = t * 2^(p(t) - a^2 log2(e) / 2), where p is the polynomial of degree 7 that fits
+// log2(Phi(-a) e^(a^2/2) / t) on 0 <= a <= 14 with the least maximum error (5.6e-7 relative; 2.5e-6 for a < 6 in float32, where
+// the exponent's rounding is most of it).  Sixteen instructions, two of them on the special-function pipe; 1 + erf(v / sqrt(2))
+// takes twice as many and loses its relative accuracy for negative v.  [16384, 3072, 768] with gelu in the epilogue: 117 -> 94 us.
+__device__ __forceinline__ float normal_cdf(float v) {
+  const float a = fabsf(v), t = __fdividef(1.f, fmaf(0.35f, a, 1.f)), x = a * 0.8493218002880191f;  // x^2 = a^2 log2(e) / 2
+  float p = -0.2692641317844391f;
+  p = fmaf(p, t, 1.0951932668685913f);
+  p = fmaf(p, t, -1.4946914911270142f);
+  p = fmaf(p, t, 0.5625093579292297f);
+  p = fmaf(p, t, -0.06951091438531876f);
+  p = fmaf(p, t, 0.5756505131721497f);
+  p = fmaf(p, t, 1.4403815269470215f);
+  p = fmaf(p, t, -2.840268850326538f);
+  const float lower = t * exp2f(fmaf(-x, x, p));
+  return v > 0.f ? 1.f - lower : lower;
+}

@@ -597,8 +597,9 @@ static int gemm_variant(int M, int N, int split_k, int sms) {
   return N > 128 && t1 >= sms / 2 ? GV_PERSISTENT : GV_TILE;
 }
 
-KB_API int kb200_gemm_bf16_run(const void* a, const void* b, void* c, const float* bias, int M, int N, int K, long long lda, long long ldb,
-                               long long ldc, int a_mn_major, int b_mn_major, int act, int out_fp32, int split_k, int variant, int* err,
+// `bias_bf16`: the bias holds bf16.
+KB_API int kb200_gemm_bf16_run(const void* a, const void* b, void* c, const void* bias, int M, int N, int K, long long lda, long long ldb,
+                               long long ldc, int a_mn_major, int b_mn_major, int act, int out_fp32, int bias_bf16, int split_k, int variant, int* err,
                                cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const int accumulate = split_k < 0 ? 1 : 0;
@@ -640,7 +641,8 @@ KB_API int kb200_gemm_bf16_run(const void* a, const void* b, void* c, const floa
     kb200_set_error("gemm_bf16: cannot raise the shared-memory limit of the kernel on this device");
     return -3;
   }
-  GemmParams p{c, bias, M, N, K, ldc, a_mn_major, b_mn_major, act, out_fp32, err, split_k, kb_per_split};
+  GemmParams p{c, bias_bf16 ? nullptr : (const float*)bias, M, N, K, ldc, a_mn_major, b_mn_major, act, out_fp32, err, split_k, kb_per_split};
+  p.bias16 = bias_bf16 ? (const __nv_bfloat16*)bias : nullptr;
   p.accumulate = accumulate;
   const int tile_m = variant == GV_PAIR256 ? 256 : 128, tile_n = variant == GV_TILE ? 128 : 256;
   const long long units = (long long)((M + tile_m - 1) / tile_m) * ((N + tile_n - 1) / tile_n) * split_k;
@@ -659,7 +661,7 @@ KB_API int kb200_gemm_bf16_run(const void* a, const void* b, void* c, const floa
 KB_API int kb200_gemm_bf16_splitk(const void* a, const void* b, void* c, const float* bias, int M, int N, int K, long long lda, long long ldb,
                                   long long ldc, int a_mn_major, int b_mn_major, int act, int out_fp32, int split_k, int* err,
                                   cudaStream_t stream) {
-  return kb200_gemm_bf16_run(a, b, c, bias, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, act, out_fp32, split_k, GV_AUTO, err, stream);
+  return kb200_gemm_bf16_run(a, b, c, bias, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, act, out_fp32, 0, split_k, GV_AUTO, err, stream);
 }
 
 KB_API int kb200_gemm_bf16(const void* a, const void* b, void* c, const float* bias, int M, int N, int K, long long lda, long long ldb,

@@ -38,6 +38,7 @@ struct GemmParams {
   int int8 = 0;                      // 1: signed 8-bit operands (kind::i8), int32 accumulators
   const float* row_scale = nullptr;  // [M] and [N] factors applied to the accumulator (int8 de-quantisation)
   const float* col_scale = nullptr;
+  const __nv_bfloat16* bias16 = nullptr;  // a bias in bf16 (instead of `bias`): a layer's 16-bit read of it needs no cast
   int accumulate = 0;                // 1: add the fp32 tile into C (TMA reduce store) instead of overwriting it
 };
 
@@ -147,7 +148,7 @@ __device__ __forceinline__ float apply_act(float v, int act) {
       return 0.5f * v * (1.f + tanhf(u));
     }
     case ACT_SILU: return v / (1.f + __expf(-v));
-    case ACT_GELU_ERF: return 0.5f * v * (1.f + erff(v * 0.7071067811865476f));
+    case ACT_GELU_ERF: return v * normal_cdf(v);
     default: return v;
   }
 }
@@ -188,6 +189,9 @@ __device__ __forceinline__ void store_rows_tma(uint32_t tmem_row, int ncols, int
       if (p.bias != nullptr) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] += __ldg(p.bias + min(col0 + j, p.N - 1));
+      } else if (p.bias16 != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] += __bfloat162float(p.bias16[min(col0 + j, p.N - 1)]);
       }
       if (p.act != ACT_NONE) {
 #pragma unroll
@@ -210,6 +214,9 @@ __device__ __forceinline__ void store_rows_tma(uint32_t tmem_row, int ncols, int
         if (p.bias != nullptr) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] += __ldg(p.bias + min(col0 + h * 32 + j, p.N - 1));
+        } else if (p.bias16 != nullptr) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] += __bfloat162float(p.bias16[min(col0 + h * 32 + j, p.N - 1)]);
         }
         if (p.act != ACT_NONE) {
 #pragma unroll

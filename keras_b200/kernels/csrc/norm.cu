@@ -538,6 +538,70 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const T* __restrict
   }
 }
 
+// dz = dy * act'(z) and, in the same pass, the column sums of dz (the bias gradient of the layer in front): three tensors moved where
+// the library's derivative and a separate sum move four.  [16384, 3072] gelu: 83 + 20 -> 73 us; the traffic takes 45.
+enum { AB_RELU = 1, AB_SILU = 3, AB_GELU = 4 };
+template <int ACT>
+__device__ __forceinline__ float act_grad(float z) {
+  if (ACT == AB_RELU) return z > 0.f ? 1.f : 0.f;
+  if (ACT == AB_SILU) {
+    const float s = 1.f / (1.f + __expf(-z));
+    return s * (1.f + z * (1.f - s));
+  }
+  return fmaf(z * 0.3989422804014327f, __expf(-0.5f * z * z), normal_cdf(z));
+}
+
+template <int ACT>
+__global__ void __launch_bounds__(256) act_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ z,
+                                                      __nv_bfloat16* __restrict__ dz, long long rows, int cols, float* __restrict__ partial) {
+  constexpr int VN = 8, U = 2;
+  __shared__ float sm[8][32 * VN + 1];
+  const int cv = threadIdx.x & 31, rl = threadIdx.x >> 5;
+  const int c0 = (blockIdx.x * 32 + cv) * VN;
+  const long long per = (rows + gridDim.y - 1) / gridDim.y;
+  const long long r0 = (long long)blockIdx.y * per, r1 = min(rows, r0 + per);
+  float acc[VN] = {};
+  if (c0 < cols) {
+    for (long long r = r0 + rl; r < r1; r += 8 * U) {
+      uint4 g[U], q[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (r + 8 * u < r1) {
+          g[u] = *reinterpret_cast<const uint4*>(dy + (r + 8 * u) * cols + c0);
+          q[u] = *reinterpret_cast<const uint4*>(z + (r + 8 * u) * cols + c0);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (r + 8 * u >= r1) continue;
+        float gv[VN], zv[VN];
+        unpack8(reinterpret_cast<const bf16x8&>(g[u]), gv);
+        unpack8(reinterpret_cast<const bf16x8&>(q[u]), zv);
+#pragma unroll
+        for (int j = 0; j < VN; ++j) gv[j] *= act_grad<ACT>(zv[j]);
+        const bf16x8 out = pack8(gv);
+        *reinterpret_cast<bf16x8*>(dz + (r + 8 * u) * cols + c0) = out;
+        unpack8(out, gv);  // the sum is that of the values as stored
+#pragma unroll
+        for (int j = 0; j < VN; ++j) acc[j] += gv[j];
+      }
+    }
+  }
+  if (partial == nullptr) return;
+#pragma unroll
+  for (int j = 0; j < VN; ++j) sm[rl][cv * VN + j] = acc[j];
+  __syncthreads();
+  for (int c = threadIdx.x; c < 32 * VN; c += 256) {
+    const int col = blockIdx.x * 32 * VN + c;
+    if (col < cols) {
+      float s = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) s += sm[k][c];
+      partial[(long long)blockIdx.y * cols + col] = s;
+    }
+  }
+}
+
 KB_API int kb200_colsum_slabs(long long rows, int cols, int dtype) {
   const int vn = dtype == 1 ? 8 : 4;
   const int col_blocks = (cols + 32 * vn - 1) / (32 * vn);
@@ -569,5 +633,28 @@ KB_API int kb200_colsum(const void* x, long long ld, long long rows, int cols, f
   dim3 grid2((cols + 31) / 32, 1);
   norm_partial_reduce2_kernel<<<grid2, 1024, 0, stream>>>(partial, out, nullptr, nullptr, slabs, cols, accumulate);
   KB_CHECK_LAUNCH("colsum_reduce");
+  return 0;
+}
+
+// dz = dy * act'(z) on contiguous bf16 [rows, cols] (cols a multiple of 8, 16-byte aligned bases), act: 1 relu, 3 silu, 4 gelu (erf).
+// With partial (scratch as for kb200_colsum) the column sums of dz go to out, or are added to it (accumulate).
+KB_API int kb200_act_bwd(const void* dy, const void* z, void* dz, long long rows, int cols, int act, float* partial, float* out, int accumulate,
+                         cudaStream_t stream) {
+  if (rows <= 0 || cols <= 0) return 0;
+  if (cols % 8 || (((uintptr_t)dy | (uintptr_t)z | (uintptr_t)dz) & 15) || (act != AB_RELU && act != AB_SILU && act != AB_GELU)) {
+    kb200_set_error("act_bwd: columns must be a multiple of 8, bases aligned, the activation relu, silu or gelu");
+    return -2;
+  }
+  const int slabs = kb200_colsum_slabs(rows, cols, 1);
+  dim3 grid((cols + 255) / 256, slabs);
+  const __nv_bfloat16 *g = (const __nv_bfloat16*)dy, *q = (const __nv_bfloat16*)z;
+  if (act == AB_RELU) act_bwd_kernel<AB_RELU><<<grid, 256, 0, stream>>>(g, q, (__nv_bfloat16*)dz, rows, cols, partial);
+  else if (act == AB_SILU) act_bwd_kernel<AB_SILU><<<grid, 256, 0, stream>>>(g, q, (__nv_bfloat16*)dz, rows, cols, partial);
+  else act_bwd_kernel<AB_GELU><<<grid, 256, 0, stream>>>(g, q, (__nv_bfloat16*)dz, rows, cols, partial);
+  KB_CHECK_LAUNCH("act_bwd");
+  if (partial != nullptr) {
+    norm_partial_reduce2_kernel<<<dim3((cols + 31) / 32, 1), 1024, 0, stream>>>(partial, out, nullptr, nullptr, slabs, cols, accumulate);
+    KB_CHECK_LAUNCH("act_bwd_reduce");
+  }
   return 0;
 }

@@ -73,6 +73,7 @@ def gemm(a, b, a_mn, b_mn, M, N, K, bias=None, act=0, out_dtype=torch.bfloat16, 
     """Raw launch. ``a``/``b`` are 2-D bf16 tensors in the storage layout named by the major flags.
 
     ``split_k > 1`` accumulates K slices into a zeroed fp32 buffer (TMA reduce stores) and casts to ``out_dtype``.
+    ``bias``: fp32 or bf16.
     ``accumulate_into``: fp32 [M, N] tensor that the product is added to in place (returned)."""
     lib = kops._lib()
     err = _err_flag(a.device)
@@ -91,11 +92,22 @@ def gemm(a, b, a_mn, b_mn, M, N, K, bias=None, act=0, out_dtype=torch.bfloat16, 
         kops._check(code, "gemm_bf16")
         return acc if out_dtype == torch.float32 else acc.to(out_dtype)
     out = torch.empty((M, N), dtype=out_dtype, device=a.device)
-    code = lib.kb200_gemm_bf16(kops._p(a), kops._p(b), kops._p(out), kops._p(bias), kops._i(M), kops._i(N), kops._i(K), kops._ll(a.stride(0)),
-                               kops._ll(b.stride(0)), kops._ll(out.stride(0)), kops._i(a_mn), kops._i(b_mn), kops._i(act),
-                               kops._i(1 if out_dtype == torch.float32 else 0), kops._p(err), kops._stream())
+    code = lib.kb200_gemm_bf16_run(kops._p(a), kops._p(b), kops._p(out), kops._p(bias), kops._i(M), kops._i(N), kops._i(K),
+                                   kops._ll(a.stride(0)), kops._ll(b.stride(0)), kops._ll(out.stride(0)), kops._i(a_mn), kops._i(b_mn), kops._i(act),
+                                   kops._i(1 if out_dtype == torch.float32 else 0), kops._i(1 if bias is not None and bias.dtype == torch.bfloat16 else 0),
+                                   kops._i(1), kops._i(0), kops._p(err), kops._stream())
     kops._check(code, "gemm_bf16")
     return out
+
+
+_ACT_FN = {1: torch.relu, 3: torch.nn.functional.silu, 4: torch.nn.functional.gelu}
+
+
+def _bias_operand(bias):
+    """A bias as the epilogue reads it: fp32 or bf16, contiguous."""
+    if bias is None:
+        return None
+    return (bias if bias.dtype in (torch.float32, torch.bfloat16) else bias.float()).detach().contiguous()
 
 
 class GemmFn(torch.autograd.Function):
@@ -105,21 +117,26 @@ class GemmFn(torch.autograd.Function):
     the padded output keeps its 16-byte row pitch and the caller sees its first ``N`` columns as a view."""
 
     @staticmethod
-    def forward(ctx, x, w, bias, grad_target=None, bias_target=None):
-        """``grad_target``: the fp32 parameter behind ``w`` (its bf16 shadow) when its ``.grad`` is persistent fp32 storage: the
+    def forward(ctx, x, w, bias, grad_target=None, bias_target=None, act=0):
+        """``act``: code of the activation behind the product (relu, silu, gelu): its derivative and the bias gradient are one pass.
+        (Its value as a second output of the epilogue gains 12 of 130 us at [16384, 3072, 768] and nothing at smaller products.)
+        ``grad_target``: the fp32 parameter behind ``w`` (its bf16 shadow) when its ``.grad`` is persistent fp32 storage: the
         weight gradient is then accumulated there by the GEMM itself and no bf16 gradient tensor is produced."""
         M, K = x.shape
         N = w.shape[1]
         ctx.grad_target = grad_target
         ctx.bias_target = bias_target
         Np = (N + 7) // 8 * 8
-        b32 = bias.float().contiguous() if bias is not None else None
+        b = _bias_operand(bias)
         if Np != N:
             w = kops.pad_columns(w, Np)
-            if b32 is not None:
-                b32 = torch.nn.functional.pad(b32, (0, Np - N))
-        out = gemm(x, w, 0, 1, M, Np, K, bias=b32)
-        ctx.save_for_backward(x, w)
+            if b is not None:
+                b = torch.nn.functional.pad(b, (0, Np - N))
+        out, pre = gemm(x, w, 0, 1, M, Np, K, bias=b), None
+        if act:
+            pre, out = out, _ACT_FN[act](out)
+        ctx.save_for_backward(x, w, pre)
+        ctx.act = act
         ctx.has_bias = bias is not None
         ctx.bias_dtype = bias.dtype if bias is not None else None
         ctx.n = N
@@ -127,9 +144,16 @@ class GemmFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        x, w = ctx.saved_tensors
+        x, w, pre = ctx.saved_tensors
         M, K = x.shape
         N, Np = ctx.n, w.shape[1]
+        sums = bias_slot = None
+        if ctx.act:
+            dy = dy.contiguous()
+            dy = dy if dy.data_ptr() % 16 == 0 else dy.clone()
+            wanted = ctx.has_bias and ctx.needs_input_grad[2]
+            bias_slot = shadow.grad_slot(ctx.bias_target, (N,)) if wanted else None
+            dy, sums = kops.activation_backward(dy, pre, ctx.act, wanted, bias_slot.view(N) if bias_slot is not None else None)
         if Np != N:
             if dy.dtype == torch.bfloat16 and dy.stride(1) == 1 and dy.stride(0) == Np and dy.data_ptr() % 16 == 0:
                 # the gradient is itself the leading columns of a padded buffer (produced for a padded logits view)
@@ -154,13 +178,15 @@ class GemmFn(torch.autograd.Function):
                 dw = gemm(x, dy, 1, 1, K, Np, M, split_k=split)
                 if Np != N:
                     dw = dw[:, :N]
-        if ctx.has_bias and ctx.needs_input_grad[2]:
+        if sums is not None:
+            db = sums.to(ctx.bias_dtype) if bias_slot is None else None
+        elif ctx.has_bias and ctx.needs_input_grad[2]:
             g = shadow.grad_slot(ctx.bias_target, (N,)) if Np == N else None
             if g is not None:
                 kops.column_sum(dy, accumulate_into=g.view(N))  # db stays None: already accumulated
             else:
                 db = kops.column_sum(dy)[:N].to(ctx.bias_dtype)
-        return (dx, dw, db, None, None)[: len(ctx.needs_input_grad)]
+        return (dx, dw, db, None, None, None)[: len(ctx.needs_input_grad)]
 
 
 def _qualifies(x2, w, padded=False):
@@ -241,7 +267,7 @@ def dense(x, kernel, bias, activation_name, kernel_shape=None, value=None):
         act = _ACT.get(name)
         fused_act = act is not None
         N = w.shape[1]
-        b32 = b.float().contiguous() if b is not None else None
+        b32 = _bias_operand(b)
         if N % 8:
             w = kops.pad_columns(w, N + 8 - N % 8) if wide is None else wide
             b32 = torch.nn.functional.pad(b32, (0, 8 - N % 8)) if b32 is not None else None
@@ -251,5 +277,7 @@ def dense(x, kernel, bias, activation_name, kernel_shape=None, value=None):
         return out.reshape(tuple(lead) + (N,)), fused_act
     target = _grad_target(kernel, w) if isinstance(kernel, Variable) else None
     bias_target = _grad_target(bias, b) if isinstance(bias, Variable) else None
-    out = GemmFn.apply(x2, w, b, target, bias_target)
-    return out.reshape(tuple(lead) + (w.shape[1],)), activation_name in (None, "linear")
+    # relu, silu and gelu come with the product: their derivative is taken together with the bias gradient
+    act = {"relu": 1, "silu": 3, "swish": 3, "gelu": 4}.get(activation_name, 0) if w.shape[1] % 8 == 0 else 0
+    out = GemmFn.apply(x2, w, b, target, bias_target, act)
+    return out.reshape(tuple(lead) + (w.shape[1],)), act != 0 or activation_name in (None, "linear")

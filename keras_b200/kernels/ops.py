@@ -36,7 +36,7 @@ def _stream():
     if getattr(_TL, "dev", None) != dev:
         loader.get().kb200_bind_device(_i(dev))
         _TL.dev = dev
-    return _vp(torch.cuda.current_stream().cuda_stream)
+    return _vp(torch._C._cuda_getCurrentRawStream(dev))
 
 
 def _lib():
@@ -438,6 +438,21 @@ def column_sum(x, accumulate_into=None):
     _check(lib.kb200_colsum(_p(x), _ll(x.stride(0)), _ll(rows), _i(cols), _p(partial), _p(out), _i(_dt(x)), _i(0 if accumulate_into is None else 1),
                             _stream()), "colsum")
     return out
+
+
+def activation_backward(dy, z, act, want_sums=False, accumulate_into=None):
+    """``(dy * act'(z), its column sums or None)`` for contiguous bf16 matrices, in one pass; ``act`` as the GEMM numbers it."""
+    lib = _lib()
+    rows, cols = z.shape
+    dz = torch.empty_like(z)
+    partial = out = None
+    if want_sums:
+        lib.kb200_colsum_slabs.restype = ctypes.c_int
+        partial = torch.empty((lib.kb200_colsum_slabs(_ll(rows), _i(cols), _i(1)), cols), dtype=torch.float32, device=z.device)
+        out = torch.empty(cols, dtype=torch.float32, device=z.device) if accumulate_into is None else accumulate_into
+    _check(lib.kb200_act_bwd(_p(dy), _p(z), _p(dz), _ll(rows), _i(cols), _i(act), _p(partial), _p(out), _i(0 if accumulate_into is None else 1), _stream()),
+           "act_bwd")
+    return dz, out
 
 
 # ----------------------------------------------------------------- softmax cross-entropy

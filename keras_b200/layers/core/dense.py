@@ -18,6 +18,10 @@ from keras_b200.layers.core.calibrated_kernel import CalibratedKernel
 from keras_b200.layers.layer import Layer
 
 
+# activations that the GEMM's epilogue knows
+_EPILOGUE_ACTIVATIONS = (activations.linear, activations.relu, activations.silu, activations.gelu)
+
+
 @keras_export("keras.layers.Dense")
 class Dense(CalibratedKernel, Layer):
     def __init__(self, units, activation=None, use_bias=True, kernel_initializer="glorot_uniform", bias_initializer="zeros",
@@ -83,7 +87,9 @@ class Dense(CalibratedKernel, Layer):
                 return out
         kernel = self.kernel
         act = self.activation
-        fused = dispatch.dense(inputs, kernel, self.bias, getattr(act, "__name__", None))
+        # by identity: a user's own function may well be called "gelu"
+        name = None if act is None else getattr(act, "__name__", None) if act in _EPILOGUE_ACTIVATIONS else "other"
+        fused = dispatch.dense(inputs, kernel, self.bias, name)
         if fused is not None:
             out, act_done = fused
             if not act_done and act is not None and act is not activations.linear:

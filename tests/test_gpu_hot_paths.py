@@ -58,7 +58,7 @@ def test_gemm_variants_agree_with_the_product_in_64_bits(M, N, K, variant):
             with_bias = split == 1
             code = lib.kb200_gemm_bf16_run(K_._p(a), K_._p(b), K_._p(c), K_._p(bias if with_bias else None), K_._i(M), K_._i(N), K_._i(K),
                                            K_._ll(a.stride(0)), K_._ll(b.stride(0)), K_._ll(N), K_._i(a_mn), K_._i(b_mn), K_._i(1 if with_bias else 0),
-                                           K_._i(fp32), K_._i(split), K_._i(variant), K_._p(err), K_._stream())
+                                           K_._i(fp32), K_._i(0), K_._i(split), K_._i(variant), K_._p(err), K_._stream())
             K_._check(code, "gemm_bf16")
             want = torch.relu(ref + bias) if with_bias else ref + 2.0 if add else ref
             rel = ((c.double() - want).norm() / want.norm()).item()
@@ -502,3 +502,72 @@ def test_padded_matrices(rows, cols):
     want = total + padded[:, :cols].float()
     assert torch.equal(kops.add_rows(total, padded[:, :cols]), want)
     assert torch.equal(kops.add_rows(total, w), want + w.float())
+
+
+@pytest.mark.parametrize("activation", ["relu", "silu", "gelu"])
+@pytest.mark.parametrize("rows,width,use_bias", [((3, 5), 64, True), ((1000,), 264, True), ((5000,), 512, False), ((77, 260), 1024, True), ((20100,), 512, True)])
+def test_dense_with_an_activation_and_its_gradient(activation, rows, width, use_bias):
+    import keras_b200 as keras
+
+    old = keras.config.dtype_policy()
+    keras.config.set_dtype_policy("mixed_bfloat16")
+    try:
+        layer = keras.layers.Dense(width, activation=activation, use_bias=use_bias)
+        plain = keras.layers.Dense(width, use_bias=use_bias)
+    finally:
+        keras.config.set_dtype_policy(old)
+    torch.manual_seed(width)
+    x = torch.randn(rows + (256,), device="cuda").bfloat16().requires_grad_(True)
+    dy = torch.randn(rows + (width,), device="cuda").bfloat16()
+    layer(x), plain(x)
+    for a, b in zip(plain.weights, layer.weights):
+        a.assign(b.value + 0.1 * torch.randn(tuple(b.shape), device="cuda"))
+        b.assign(a.value)
+    results = []
+    for run in (layer, lambda t: getattr(torch.nn.functional, activation)(plain(t))):
+        y = run(x)
+        which = layer if run is layer else plain
+        results.append([y.detach()] + list(torch.autograd.grad(y, [x] + [v.value for v in which.trainable_variables], dy)))
+    for a, b in zip(*results):
+        # the same rounded value ahead of the activation; each result is rounded once more
+        assert ((a.float() - b.float()).norm() / b.float().norm()).item() < 2.0 ** -8
+
+
+def test_a_function_of_the_users_own_is_not_taken_for_a_known_activation():
+    import keras_b200 as keras
+
+    def gelu(x):
+        return x * 3.0
+
+    old = keras.config.dtype_policy()
+    keras.config.set_dtype_policy("mixed_bfloat16")
+    try:
+        layer = keras.layers.Dense(256, activation=gelu)
+    finally:
+        keras.config.set_dtype_policy(old)
+    x = torch.randn(256, 256, device="cuda").bfloat16()
+    for grad in (True, False):
+        with torch.set_grad_enabled(grad):
+            y, want = layer(x), 3.0 * torch.matmul(x.float(), layer.kernel.value.float())
+            assert ((y.float() - want).norm() / want.norm()).item() < 2.0 ** -7
+
+
+def test_exact_gelu_of_the_epilogue_and_its_derivative_over_the_whole_range():
+    from keras_b200.kernels import gemm, ops as kops
+
+    # the product with the identity hands every value of x to the epilogue as it is
+    x = torch.cat([torch.linspace(-14, 14, 64 * 1000 - 64), torch.tensor([0.0, -0.0, 1e-30, -1e-30] * 8 + [30.0, -30.0, 1e4, -1e4] * 8)]).reshape(1000, 64).cuda().bfloat16()
+    eye = torch.eye(64, device="cuda").bfloat16()
+    xe = x.double()
+    cdf = 0.5 * torch.special.erfc(-xe * 0.5 ** 0.5)  # 1 + erf cancels for negative values, in 64 bits too
+    want, slope = xe * cdf, cdf + xe * torch.exp(-0.5 * xe * xe) * 0.3989422804014327
+    out = gemm.gemm(x, eye, 0, 1, 1000, 64, 64, act=4, out_dtype=torch.float32)
+    # float32: 2.5e-6 of the value (the exponent's rounding grows with x^2 beyond 6) and nothing below 1e-30
+    assert torch.all((out.double() - want).abs() <= 2e-5 * want.abs() + 1e-30)
+    small = x.abs() < 6
+    assert torch.all((out.double() - want).abs()[small] <= 4e-6 * want.abs()[small] + 1e-30)
+    one = torch.ones_like(x)
+    dz, _ = kops.activation_backward(one, x, 4)
+    assert torch.all((dz.double() - slope).abs() <= 2.0 ** -8 * slope.abs() + 2e-6)  # one rounding to bf16; the slope itself crosses zero
+    nan = torch.full((8, 64), float("nan"), device="cuda").bfloat16()
+    assert gemm.gemm(nan, eye, 0, 1, 8, 64, 64, act=4).isnan().all() and kops.activation_backward(one[:8].contiguous(), nan, 4)[0].isnan().all()
