@@ -363,7 +363,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
           for (int c = 0; c < D / 64; ++c)
             tma_store_4d(&map_o, sQ + (uint32_t)(i * TILE + c * 16384) + (uint32_t)(q * 32) * 128u, c * 64, first + q * 32, h, b);
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-          asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the writes land before the grid ends
         }
         if (qi < p.Tq && p.lse != nullptr)
           p.lse[((long long)b * p.H + h) * p.Tq + qi] = (l != 0.f) ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;

@@ -460,7 +460,7 @@ conv_igemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_acc_empty(s, acc));
     }
-    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the writes land before the grid ends
     if (p.stats != nullptr) {
       // combine the warps' column sums in a fixed order (reproducible) and write one row pair per CTA
       __syncwarp();  // lane 0 has waited for this warp's stores: the staging buffers are free
@@ -692,7 +692,7 @@ conv_wgrad_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_acc_empty(s, 0));
     }
-    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the writes land before the grid ends
     if (!ok) {
       if (lane == 0 && p.err) atomicExch(p.err, 33);
       *abort_flag = 1;

@@ -21,7 +21,10 @@
 namespace {
 using namespace kbgemm;
 
-__global__ void __launch_bounds__(THREADS, 2)
+// STAGES: three leave room for two CTAs an SM, which hide each other's latency; a grid of at most one CTA an SM has no second one and
+// takes six, or its loop waits for L2 (600 ns a 64-element K block with three: [2664, 512, 2048] 12.1 -> 10.7 us).
+template <int STAGES>
+__global__ void __launch_bounds__(THREADS, STAGES == 3 ? 2 : 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -41,8 +44,29 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   const int m0 = (blockIdx.x / n_tiles) * BM;
   const int n0 = (blockIdx.x % n_tiles) * BN;
   const int k_blocks = (p.K + BK - 1) / BK;
+  auto load_block = [&](int kb) {
+    const int s = kb % STAGES, k0 = kb * BK;
+    const uint32_t sa = base + s * STAGE_BYTES, sb = sa + A_TILE_BYTES;
+    mbar_expect_tx(full_bar(s), STAGE_BYTES);
+    if (p.a_mn_major) {
+      tma_load_2d(sa, &map_a, full_bar(s), m0, k0);
+      tma_load_2d(sa + 8192, &map_a, full_bar(s), m0 + 64, k0);
+    } else {
+      tma_load_2d(sa, &map_a, full_bar(s), k0, m0);
+    }
+    if (p.b_mn_major) {
+      tma_load_2d(sb, &map_b, full_bar(s), n0, k0);
+      tma_load_2d(sb + 8192, &map_b, full_bar(s), n0 + 64, k0);
+    } else {
+      tma_load_2d(sb, &map_b, full_bar(s), k0, n0);
+    }
+  };
+  const int first_blocks = min(STAGES, k_blocks);  // loaded ahead of the barrier below, while TMEM is being allocated
 
   if (threadIdx.x == 0) {
+    prefetch_map(&map_a);
+    prefetch_map(&map_b);
+    prefetch_map(&map_c);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
@@ -50,6 +74,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     mbar_init(tmem_full_bar, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    for (int kb = 0; kb < first_blocks; ++kb) load_block(kb);
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "r"(TMEM_COLS) : "memory");
@@ -63,28 +89,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one()) {
-      int issued = 0;
+      int issued = first_blocks;
       bool ok = true;
-      for (int kb = 0; kb < k_blocks && ok; ++kb) {
-        const int s = kb % STAGES;
-        const uint32_t parity = ((kb / STAGES) & 1) ^ 1;
-        ok = mbar_wait(empty_bar(s), parity, abort_flag);
+      for (int kb = first_blocks; kb < k_blocks && ok; ++kb) {
+        ok = mbar_wait(empty_bar(kb % STAGES), ((kb / STAGES) & 1) ^ 1, abort_flag);
         if (!ok) break;
-        const uint32_t sa = base + s * STAGE_BYTES, sb = sa + A_TILE_BYTES;
-        mbar_expect_tx(full_bar(s), STAGE_BYTES);
-        const int k0 = kb * BK;
-        if (p.a_mn_major) {
-          tma_load_2d(sa, &map_a, full_bar(s), m0, k0);
-          tma_load_2d(sa + 8192, &map_a, full_bar(s), m0 + 64, k0);
-        } else {
-          tma_load_2d(sa, &map_a, full_bar(s), k0, m0);
-        }
-        if (p.b_mn_major) {
-          tma_load_2d(sb, &map_b, full_bar(s), n0, k0);
-          tma_load_2d(sb + 8192, &map_b, full_bar(s), n0 + 64, k0);
-        } else {
-          tma_load_2d(sb, &map_b, full_bar(s), k0, n0);
-        }
+        load_block(kb);
         issued = kb + 1;
       }
       if (!ok) {
@@ -139,7 +149,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       // every MMA of this CTA's only tile has completed, so the operand ring is free: stage 0 holds the staging buffers
       uint32_t stores = 0;
       store_rows_tma(tmem_base + ((uint32_t)(q * 32) << 16), BN, n0, m0 + q * 32, base + (uint32_t)(warp - 2) * 8192u, stores, &map_c, p, lane);
-      if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+      if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // staging read out; the writes land before the grid ends
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -182,6 +192,9 @@ gemm_bf16_tcgen05_persistent(const __grid_constant__ CUtensorMap map_a, const __
   const int kb_per = split > 1 ? p.kb_per_split : k_blocks_all;
 
   if (threadIdx.x == 0) {
+    prefetch_map(&map_a);
+    prefetch_map(&map_b);
+    prefetch_map(&map_c);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
@@ -313,7 +326,7 @@ gemm_bf16_tcgen05_persistent(const __grid_constant__ CUtensorMap map_a, const __
       __syncwarp();
       if (lane == 0) mbar_arrive(acc_empty_bar(acc));
     }
-    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // staging read out; the writes land before the grid ends
     if (!ok) {
       if (lane == 0 && p.err) atomicExch(p.err, 13);
       *abort_flag = 1;
@@ -431,6 +444,9 @@ gemm_bf16_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_c
   };
 
   if (threadIdx.x == 0) {
+    prefetch_map(&map_a);
+    prefetch_map(&map_b);
+    prefetch_map(&map_c);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
@@ -552,7 +568,7 @@ gemm_bf16_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_c
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(map_to_rank(acc_empty_bar(acc), 0));
     }
-    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // staging read out; the writes land before the grid ends
     if (!ok) {
       if (lane == 0 && p.err) atomicExch(p.err, 23);
       *abort_flag = 1;
@@ -633,8 +649,12 @@ KB_API int kb200_gemm_bf16_run(const void* a, const void* b, void* c, const void
     kb200_set_error("gemm_bf16: cuTensorMapEncodeTiled failed");
     return -3;
   }
+  constexpr int LONG = 6;
+  constexpr int smem_v1 = SMEM_BYTES, smem_long = SMEM_BYTES + (LONG - STAGES) * STAGE_BYTES;
+  static bool attr_long[KB_MAX_DEVICES] = {false};
   static bool attr_v1[KB_MAX_DEVICES] = {false}, attr_v2[KB_MAX_DEVICES] = {false}, attr_v3[KB_MAX_DEVICES] = {false};
-  const bool allowed = variant == GV_TILE         ? kb_allow_smem(gemm_bf16_tcgen05_kernel, SMEM_BYTES, attr_v1)
+  const bool allowed = variant == GV_TILE         ? kb_allow_smem(gemm_bf16_tcgen05_kernel<STAGES>, smem_v1, attr_v1) &&
+                                                        kb_allow_smem(gemm_bf16_tcgen05_kernel<LONG>, smem_long, attr_long)
                        : variant == GV_PERSISTENT ? kb_allow_smem(gemm_bf16_tcgen05_persistent, v2::SMEM_BYTES, attr_v2)
                                                   : kb_allow_smem(gemm_bf16_tcgen05_pair, v3::SMEM_BYTES, attr_v3);
   if (!allowed) {
@@ -647,7 +667,10 @@ KB_API int kb200_gemm_bf16_run(const void* a, const void* b, void* c, const void
   const int tile_m = variant == GV_PAIR256 ? 256 : 128, tile_n = variant == GV_TILE ? 128 : 256;
   const long long units = (long long)((M + tile_m - 1) / tile_m) * ((N + tile_n - 1) / tile_n) * split_k;
   if (variant == GV_TILE) {
-    gemm_bf16_tcgen05_kernel<<<(unsigned)units, THREADS, SMEM_BYTES, stream>>>(map_a, map_b, map_c, p);
+    if (units <= sm_count)
+      gemm_bf16_tcgen05_kernel<LONG><<<(unsigned)units, THREADS, smem_long, stream>>>(map_a, map_b, map_c, p);
+    else
+      gemm_bf16_tcgen05_kernel<STAGES><<<(unsigned)units, THREADS, smem_v1, stream>>>(map_a, map_b, map_c, p);
   } else if (variant == GV_PERSISTENT) {
     gemm_bf16_tcgen05_persistent<<<(unsigned)(units < sm_count ? units : sm_count), THREADS, v2::SMEM_BYTES, stream>>>(map_a, map_b, map_c, p);
   } else {

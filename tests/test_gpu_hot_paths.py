@@ -39,7 +39,7 @@ GEMM_VARIANTS = {1: "one tile a CTA", 2: "persistent", 3: "CTA pairs"}
 
 
 @pytest.mark.parametrize("variant", sorted(GEMM_VARIANTS))
-@pytest.mark.parametrize("M,N,K", [(256, 256, 64), (264, 520, 1000), (136, 1000, 72), (2664, 512, 520), (2049 * 8, 264, 136)])
+@pytest.mark.parametrize("M,N,K", [(256, 256, 64), (264, 520, 384), (264, 520, 392), (16392, 264, 200), (264, 520, 1000), (136, 1000, 72), (2664, 512, 520), (2049 * 8, 264, 136)])
 def test_gemm_variants_agree_with_the_product_in_64_bits(M, N, K, variant):
     from keras_b200.kernels import ops as K_
 
