@@ -89,9 +89,15 @@ def _kernel_mask(mask, q, k, is_causal):
         return None
 
 
-def flash_attention(q, k, v, mask, scale, is_causal):
+def flash_attention(q, k, v, mask, scale, is_causal, row_mask=None):
     """Attention on this package's kernel, or ``None`` when the call does not fit it (other head sizes, unaligned layouts, a scale
-    that is not positive) or the kernel is not selected for training."""
+    that is not positive) or the kernel is not selected for training.
+
+    ``row_mask`` (with ``mask``, not causal): bool ``[B, Tq]``; a row at zero has every key masked.  A padding mask as one byte a row
+    and one a key, instead of their product over ``[B, Tq, Tk]``: 32 x 384 x 12 heads of 64 104 -> 50.5 us (unmasked 45.4)."""
+    if row_mask is not None and (mask is None or is_causal or row_mask.dtype != torch.bool or row_mask.device != q.device
+                                 or tuple(row_mask.shape) != tuple(q.shape[:2]) or row_mask.stride(1) != 1):
+        return None
     if not (_ok(q) and _ok(k) and _ok(v)):
         return None
     D = q.shape[-1]
@@ -112,4 +118,4 @@ def flash_attention(q, k, v, mask, scale, is_causal):
         if mask is None:
             return None
         is_causal = False
-    return forward(q, k, v, float(scale), bool(is_causal), mask)[0]
+    return forward(q, k, v, float(scale), bool(is_causal), mask, row_mask)[0]

@@ -328,12 +328,12 @@ def softmax_cross_entropy(logits, labels):
     return _ops().FusedSoftmaxXent.apply(logits, labels)
 
 
-def flash_attention(q, k, v, mask, scale, is_causal):
+def flash_attention(q, k, v, mask, scale, is_causal, row_mask=None):
     if not enabled(q):
         return None
     from keras_b200.kernels import attention
 
-    return attention.flash_attention(q, k, v, mask, scale, is_causal)
+    return attention.flash_attention(q, k, v, mask, scale, is_causal, row_mask)
 
 
 # ---------------------------------------------------------------------------- recurrent layers

@@ -9,9 +9,12 @@ every other case builds explicit einsum equations over the attention axes.
 import math
 import string
 
+import torch
+
 from keras_b200 import constraints, initializers, ops, regularizers
 from keras_b200.core import config
 from keras_b200.core.export_registry import keras_export
+from keras_b200.kernels import dispatch
 from keras_b200.layers.activations.activation_layers import Softmax
 from keras_b200.layers.core.einsum_dense import EinsumDense
 from keras_b200.layers.layer import Layer
@@ -223,7 +226,9 @@ class MultiHeadAttention(Layer):
     def _attend(self, query, value, key, query_mask, value_mask, key_mask, attention_mask, return_attention_scores, training, use_causal_mask):
         causal_only = (use_causal_mask and query_mask is None and value_mask is None and key_mask is None and attention_mask is None
                        and self._sliding_window is None and type(self)._compute_attention is MultiHeadAttention._compute_attention)
-        if causal_only:
+        padding_only = (query_mask is not None and (value_mask is not None or key_mask is not None) and attention_mask is None and not use_causal_mask
+                        and not return_attention_scores and self._takes_padding())
+        if causal_only or padding_only:
             attention_mask = None
         else:
             attention_mask = self._compute_attention_mask(query, value, query_mask=query_mask, value_mask=value_mask, key_mask=key_mask,
@@ -238,8 +243,14 @@ class MultiHeadAttention(Layer):
         q = self._query_dense(query)
         k = self._key_dense(key)
         v = self._value_dense(value)
-        extra = {"use_causal_mask": True} if causal_only else {}
-        out, scores = self._compute_attention(q, k, v, attention_mask, training, return_attention_scores, **extra)
+        out = scores = None
+        if padding_only:
+            out = self._attend_padded(q, k, v, query_mask, value_mask, key_mask)
+            if out is None:
+                attention_mask = self._compute_attention_mask(query, value, query_mask=query_mask, value_mask=value_mask, key_mask=key_mask)
+        if out is None:
+            extra = {"use_causal_mask": True} if causal_only else {}
+            out, scores = self._compute_attention(q, k, v, attention_mask, training, return_attention_scores, **extra)
         if gate is not None:
             out = ops.multiply(out, gate)
         out = self._output_dense(out)
@@ -253,6 +264,23 @@ class MultiHeadAttention(Layer):
                 scores = tensor_parallel.gather_dim(scores, 1, *tp[1:])
             return out, scores
         return out
+
+    def _takes_padding(self):
+        """Whether masks of whole rows and keys may go to the fused kernel as they are: no subclass looks at their product."""
+        cls = type(self)
+        return (cls._compute_attention is MultiHeadAttention._compute_attention and cls._compute_attention_mask is MultiHeadAttention._compute_attention_mask
+                and self._sliding_window is None and self._dropout == 0.0 and tuple(self._attention_axes) == (1,) and self._flash_attention is not False)
+
+    def _attend_padded(self, q, k, v, query_mask, value_mask, key_mask):
+        """Attention under one mask of the rows and one (or two) of the keys, their product over ``[B, T, S]`` never built; ``None``
+        where the fused kernel does not take the call."""
+        masks = [m for m in (query_mask, value_mask, key_mask) if m is not None]
+        if not all(isinstance(t, torch.Tensor) for t in (q, k, v, *masks)) or q.ndim != 4 or any(m.dtype != torch.bool or m.ndim != 2 for m in masks):
+            return None
+        if any(m.shape != (k.shape[0], k.shape[1]) for m in masks[1:]):
+            return None
+        keys = masks[1] if len(masks) == 2 else masks[1] & masks[2]
+        return dispatch.flash_attention(q, k, v, keys[:, None, None, :], self._inverse_sqrt_key_dim, False, row_mask=query_mask)
 
     def _compute_attention_mask(self, query, value, query_mask=None, value_mask=None, key_mask=None, attention_mask=None, use_causal_mask=False):
         auto = None

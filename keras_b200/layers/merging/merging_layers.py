@@ -93,7 +93,8 @@ class Merge(Layer):
             return None
         out = mask[0]
         for m in mask[1:]:
-            out = ops.logical_or(out, m)
+            if m is not out or out.dtype not in (torch.bool, "bool"):  # a residual branch carries the very mask of its input
+                out = ops.logical_or(out, m)
         return out
 
 

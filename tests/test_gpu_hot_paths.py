@@ -176,6 +176,38 @@ def test_attention_with_masked_rows_and_keys(D, T):
     assert ((out.double() - want).norm() / want.norm()).item() < 2.0 ** -8
 
 
+@pytest.mark.parametrize("masks", ["both", "query+key", "three", "query only", "of integers"])
+def test_attention_layer_with_padding(masks):
+    """Rows and keys that are padding: the layer against itself with their product as an explicit mask."""
+    import keras_b200 as keras
+    from keras_b200.kernels import attention
+
+    T, S = 77, 77 if masks == "both" else 130
+    layer = keras.layers.MultiHeadAttention(4, 64, dtype="bfloat16")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q = torch.randn((3, T, 256), generator=g, device="cuda").bfloat16()
+    v = q if masks == "both" else torch.randn((3, S, 256), generator=g, device="cuda").bfloat16()
+    rows = torch.arange(T, device="cuda") < torch.tensor([[T], [1], [T // 2]], device="cuda")
+    keys = rows if masks == "both" else torch.arange(S, device="cuda") < torch.tensor([[S], [70], [3]], device="cuda")
+    other = torch.rand((3, S), generator=g, device="cuda") < 0.8
+    given, seen = {"both": ({"value_mask": keys}, keys), "query+key": ({"key_mask": keys}, keys), "of integers": ({"value_mask": keys.to(torch.int32)}, keys),
+                   "three": ({"value_mask": keys, "key_mask": other}, keys & other), "query only": ({}, torch.ones_like(keys))}[masks]
+    with torch.no_grad():
+        want = layer(q, v, attention_mask=rows[:, :, None] & seen[:, None, :])
+        calls, plain = [], attention.forward
+        attention.forward = lambda *a, **k: calls.append(a) or plain(*a, **k)
+        try:
+            got = layer(q, v, query_mask=rows, **given)
+        finally:
+            attention.forward = plain
+        attention.check_errors()
+        assert torch.equal(got, want) and len(calls) == 1
+        assert (calls[0][-1] is rows) == (masks in ("both", "query+key", "three"))
+    # training keeps the product; its library kernel answers rows without any key with zeros, so only the others are compared
+    out, want = layer(q.clone().requires_grad_(True), v, query_mask=rows, **given)[rows], want[rows]
+    assert ((out.double() - want.double()).norm() / want.double().norm()).item() < 2.0 ** -6
+
+
 def test_attention_keeps_a_nan_to_the_rows_that_see_it():
     from keras_b200.kernels import attention
 
