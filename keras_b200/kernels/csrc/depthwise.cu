@@ -7,9 +7,12 @@
 // strip of 4 pixels of a row: a row of input vectors is loaded once, all loads in flight together, unpacked once and used for every
 // pixel of the strip; the rows above and below come from L1 / L2, where the neighbouring strips left them.  Sums are fp32 in a fixed
 // order; the weight gradient sums strips per thread, then per CTA, then with one fp32 atomic add per CTA and weight.
+// The lanes of a warp take whole pixels side by side (dw_grid) and two channels share a multiply-add instruction: at stride 2, 56x56x144,
+// forward 65 -> 42 us, data gradient 80 -> 52, weight gradient 78 -> 58; 28x28x192 at stride 1 37 -> 35, 37 -> 35, 49 -> 42; 5x5 there
+// 66 -> 61, 66 -> 61, 87 -> 64.  (A thread that walks down its strip and keeps three rows of sums, 196 registers, was no quicker: 37 us.)
 // us, this / the library (which pads and re-lays in passes of its own at stride 2), 128 images:
-//   56x56x144 3x3 /2   forward 64 / 208   both gradients 160 / 394      28x28x192 5x5   forward 67 / 66   gradients 153 / 230
-//   28x28x192 3x3      forward 38 / 32    both gradients  84 / 120      56x56x96 7x7 (64 images)   119 / 115   287 / 673
+//   56x56x144 3x3 /2   forward 42 / 208   both gradients 110 / 395     28x28x192 5x5   forward 61 / 66   gradients 125 / 230
+//   28x28x192 3x3      forward 35 / 31    both gradients  77 / 121     56x56x96 7x7 (64 images)   109 / 115   251 / 673
 #include "common.cuh"
 
 namespace {
@@ -23,40 +26,67 @@ struct DwArgs {
   const __nv_bfloat16* dy;  // weight gradient
   float* dw;                // weight gradient, [K, K, C], added to
   int N, H, W, C, OH, OW, pt, pl;
-  int cx_log2;              // channel vectors of a CTA
+  int cx;                   // channel vectors of a CTA
 };
 
+// Two floats in a 64-bit register: one fused multiply-add does both (each rounded as by itself).
+using f2 = unsigned long long;
 __device__ __forceinline__ uint4 load_vec(const __nv_bfloat16* p) { return *reinterpret_cast<const uint4*>(p); }
-__device__ __forceinline__ void unpack_vec(const uint4& r, float* f) { unpack8(reinterpret_cast<const bf16x8&>(r), f); }
+__device__ __forceinline__ f2 pair_of(uint32_t u) {
+  f2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(u << 16), "r"(u & 0xffff0000u));
+  return d;
+}
+__device__ __forceinline__ void unpack_vec(const uint4& r, f2* f) {
+  f[0] = pair_of(r.x), f[1] = pair_of(r.y), f[2] = pair_of(r.z), f[3] = pair_of(r.w);
+}
+__device__ __forceinline__ void fma2(f2& acc, f2 a, f2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+__device__ __forceinline__ uint32_t pack_pair(f2 v) {
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+  const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
+  return reinterpret_cast<const uint32_t&>(b);
+}
+__device__ __forceinline__ void store_vec(__nv_bfloat16* p, const f2* v) {
+  *reinterpret_cast<uint4*>(p) = make_uint4(pack_pair(v[0]), pack_pair(v[1]), pack_pair(v[2]), pack_pair(v[3]));
+}
+// Weights in shared memory, as floats: [taps][half of a vector][32 vectors][4].  Channels side by side give no bank conflicts, and a
+// pitch known here makes every address an immediate.
+constexpr int SW_HALF = 32 * 4, SW_TAP = 2 * SW_HALF;
+__device__ __forceinline__ void load_tap(const float* sw, f2* w) {
+  *reinterpret_cast<ulonglong2*>(w) = *reinterpret_cast<const ulonglong2*>(sw);
+  *reinterpret_cast<ulonglong2*>(w + 2) = *reinterpret_cast<const ulonglong2*>(sw + SW_HALF);
+}
 
-// Stage the CTA's weights as floats: [taps][channels of the CTA].  FLIP: the taps in reverse order (data gradient at stride 1).
+// Stage the CTA's weights.  FLIP: the taps in reverse order (data gradient at stride 1).
 template <int K, bool FLIP>
 __device__ __forceinline__ void stage_weights(const DwArgs& a, float* sw, int cvec0, int cx) {
   const int ch = cx * 8;
   for (int i = threadIdx.x; i < K * K * ch; i += THREADS) {
-    const int tap = i / ch, c = cvec0 * 8 + i % ch;
-    sw[i] = c < a.C ? __bfloat162float(a.w[(size_t)(FLIP ? K * K - 1 - tap : tap) * a.C + c]) : 0.f;
+    const int tap = i / ch, at = i % ch, c = cvec0 * 8 + at;
+    sw[tap * SW_TAP + (at >> 2 & 1) * SW_HALF + (at >> 3) * 4 + (at & 3)] =
+        c < a.C ? __bfloat162float(a.w[(size_t)(FLIP ? K * K - 1 - tap : tap) * a.C + c]) : 0.f;
   }
   __syncthreads();
 }
 
 // FLIP = false: forward.  FLIP = true (stride 1): data gradient, the same sum with mirrored taps; the launcher mirrors the padding.
 template <int K, int S, bool FLIP>
-__global__ void __launch_bounds__(THREADS, K == 3 ? 1 : 2) depthwise_kernel(const DwArgs a) {
+__global__ void __launch_bounds__(THREADS, 2) depthwise_kernel(const DwArgs a) {
   extern __shared__ float sw[];
-  const int cx = 1 << a.cx_log2, cvecs = a.C / 8, ch = cx * 8;
-  const int tx = threadIdx.x & (cx - 1), cv = blockIdx.y * cx + tx;
+  const int cx = a.cx, cvecs = a.C / 8, per = THREADS / cx, slot = threadIdx.x / cx;
+  const int tx = threadIdx.x - slot * cx, cv = blockIdx.y * cx + tx;
   stage_weights<K, FLIP>(a, sw, blockIdx.y * cx, cx);
-  if (cv >= cvecs) return;
+  if (cv >= cvecs || slot >= per) return;
   const unsigned strips = (a.OW + TW - 1) / TW;
-  const unsigned total = (unsigned)(a.N * a.OH * strips), step = gridDim.x * (THREADS >> a.cx_log2);
+  const unsigned total = (unsigned)(a.N * a.OH * strips), step = gridDim.x * per;
   constexpr int IN = (TW - 1) * S + K;
-  for (unsigned t = blockIdx.x * (THREADS >> a.cx_log2) + (threadIdx.x >> a.cx_log2); t < total; t += step) {
+  for (unsigned t = blockIdx.x * per + slot; t < total; t += step) {
     const unsigned line = t / strips;  // 32-bit divisions: the launcher keeps the pixels below 2^30
     const int ow0 = (int)(t - line * strips) * TW, oh = (int)(line % a.OH);
     const long long n = line / a.OH;
     const int iw0 = ow0 * S - a.pl, ih0 = oh * S - a.pt;
-    float acc[TW][8] = {};
+    f2 acc[TW][4] = {};
 #pragma unroll
     for (int r = 0; r < K; ++r) {
       const int ih = ih0 + r;
@@ -65,22 +95,19 @@ __global__ void __launch_bounds__(THREADS, K == 3 ? 1 : 2) depthwise_kernel(cons
       uint4 raw[IN];
 #pragma unroll
       for (int i = 0; i < IN; ++i) raw[i] = (unsigned)(iw0 + i) < (unsigned)a.W ? load_vec(row + (long long)i * a.C) : make_uint4(0, 0, 0, 0);
-      float w[K][8];
+      f2 w[K][4];
 #pragma unroll
-      for (int s = 0; s < K; ++s) {
-        *reinterpret_cast<float4*>(w[s]) = *reinterpret_cast<const float4*>(sw + (r * K + s) * ch + tx * 8);
-        *reinterpret_cast<float4*>(w[s] + 4) = *reinterpret_cast<const float4*>(sw + (r * K + s) * ch + tx * 8 + 4);
-      }
+      for (int s = 0; s < K; ++s) load_tap(sw + (r * K + s) * SW_TAP + tx * 4, w[s]);
 #pragma unroll
       for (int i = 0; i < IN; ++i) {
-        float v[8];
+        f2 v[4];
         unpack_vec(raw[i], v);
 #pragma unroll
         for (int j = 0; j < TW; ++j) {
           const int s = i - j * S;
           if (s >= 0 && s < K) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) acc[j][e] += v[e] * w[s][e];
+            for (int e = 0; e < 4; ++e) fma2(acc[j][e], v[e], w[s][e]);
           }
         }
       }
@@ -88,32 +115,32 @@ __global__ void __launch_bounds__(THREADS, K == 3 ? 1 : 2) depthwise_kernel(cons
     __nv_bfloat16* out = a.y + ((n * a.OH + oh) * a.OW + ow0) * a.C + cv * 8;
 #pragma unroll
     for (int j = 0; j < TW; ++j)
-      if (ow0 + j < a.OW) *reinterpret_cast<bf16x8*>(out + (long long)j * a.C) = pack8(acc[j]);
+      if (ow0 + j < a.OW) store_vec(out + (long long)j * a.C, acc[j]);
   }
 }
 
 // Strips of 2 with 64 registers (four CTAs an SM) hide the latency of the few loads a strip has better than strips of 4: [128, 56, 56,
-// 144] 3x3 116 -> 81 us, 5x5 152 -> 126.
+// 144] 3x3 116 -> 81 us, 5x5 152 -> 126 (before the lanes took whole pixels).
 // Data gradient at stride 2: dx[ih, iw] = sum dy[oh, ow] w[ih + pt - 2 oh, iw + pl - 2 ow].  Strips start where iw + pl is even, so that the
 // taps of each pixel are known at compile time.
 template <int K>
 __global__ void __launch_bounds__(THREADS, 4) depthwise_dgrad2_kernel(const DwArgs a) {
   extern __shared__ float sw[];
   constexpr int S = 2, TW = TW2;
-  const int cx = 1 << a.cx_log2, cvecs = a.C / 8, ch = cx * 8;
-  const int tx = threadIdx.x & (cx - 1), cv = blockIdx.y * cx + tx;
+  const int cx = a.cx, cvecs = a.C / 8, per = THREADS / cx, slot = threadIdx.x / cx;
+  const int tx = threadIdx.x - slot * cx, cv = blockIdx.y * cx + tx;
   stage_weights<K, false>(a, sw, blockIdx.y * cx, cx);
-  if (cv >= cvecs) return;
+  if (cv >= cvecs || slot >= per) return;
   const int off = a.pl & 1;
   const unsigned strips = (a.W + off + TW - 1) / TW;
-  const unsigned total = (unsigned)(a.N * a.H * strips), step = gridDim.x * (THREADS >> a.cx_log2);
+  const unsigned total = (unsigned)(a.N * a.H * strips), step = gridDim.x * per;
   constexpr int BACK = (K - 1) / S, COLS = BACK + (TW - 1) / S + 1;  // output columns base/2 - BACK ... base/2 + (TW - 1)/2
-  for (unsigned t = blockIdx.x * (THREADS >> a.cx_log2) + (threadIdx.x >> a.cx_log2); t < total; t += step) {
+  for (unsigned t = blockIdx.x * per + slot; t < total; t += step) {
     const unsigned line = t / strips;
     const int iw0 = (int)(t - line * strips) * TW - off, ih = (int)(line % a.H);
     const long long n = line / a.H;
     const int ow0 = (iw0 + a.pl) / S - BACK;
-    float acc[TW][8] = {};
+    f2 acc[TW][4] = {};
 #pragma unroll
     for (int r = 0; r < K; ++r) {
       const int hh = ih + a.pt - r;
@@ -124,22 +151,19 @@ __global__ void __launch_bounds__(THREADS, 4) depthwise_dgrad2_kernel(const DwAr
       uint4 raw[COLS];
 #pragma unroll
       for (int i = 0; i < COLS; ++i) raw[i] = (unsigned)(ow0 + i) < (unsigned)a.OW ? load_vec(row + (long long)i * a.C) : make_uint4(0, 0, 0, 0);
-      float w[K][8];
+      f2 w[K][4];
 #pragma unroll
-      for (int s = 0; s < K; ++s) {
-        *reinterpret_cast<float4*>(w[s]) = *reinterpret_cast<const float4*>(sw + (r * K + s) * ch + tx * 8);
-        *reinterpret_cast<float4*>(w[s] + 4) = *reinterpret_cast<const float4*>(sw + (r * K + s) * ch + tx * 8 + 4);
-      }
+      for (int s = 0; s < K; ++s) load_tap(sw + (r * K + s) * SW_TAP + tx * 4, w[s]);
 #pragma unroll
       for (int i = 0; i < COLS; ++i) {
-        float v[8];
+        f2 v[4];
         unpack_vec(raw[i], v);
 #pragma unroll
         for (int j = 0; j < TW; ++j) {
           const int s = j - S * (i - BACK);
           if (s >= 0 && s < K) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) acc[j][e] += v[e] * w[s][e];
+            for (int e = 0; e < 4; ++e) fma2(acc[j][e], v[e], w[s][e]);
           }
         }
       }
@@ -147,29 +171,29 @@ __global__ void __launch_bounds__(THREADS, 4) depthwise_dgrad2_kernel(const DwAr
     __nv_bfloat16* out = a.y + ((n * a.H + ih) * a.W + iw0) * a.C + cv * 8;
 #pragma unroll
     for (int j = 0; j < TW; ++j)
-      if ((unsigned)(iw0 + j) < (unsigned)a.W) *reinterpret_cast<bf16x8*>(out + (long long)j * a.C) = pack8(acc[j]);
+      if ((unsigned)(iw0 + j) < (unsigned)a.W) store_vec(out + (long long)j * a.C, acc[j]);
   }
 }
 
 // R rows of taps a thread (all of them for 3x3, whose 72 sums fit the registers; else one, blockIdx.z): dw[r, s] += x[oh*S - pt + r, ow*S - pl + s] dy[oh, ow]
 template <int K, int S, int R>
-__global__ void __launch_bounds__(THREADS, K == 3 ? 1 : 2) depthwise_wgrad_kernel(const DwArgs a) {
-  extern __shared__ float red[];  // [THREADS / cx strips] folded to warps: [8 warps][cx * 8]
-  const int cx = 1 << a.cx_log2, cvecs = a.C / 8;
-  const int tx = threadIdx.x & (cx - 1), cv = blockIdx.y * cx + tx;
+__global__ void __launch_bounds__(THREADS, K == 5 ? 2 : 1) depthwise_wgrad_kernel(const DwArgs a) {
+  __shared__ float red[THREADS * 8];
+  const int cx = a.cx, cvecs = a.C / 8, per = THREADS / cx, slot = threadIdx.x / cx;
+  const int tx = threadIdx.x - slot * cx, cv = blockIdx.y * cx + tx;
   const int r_first = blockIdx.z * R;
-  const bool active = cv < cvecs;
+  const bool active = cv < cvecs && slot < per;
   const unsigned strips = (a.OW + TW - 1) / TW;
-  const unsigned total = active ? (unsigned)(a.N * a.OH * strips) : 0u, step = gridDim.x * (THREADS >> a.cx_log2);
+  const unsigned total = active ? (unsigned)(a.N * a.OH * strips) : 0u, step = gridDim.x * per;
   constexpr int IN = (TW - 1) * S + K;
-  float acc[R][K][8] = {};
-  for (unsigned t = blockIdx.x * (THREADS >> a.cx_log2) + (threadIdx.x >> a.cx_log2); t < total; t += step) {
+  f2 acc[R][K][4] = {};
+  for (unsigned t = blockIdx.x * per + slot; t < total; t += step) {
     const unsigned line = t / strips;
     const int ow0 = (int)(t - line * strips) * TW, oh = (int)(line % a.OH);
     const long long n = line / a.OH;
     const int iw0 = ow0 * S - a.pl;
     const __nv_bfloat16* grow = a.dy + ((n * a.OH + oh) * a.OW + ow0) * a.C + cv * 8;
-    float g[TW][8];
+    f2 g[TW][4];
 #pragma unroll
     for (int j = 0; j < TW; ++j) unpack_vec(ow0 + j < a.OW ? load_vec(grow + (long long)j * a.C) : make_uint4(0, 0, 0, 0), g[j]);
 #pragma unroll
@@ -182,66 +206,53 @@ __global__ void __launch_bounds__(THREADS, K == 3 ? 1 : 2) depthwise_wgrad_kerne
       for (int i = 0; i < IN; ++i) raw[i] = (unsigned)(iw0 + i) < (unsigned)a.W ? load_vec(row + (long long)i * a.C) : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int i = 0; i < IN; ++i) {
-        float v[8];
+        f2 v[4];
         unpack_vec(raw[i], v);
 #pragma unroll
         for (int j = 0; j < TW; ++j) {
           const int s = i - j * S;
           if (s >= 0 && s < K) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) acc[r][s][e] += v[e] * g[j][e];
+            for (int e = 0; e < 4; ++e) fma2(acc[r][s][e], v[e], g[j][e]);
           }
         }
       }
     }
   }
-  // threads of a warp that own the same channels differ by multiples of cx; then the warps
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // one tap at a time: the CTA's threads hand their sums over, cx * 8 channels times `groups` threads add them up
+  const int lanes = cx * 8, groups = THREADS / lanes, group = threadIdx.x / lanes, ci = threadIdx.x - group * lanes;
+  const int c = blockIdx.y * lanes + ci;
 #pragma unroll
   for (int r = 0; r < R; ++r)
 #pragma unroll
     for (int s = 0; s < K; ++s) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e)
-        for (int o = 16; o >= cx; o >>= 1) acc[r][s][e] += __shfl_xor_sync(0xffffffffu, acc[r][s][e], o);
       __syncthreads();
-      if (lane < cx) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) red[(warp * cx + lane) * 8 + e] = acc[r][s][e];
-      }
+      *reinterpret_cast<ulonglong2*>(red + threadIdx.x * 8) = make_ulonglong2(acc[r][s][0], acc[r][s][1]);
+      *reinterpret_cast<ulonglong2*>(red + threadIdx.x * 8 + 4) = make_ulonglong2(acc[r][s][2], acc[r][s][3]);
       __syncthreads();
-      for (int i = threadIdx.x; i < cx * 8; i += THREADS) {
-        const int c = blockIdx.y * cx * 8 + i;
-        if (c < a.C) {
-          float sum = 0.f;
-#pragma unroll
-          for (int w = 0; w < THREADS / 32; ++w) sum += red[w * cx * 8 + i];
-          atomicAdd(a.dw + (size_t)((r_first + r) * K + s) * a.C + c, sum);
-        }
+      if (group < groups && c < a.C) {
+        float sum = 0.f;
+        for (int i = group; i < per; i += groups) sum += red[i * lanes + ci];
+        atomicAdd(a.dw + (size_t)((r_first + r) * K + s) * a.C + c, sum);
       }
     }
 }
 
 struct DwGrid {
   dim3 grid;
-  int cx_log2;
+  int cx;
 };
 
-// Channel vectors of a CTA: the power of two up to 32 that wastes the fewest threads; CTAs along the pixels: `waves` residencies at most.
-DwGrid dw_grid(int C, long long strips, int ctas_per_sm, int z) {
+// Channel vectors of a CTA: eight (128 bytes, whole lines, and few distinct weights a warp) where that divides them, else an even share of
+// at most 32, so that a warp reads pixels whole.  (A power of two that divides 18 vectors is 2: 32 bytes of each pixel, and an L1 that
+// found 31 % of the sectors that are read again.)  The weight gradient has no weights to read and takes the share always.
+DwGrid dw_grid(int C, long long strips, int ctas_per_sm, int z, bool eights) {
   const int cvecs = C / 8;
-  int best = 0;
-  long long least = -1;
-  for (int l = 0; l <= 5; ++l) {
-    const long long lanes = (long long)((cvecs + (1 << l) - 1) >> l) << l;
-    if (least < 0 || lanes <= least) {
-      least = lanes;
-      best = l;
-    }
-  }
   DwGrid g;
-  g.cx_log2 = best;
-  const int gy = (cvecs + (1 << best) - 1) >> best, per = THREADS >> best;
+  g.cx = (cvecs + (cvecs + 31) / 32 - 1) / ((cvecs + 31) / 32);
+  if (eights && cvecs % 8 == 0) g.cx = 8;
+  const int gy = (cvecs + g.cx - 1) / g.cx;
+  const int per = THREADS / g.cx;
   long long gx = (strips + per - 1) / per, cap = (long long)kb_sm_count() * ctas_per_sm / ((long long)gy * z);
   if (cap < 1) cap = 1;
   if (gx > cap) gx = cap;
@@ -252,10 +263,10 @@ DwGrid dw_grid(int C, long long strips, int ctas_per_sm, int z) {
 template <int K>
 int dw_launch(int mode, DwArgs a, int S, cudaStream_t st) {
   const long long out_strips = (long long)a.N * a.OH * ((a.OW + TW - 1) / TW), in_strips = (long long)a.N * a.H * ((a.W + 1 + TW2 - 1) / TW2);
-  const DwGrid g = mode == 0 ? dw_grid(a.C, out_strips, 16, 1) : mode == 1 ? dw_grid(a.C, in_strips, 16, 1) : dw_grid(a.C, out_strips, 2, K == 3 ? 1 : K);
-  a.cx_log2 = g.cx_log2;
-  const int smem = mode == 2 ? (THREADS / 32) * (1 << a.cx_log2) * 8 * 4 : K * K * (1 << a.cx_log2) * 8 * 4;
-  if (smem > 48 * 1024) {  // 7x7 with 32 vectors: 50 KB
+  const DwGrid g = mode == 0 ? dw_grid(a.C, out_strips, 16, 1, true) : mode == 1 ? dw_grid(a.C, in_strips, 16, 1, true) : dw_grid(a.C, out_strips, 2, K == 3 ? 1 : K, false);
+  a.cx = g.cx;
+  const int smem = mode == 2 ? 0 : K * K * SW_TAP * 4;
+  if (smem > 48 * 1024) {  // 7x7: 49 KB and more
     static bool f1[KB_MAX_DEVICES] = {false}, f2[KB_MAX_DEVICES] = {false}, b1[KB_MAX_DEVICES] = {false}, b2[KB_MAX_DEVICES] = {false};
     if (!kb_allow_smem(depthwise_kernel<K, 1, false>, smem, f1) || !kb_allow_smem(depthwise_kernel<K, 2, false>, smem, f2) ||
         !kb_allow_smem(depthwise_kernel<K, 1, true>, smem, b1) || !kb_allow_smem(depthwise_dgrad2_kernel<K>, smem, b2)) {
