@@ -46,11 +46,14 @@ __device__ __forceinline__ void xe_store(T* p, const float* v) {
   *reinterpret_cast<uint4*>(p) = raw;
 }
 
+// The running maximum starts at the lowest finite value, not at -inf: a masked class (-inf) then adds exp(-inf) = 0 from the first on, and
+// needs no test of its own (one in this loop cost [16384, 50257] fp32 520 -> 1176 us).
+constexpr float XE_LOWEST = -3.402823466e38f;
 __device__ __forceinline__ void xe_online(float v, float& m, float& s) {
   if (v > m) {
     s = s * __expf(m - v) + 1.f;
     m = v;
-  } else if (v != -INFINITY) {  // a masked class adds nothing, also while the maximum itself is still -inf
+  } else {
     s += __expf(v - m);
   }
 }
@@ -62,7 +65,7 @@ __global__ void __launch_bounds__(XE_THREADS) xent_fwd_kernel(const T* __restric
   constexpr int VN = XeVec<T>::N;
   const long long row = blockIdx.x;
   const T* l = logits + row * ld;
-  float m = -INFINITY, s = 0.f;
+  float m = XE_LOWEST, s = 0.f;
   const int body = vec ? (V / VN) * VN : 0;
   for (int i = threadIdx.x * VN; i < body; i += XE_THREADS * VN) {
     float v[VN];
@@ -75,11 +78,11 @@ __global__ void __launch_bounds__(XE_THREADS) xent_fwd_kernel(const T* __restric
       m = vm;
     }
 #pragma unroll
-    for (int j = 0; j < VN; ++j) s += v[j] == -INFINITY ? 0.f : __expf(v[j] - m);
+    for (int j = 0; j < VN; ++j) s += __expf(v[j] - m);
   }
   for (int i = body + threadIdx.x; i < V; i += XE_THREADS) xe_online(to_f32<T>(l[i]), m, s);
   const float gm = block_max(m, red);
-  s = (m == -INFINITY) ? 0.f : s * __expf(m - gm);
+  s *= __expf(m - gm);
   s = block_sum(s, red);
   if (threadIdx.x == 0) {
     const float lse = gm + logf(s);
@@ -140,7 +143,7 @@ __global__ void __launch_bounds__(256) xent_narrow_fwd_kernel(const T* __restric
   const T* l = logits + (live ? row : 0) * ld;
   const int n = live ? V : 0;
   const int body = vec ? (n / VN) * VN : 0;
-  float m = -INFINITY, s = 0.f;
+  float m = XE_LOWEST, s = 0.f;
   for (int i = gl * VN; i < body; i += G * VN) {
     float v[VN];
     xe_load<T>(l + i, v);
@@ -152,13 +155,13 @@ __global__ void __launch_bounds__(256) xent_narrow_fwd_kernel(const T* __restric
       m = vm;
     }
 #pragma unroll
-    for (int j = 0; j < VN; ++j) s += v[j] == -INFINITY ? 0.f : __expf(v[j] - m);
+    for (int j = 0; j < VN; ++j) s += __expf(v[j] - m);
   }
   for (int i = body + gl; i < n; i += G) xe_online(to_f32<T>(l[i]), m, s);
   float gm = m;
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) gm = fmaxf(gm, __shfl_xor_sync(0xffffffffu, gm, o));
-  s = (m == -INFINITY) ? 0.f : s * __expf(m - gm);
+  s *= __expf(m - gm);
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (live && gl == 0) {

@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,V,ld", [(1, 64, 64), (77, 64, 64), (513, 65, 72), (100, 100, 100), (33, 129, 136), (7, 1000, 1000), (19, 2047, 2047),
-                                       (9, 2048, 2048), (5, 2049, 2056)])
+                                       (9, 2048, 2048), (5, 2049, 2056), (5, 5001, 5001)])
 def test_cross_entropy_of_narrow_and_wide_rows(rows, V, ld, dtype):
     from keras_b200.kernels import ops as kops
 
@@ -18,6 +18,7 @@ def test_cross_entropy_of_narrow_and_wide_rows(rows, V, ld, dtype):
     buf = (torch.randn(rows, ld, device="cuda") * 3).to(dtype)
     if V > 70:
         buf[:, 3:17] = float("-inf")  # masked classes
+        buf[0, 17:20] = torch.finfo(dtype).min  # masks of the lowest value
     logits = buf[:, :V].detach().requires_grad_(True)
     labels = torch.randint(20, V, (rows,), device="cuda")
     if rows > 2:
