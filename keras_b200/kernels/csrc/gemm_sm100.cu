@@ -681,17 +681,6 @@ KB_API int kb200_gemm_bf16_run(const void* a, const void* b, void* c, const void
   return 0;
 }
 
-KB_API int kb200_gemm_bf16_splitk(const void* a, const void* b, void* c, const float* bias, int M, int N, int K, long long lda, long long ldb,
-                                  long long ldc, int a_mn_major, int b_mn_major, int act, int out_fp32, int split_k, int* err,
-                                  cudaStream_t stream) {
-  return kb200_gemm_bf16_run(a, b, c, bias, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, act, out_fp32, 0, split_k, GV_AUTO, err, stream);
-}
-
-KB_API int kb200_gemm_bf16(const void* a, const void* b, void* c, const float* bias, int M, int N, int K, long long lda, long long ldb,
-                           long long ldc, int a_mn_major, int b_mn_major, int act, int out_fp32, int* err, cudaStream_t stream) {
-  return kb200_gemm_bf16_splitk(a, b, c, bias, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, act, out_fp32, 1, err, stream);
-}
-
 // C[M,N] = act(alpha * (A x B^T) + bias) with one-byte floating-point operands on kind::f8f6f4 tensor-core instructions.
 //   A: [M, K] bytes, row pitch lda bytes;  B: [N, K] bytes, row pitch ldb bytes (both K-major)
 //   a_format / b_format: 0 = e4m3, 1 = e5m2;  alpha: device scalar (product of the operands' scales) or null

@@ -79,16 +79,16 @@ def gemm(a, b, a_mn, b_mn, M, N, K, bias=None, act=0, out_dtype=torch.bfloat16, 
     err = _err_flag(a.device)
     if accumulate_into is not None:
         acc = accumulate_into
-        code = lib.kb200_gemm_bf16_splitk(kops._p(a), kops._p(b), kops._p(acc), None, kops._i(M), kops._i(N), kops._i(K), kops._ll(a.stride(0)),
-                                          kops._ll(b.stride(0)), kops._ll(acc.stride(0)), kops._i(a_mn), kops._i(b_mn), kops._i(0), kops._i(1),
-                                          kops._i(-max(1, split_k)), kops._p(err), kops._stream())
+        code = lib.kb200_gemm_bf16_run(kops._p(a), kops._p(b), kops._p(acc), None, kops._i(M), kops._i(N), kops._i(K), kops._ll(a.stride(0)),
+                                       kops._ll(b.stride(0)), kops._ll(acc.stride(0)), kops._i(a_mn), kops._i(b_mn), kops._i(0), kops._i(1),
+                                       kops._i(0), kops._i(-max(1, split_k)), kops._i(0), kops._p(err), kops._stream())
         kops._check(code, "gemm_bf16")
         return acc
     if split_k > 1 and bias is None and act == 0:
         acc = torch.zeros((M, N), dtype=torch.float32, device=a.device)
-        code = lib.kb200_gemm_bf16_splitk(kops._p(a), kops._p(b), kops._p(acc), None, kops._i(M), kops._i(N), kops._i(K), kops._ll(a.stride(0)),
-                                          kops._ll(b.stride(0)), kops._ll(acc.stride(0)), kops._i(a_mn), kops._i(b_mn), kops._i(0), kops._i(1),
-                                          kops._i(split_k), kops._p(err), kops._stream())
+        code = lib.kb200_gemm_bf16_run(kops._p(a), kops._p(b), kops._p(acc), None, kops._i(M), kops._i(N), kops._i(K), kops._ll(a.stride(0)),
+                                       kops._ll(b.stride(0)), kops._ll(acc.stride(0)), kops._i(a_mn), kops._i(b_mn), kops._i(0), kops._i(1),
+                                       kops._i(0), kops._i(split_k), kops._i(0), kops._p(err), kops._stream())
         kops._check(code, "gemm_bf16")
         return acc if out_dtype == torch.float32 else acc.to(out_dtype)
     out = torch.empty((M, N), dtype=out_dtype, device=a.device)
