@@ -6,6 +6,8 @@ tracing on the meta device); the caller then uses its library path.  On a CUDA d
 library must be loadable: a missing build raises instead of silently falling back.
 """
 
+import weakref
+
 import torch
 
 from keras_b200.core import config
@@ -63,32 +65,40 @@ def int8_quantize_rows(x, quantizer):
     return q.reshape(lead + (x.shape[-1],)), scale.reshape(lead + (1,)), inv
 
 
+def _i8_owner(t):
+    return t if t._base is None else t._base
+
+
+def _i8_kept(cache, t):
+    """What was made from ``t`` while the tensor that owns its memory lives and is unchanged; an address alone may be another's by now."""
+    entry = cache.get(t.data_ptr())
+    return entry[2] if entry is not None and entry[0]() is _i8_owner(t) and entry[1] == (t._version, t.stride()) else None
+
+
+def _i8_keep(cache, t, made):
+    if len(cache) > 256:
+        cache.clear()
+    cache[t.data_ptr()] = (weakref.ref(_i8_owner(t)), (t._version, t.stride()), made)
+
+
 def _i8_operands(kernel, kernel_scale):
     """Per int8 kernel [K, N], cached: the kernel transposed to [Np, K] (the GEMM wants both operands K-major; N padded to
     a multiple of 8 with zero rows) and 1 / kernel_scale as fp32 [Np]."""
     K, N = kernel.shape
     Np = (N + 7) // 8 * 8
-    key = kernel.data_ptr()
-    hit = _I8_TRANSPOSED.get(key)
-    if hit is None or hit[0] != kernel._version or hit[1].shape != (Np, K):
-        if len(_I8_TRANSPOSED) > 256:
-            _I8_TRANSPOSED.clear()
-        bt = kernel.t().contiguous()
+    hit = _i8_kept(_I8_TRANSPOSED, kernel)
+    if hit is None or hit.shape != (Np, K):
+        hit = kernel.t().contiguous()
         if Np != N:
-            bt = torch.nn.functional.pad(bt, (0, 0, 0, Np - N))
-        hit = (kernel._version, bt)
-        _I8_TRANSPOSED[key] = hit
-    ckey = kernel_scale.data_ptr()
-    chit = _I8_COL_SCALE.get(ckey)
-    if chit is None or chit[0] != kernel_scale._version or chit[1].numel() != Np:
-        if len(_I8_COL_SCALE) > 256:
-            _I8_COL_SCALE.clear()
+            hit = torch.nn.functional.pad(hit, (0, 0, 0, Np - N))
+        _i8_keep(_I8_TRANSPOSED, kernel, hit)
+    col = _i8_kept(_I8_COL_SCALE, kernel_scale)
+    if col is None or col.numel() != Np:
         col = torch.reciprocal(kernel_scale.detach().reshape(-1).float())
         if Np != N:
             col = torch.nn.functional.pad(col, (0, Np - N))
-        chit = (kernel_scale._version, col)
-        _I8_COL_SCALE[ckey] = chit
-    return hit[1], chit[1], Np
+        _i8_keep(_I8_COL_SCALE, kernel_scale, col)
+    return hit, col, Np
 
 
 def int8_matmul(q_inputs, kernel, inputs_scale, kernel_scale, out_dtype=torch.bfloat16, inv_inputs_scale=None, bias=None, act=0):

@@ -604,3 +604,25 @@ def test_exact_gelu_of_the_epilogue_and_its_derivative_over_the_whole_range():
     assert torch.all((dz.double() - slope).abs() <= 2.0 ** -8 * slope.abs() + 2e-6)  # one rounding to bf16; the slope itself crosses zero
     nan = torch.full((8, 64), float("nan"), device="cuda").bfloat16()
     assert gemm.gemm(nan, eye, 0, 1, 8, 64, 64, act=4).isnan().all() and kops.activation_backward(one[:8].contiguous(), nan, 4)[0].isnan().all()
+
+
+def test_int8_operands_are_not_taken_for_those_of_a_freed_kernel():
+    """Kernels that take one another's place in memory (unpacked int4 kernels of equal layers, a second model): each its own product."""
+    from keras_b200.kernels import dispatch
+
+    x = torch.randint(-127, 128, (64, 256), device="cuda", dtype=torch.int8)
+    one = torch.ones((64, 1), device="cuda")
+    seen = set()
+    for seed in range(4):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        kernel = torch.randint(-127, 128, (256, 128), generator=g, device="cuda", dtype=torch.int8)
+        scale = torch.rand(128, generator=g, device="cuda") + 0.5
+        seen.add(kernel.data_ptr())
+        for view in (kernel, kernel.reshape(256, 8, 16).reshape(256, -1), kernel):
+            out = dispatch.int8_matmul(x, view, one, scale, out_dtype=torch.float32)
+            want = (x.double() @ kernel.double()) / scale.double()
+            assert torch.allclose(out.double(), want, rtol=1e-6, atol=1e-3)  # exact integer sums below 2^24, a reciprocal and a product rounded
+        kernel.neg_()  # changed in place
+        assert torch.allclose(dispatch.int8_matmul(x, kernel, one, scale, out_dtype=torch.float32).double(), -want, rtol=1e-6, atol=1e-3)
+        del kernel, view, scale
+    assert len(seen) < 4  # memory was reused
