@@ -593,6 +593,17 @@ def add_rows(dst, src):
     return dst.add_(src)
 
 
+def copy_and_cast(src, dst, dst16):
+    """``dst.copy_(src)`` and ``dst16.copy_(src)`` (bf16) of one fp32 tensor, from one read of it where it is laid out for that."""
+    if (src.is_cuda and src.device == dst.device == dst16.device and src.dtype == dst.dtype == torch.float32 and dst16.dtype == torch.bfloat16
+            and src.is_contiguous() and dst.is_contiguous() and dst16.is_contiguous() and src.shape == dst.shape == dst16.shape
+            and src.numel() % 8 == 0 and not (src.data_ptr() | dst.data_ptr() | dst16.data_ptr()) % 16):
+        _check(_lib().kb200_copy_cast(_p(src), _p(dst), _p(dst16), _ll(src.numel()), _stream()), "copy_cast")
+    else:
+        dst.copy_(src, non_blocking=True)
+        dst16.copy_(dst)
+
+
 def cast_f32_to_bf16(src, dst):
     lib = _lib()
     _check(lib.kb200_cast_f32_bf16(_p(src), _p(dst), _ll(src.numel()), _stream()), "cast_f32_bf16")

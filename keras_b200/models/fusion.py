@@ -12,6 +12,8 @@ consumer node is reached so the residual operand is available.  Patterns only fi
 with a channels-last BN; otherwise execution is node by node as written.
 """
 
+import threading
+
 import torch
 
 from keras_b200 import activations
@@ -187,6 +189,34 @@ def run_pool_padded(layer, x, pairs):
     return layer(ops.pad(x, pads))
 
 
+class RecordedInputs(threading.local):
+    """The batch of a step that is being recorded in this thread.  Its cast to bf16 is left to whoever copies a batch in, which reads
+    it anyway: ``casts`` maps the place of a batch tensor to the bf16 tensor that the recorded step reads."""
+
+    def __init__(self):
+        self.end()
+
+    def begin(self, leaves):
+        self._leaves = [(leaf, leaf._version) if isinstance(leaf, torch.Tensor) else None for leaf in leaves]
+        self.casts = {}
+
+    def end(self):
+        casts = getattr(self, "casts", None)
+        self._leaves, self.casts = (), {}
+        return casts
+
+    def cast(self, x, dtype):
+        for i, entry in enumerate(self._leaves):
+            if entry is not None and entry[0] is x and entry[1] == x._version and x.is_cuda and x.dtype == torch.float32 and dtype == torch.bfloat16:
+                if i not in self.casts:
+                    self.casts[i] = torch.empty_like(x, dtype=dtype)
+                return self.casts[i]
+        return None
+
+
+recorded_inputs = RecordedInputs()
+
+
 def shared_cast(layer, x, casts):
     """``x`` in the layer's compute dtype, cast once for all the convolutions of a pass that read it (the input of a block with a
     projected shortcut: [256, 56, 56, 256] in float32 is 185 us a cast).  Only where no gradient flows back, which would
@@ -198,7 +228,8 @@ def shared_cast(layer, x, casts):
         return x  # an fp32 input with few channels is cast inside the patch kernel
     kept = casts.get((id(x), td))
     if kept is None or kept[0] is not x:
-        kept = casts[(id(x), td)] = (x, x.to(td))
+        recorded = recorded_inputs.cast(x, td)
+        kept = casts[(id(x), td)] = (x, x.to(td) if recorded is None else recorded)
     return kept[1]
 
 

@@ -61,6 +61,7 @@ class GraphedTrainStep:
         self._seen = 0
         self.disabled = None         # reason string once capture is ruled out for good
         self.static_leaves = None
+        self.input_casts = {}        # place of a batch tensor -> its bf16 rounding, which the recorded step reads
         self.structure = None
         self.out_structure = None
         self.out_leaves = None
@@ -150,6 +151,8 @@ class GraphedTrainStep:
         return logs
 
     def _capture(self, data, leaves, sig):
+        from keras_b200.models import fusion
+
         model = self.model
         self.structure = data
         static = [torch.empty_like(leaf).copy_(leaf) if isinstance(leaf, torch.Tensor) else leaf for leaf in leaves]
@@ -158,6 +161,7 @@ class GraphedTrainStep:
         graph = torch.cuda.CUDAGraph()
         launches_before = kops.launch_count()
         seed_generator.begin_capture()
+        fusion.recorded_inputs.begin(static)
         try:
             with torch.cuda.graph(graph, stream=self._stream):
                 logs = model.train_step(static_data)
@@ -167,6 +171,7 @@ class GraphedTrainStep:
                                 if isinstance(leaf, torch.Tensor) and leaf.ndim == 0 and leaf.is_floating_point() and leaf.is_cuda]
                 packed = torch.stack([out_leaves[i].detach().float() for i in packed_index]) if packed_index else None
         except Exception as e:  # capture ruled out: the step that was being captured has not run, so run it eagerly
+            fusion.recorded_inputs.end()
             seed_generator.end_capture()
             self.disabled = f"capture failed: {type(e).__name__}: {e}"
             self.failure_traceback = traceback.format_exc()
@@ -177,13 +182,14 @@ class GraphedTrainStep:
             self._resync_host_state()
             torch.cuda.empty_cache()  # what the side-stream steps cached is of no use to the eager steps on the main stream
             return model.train_step(data)
+        input_casts = fusion.recorded_inputs.end()
         seed_generator.end_capture()
         self._resync_host_state()
         torch.cuda.empty_cache()      # the graph owns its pool; the warm-up's cached blocks go back to the device
         # launcher calls recorded into the graph: nothing ran yet, each replay runs that many kernels' launchers
         self.launches_per_replay = kops.launch_count() - launches_before
         kops.add_launches(-self.launches_per_replay)
-        self.graph, self.signature, self.static_leaves = graph, sig, static
+        self.graph, self.signature, self.static_leaves, self.input_casts = graph, sig, static, input_casts
         self.out_structure, self.out_type = raw, type(logs)
         self.out_leaves, self.out_packed, self.out_packed_index = out_leaves, packed, packed_index
         # capture records the step without running it: this batch is the first replay
@@ -198,9 +204,14 @@ class GraphedTrainStep:
 
     def _replay(self, leaves, copy_inputs=True):
         if copy_inputs:
-            for dst, src in zip(self.static_leaves, leaves):
-                if isinstance(dst, torch.Tensor):
+            for i, (dst, src) in enumerate(zip(self.static_leaves, leaves)):
+                if i in self.input_casts:
+                    kops.copy_and_cast(src, dst, self.input_casts[i])
+                elif isinstance(dst, torch.Tensor):
                     dst.copy_(src, non_blocking=True)
+        else:
+            for i, cast in self.input_casts.items():
+                cast.copy_(self.static_leaves[i])
         engine = getattr(self.model, "_parallel_engine", None)
         if engine is not None:
             engine.check()

@@ -626,3 +626,45 @@ def test_int8_operands_are_not_taken_for_those_of_a_freed_kernel():
         assert torch.allclose(dispatch.int8_matmul(x, kernel, one, scale, out_dtype=torch.float32).double(), -want, rtol=1e-6, atol=1e-3)
         del kernel, view, scale
     assert len(seen) < 4  # memory was reused
+
+
+@pytest.mark.parametrize("n", [8, 4096, 8 * 148 * 16 * 256 * 2 + 8, 999])
+def test_copy_and_cast(n):
+    from keras_b200.kernels import ops as kops
+
+    src = torch.randn(n, device="cuda")
+    src[:3] = torch.tensor([float("nan"), float("inf"), -3.4e38])
+    dst, dst16 = torch.zeros_like(src), torch.zeros(n, device="cuda", dtype=torch.bfloat16)
+    kops.copy_and_cast(src, dst, dst16)
+    assert torch.equal(dst[1:], src[1:]) and dst[0].isnan() and torch.equal(dst16[1:], src[1:].to(torch.bfloat16)) and dst16[0].isnan()
+
+
+def test_recorded_step_reads_the_rounded_batch_of_each_replay():
+    """A float32 batch into convolutions, also read as it is: each replay answers as the eager step does, batch by batch."""
+    import keras_b200 as keras
+
+    def build():
+        keras.utils.set_random_seed(3)
+        keras.config.set_dtype_policy("mixed_bfloat16")
+        try:
+            x = keras.Input((16, 16, 64))
+            a, b = (keras.layers.ReLU()(keras.layers.BatchNormalization()(keras.layers.Conv2D(64, k, padding="same", use_bias=False)(x))) for k in (1, 3))
+        finally:
+            keras.config.set_dtype_policy("float32")
+        h = keras.layers.GlobalAveragePooling2D(dtype="float32")(keras.layers.Add(dtype="float32")([a, b, x]))
+        m = keras.Model(x, keras.layers.Dense(4, dtype="float32")(h))
+        m.compile(keras.optimizers.SGD(0.01), keras.losses.SparseCategoricalCrossentropy(from_logits=True))
+        return m
+
+    gc.collect()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    batches = [(torch.randn((32, 16, 16, 64), generator=g, device="cuda"), torch.randint(0, 4, (32,), generator=g, device="cuda")) for _ in range(8)]
+    losses = []
+    for jit in ("auto", False):
+        m = build()
+        m.jit_compile = jit
+        losses.append([float(m.train_on_batch(*b)) for b in batches])
+        if jit == "auto":
+            assert m._graphed_step.replays > 0 and list(m._graphed_step.input_casts) == [0]
+    # the same kernels on the same values; weight gradients are summed by atomics in another order
+    assert losses[0] == pytest.approx(losses[1], rel=1e-4)
