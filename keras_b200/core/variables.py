@@ -75,8 +75,6 @@ class Variable:
         self._shard_spec = None
         self._value = None
         self._shadow = None
-        self._copy = None
-        self._copy_allowed = True
         if isinstance(initializer, str):
             from keras_b200 import initializers
 
@@ -217,73 +215,10 @@ class Variable:
             scope = global_state.get_global_attribute("autocast_scope")
             if scope is not None and scope.torch_dtype is not None and value.dtype != scope.torch_dtype:
                 shadow = self._shadow
-                if value is self._value:
-                    if shadow is not None:
-                        if shadow[0] == scope.torch_dtype:
-                            return shadow[1](value)
-                    elif self._copy_allowed and not torch.is_grad_enabled():
-                        copy = self._inference_copy(value, scope.torch_dtype)
-                        if copy is not None:
-                            return copy
+                if shadow is not None and value is self._value and shadow[0] == scope.torch_dtype:
+                    return shadow[1](value)
                 return value.to(scope.torch_dtype)
         return value
-
-    def _inference_copy(self, value, dtype, padded=False):
-        """The 16-bit copy of a CUDA variable that inference reads instead of casting it at every call, or ``None``.
-
-        It is made when the variable is read a second time without having changed in between, so weights that move between
-        reads (evaluation inside a training loop) are cast as before and hold no memory.  It belongs to one state of the
-        variable: its version counter, its storage, and the copy's own version counter (nobody has written into it).  Recording
-        (a CUDA graph, a tracer, a dispatch mode, function transforms) reads the variable itself, so that what is recorded follows
-        later updates.  Kernels that write variables through raw pointers switch it off (``written_through_pointers``).
-
-        ``padded``: a matrix whose rows are zero-padded to a multiple of 8 elements, for the GEMM; returns the wide matrix."""
-        if (type(value) is not torch.nn.Parameter or not value.is_cuda or torch.cuda.is_current_stream_capturing() or torch._C._is_tracing()
-                or torch._C._len_torch_dispatch_stack() or torch._C._are_functorch_transforms_active() or torch.compiler.is_compiling()):
-            return None
-        state = (value._version, value.data_ptr(), dtype, padded)
-        seen = self._copy
-        if seen is None or seen[0] != state:
-            self._copy = (state, None, 0, 0, None)
-            return None
-        copy = seen[1]
-        if copy is None:
-            return self._make_inference_copy(value, dtype, padded, state)
-        if copy._version != seen[2]:
-            self._copy = None
-            return None
-        if torch._C._cuda_getCurrentRawStream(copy.device.index) != seen[3]:
-            stream = torch.cuda.current_stream(copy.device)  # made on another stream: wait for it, and keep its memory while this one reads
-            stream.wait_stream(seen[4])
-            copy.record_stream(stream)
-        return copy
-
-    def _make_inference_copy(self, value, dtype, padded, state):
-        if (value.dtype != torch.float32 or dtype not in (torch.bfloat16, torch.float16) or torch.is_inference_mode_enabled()
-                or self._shard_slices is not None or global_state.get_global_attribute("distribution") is not None):
-            self._copy_allowed = self._shard_slices is None  # the other conditions may pass
-            return None
-        rows, cols = (value.numel() // value.shape[-1], value.shape[-1]) if value.ndim else (1, 1)
-        width = -(-cols // 8) * 8 if padded else cols
-        if rows * width >= 1 << 23:
-            # a copy of 16 MB and more has to leave room: it takes at most a quarter of what is free
-            spare = torch.cuda.mem_get_info(value.device)[0] + torch.cuda.memory_reserved(value.device) - torch.cuda.memory_allocated(value.device)
-            if rows * width * 8 > spare:
-                return None
-        if padded:
-            copy = torch.empty((rows, width), dtype=dtype, device=value.device)
-            copy[:, :cols].copy_(value)
-            copy[:, cols:].zero_()
-        else:
-            copy = value.detach().to(dtype)
-        stream = torch.cuda.current_stream(value.device)
-        self._copy = (state, copy, copy._version, stream.cuda_stream, stream)
-        return copy
-
-    def written_through_pointers(self):
-        """From now on kernels write this variable without its version counter noticing: no copy of it can be trusted."""
-        self._copy_allowed = False
-        self._copy = None
 
     def _direct_assign(self, value):
         with torch.no_grad():

@@ -387,8 +387,6 @@ def _plan_for(opt, grads, variables, slot_lists):
     from keras_b200.kernels import shadow
 
     shadows = shadow.shadows_for(variables)
-    for v in variables:
-        v.written_through_pointers()
     plan = _ops().OptimizerPlan(params, list(grads), slots[0], slots[1] if len(slots) > 1 else None, shadows, [0.0] * len(params))
     opt._fused_plan = (key, plan)
     return plan

@@ -14,8 +14,6 @@ import os
 
 import torch
 
-from keras_b200.core import global_state
-from keras_b200.core.scopes import get_stateless_scope
 from keras_b200.kernels import ops as kops
 from keras_b200.kernels import shadow
 
@@ -189,8 +187,8 @@ class GemmFn(torch.autograd.Function):
         return (dx, dw, db, None, None, None)[: len(ctx.needs_input_grad)]
 
 
-def _qualifies(x2, w, padded=False):
-    if not (_ok_2d(x2) and (padded or _ok_2d(w, any_width=True))):
+def _qualifies(x2, w):
+    if not (_ok_2d(x2) and _ok_2d(w, any_width=True)):
         return False
     M, K = x2.shape
     N = w.shape[1]
@@ -225,40 +223,19 @@ def _grad_target(variable, w):
     return p
 
 
-def _wide_weight(variable, x):
-    """``(weight, wide)`` of an fp32 matrix variable whose width is no multiple of 8 (a vocabulary), read for inference in bf16:
-    ``wide`` is its kept zero-padded copy and ``weight`` a view of it, or ``wide`` is ``None`` and ``weight`` a cast (the first time).
-    ``None`` when the variable is not read that way."""
-    shape, value = variable.shape, variable._value
-    if torch.is_grad_enabled() or len(shape) != 2 or shape[1] % 8 == 0 or shape[1] < 256 or not variable._copy_allowed or variable._shadow is not None:
-        return None
-    scope = global_state.get_global_attribute("autocast_scope")
-    if (not variable._autocast or variable._shard_slices is not None or value is None or value.dtype != torch.float32 or scope is None
-            or scope.torch_dtype != torch.bfloat16 or x.dtype != torch.bfloat16 or shape[0] % 8
-            or get_stateless_scope() is not None or global_state.get_global_attribute("symbolic_scope") is not None):
-        return None
-    wide = variable._inference_copy(value, torch.bfloat16, padded=True)
-    return (value.to(torch.bfloat16), None) if wide is None else (wide[:, : shape[1]], wide)
-
-
 def dense(x, kernel, bias, activation_name, kernel_shape=None, value=None):
-    """``value``: what ``kernel`` (a ``Variable``) reads as, when the caller has already read it.  Returns ``(output, activation_applied)`` or ``None``.  ``kernel`` may be a ``Variable`` (reshaped to the 2-D
-    ``kernel_shape`` when given) or a tensor."""
+    """Returns ``(output, activation_applied)`` or ``None``.  ``kernel`` may be a ``Variable`` (reshaped to the 2-D ``kernel_shape`` when
+    given) or a tensor; ``value``: what the ``Variable`` reads as, when the caller has already read it."""
     from keras_b200.core.variables import Variable
 
-    wide = None
-    if isinstance(kernel, Variable):
-        read = _wide_weight(kernel, x) if kernel_shape is None and isinstance(x, torch.Tensor) else None
-        w, wide = (kernel.value if value is None else value, None) if read is None else read
-    else:
-        w = kernel
+    w = (kernel.value if value is None else value) if isinstance(kernel, Variable) else kernel
     if kernel_shape is not None:
         w = w.reshape(kernel_shape)
     if not isinstance(x, torch.Tensor) or x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or w.ndim != 2 or x.ndim < 2:
         return None
     lead = x.shape[:-1]
     x2 = x.reshape(-1, x.shape[-1])
-    if not _qualifies(x2, w, wide is not None):
+    if not _qualifies(x2, w):
         return None
     b = bias.value if isinstance(bias, Variable) else bias
     needs_grad = torch.is_grad_enabled() and (x2.requires_grad or w.requires_grad or (b is not None and b.requires_grad))
@@ -269,7 +246,7 @@ def dense(x, kernel, bias, activation_name, kernel_shape=None, value=None):
         N = w.shape[1]
         b32 = _bias_operand(b)
         if N % 8:
-            w = kops.pad_columns(w, N + 8 - N % 8) if wide is None else wide
+            w = kops.pad_columns(w, N + 8 - N % 8)
             b32 = torch.nn.functional.pad(b32, (0, 8 - N % 8)) if b32 is not None else None
         out = gemm(x2, w, 0, 1, x2.shape[0], w.shape[1], x2.shape[1], bias=b32, act=act or 0)
         if N % 8:

@@ -256,46 +256,82 @@ def _plain(model, x):
     return h
 
 
+def _agrees(model, x):
+    with torch.no_grad():
+        return torch.allclose(model(x, training=False).float(), _plain(model, x).float(), atol=0.05, rtol=0.02)
+
+
 @pytest.mark.parametrize("vocab", [300, 301, 304])
-def test_inference_copies_of_weights_follow_every_change(vocab):
+def test_inference_follows_every_change_of_its_weights(vocab):
+    """Also those that no version counter shows: writes through ``data``, replays of a recorded update, the fused optimizer."""
     import keras_b200 as keras
 
     keras.utils.set_random_seed(0)
     model = _bf16_model(vocab)
     x = torch.randn(8, 16, 64, device="cuda")
-    kernels = [layer.kernel for layer in model.layers[1:]]
-
-    def check(times=3):
-        for _ in range(times):
-            with torch.no_grad():
-                out = model(x, training=False)
-                want = _plain(model, x)
-            assert torch.allclose(out.float(), want.float(), atol=0.05, rtol=0.02)
-
-    check()
-    assert all(k._copy is not None and k._copy[1] is not None for k in kernels)  # kept from the second call on
-    assert kernels[1]._copy[1].shape == (64, -(-vocab // 8) * 8)
-    kernels[0].assign(torch.randn(64, 64, device="cuda") * 0.1)  # a variable update
-    check()
+    first, second = (layer.kernel for layer in model.layers[1:])
+    assert all(_agrees(model, x) for _ in range(3))
+    first.assign(torch.randn(64, 64, device="cuda") * 0.1)
+    assert all(_agrees(model, x) for _ in range(3))
     with torch.no_grad():
-        kernels[1].value.mul_(2.0)  # in place on the parameter
-    check()
-    with torch.no_grad():
-        kernels[0]._copy[1].zero_()  # somebody wrote into what was read
-    check()
-    weights = [w * 0.5 for w in model.get_weights()]
-    model.set_weights(weights)
-    check()
-    # updates by the fused optimizer write through raw pointers
+        second.value.mul_(2.0)
+    assert all(_agrees(model, x) for _ in range(3))
+    second.value.data.mul_(-1.5)
+    assert all(_agrees(model, x) for _ in range(3))
+    model.set_weights([w * 0.5 for w in model.get_weights()])
+    assert all(_agrees(model, x) for _ in range(3))
+    gc.collect()  # a recorded step of an earlier model, released during a capture, would invalidate it
+    update = torch.cuda.CUDAGraph()
+    with torch.no_grad(), torch.cuda.graph(update):
+        first.value.mul_(-1.25)
+    for _ in range(3):
+        update.replay()
+        assert all(_agrees(model, x) for _ in range(2))
     model.compile(optimizer=keras.optimizers.SGD(0.5, momentum=0.9), loss="mse")
     y = torch.randn(8, 16, vocab, device="cuda")
     for _ in range(6):
         model.train_on_batch(x, y)
-        check(2)
-    assert all(k._copy is None for k in kernels)
+        assert all(_agrees(model, x) for _ in range(2))
 
 
-def test_inference_copies_stay_out_of_recordings_and_transforms():
+def test_validation_reads_the_statistic_that_recorded_steps_wrote():
+    """A state that ``call`` assigns under ``mixed_bfloat16``: replays of the recorded step write it without any version counter moving."""
+    import keras_b200 as keras
+
+    class Scaled(keras.layers.Layer):
+        def build(self, shape):
+            self.seen = self.add_weight(shape=(), initializer="zeros", trainable=False, name="seen")
+
+        def call(self, t, training=False):
+            if training:
+                self.seen.assign_add(keras.ops.ones((), dtype="float32"))
+            return t + keras.ops.cast(self.seen, t.dtype)
+
+    def fitted(jit):
+        keras.utils.set_random_seed(7)
+        old = keras.config.dtype_policy()
+        keras.config.set_dtype_policy("mixed_bfloat16")
+        try:
+            x = keras.Input((64,))
+            m = keras.Model(x, keras.layers.Dense(8)(Scaled()(x)))
+        finally:
+            keras.config.set_dtype_policy(old)
+        m.compile(keras.optimizers.SGD(0.0), "mse", jit_compile=jit)
+        seen = []
+        for _ in range(3):
+            for _ in range(5):
+                m.train_on_batch(data, target)
+            with torch.no_grad():
+                seen += [m(data, training=False).float() for _ in range(4)]
+        return seen
+
+    gc.collect()
+    data, target = torch.randn(32, 64, device="cuda"), torch.zeros(32, 8, device="cuda")
+    for a, b in zip(fitted("auto"), fitted(False)):
+        assert torch.equal(a, b)
+
+
+def test_inference_of_a_recorded_model_and_under_inference_mode():
     import keras_b200 as keras
 
     keras.utils.set_random_seed(1)
@@ -304,7 +340,7 @@ def test_inference_copies_stay_out_of_recordings_and_transforms():
     with torch.no_grad():
         for _ in range(3):
             model(x, training=False)
-        gc.collect()  # a recorded step of an earlier model, released during a capture, would invalidate it
+        gc.collect()
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
             out = model(x, training=False)
@@ -312,15 +348,35 @@ def test_inference_copies_stay_out_of_recordings_and_transforms():
             layer.kernel.value.mul_(-1.5)
         graph.replay()
         assert torch.allclose(out.float(), _plain(model, x).float(), atol=0.05, rtol=0.02)
-        with torch.inference_mode():
-            assert torch.allclose(model(x, training=False).float(), _plain(model, x).float(), atol=0.05, rtol=0.02)
-    # with gradients on, the variable itself is read
+    with torch.inference_mode():
+        assert _agrees(model, x)
+        built_inside = _bf16_model(301)
+        assert all(_agrees(built_inside, x) for _ in range(3))
+    assert all(_agrees(built_inside, x) for _ in range(3))
     loss = model(x, training=True).float().square().mean()
     loss.backward()
     assert all(v.value.grad is not None for v in model.trainable_variables)
 
 
-def test_inference_copies_across_streams():
+def test_inference_leaves_nothing_behind():
+    """Neither memory nor anything that keeps a variable from being copied or pickled."""
+    import copy
+    import pickle
+
+    model = _bf16_model(301, 512)
+    x = torch.randn(1, 16, 512, device="cuda")
+    with torch.no_grad():
+        model(x, training=False)
+        held = torch.cuda.memory_allocated()
+        for _ in range(3):
+            model(x, training=False)
+    assert torch.cuda.memory_allocated() == held
+    kernel = model.layers[2].kernel
+    for twin in (copy.deepcopy(kernel), pickle.loads(pickle.dumps(kernel))):
+        assert torch.equal(twin.value.cpu(), kernel.value.cpu())
+
+
+def test_inference_on_two_streams():
     import keras_b200 as keras
 
     keras.utils.set_random_seed(2)
@@ -332,10 +388,11 @@ def test_inference_copies_across_streams():
         side.wait_stream(torch.cuda.current_stream())
         for _ in range(2):
             with torch.cuda.stream(side):
-                model(x, training=False)  # the copies are made on this stream
-        out = model(x, training=False)
-        assert torch.allclose(out.float(), want, atol=0.05, rtol=0.02)
-        assert model.layers[2].kernel._copy[3] == side.cuda_stream
+                there = model(x, training=False)
+        here = model(x, training=False)
+        torch.cuda.synchronize()
+        for out in (there, here):
+            assert torch.allclose(out.float(), want, atol=0.05, rtol=0.02)
 
 
 @pytest.mark.parametrize("K", [3, 5, 7])
