@@ -100,8 +100,10 @@ def flash_attention(q, k, v, mask, scale, is_causal, row_mask=None):
         return None
     if not (_ok(q) and _ok(k) and _ok(v)):
         return None
+    # the kernel takes every size but the query's heads and rows from the query and the keys: what the library would broadcast is left to it
     D = q.shape[-1]
-    if D not in (64, 128) or k.shape[-1] != D or v.shape[-1] != D or q.shape[2] % k.shape[2] or k.shape[1] != v.shape[1]:
+    if (D not in (64, 128) or k.shape != v.shape or k.shape[0] != q.shape[0] or k.shape[-1] != D or not q.device == k.device == v.device
+            or 0 in q.shape or 0 in k.shape or q.shape[2] % k.shape[2]):
         return None
     needs_grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
     mode = os.environ.get("KERAS_B200_FLASH_ATTENTION", "inference")
@@ -109,7 +111,7 @@ def flash_attention(q, k, v, mask, scale, is_causal, row_mask=None):
         return None
     if scale is None:
         scale = D ** -0.5
-    if not scale > 0 or 0 in q.shape or 0 in k.shape:
+    if not scale > 0:
         return None
     if needs_grad:
         return FlashAttentionFn.apply(q, k, v, float(scale), bool(is_causal))

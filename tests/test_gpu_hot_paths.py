@@ -236,6 +236,28 @@ def test_attention_strides_and_refusals():
     assert attention.flash_attention(q.detach().requires_grad_(True), k, v, wide[..., :200], 0.125, False) is None
 
 
+def test_attention_leaves_broadcast_operands_to_the_library():
+    """Keys and values of fewer batch elements (or heads) than the query's: the kernel would read behind them."""
+    import keras_b200 as keras
+    from keras_b200.kernels import attention
+
+    g = torch.Generator(device="cuda").manual_seed(11)
+    q, k, v = (torch.randn((b, 40, 4, 64), generator=g, device="cuda").bfloat16() for b in (3, 1, 1))
+    mask = torch.rand((3, 1, 40, 40), generator=g, device="cuda") < 0.7
+    mask[..., 0] = True
+    with torch.no_grad():
+        for m in (mask, None):
+            assert attention.flash_attention(q, k, v, m, 0.125, False) is None
+            out = keras.ops.dot_product_attention(q, k, v, mask=m)
+            want = _attention_in_64_bits(q, k, v, 0.125, False, m)
+            assert ((out.double() - want).norm() / want.norm()).item() < 2.0 ** -7
+        three = k.expand(3, 40, 4, 64)
+        for keys, values in ((three, v), (k, v.expand(3, 40, 4, 64)), (three, three[:, :, :2]), (three[:, :, :2], three), (three, three[:, :30])):
+            assert attention.flash_attention(q, keys, values, mask, 0.125, False) is None
+        assert attention.flash_attention(q[:1], three, three, None, 0.125, False) is None
+        assert attention.flash_attention(q, three[:, :, :0], three[:, :, :0], None, 0.125, False) is None
+
+
 def _bf16_model(vocab=300, d=64):
     import keras_b200 as keras
 
