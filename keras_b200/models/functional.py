@@ -294,7 +294,7 @@ class _FusionCtx:
     def __init__(self, mod, training):
         self.mod, self.training = mod, training
         self.Deferred, self.NoBias, self.run_bn, self.build_plan, self.applicable = mod.Deferred, mod.NoBias, mod.run_bn, mod.build_plan, mod.applicable
-        self.relu_cap, self.shared_cast = mod._relu_cap, mod.shared_cast
+        self.relu_cap, self.shared_cast = mod.relu_cap, mod.shared_cast
         self.run_conv_nobias, self.run_pool_padded, self.Padded = mod.run_conv_nobias, mod.run_pool_padded, mod.Padded
 
 

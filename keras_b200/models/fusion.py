@@ -12,6 +12,7 @@ consumer node is reached so the residual operand is available.  Patterns only fi
 with a channels-last BN; otherwise execution is node by node as written.
 """
 
+import math
 import threading
 
 import torch
@@ -48,21 +49,30 @@ class NoBias:
         self.x, self.bias, self.stats = x, bias, stats
 
 
-def _is_relu(op):
-    if isinstance(op, ReLU):
-        return op.max_value is None and op.negative_slope == 0.0 and op.threshold == 0.0
-    if isinstance(op, Activation):
-        return getattr(op.activation, "__name__", "") == "relu"
-    return False
+def _plain(node, *types):
+    """Whether a node is its stock layer and nothing more, so that a kernel may stand for the whole call: the exact class (a subclass may
+    compute anything), called on its inputs alone (a BatchNormalization may have been told its ``training``), with no regularizer of
+    its output to report and its input cast as the policy says."""
+    op, arguments = node.operation, node.arguments
+    return (type(op) in types and "call" not in vars(op) and op.activity_regularizer is None and op.autocast and len(arguments.args) == 1
+            and all(v is None for v in arguments.kwargs.values()))
 
 
-def _relu_cap(op):
-    """Upper bound of a ReLU layer with the sixes' strict derivative (the library's ``relu6``), or ``None``."""
-    if isinstance(op, ReLU):
-        six = op.max_value == 6.0 and op.negative_slope == 0.0 and op.threshold == 0.0
-    else:
-        six = isinstance(op, Activation) and op.activation is activations.relu6
-    return 6.0 if six else None
+def _rectifier_bound(node):
+    """Upper bound of a rectifier layer (infinity for a plain one, six with the strict derivative of the library's ``relu6``), or ``None``."""
+    op = node.operation
+    if not _plain(node, ReLU, Activation):
+        return None
+    if isinstance(op, Activation):  # by identity: a user's own function may well be called "relu"
+        return math.inf if op.activation is activations.relu else 6.0 if op.activation is activations.relu6 else None
+    if op.negative_slope != 0.0 or op.threshold != 0.0:
+        return None
+    return math.inf if op.max_value is None else 6.0 if op.max_value == 6.0 else None
+
+
+def relu_cap(op):
+    """Upper bound of a layer that ``build_plan`` took for a rectifier, or ``None``."""
+    return None if (op.max_value is None if isinstance(op, ReLU) else op.activation is activations.relu) else 6.0
 
 
 def build_plan(function):
@@ -77,7 +87,7 @@ def build_plan(function):
     plan = {}
     for n in nodes:
         op = n.operation
-        if not isinstance(op, BatchNormalization) or op.renorm or op.synchronized or len(n.outputs) != 1:
+        if not _plain(n, BatchNormalization) or op.renorm or op.synchronized or len(n.outputs) != 1:
             continue
         out = n.outputs[0]
         if id(out) in output_ids:
@@ -86,6 +96,8 @@ def build_plan(function):
         if len(cons) != 1:
             continue
         c = cons[0]
+        if getattr(c.operation, "compute_dtype", None) != op.compute_dtype:
+            continue  # the consumer casts first
         if plan.get(id(c)) in ("consume_add", "consume_add_relu"):
             # second BN operand of an already planned Add: deferred too, so that its producing convolution can
             # drop its bias; the executor materialises it before the fused BN+Add of the first operand
@@ -93,10 +105,10 @@ def build_plan(function):
             continue
         if id(c) in plan:
             continue
-        if (_is_relu(c.operation) or _relu_cap(c.operation) is not None) and len(c.input_tensors) == 1:
+        if _rectifier_bound(c) is not None and len(c.input_tensors) == 1:
             plan[id(n)] = "defer_bn"
             plan[id(c)] = "consume_relu"
-        elif isinstance(c.operation, Add) and len(c.input_tensors) == 2 and len(c.outputs) == 1:
+        elif _plain(c, Add) and len(c.input_tensors) == 2 and len(c.outputs) == 1:
             other = [t for t in c.input_tensors if t is not out]
             if len(other) != 1 or tuple(other[0].shape) != tuple(out.shape):
                 continue
@@ -104,13 +116,14 @@ def build_plan(function):
             plan[id(c)] = "consume_add"
             add_out = c.outputs[0]
             cc = consumers.get(id(add_out), [])
-            if id(add_out) not in output_ids and len(cc) == 1 and _is_relu(cc[0].operation) and id(cc[0]) not in plan:
+            if (id(add_out) not in output_ids and len(cc) == 1 and _rectifier_bound(cc[0]) == math.inf and id(cc[0]) not in plan
+                    and cc[0].operation.compute_dtype == op.compute_dtype):
                 plan[id(c)] = "consume_add_relu"
                 plan[id(cc[0])] = "identity"
     # Convolution bias feeding a fused BN: the normalised output does not depend on it (training
     # mode) and its gradient is exactly zero, so the add and the bias-gradient reduction are dropped;
     # the bias only enters the moving-mean update (and the shift in inference mode).
-    from keras_b200.layers.convolutional.base_conv import BaseConv
+    from keras_b200.layers.convolutional.base_conv import Conv1D, Conv2D, Conv3D
 
     producers = {}
     for n in nodes:
@@ -123,9 +136,9 @@ def build_plan(function):
         if src is None or id(src) in plan:
             continue
         op = src.operation
-        if not isinstance(op, BaseConv) or op.lora_enabled or op.data_format != "channels_last":
+        if not _plain(src, Conv1D, Conv2D, Conv3D) or op.lora_enabled or op.data_format != "channels_last":
             continue
-        if getattr(op.activation, "__name__", "linear") != "linear" or op.activity_regularizer is not None:
+        if op.activation is not None and op.activation is not activations.linear:
             continue
         out = src.outputs[0]
         if id(out) in output_ids or len(consumers.get(id(out), [])) != 1 or len(src.input_tensors) != 1:
@@ -140,7 +153,7 @@ def build_plan(function):
 
     for n in nodes:
         op = n.operation
-        if not isinstance(op, ZeroPadding2D) or op.data_format != "channels_last" or id(n) in plan or len(n.input_tensors) != 1:
+        if not _plain(n, ZeroPadding2D) or op.data_format != "channels_last" or id(n) in plan or len(n.input_tensors) != 1:
             continue
         out = n.outputs[0]
         cons = consumers.get(id(out), [])
@@ -148,7 +161,7 @@ def build_plan(function):
             continue
         c = cons[0]
         cop = c.operation
-        if isinstance(cop, MaxPooling2D) and cop.padding == "valid" and cop.data_format == "channels_last" and id(c) not in plan:
+        if _plain(c, MaxPooling2D) and cop.padding == "valid" and cop.data_format == "channels_last" and id(c) not in plan:
             plan[id(n)] = "pad_fold"
             plan[id(c)] = "pool_padded"
         elif plan.get(id(c)) == "conv_fold_bias" and cop.rank == 2 and cop.padding == "valid" and all(lo == hi for lo, hi in op.padding):
@@ -277,6 +290,11 @@ def run_bn(layer, x, training, residual=None, relu=False, pre_bias=None, stats=N
     from keras_b200.kernels import dispatch
 
     train = bool(training) and layer.trainable
+    td = layer._compute_torch_dtype()
+    if x.dtype != td and x.dtype.is_floating_point:
+        x, stats = x.to(td), None
+    if residual is not None and residual.dtype != td and residual.dtype.is_floating_point:
+        residual = residual.to(td)
     bias_value = pre_bias._value if pre_bias is not None else None
     out = dispatch.batch_norm(layer, x, train, residual=residual, relu=relu, pre_bias=bias_value, conv_stats=stats, cap=cap)
     if out is not None:

@@ -178,6 +178,9 @@ class Function(Operation):
                     x, pre_bias, stats = x.x, x.bias, x.stats
                 elif isinstance(x, fusion.Deferred):
                     x = fusion.run_bn(x.layer, x.x, training, pre_bias=x.pre_bias, stats=x.stats)
+                if getattr(x, "_keras_mask", None) is not None:  # the layer's own call: statistics of the real positions, and the mask goes on
+                    env[id(outs[0])] = (node.operation if operation_fn is None else operation_fn(node.operation))(x)
+                    continue
                 env[id(outs[0])] = fusion.Deferred(node.operation, x, pre_bias, stats)
                 continue
             if role == "consume_relu":

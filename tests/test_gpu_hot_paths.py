@@ -519,6 +519,107 @@ def test_model_with_relu6_folds_it_into_the_normalisation():
     assert list(plan.values()).count("consume_relu") == 2  # the bound of four keeps its own layer
 
 
+def _odd_chains():
+    """Chains in which one layer is more than the fused kernel that could stand for its neighbours: ``{name: (input shape, build)}``."""
+    import keras_b200 as keras
+
+    L = keras.layers
+
+    def relu(t):
+        return t * 0 + 7
+
+    def linear(t):
+        return t * 0 + 2
+
+    class Rectifier(L.ReLU):
+        def call(self, t):
+            return t * 0 + 5
+
+    class Norm(L.BatchNormalization):
+        def call(self, t, training=None, mask=None):
+            return t * 0 - 3
+
+    class Sum(L.Add):
+        def _merge_function(self, inputs):
+            return inputs[0] * 0 + 4
+
+    class Conv(L.Conv2D):
+        def call(self, t):
+            return t * 0 + 9
+
+    class Frame(L.ZeroPadding2D):
+        def call(self, t):
+            return torch.nn.functional.pad(t, (0, 0, 1, 1, 1, 1), value=100.0)
+
+    conv = lambda t, **k: L.Conv2D(16, 1, **k)(t)  # noqa: E731
+    norm = lambda t, **k: L.BatchNormalization(**k)(t)  # noqa: E731
+    image = (8, 8, 16)
+    return {
+        "relu6 in float32": (image, lambda x: L.ReLU(6.0, dtype="float32")(norm(conv(x)))),
+        "relu in float32": (image, lambda x: L.ReLU(dtype="float32")(norm(conv(x)))),
+        "norm in float32": (image, lambda x: L.ReLU(6.0)(norm(conv(x), dtype="float32"))),
+        "sum in float32": (image, lambda x: L.ReLU()(L.Add(dtype="float32")([norm(conv(x)), x]))),
+        "rectified sum in float32": (image, lambda x: L.ReLU(dtype="float32")(L.Add()([norm(conv(x)), x]))),
+        "relu6 with a penalty": (image, lambda x: L.ReLU(6.0, activity_regularizer="l2")(norm(conv(x)))),
+        "relu with a penalty": (image, lambda x: L.ReLU(activity_regularizer="l2")(norm(conv(x)))),
+        "norm with a penalty": (image, lambda x: L.ReLU()(norm(conv(x), activity_regularizer="l2"))),
+        "sum with a penalty": (image, lambda x: L.Add(activity_regularizer="l2")([norm(conv(x)), x])),
+        "relu6 of one's own": (image, lambda x: Rectifier(6.0)(norm(conv(x)))),
+        "relu of one's own": (image, lambda x: Rectifier()(norm(conv(x)))),
+        "function called relu": (image, lambda x: L.Activation(relu)(norm(conv(x)))),
+        "convolution with a function called linear": (image, lambda x: L.ReLU()(norm(conv(x, activation=linear)))),
+        "norm of one's own": (image, lambda x: L.ReLU(6.0)(Norm()(conv(x)))),
+        "sum of one's own": (image, lambda x: Sum()([norm(conv(x)), x])),
+        "convolution of one's own": (image, lambda x: L.ReLU(6.0)(norm(Conv(16, 1)(x)))),
+        "padding of one's own": (image, lambda x: L.MaxPooling2D(3, 2)(Frame(1)(x))),
+        "frozen norm": (image, lambda x: L.ReLU(6.0)(L.BatchNormalization()(x, training=False))),
+        "masked norm": ((6, 8), lambda x: L.ReLU(6.0)(norm(L.Masking()(x)))),
+    }
+
+
+@pytest.mark.parametrize("policy", ["float32", "mixed_bfloat16"])
+@pytest.mark.parametrize("training", [False, True])
+def test_folded_chains_answer_as_their_layers_do(policy, training):
+    """Results, their type, penalties and masks of a whole model against its layers called one by one."""
+    import keras_b200 as keras
+
+    old = keras.config.dtype_policy()
+    for name, (shape, build) in _odd_chains().items():
+        keras.utils.set_random_seed(5)
+        keras.config.set_dtype_policy(policy)
+        try:
+            x = keras.Input(shape)
+            model = keras.Model(x, build(x))
+        finally:
+            keras.config.set_dtype_policy(old)
+        data = torch.randn((4,) + shape, device="cuda") * 2
+        data[:, 3:] = data[:, 3:] * (len(shape) == 3)  # positions of a sequence that are masked
+        state = [v.value.clone() for v in model.weights]
+        with torch.no_grad():
+            got = model(data, training=training)
+            penalties = len(model.losses)
+            after = [v.value.clone() for v in model.weights]
+            for v, s in zip(model.weights, state):
+                v.assign(s)
+            env = {id(t): data for t in model.inputs}
+            for node in model._ordered_nodes():
+                if node.input_tensors:
+                    args, kwargs = node.arguments.fill_in(env)
+                    if not isinstance(node.operation, keras.layers.BatchNormalization) or "training" in kwargs:
+                        env[id(node.outputs[0])] = node.operation(*args, **kwargs)
+                    else:
+                        env[id(node.outputs[0])] = node.operation(*args, training=training)
+        want = env[id(model.outputs[0])]
+        assert got.dtype == want.dtype == keras.ops.zeros((), dtype=model.outputs[0].dtype).dtype, name
+        assert (getattr(got, "_keras_mask", None) is None) == (getattr(want, "_keras_mask", None) is None), name
+        assert penalties == sum(layer.activity_regularizer is not None for layer in model.layers), name
+        # a fused chain keeps float32 between its parts where layers of their own round to the compute type
+        step = 2.0 ** -6 if policy != "float32" else 1e-4
+        assert torch.allclose(got.float(), want.float(), rtol=step, atol=step), name
+        for a, v in zip(after, model.weights):
+            assert torch.allclose(a, v.value, rtol=step, atol=step), name
+
+
 @pytest.mark.parametrize("relu,res", [(True, True), (True, False), (False, False)])
 @pytest.mark.parametrize("rows,C", [(20011, 144), (15003, 192), (70001, 48), (3001, 960), (9001, 320), (2200, 1000), (600, 4096), (30, 24)])
 def test_batch_norm_at_channel_counts_that_are_no_power_of_two(rows, C, relu, res):

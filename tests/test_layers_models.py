@@ -147,3 +147,35 @@ def test_float8_dense_updates_scales_through_optimizer():
     assert hist[0] == pytest.approx(np.abs(x).max(), rel=1e-5) and hist.shape == (4,)
     model.train_on_batch(x, y)
     assert dense.inputs_scale.numpy() == pytest.approx(np.abs(x).max() / 448.0, rel=1e-4)
+
+
+def test_only_stock_chains_are_planned_for_fused_kernels():
+    from keras_b200.models import fusion
+
+    L = keras.layers
+
+    def roles(build):
+        x = keras.Input((8, 8, 16))
+        model = keras.Model(x, build(x))
+        plan = fusion.build_plan(model)
+        return [plan.get(id(n)) for n in model._ordered_nodes() if n.input_tensors]
+
+    def relu(t):
+        return t * 2
+
+    class Mine(L.ReLU):
+        pass
+
+    norm = lambda x, **k: L.BatchNormalization(**k)(x)  # noqa: E731
+    for rectifier in (L.ReLU(), L.ReLU(6.0), L.Activation("relu"), L.Activation("relu6")):
+        assert roles(lambda x: rectifier(norm(x))) == ["defer_bn", "consume_relu"]
+    for rectifier in (Mine(), Mine(6.0), L.ReLU(5.0), L.ReLU(negative_slope=0.1), L.Activation(relu), L.ReLU(activity_regularizer="l2"), L.ReLU(dtype="bfloat16"),
+                      L.ReLU(6.0, autocast=False)):
+        assert roles(lambda x: rectifier(norm(x))) == [None, None]
+    assert roles(lambda x: L.ReLU()(L.BatchNormalization()(x, training=False))) == [None, None]
+    assert roles(lambda x: L.ReLU()(norm(x, activity_regularizer="l2"))) == [None, None]
+    assert roles(lambda x: L.ReLU()(norm(L.Conv2D(8, 1)(x)))) == ["conv_fold_bias", "defer_bn", "consume_relu"]
+    assert roles(lambda x: L.ReLU()(norm(L.Conv2D(8, 1, activation="relu")(x)))) == [None, "defer_bn", "consume_relu"]
+    assert sorted(map(str, roles(lambda x: L.ReLU()(L.Add()([norm(x), x]))))) == ["consume_add_relu", "defer_bn", "identity"]
+    assert sorted(map(str, roles(lambda x: L.ReLU(6.0)(L.Add()([norm(x), x]))))) == ["None", "consume_add", "defer_bn"]
+    assert set(roles(lambda x: L.Add(dtype="bfloat16")([norm(x), x]))) == {None}  # casts stand between them
