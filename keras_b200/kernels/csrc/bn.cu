@@ -100,7 +100,8 @@ static int bn_resident_blocks(K kernel) {
   return n;
 }
 
-// ReLU mask of a row vector: from the saved bit mask (one byte per thread vector), else from y > 0, else all ones.
+// ReLU mask of a row vector: from the saved bit mask (one byte per thread vector), else closed where y <= 0 (a NaN is open, as in the library),
+// else all ones.
 template <typename T>
 __device__ __forceinline__ unsigned bn_mask_bits(const typename Vec<T>::Raw& ry, bool have_y, const unsigned char* bits, long long vec_index) {
   constexpr int V = Vec<T>::N;
@@ -110,7 +111,7 @@ __device__ __forceinline__ unsigned bn_mask_bits(const typename Vec<T>::Raw& ry,
   Vec<T>::unpack(ry, yv);
   unsigned m = 0;
 #pragma unroll
-  for (int k = 0; k < V; ++k) m |= (yv[k] > 0.f ? 1u : 0u) << k;
+  for (int k = 0; k < V; ++k) m |= (yv[k] <= 0.f ? 0u : 1u) << k;
   return m;
 }
 
@@ -203,6 +204,9 @@ __global__ void __launch_bounds__(BN_THREADS, 2) bn_reduce_kernel(const T* __res
   }
 }
 
+// The difference of two roundings may be a little below zero; NaN stays NaN (a channel with an infinity or a NaN in it), where fmaxf makes it zero.
+__device__ __forceinline__ float bn_variance(float v) { return v < 0.f ? 0.f : v; }
+
 // pre_bias: bias of the producing convolution that was folded away (the normalised output does not
 // depend on it; only the moving mean does).
 __global__ void bn_finalize_kernel(const float* __restrict__ sums, const float* __restrict__ gamma, const float* __restrict__ beta,
@@ -212,7 +216,7 @@ __global__ void bn_finalize_kernel(const float* __restrict__ sums, const float* 
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   const float mean = sums[c] * inv_m;
-  const float var = fmaxf(sums[C + c] * inv_m - mean * mean, 0.f);
+  const float var = bn_variance(sums[C + c] * inv_m - mean * mean);
   const float invstd = rsqrtf(var + eps);
   const float g = gamma ? gamma[c] : 1.f, b = beta ? beta[c] : 0.f;
   mean_out[c] = mean;
@@ -248,7 +252,7 @@ __global__ void bn_finalize_partials_kernel(const float* __restrict__ partials, 
   q = warp_sum(q);
   if (lane != 0) return;
   const float mean = s * inv_m;
-  const float var = fmaxf(q * inv_m - mean * mean, 0.f);
+  const float var = bn_variance(q * inv_m - mean * mean);
   const float invstd = rsqrtf(var + eps);
   const float g = gamma ? gamma[c] : 1.f, b = beta ? beta[c] : 0.f;
   mean_out[c] = mean;
@@ -277,7 +281,7 @@ __global__ void bn_bwd_coeff_kernel(const float* __restrict__ sums, const float*
   coef[2 * C + c] = a * (mu * is * s2 - s1);
 }
 
-// MODE 0: y  = relu?(x*p0 + p1 (+ res)), bits = (y > 0)      (p0 = scale, p1 = shift)
+// MODE 0: y  = relu?(x*p0 + p1 (+ res)), bits = !(y <= 0)     (p0 = scale, p1 = shift)
 // MODE 1: dx = p0*dy' + p1*x + p2, dres = dy'                 (in0 = dy, in1 = x, mask from bits or y)
 // U rows in flight per thread: 4, or 8 for the forward pass without a residual input (one stream of loads only)
 template <typename T, int MODE, int U = BN_U>
@@ -333,8 +337,8 @@ __global__ void __launch_bounds__(BN_THREADS, 2) bn_apply_kernel(const T* __rest
         for (int k = 0; k < V; ++k) {
           float t = v0[k] * a[k] + b[k];
           if (has1) t += v1[k];
-          bool pass = t > 0.f;
-          o[k] = relu ? fmaxf(t, 0.f) : t;
+          bool pass = !(t <= 0.f);  // so that a NaN passes, and its gradient: fmaxf would make it a zero
+          o[k] = relu && !pass ? 0.f : t;
           if (capped && to_f32<T>(from_f32<T>(t)) >= cap) {  // decided on the value that is stored, as a separate layer would
             o[k] = cap;
             pass = false;

@@ -95,7 +95,7 @@ __device__ __forceinline__ uint4 bs_pack8(const float* f) {
   return q;
 }
 
-// MODE 0: y = relu?(in0*p0 + p1 + in1), bits_out = (y > 0)                          in0 = x, in1 = residual
+// MODE 0: y = relu?(in0*p0 + p1 + in1), bits_out = !(y <= 0)                         in0 = x, in1 = residual
 // MODE 1: sums[c] += sum d, sums[C + c] += p1[c] * sum d*(in1 - p0[c]),  d = mask ? in0 : 0   in0 = dy, in1 = x, p0 = mean, p1 = invstd
 // MODE 2: out0 = p0*d + p1*in1 + p2, out1 = d (optional)                             in0 = dy, in1 = x
 template <int MODE>
@@ -176,8 +176,9 @@ __global__ void __launch_bounds__(BS_THREADS, 1) bn_stream_kernel(const BsParams
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const float y = v0[k] * a[k] + b[k] + v1[k];
-          m |= (y > 0.f ? 1u : 0u) << k;
-          o[k] = p.relu ? fmaxf(y, 0.f) : y;
+          const bool pass = !(y <= 0.f);  // a NaN passes
+          m |= (pass ? 1u : 0u) << k;
+          o[k] = p.relu && !pass ? 0.f : y;
         }
         *reinterpret_cast<uint4*>(p.out0 + gv * 8) = bs_pack8(o);
         if (p.bits_out != nullptr) p.bits_out[gv] = (unsigned char)m;

@@ -519,6 +519,41 @@ def test_model_with_relu6_folds_it_into_the_normalisation():
     assert list(plan.values()).count("consume_relu") == 2  # the bound of four keeps its own layer
 
 
+@pytest.mark.parametrize("rows,C", [(64, 16), (4096, 1024), (20011, 144)])  # registers, the ring of bulk copies, both at no power of two
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("kind", ["relu", "relu6", "relu + residual"])
+def test_batch_norm_with_a_rectifier_keeps_nan(rows, C, dtype, kind):
+    """A channel whose statistics are no numbers stays so, values and gradients, as the layers one by one have it."""
+    from keras_b200.kernels import ops as kops
+
+    g = torch.Generator(device="cuda").manual_seed(C)
+    x = torch.randn((rows, C), generator=g, device="cuda").to(dtype)
+    x[3, 5], x[4, 6], x[5, 7] = float("nan"), float("inf"), 3.0
+    res = torch.randn((rows, C), generator=g, device="cuda").to(dtype).requires_grad_(True) if "residual" in kind else None
+    if res is not None:
+        with torch.no_grad():
+            res[7, 9] = float("nan")
+    x.requires_grad_(True)
+    gamma, beta = torch.ones(C, device="cuda", requires_grad=True), torch.zeros(C, device="cuda", requires_grad=True)
+    mean, var = torch.zeros(C, device="cuda"), torch.ones(C, device="cuda")
+    y = kops.FusedBatchNormAct.apply(x, gamma, beta, res, mean, var, 0.9, 1e-3, True, None, None, None, 6.0 if kind == "relu6" else None)
+    bad = torch.zeros((rows, C), dtype=torch.bool, device="cuda")
+    bad[:, 5:7] = True
+    grad_bad = bad.clone()
+    if res is not None:
+        bad[7, 9] = True
+    assert torch.equal(y.isnan(), bad)
+    assert torch.equal(mean.isfinite(), ~bad[0]) and torch.equal(var.isnan(), bad[0])
+    y.backward(torch.ones_like(y))
+    assert torch.equal(x.grad.isnan(), grad_bad)
+    if res is not None:
+        assert res.grad[7, 9].item() == 1.0  # the gradient passes where the sum is no number
+    scale = torch.ones(C, device="cuda")
+    scale[5] = float("nan")
+    out = kops.bn_inference(x.detach(), scale, beta.detach(), None, True, 6.0 if kind == "relu6" else None)
+    assert out[:, 5].isnan().all() and out[3, 5].isnan() and not out[:, 8].isnan().any()
+
+
 def _odd_chains():
     """Chains in which one layer is more than the fused kernel that could stand for its neighbours: ``{name: (input shape, build)}``."""
     import keras_b200 as keras
