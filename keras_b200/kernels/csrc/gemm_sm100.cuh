@@ -144,7 +144,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
 
 __device__ __forceinline__ float apply_act(float v, int act) {
   switch (act) {
-    case ACT_RELU: return fmaxf(v, 0.f);
+    case ACT_RELU: return v <= 0.f ? 0.f : v;  // a NaN stays one
     case ACT_GELU_TANH: {
       const float u = 0.7978845608028654f * (v + 0.044715f * v * v * v);
       return 0.5f * v * (1.f + tanhf(u));

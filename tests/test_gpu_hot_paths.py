@@ -781,6 +781,18 @@ def test_dense_with_an_activation_and_its_gradient(activation, rows, width, use_
         assert ((a.float() - b.float()).norm() / b.float().norm()).item() < 2.0 ** -8
 
 
+@pytest.mark.parametrize("rows", [8, 1001, 5000])
+def test_dense_with_a_relu_keeps_nan_in_inference(rows):
+    import keras_b200 as keras
+
+    layer = keras.layers.Dense(256, activation="relu", dtype="bfloat16")
+    x = torch.randn(rows, 512, device="cuda").bfloat16()
+    x[5, 7] = float("nan")
+    with torch.no_grad():
+        out = layer(x)
+    assert out[5].isnan().all() and not out[:5].isnan().any() and not out[6:].isnan().any() and (out[:5] >= 0).all()
+
+
 def test_a_function_of_the_users_own_is_not_taken_for_a_known_activation():
     import keras_b200 as keras
 
