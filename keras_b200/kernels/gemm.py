@@ -126,14 +126,15 @@ class GemmFn(torch.autograd.Function):
         ctx.bias_target = bias_target
         Np = (N + 7) // 8 * 8
         b = _bias_operand(bias)
+        wide = w
         if Np != N:
-            w = kops.pad_columns(w, Np)
+            wide = kops.pad_columns(w, Np)
             if b is not None:
                 b = torch.nn.functional.pad(b, (0, Np - N))
-        out, pre = gemm(x, w, 0, 1, M, Np, K, bias=b), None
+        out, pre = gemm(x, wide, 0, 1, M, Np, K, bias=b), None
         if act:
             pre, out = out, _ACT_FN[act](out)
-        ctx.save_for_backward(x, w, pre)
+        ctx.save_for_backward(x, w, bias, pre, wide if Np != N else None)
         ctx.act = act
         ctx.has_bias = bias is not None
         ctx.bias_dtype = bias.dtype if bias is not None else None
@@ -142,7 +143,13 @@ class GemmFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        x, w, pre = ctx.saved_tensors
+        x, w, bias, pre, wide = ctx.saved_tensors
+        if torch.is_grad_enabled():  # a gradient of this gradient is wanted: differentiate the same layer from library operations
+            operands = [t for t, need in zip((x, w, bias), ctx.needs_input_grad) if need]
+            out = torch.matmul(x, w) if bias is None else torch.matmul(x, w) + bias.to(x.dtype)
+            grads = iter(torch.autograd.grad(_ACT_FN[ctx.act](out) if ctx.act else out, operands, dy, create_graph=True))
+            return tuple(next(grads) if need else None for need in ctx.needs_input_grad[:3]) + (None,) * (len(ctx.needs_input_grad) - 3)
+        w = w if wide is None else wide
         M, K = x.shape
         N, Np = ctx.n, w.shape[1]
         sums = bias_slot = None

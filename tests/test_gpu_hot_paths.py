@@ -781,6 +781,35 @@ def test_dense_with_an_activation_and_its_gradient(activation, rows, width, use_
         assert ((a.float() - b.float()).norm() / b.float().norm()).item() < 2.0 ** -8
 
 
+@pytest.mark.parametrize("rows,width", [(1000, 256), (1001, 256), (1001, 301)])
+@pytest.mark.parametrize("activation", [None, "gelu", "silu"])
+def test_second_derivatives_of_a_dense_layer(rows, width, activation):
+    """A penalty on the gradient of the input: it reaches the weights, at every route of the product."""
+    import keras_b200 as keras
+
+    old = keras.config.dtype_policy()
+    keras.config.set_dtype_policy("mixed_bfloat16")
+    try:
+        layer = keras.layers.Dense(width, activation=activation)
+    finally:
+        keras.config.set_dtype_policy(old)
+    torch.manual_seed(rows + width)
+    x = torch.randn(rows, 256, device="cuda").bfloat16().requires_grad_(True)
+    layer(x)
+    layer.bias.assign(torch.randn(width, device="cuda") * 0.3)
+    y = layer(x)
+    (g,) = torch.autograd.grad(y.float().square().sum(), x, create_graph=True)
+    got = torch.autograd.grad(g.float().square().sum(), [layer.kernel.value, layer.bias.value])
+    xe, w, b = (t.detach().double().requires_grad_(True) for t in (x, layer.kernel.value, layer.bias.value))
+    ye = torch.matmul(xe, w) + b
+    ye = ye if activation is None else getattr(torch.nn.functional, activation)(ye)
+    (ge,) = torch.autograd.grad(ye.square().sum(), xe, create_graph=True)
+    want = torch.autograd.grad(ge.square().sum(), [w, b])
+    assert ((g.double() - ge).norm() / ge.norm()).item() < 2.0 ** -6
+    for a, e in zip(got, want):  # a chain of some eight roundings to bf16
+        assert ((a.double() - e).norm() / e.norm()).item() < 2.0 ** -6
+
+
 @pytest.mark.parametrize("rows", [8, 1001, 5000])
 def test_dense_with_a_relu_keeps_nan_in_inference(rows):
     import keras_b200 as keras
