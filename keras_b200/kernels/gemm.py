@@ -160,20 +160,21 @@ class GemmFn(torch.autograd.Function):
             bias_slot = shadow.grad_slot(ctx.bias_target, (N,)) if wanted else None
             dy, sums = kops.activation_backward(dy, pre, ctx.act, wanted, bias_slot.view(N) if bias_slot is not None else None)
         if Np != N:
-            if dy.dtype == torch.bfloat16 and dy.stride(1) == 1 and dy.stride(0) == Np and dy.data_ptr() % 16 == 0:
-                # the gradient is itself the leading columns of a padded buffer (produced for a padded logits view)
-                dyp = dy.as_strided((M, Np), (Np, 1))
-                dyp[:, N:].zero_()
+            if (dy.dtype == torch.bfloat16 and dy.stride(1) == 1 and dy.stride(0) == Np and dy.data_ptr() % 16 == 0
+                    and (dy.storage_offset() + M * Np) * dy.element_size() <= dy.untyped_storage().nbytes()):
+                # The gradient is itself the leading columns of a wider buffer, often the padded logits' own.  What stands in the columns
+                # behind may be somebody else's (a concatenation's other operand): it is neither written nor summed over.
+                dy = dy.as_strided((M, Np), (Np, 1))
             else:
-                dyp = torch.empty((M, Np), dtype=torch.bfloat16, device=dy.device)
-                dyp[:, :N].copy_(dy)
-                dyp[:, N:].zero_()
-            dy = dyp
+                wide_dy = torch.empty((M, Np), dtype=torch.bfloat16, device=dy.device)
+                wide_dy[:, :N].copy_(dy)
+                wide_dy[:, N:].zero_()
+                dy = wide_dy
         elif not _ok_2d(dy):
             dy = dy.contiguous()
         dx = dw = db = None
         if ctx.needs_input_grad[0]:
-            dx = gemm(dy, w, 0, 0, M, K, Np)
+            dx = gemm(dy, w, 0, 0, M, K, N)  # the sum ends at N; below, the columns behind it stay columns of their own
         if ctx.needs_input_grad[1]:
             split = split_k_for(K, Np, M, x.device)
             g = shadow.grad_slot(ctx.grad_target, (K, N)) if Np == N and N % 4 == 0 else None

@@ -810,6 +810,28 @@ def test_second_derivatives_of_a_dense_layer(rows, width, activation):
         assert ((a.double() - e).norm() / e.norm()).item() < 2.0 ** -6
 
 
+@pytest.mark.parametrize("rows,N", [(1001, 301), (2048, 297), (1001, 303)])
+def test_gradient_of_padded_columns_leaves_its_neighbours_alone(rows, N):
+    """A product of odd width beside other columns: its gradient is a view of the whole gradient, with the same pitch as the padded one."""
+    from keras_b200.kernels import gemm
+
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randn((rows, 256), generator=g, device="cuda").bfloat16().requires_grad_(True)
+    w = torch.randn((256, N), generator=g, device="cuda").bfloat16().requires_grad_(True)
+    b = torch.randn(N, generator=g, device="cuda").requires_grad_(True)
+    other = torch.randn((rows, -N % 8), generator=g, device="cuda").bfloat16().requires_grad_(True)
+    coef = torch.randn((rows, N - N % 8 + 8), generator=g, device="cuda").bfloat16()
+    coef[0, N:] = float("inf")
+    kept = coef.clone()
+    y = torch.cat([gemm.GemmFn.apply(x, w, b), other], dim=1)
+    y.backward(coef)
+    gemm.check_errors()
+    assert torch.equal(coef, kept) and torch.equal(other.grad, kept[:, N:])
+    d = kept[:, :N].double()
+    for got, want in ((x.grad, d @ w.detach().double().t()), (w.grad, x.detach().double().t() @ d), (b.grad, d.sum(0))):
+        assert ((got.double() - want).norm() / want.norm()).item() < 2.0 ** -8
+
+
 @pytest.mark.parametrize("rows", [8, 1001, 5000])
 def test_dense_with_a_relu_keeps_nan_in_inference(rows):
     import keras_b200 as keras
