@@ -172,15 +172,8 @@ _load_user_config()
 
 # --- framework switches (read once per query; cheap) -------------------------------------
 
-# The table behind ``os.environ`` where CPython has one in bytes: a look-up there skips the encoding of the name and the
-# decoding of the value (1 us), and this question is asked some 50 times a forward pass.
-_ENV_BYTES = getattr(os.environ, "_data", None) if os.name == "posix" else None
-
-
 def fused_kernels_enabled():
     """False when ``KERAS_B200_DISABLE_FUSED_KERNELS=1``: every op then runs its library path."""
-    if _ENV_BYTES is not None:
-        return _ENV_BYTES.get(b"KERAS_B200_DISABLE_FUSED_KERNELS") != b"1"
     return os.environ.get("KERAS_B200_DISABLE_FUSED_KERNELS", "0") != "1"
 
 

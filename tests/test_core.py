@@ -105,3 +105,17 @@ def test_convolution_tiling_choices_without_a_gpu():
     assert bn == 64 and n_tiles == 1 and 0 < grid <= 148
     assert lib.kb200_conv_igemm_plan(256, 14, 14, 256, 1024, 1, 1, 0, plan) == 0
     assert plan[2] == 256 and plan[1] == 4 and plan[0] % 4 == 0
+
+
+def test_the_kernels_switch_is_read_from_the_environment_in_force(monkeypatch):
+    import os
+
+    from keras_b200.core import config
+
+    for environ in (dict(os.environ), os.environ):  # a program may put a mapping of its own in its place
+        monkeypatch.setattr(os, "environ", environ)
+        for value, on in (("1", False), ("0", True), ("", True)):
+            monkeypatch.setitem(os.environ, "KERAS_B200_DISABLE_FUSED_KERNELS", value)
+            assert config.fused_kernels_enabled() is on
+        monkeypatch.delitem(os.environ, "KERAS_B200_DISABLE_FUSED_KERNELS")
+        assert config.fused_kernels_enabled()
