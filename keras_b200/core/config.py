@@ -8,6 +8,8 @@ therefore returns a constant.
 import json
 import os
 
+import torch
+
 from keras_b200.core.export_registry import keras_export
 
 _FLOATX = "float32"
@@ -172,8 +174,15 @@ _load_user_config()
 
 # --- framework switches (read once per query; cheap) -------------------------------------
 
+_forward_ad = torch.autograd.forward_ad
+_in_function_transform = torch._C._are_functorch_transforms_active
+
+
 def fused_kernels_enabled():
-    """False when ``KERAS_B200_DISABLE_FUSED_KERNELS=1``: every op then runs its library path."""
+    """False when ``KERAS_B200_DISABLE_FUSED_KERNELS=1``, and inside the transforms of ``torch.func`` and forward-mode derivatives, which
+    kernels that work on raw pointers cannot take part in: every op then runs its library path."""
+    if _forward_ad._current_level >= 0 or _in_function_transform():
+        return False
     return os.environ.get("KERAS_B200_DISABLE_FUSED_KERNELS", "0") != "1"
 
 

@@ -23,11 +23,8 @@ def _groups(batch, units):
 
 
 def takes(sequences, initial_state, cell):
-    """float32 tensors on one device, plain reverse-mode autograd at most (function transforms and forward-mode derivatives go
-    through the composed operations), a batch and a width that the launch holds."""
+    """float32 tensors on one device, a batch and a width that the launch holds."""
     if not _plain(sequences) or sequences.ndim != 3 or sequences.shape[0] == 0 or sequences.shape[1] == 0 or len(initial_state) != 2:
-        return False
-    if torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0:
         return False
     weights = [cell.kernel, cell.recurrent_kernel] + ([cell.bias] if cell.bias is not None else [])
     if any(getattr(w, "_shard_slices", None) is not None for w in weights):

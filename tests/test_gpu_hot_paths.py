@@ -832,6 +832,54 @@ def test_gradient_of_padded_columns_leaves_its_neighbours_alone(rows, N):
         assert ((got.double() - want).norm() / want.norm()).item() < 2.0 ** -8
 
 
+def _transformed_models():
+    import keras_b200 as keras
+
+    L = keras.layers
+    old = keras.config.dtype_policy()
+    try:
+        keras.config.set_dtype_policy("mixed_bfloat16")
+        for rows in (1000, 1001):
+            for activation in (None, "relu", "gelu"):
+                x = keras.Input((rows, 256))
+                yield f"dense {rows} {activation}", keras.Model(x, L.Dense(256, activation=activation)(x)), (1, rows, 256)
+        x = keras.Input((40, 256))
+        yield "attention", keras.Model(x, L.MultiHeadAttention(4, 64)(x, x)), (2, 40, 256)
+        yield "depthwise", keras.Sequential([keras.Input((12, 12, 16)), L.DepthwiseConv2D(3, strides=2), L.BatchNormalization(), L.ReLU(6.0)]), (2, 12, 12, 16)
+        keras.config.set_dtype_policy("float32")
+        yield "lstm", keras.Sequential([keras.Input((5, 8)), L.LSTM(32)]), (3, 5, 8)
+        x = keras.Input((8, 8, 16))
+        yield "chain", keras.Model(x, L.ReLU(6.0)(L.BatchNormalization()(L.Conv2D(16, 3, padding="same")(x)))), (2, 8, 8, 16)
+    finally:
+        keras.config.set_dtype_policy(old)
+
+
+@pytest.mark.parametrize("recording", [False, True])
+def test_forward_mode_and_function_transforms_see_every_layer(recording):
+    """A tangent against the reverse mode (<J t, J t> = <t, J' J t>), and a mapped call against a single one: with and without gradients."""
+    import keras_b200 as keras
+    from torch.autograd import forward_ad
+
+    keras.utils.set_random_seed(4)
+    for name, model, shape in _transformed_models():
+        g = torch.Generator(device="cuda").manual_seed(2)
+        x, t = (torch.randn(shape, generator=g, device="cuda") for _ in range(2))
+        with torch.set_grad_enabled(recording):
+            plain = model(x, training=False)
+            with torch.nn.attention.sdpa_kernel(torch.nn.attention.SDPBackend.MATH):  # the one library attention with these derivatives
+                with forward_ad.dual_level():
+                    tangent = forward_ad.unpack_dual(model(forward_ad.make_dual(x, t), training=False)).tangent
+                also = keras.ops.jvp(lambda a: model(a, training=False), (x,), (t,))[1]
+                many = torch.func.vmap(lambda a: model(a, training=False))(torch.stack([x, x + t]))
+        assert tangent is not None, name
+        xg = x.clone().requires_grad_(True)
+        (back,) = torch.autograd.grad(model(xg, training=False), xg, tangent.detach())
+        want = (back * t).sum().item()
+        for got in (tangent, also):  # sums over thousands of products of bf16 numbers
+            assert got.detach().float().square().sum().item() == pytest.approx(want, rel=0.02 if plain.dtype == torch.bfloat16 else 1e-3), name
+        assert torch.allclose(many[0].float(), plain.float(), atol=0.03, rtol=0.03), name
+
+
 @pytest.mark.parametrize("rows", [8, 1001, 5000])
 def test_dense_with_a_relu_keeps_nan_in_inference(rows):
     import keras_b200 as keras
