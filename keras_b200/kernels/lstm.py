@@ -67,12 +67,13 @@ def _aligned(t):
 
 class LstmSequence(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, xz, bias, h0, c0, R, reverse, want_sequence):
+    def forward(ctx, xz, bias, h0, c0, R, reverse, want_sequence, recording):
         B, T = xz.shape[0], xz.shape[1]
         U = R.shape[0]
         x, h, c, r = _aligned(xz), _aligned(h0), _aligned(c0), _aligned(R)
         b = bias.detach().contiguous() if bias is not None else None
-        grad = any(ctx.needs_input_grad)
+        # needs_input_grad follows requires_grad whether gradients are recorded or not: trainable weights have it in inference too
+        grad = recording and any(ctx.needs_input_grad)
         empty = lambda *shape: torch.empty(shape, dtype=torch.float32, device=xz.device)  # noqa: E731
         hprev, hT, cT = empty(B, T, U), empty(B, U), empty(B, U)
         out = empty(B, T, U) if want_sequence else None
@@ -87,14 +88,14 @@ class LstmSequence(torch.autograd.Function):
     def backward(ctx, dout, dhT, dcT):
         xz, bias, h0, c0, R, hprev, gates, cs = ctx.saved_tensors
         if dout is None and dhT is None and dcT is None:
-            return (None,) * 7
+            return (None,) * 8
         if torch.is_grad_enabled():  # a gradient of this gradient is wanted: differentiate the composed operations
             inputs = [xz, bias, h0, c0, R]
             wanted = [t for t, need in zip(inputs, ctx.needs_input_grad) if need]
             results = _composed(xz, bias, h0, c0, R, ctx.reverse)
             pairs = [(r, g) for r, g in zip(results, (dout, dhT, dcT)) if g is not None]
             grads = iter(torch.autograd.grad([r for r, _ in pairs], wanted, [g for _, g in pairs], create_graph=True, allow_unused=True))
-            return tuple(next(grads) if need else None for need in ctx.needs_input_grad[:5]) + (None, None)
+            return tuple(next(grads) if need else None for need in ctx.needs_input_grad[:5]) + (None,) * 3
         B, T, U = hprev.shape
         need = ctx.needs_input_grad
         dout, dhT, dcT = (g.contiguous() if g is not None else None for g in (dout, dhT, dcT))
@@ -106,9 +107,9 @@ class LstmSequence(torch.autograd.Function):
         flat = dz.view(B * T, 4 * U)
         dR = torch.matmul(hprev.view(B * T, U).t(), flat) if need[4] else None
         db = flat.sum(0) if need[1] else None
-        return dz if need[0] else None, db, dh0, dc0 if need[3] else None, dR, None, None
+        return dz if need[0] else None, db, dh0, dc0 if need[3] else None, dR, None, None, None
 
 
 def run(xz, bias, h0, c0, R, reverse, want_sequence):
     """``(outputs [B, T, U] in processing order or None, last h, last c)``."""
-    return LstmSequence.apply(xz, bias, h0, c0, R, bool(reverse), bool(want_sequence))
+    return LstmSequence.apply(xz, bias, h0, c0, R, bool(reverse), bool(want_sequence), torch.is_grad_enabled())

@@ -96,6 +96,24 @@ def test_lstm_sequence_against_the_steps_in_64_bits(B, T, U, F, reverse, sequenc
     assert torch.equal(h2, h) and torch.equal(c2, c)
 
 
+@pytest.mark.parametrize("B,T,U", [(3, 1, 20), (64, 6, 256), (300, 4, 640)])
+@pytest.mark.parametrize("reverse", [False, True])
+def test_lstm_keeps_gates_only_for_a_backward_pass(B, T, U, reverse, monkeypatch):
+    """Trainable weights without gradients: no gates, no cell states, the same result bit for bit (several row tiles a group at B = 300)."""
+    from keras_b200.kernels import lstm
+
+    g = torch.Generator(device="cuda").manual_seed(U)
+    args = [torch.randn(s, generator=g, device="cuda") for s in ((B, T, 4 * U), (4 * U,), (B, U), (B, U))]
+    args.append((torch.randn((U, 4 * U), generator=g, device="cuda") * U ** -0.5).requires_grad_(True))
+    launched, plain = [], lstm._launch
+    monkeypatch.setattr(lstm, "_launch", lambda *a: launched.append(a) or plain(*a))
+    recorded = lstm.run(*args, reverse, True)
+    with torch.no_grad():
+        bare = lstm.run(*args, reverse, True)
+    assert [a[10] is None and a[11] is None for a in launched] == [False, True]
+    assert all(torch.equal(a, b) for a, b in zip(recorded, bare))
+
+
 def test_lstm_layer_routes_and_second_derivatives():
     import keras_b200 as keras
     from keras_b200.kernels import lstm
