@@ -898,6 +898,20 @@ def test_forward_mode_and_function_transforms_see_every_layer(recording):
         assert torch.allclose(many[0].float(), plain.float(), atol=0.03, rtol=0.03), name
 
 
+@pytest.mark.parametrize("act,fn", [(1, torch.relu), (3, torch.nn.functional.silu), (4, torch.nn.functional.gelu)])
+def test_activation_derivatives_at_infinities_and_nan(act, fn):
+    from keras_b200.kernels import ops as kops
+
+    values = [float("inf"), float("-inf"), float("nan"), 0.0, -0.0, 1.5, -1.5, 300.0, -300.0, 3e38, -3e38]
+    pairs = torch.cartesian_prod(torch.tensor(values), torch.tensor(values)).cuda().bfloat16()
+    dy, z = (torch.nn.functional.pad(c, (0, 128 - len(c))).reshape(8, 16).contiguous() for c in pairs.t())
+    z = z.requires_grad_(True)
+    (want,) = torch.autograd.grad(fn(z), z, dy)
+    got = kops.activation_backward(dy, z.detach(), act)[0]
+    same = (got == want) | (got.isnan() & want.isnan()) | ((got.float() - want.float()).abs() <= 2.0 ** -8 * want.float().abs() + 1e-30)
+    assert same.all(), torch.stack([dy[~same], z[~same], got[~same], want[~same]], 1)
+
+
 @pytest.mark.parametrize("rows", [8, 1001, 5000])
 def test_dense_with_a_relu_keeps_nan_in_inference(rows):
     import keras_b200 as keras
