@@ -142,7 +142,7 @@ __device__ __forceinline__ void conv_store_rows(uint32_t tmem_row, int ng0, int 
         }
         if (p.act != ACT_NONE) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = apply_act(v[j], p.act);
+          for (int j = 0; j < 32; ++j) v[j] = apply_act<false>(v[j], p.act);
         }
         if (!valid) {  // pixels beyond the image: clipped by the store, and they must not enter the statistics
 #pragma unroll

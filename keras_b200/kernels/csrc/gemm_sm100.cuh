@@ -142,6 +142,9 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
       : "memory");
 }
 
+// PRECISE: the result is stored as float32.  normal_cdf is within 1e-6 of the value, far below bf16's rounding; in float32 the library's
+// erff is nearer (1.7e-7 for |v| < 1) until 1 + erf cancels, at v = -2 as far off as normal_cdf is.
+template <bool PRECISE>
 __device__ __forceinline__ float apply_act(float v, int act) {
   switch (act) {
     case ACT_RELU: return v <= 0.f ? 0.f : v;  // a NaN stays one
@@ -150,7 +153,7 @@ __device__ __forceinline__ float apply_act(float v, int act) {
       return 0.5f * v * (1.f + tanhf(u));
     }
     case ACT_SILU: return v / (1.f + __expf(-v));
-    case ACT_GELU_ERF: return v * normal_cdf(v);
+    case ACT_GELU_ERF: return v * (PRECISE && !(v < -2.f) ? 0.5f * (1.f + erff(v * 0.7071067811865476f)) : normal_cdf(v));
     default: return v;
   }
 }
@@ -197,7 +200,7 @@ __device__ __forceinline__ void store_rows_tma(uint32_t tmem_row, int ncols, int
       }
       if (p.act != ACT_NONE) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = apply_act(v[j], p.act);
+        for (int j = 0; j < 32; ++j) v[j] = apply_act<true>(v[j], p.act);
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u)
@@ -222,7 +225,7 @@ __device__ __forceinline__ void store_rows_tma(uint32_t tmem_row, int ncols, int
         }
         if (p.act != ACT_NONE) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = apply_act(v[j], p.act);
+          for (int j = 0; j < 32; ++j) v[j] = apply_act<false>(v[j], p.act);
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {

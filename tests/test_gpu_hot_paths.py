@@ -964,6 +964,20 @@ def test_exact_gelu_of_the_epilogue_and_its_derivative_over_the_whole_range():
     assert gemm.gemm(nan, eye, 0, 1, 8, 64, 64, act=4).isnan().all() and kops.activation_backward(one[:8].contiguous(), nan, 4)[0].isnan().all()
 
 
+def test_gelu_into_float32_is_as_accurate_as_the_library():
+    from keras_b200.kernels import gemm
+
+    x = torch.cat([torch.linspace(-2, 2, 64 * 999), torch.linspace(-0.01, 0.01, 64)]).reshape(1000, 64).cuda().bfloat16()
+    xe = x.double()
+    want = xe * 0.5 * torch.special.erfc(-xe * 0.5 ** 0.5)
+    out = gemm.gemm(x, torch.eye(64, device="cuda").bfloat16(), 0, 1, 1000, 64, 64, act=4, out_dtype=torch.float32).double()
+    off = (out - want).abs() / want.abs().clamp_min(1e-30)
+    # half an ulp (2^-24) each for the sum and two products, up to two ulps of erf; relative to 1 + erf, which is 0.317 at -1 and 0.0455 at -2
+    for low, high, bound in ((0, 2, 5 * 2.0 ** -24), (-1, 0, 5 * 2.0 ** -24 / 0.317), (-2, -1, 5 * 2.0 ** -24 / 0.0455)):
+        assert off[(x >= low) & (x <= high)].max().item() <= bound
+    assert off[(x >= -1) & (x <= 1)].square().mean().sqrt().item() < 1e-7
+
+
 def test_int8_operands_are_not_taken_for_those_of_a_freed_kernel():
     """Kernels that take one another's place in memory (unpacked int4 kernels of equal layers, a second model): each its own product."""
     from keras_b200.kernels import dispatch
