@@ -22,6 +22,11 @@ from keras_b200.layers.layer import Layer
 _EPILOGUE_ACTIVATIONS = (activations.linear, activations.relu, activations.silu, activations.gelu)
 
 
+def epilogue_name(act):
+    """The name by which the GEMM knows an activation: by identity, for a user's own function may well be called "gelu"."""
+    return None if act is None else act.__name__ if act in _EPILOGUE_ACTIVATIONS else "other"
+
+
 @keras_export("keras.layers.Dense")
 class Dense(CalibratedKernel, Layer):
     def __init__(self, units, activation=None, use_bias=True, kernel_initializer="glorot_uniform", bias_initializer="zeros",
@@ -87,9 +92,7 @@ class Dense(CalibratedKernel, Layer):
                 return out
         kernel = self.kernel
         act = self.activation
-        # by identity: a user's own function may well be called "gelu"
-        name = None if act is None else getattr(act, "__name__", None) if act in _EPILOGUE_ACTIVATIONS else "other"
-        fused = dispatch.dense(inputs, kernel, self.bias, name)
+        fused = dispatch.dense(inputs, kernel, self.bias, epilogue_name(act))
         if fused is not None:
             out, act_done = fused
             if not act_done and act is not None and act is not activations.linear:
@@ -259,7 +262,7 @@ class Dense(CalibratedKernel, Layer):
             # inference on the device: quantise the rows, then one GEMM whose epilogue de-scales, adds the bias and activates
             act = self.activation
             fused = dispatch.int8_dense(inputs, self._kernel.value, self.kernel_scale.value, self.inputs_quantizer,
-                                        self.bias._value if self.bias is not None else None, getattr(act, "__name__", None))
+                                        self.bias._value if self.bias is not None else None, epilogue_name(act))
             if fused is not None:
                 out, act_done = fused
                 return out if act_done or act is None or act is activations.linear else act(out)

@@ -15,6 +15,7 @@ from keras_b200 import activations, constraints, initializers, ops, quantizers, 
 from keras_b200.core.export_registry import keras_export
 from keras_b200.kernels import dispatch
 from keras_b200.layers.core.calibrated_kernel import CalibratedKernel
+from keras_b200.layers.core.dense import epilogue_name
 from keras_b200.layers.layer import Layer
 
 
@@ -475,7 +476,7 @@ class EinsumDense(CalibratedKernel, Layer):
 
                 act = self.activation
                 fused = dispatch.int8_dense(x2, kv.reshape(kdim, -1), self.kernel_scale.value.reshape(-1), quantizer,
-                                            self.bias._value if self.bias is not None else None, getattr(act, "__name__", None))
+                                            self.bias._value if self.bias is not None else None, epilogue_name(act))
                 if fused is not None:
                     out, act_done = fused
                     out = out.reshape(tuple(lead) + tuple(kv.shape[nk:]))

@@ -943,6 +943,29 @@ def test_a_function_of_the_users_own_is_not_taken_for_a_known_activation():
             assert ((y.float() - want).norm() / want.norm()).item() < 2.0 ** -7
 
 
+def test_a_quantised_layer_calls_the_function_it_was_given():
+    import keras_b200 as keras
+
+    def gelu(x):
+        return x * 0 + 3.0
+
+    x = torch.randn(128, 64, device="cuda")
+    for layer in (keras.layers.Dense(64, activation=gelu), keras.layers.EinsumDense("ab,bc->ac", output_shape=64, bias_axes="c", activation=gelu)):
+        layer(x)
+        layer.quantize("int8")
+        with torch.no_grad():
+            assert torch.equal(layer(x), torch.full((128, 64), 3.0, device="cuda"))
+    for name in ("relu", "gelu", "silu"):
+        layer = keras.layers.Dense(64, activation=name)
+        layer(x)
+        layer.quantize("int8")
+        with torch.no_grad():
+            out = layer(x)
+            layer.activation = keras.activations.linear
+            want = getattr(torch.nn.functional, name)(layer(x))
+        assert torch.allclose(out, want, atol=1e-5, rtol=1e-5)
+
+
 def test_exact_gelu_of_the_epilogue_and_its_derivative_over_the_whole_range():
     from keras_b200.kernels import gemm, ops as kops
 
