@@ -714,12 +714,18 @@ def dot_product_attention(query, key, value, bias=None, mask=None, scale=None, i
         if is_causal:
             attn_mask = attn_mask & torch.ones((T, S), dtype=torch.bool, device=q.device).tril()
             is_causal = False
+        # A row with every position masked attends uniformly (keras/src/backend/torch/nn.py:1539): a query of zeros that sees them all.  Left to
+        # the large negative below, the library's kernels overflow to zeros on the GPU, and their backward passes, which recompute the
+        # probabilities from a log-sum that the negative has swallowed, take each for one.
+        empty = ~attn_mask.any(dim=-1, keepdim=True)
+        qh = torch.where(empty, torch.zeros((), dtype=d, device=q.device), qh)
+        attn_mask = attn_mask | empty
     if bias is not None:
         b = _t(bias).to(d)
-        attn_mask = b if attn_mask is None else b + _attention_mask_bias(attn_mask, d)
+        if attn_mask is not None:
+            b = torch.where(empty, torch.zeros((), dtype=d, device=b.device), b) + _attention_mask_bias(attn_mask, d)
+        attn_mask = b
     elif attn_mask is not None:
-        # a large finite negative instead of -inf: a row with every position masked attends uniformly instead of producing
-        # zeros or NaN (keras/src/backend/torch/nn.py:1539)
         attn_mask = _attention_mask_bias(attn_mask, d)
     out = F.scaled_dot_product_attention(qh, kh, vh, attn_mask=attn_mask, is_causal=is_causal and attn_mask is None, scale=scale, enable_gqa=(K != N))
     return out.transpose(1, 2)

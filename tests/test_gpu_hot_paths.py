@@ -222,9 +222,43 @@ def test_attention_layer_with_padding(masks):
         attention.check_errors()
         assert torch.equal(got, want) and len(calls) == 1
         assert (calls[0][-1] is rows) == (masks in ("both", "query+key", "three"))
-    # training keeps the product; its library kernel answers rows without any key with zeros, so only the others are compared
-    out, want = layer(q.clone().requires_grad_(True), v, query_mask=rows, **given)[rows], want[rows]
+    # training keeps the product, for the library
+    out = layer(q.clone().requires_grad_(True), v, query_mask=rows, **given)
     assert ((out.double() - want.double()).norm() / want.double().norm()).item() < 2.0 ** -6
+
+
+def _uniform_rows(keras, dtype, causal, biased, device):
+    g = torch.Generator(device=device).manual_seed(9)
+    q, k, v, dy = (torch.randn((2, 40, 4, 64), generator=g, device=device).to(dtype) for _ in range(4))
+    mask = torch.rand((2, 1, 40, 40), generator=g, device=device) < 0.5
+    mask[..., 0] = True
+    mask[:, :, 3] = mask[1, :, 20:25] = False
+    bias = torch.randn((4, 40, 40), generator=g, device=device).to(dtype) if biased else None
+    args = [t.requires_grad_(True) for t in (q, k, v)]
+    out = keras.ops.dot_product_attention(*args, bias=bias, mask=mask, is_causal=causal)
+    grads = torch.autograd.grad(out, args, dy)
+    with torch.no_grad():
+        inferred = keras.ops.dot_product_attention(q, k, v, bias=bias, mask=mask, is_causal=causal)
+    seen = mask & torch.ones((40, 40), dtype=torch.bool, device=device).tril() if causal else mask
+    empty = ~seen.any(-1, keepdim=True)
+    exact = [t.detach().double().requires_grad_(True) for t in args]
+    qe, ke, ve = (t.transpose(1, 2) for t in exact)
+    s = torch.matmul(qe, ke.transpose(-1, -2)) / 8 + (bias.double() if biased else 0)
+    s = s.masked_fill(~seen, -1e30).masked_fill(empty, 0.0)
+    want = torch.matmul(torch.softmax(s, -1), ve).transpose(1, 2)
+    bound = {torch.bfloat16: 2.0 ** -6, torch.float16: 2.0 ** -9, torch.float32: 1e-5}[dtype]  # a few roundings of scores and probabilities
+    for a, e in zip([out, inferred, *grads], [want, want, *torch.autograd.grad(want, exact, dy.double())]):
+        assert ((a.double() - e).norm() / e.norm()).item() < bound
+    rows = empty.squeeze(-1).expand(2, 4, 40).transpose(1, 2)
+    assert torch.allclose(out[rows].float(), v.float().mean(1, keepdim=True).expand(v.shape)[rows], atol=0.02)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("causal,biased", [(False, False), (True, False), (False, True)])
+def test_attention_of_rows_without_a_key_is_uniform_in_training_too(dtype, causal, biased):
+    import keras_b200 as keras
+
+    _uniform_rows(keras, dtype, causal, biased, "cuda")
 
 
 def test_attention_keeps_a_nan_to_the_rows_that_see_it():

@@ -115,3 +115,10 @@ def test_image_augmentation_geometry_and_boxes():
     assert tuple(crop(np.zeros((2, 8, 8, 3), "float32")).shape) == (2, 4, 4, 3)
     mix = layers.MixUp(seed=0)({"images": np.random.rand(4, 8, 8, 3).astype("float32"), "labels": np.eye(4, dtype="float32")})
     np.testing.assert_allclose(mix["labels"].sum(1).numpy(), 1.0, rtol=1e-6)
+
+
+@pytest.mark.parametrize("causal,biased", [(False, False), (True, False), (False, True)])
+def test_attention_of_rows_without_a_key_is_uniform_and_has_its_gradients(causal, biased):
+    from tests.test_gpu_hot_paths import _uniform_rows
+
+    _uniform_rows(keras, torch.float32, causal, biased, "cpu")
