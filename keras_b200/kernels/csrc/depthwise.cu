@@ -6,14 +6,18 @@
 // Every pass is bound by its tensors' traffic (9 to 49 multiply-adds a value).  A thread owns 8 channels (one 16-byte vector) and a
 // strip of 4 pixels of a row: a row of input vectors is loaded once, all loads in flight together, unpacked once and used for every
 // pixel of the strip; the rows above and below come from L1 / L2, where the neighbouring strips left them.  Sums are fp32 in a fixed
-// order; the weight gradient sums strips per thread, then per CTA, then with one fp32 atomic add per CTA and weight.
+// order; the weight gradient sums strips per thread, then per CTA, then over the CTAs' partial sums, each time in a fixed order, so that it
+// is the same bit for bit from run to run (an atomic add per CTA and weight took 55 us where this takes 60 at 56x56x144 and stride 2, 40 / 45 at
+// 28x28x192, 62 / 66 with 5x5 there).
 // The lanes of a warp take whole pixels side by side (dw_grid) and two channels share a multiply-add instruction: at stride 2, 56x56x144,
 // forward 65 -> 42 us, data gradient 80 -> 52, weight gradient 78 -> 58; 28x28x192 at stride 1 37 -> 35, 37 -> 35, 49 -> 42; 5x5 there
-// 66 -> 61, 66 -> 61, 87 -> 64.  (A thread that walks down its strip and keeps three rows of sums, 196 registers, was no quicker: 37 us.)
+// 66 -> 61, 66 -> 61, 87 -> 64 (the weight gradients with atomics).  (A thread that walks down its strip and keeps three rows of sums, 196 registers, was no quicker: 37 us.)
 // us, this / the library (which pads and re-lays in passes of its own at stride 2), 128 images:
-//   56x56x144 3x3 /2   forward 42 / 208   both gradients 110 / 395     28x28x192 5x5   forward 61 / 66   gradients 125 / 230
-//   28x28x192 3x3      forward 35 / 31    both gradients  77 / 121     56x56x96 7x7 (64 images)   109 / 115   251 / 673
+//   56x56x144 3x3 /2   forward 42 / 208   both gradients 114 / 395     28x28x192 5x5   forward 61 / 66   gradients 129 / 230
+//   28x28x192 3x3      forward 35 / 31    both gradients  82 / 121     56x56x96 7x7 (64 images)   109 / 115   257 / 673
 #include "common.cuh"
+
+extern "C" int kb200_sum_slabs(const float* partial, float* out, int slabs, int cols, int accumulate, cudaStream_t stream);
 
 namespace {
 
@@ -24,7 +28,7 @@ struct DwArgs {
   const __nv_bfloat16* w;   // [K, K, C]
   __nv_bfloat16* y;         // forward: output;  data gradient: dx
   const __nv_bfloat16* dy;  // weight gradient
-  float* dw;                // weight gradient, [K, K, C], added to
+  float* partial;           // weight gradient: [gridDim.x][K, K, C]
   int N, H, W, C, OH, OW, pt, pl;
   int cx;                   // channel vectors of a CTA
 };
@@ -219,9 +223,10 @@ __global__ void __launch_bounds__(THREADS, K == 5 ? 2 : 1) depthwise_wgrad_kerne
       }
     }
   }
-  // one tap at a time: the CTA's threads hand their sums over, cx * 8 channels times `groups` threads add them up
+  // one tap at a time: the CTA's threads hand their sums over, cx * 8 channels times `groups` threads add them up, then the groups' sums
   const int lanes = cx * 8, groups = THREADS / lanes, group = threadIdx.x / lanes, ci = threadIdx.x - group * lanes;
   const int c = blockIdx.y * lanes + ci;
+  float* out = a.partial + (size_t)blockIdx.x * K * K * a.C;
 #pragma unroll
   for (int r = 0; r < R; ++r)
 #pragma unroll
@@ -230,11 +235,17 @@ __global__ void __launch_bounds__(THREADS, K == 5 ? 2 : 1) depthwise_wgrad_kerne
       *reinterpret_cast<ulonglong2*>(red + threadIdx.x * 8) = make_ulonglong2(acc[r][s][0], acc[r][s][1]);
       *reinterpret_cast<ulonglong2*>(red + threadIdx.x * 8 + 4) = make_ulonglong2(acc[r][s][2], acc[r][s][3]);
       __syncthreads();
-      if (group < groups && c < a.C) {
-        float sum = 0.f;
+      float sum = 0.f;
+      if (group < groups)
         for (int i = group; i < per; i += groups) sum += red[i * lanes + ci];
-        atomicAdd(a.dw + (size_t)((r_first + r) * K + s) * a.C + c, sum);
+      if (groups > 1) {
+        __syncthreads();
+        red[threadIdx.x] = sum;
+        __syncthreads();
+        if (group == 0)
+          for (int g = 1; g < groups; ++g) sum += red[g * lanes + ci];
       }
+      if (group == 0 && c < a.C) out[(size_t)((r_first + r) * K + s) * a.C + c] = sum;
     }
 }
 
@@ -260,10 +271,16 @@ DwGrid dw_grid(int C, long long strips, int ctas_per_sm, int z, bool eights) {
   return g;
 }
 
+long long out_strips(int N, int OH, int OW) { return (long long)N * OH * ((OW + TW - 1) / TW); }
+
+DwGrid wgrad_grid(int N, int OH, int OW, int C, int K) { return dw_grid(C, out_strips(N, OH, OW), 2, K == 3 ? 1 : K, false); }
+
 template <int K>
 int dw_launch(int mode, DwArgs a, int S, cudaStream_t st) {
-  const long long out_strips = (long long)a.N * a.OH * ((a.OW + TW - 1) / TW), in_strips = (long long)a.N * a.H * ((a.W + 1 + TW2 - 1) / TW2);
-  const DwGrid g = mode == 0 ? dw_grid(a.C, out_strips, 16, 1, true) : mode == 1 ? dw_grid(a.C, in_strips, 16, 1, true) : dw_grid(a.C, out_strips, 2, K == 3 ? 1 : K, false);
+  const long long in_strips = (long long)a.N * a.H * ((a.W + 1 + TW2 - 1) / TW2);
+  const DwGrid g = mode == 0   ? dw_grid(a.C, out_strips(a.N, a.OH, a.OW), 16, 1, true)
+                   : mode == 1 ? dw_grid(a.C, in_strips, 16, 1, true)
+                               : wgrad_grid(a.N, a.OH, a.OW, a.C, K);
   a.cx = g.cx;
   const int smem = mode == 2 ? 0 : K * K * SW_TAP * 4;
   if (smem > 48 * 1024) {  // 7x7: 49 KB and more
@@ -295,10 +312,16 @@ int dw_launch(int mode, DwArgs a, int S, cudaStream_t st) {
 }
 }  // namespace
 
-// mode 0: y = conv(x, w);  1: y = dx from x = dy;  2: dw (fp32, added to) from x and dy.  x: [N, H, W, C], dy: [N, OH, OW, C], w: [K, K, C]; C a multiple
-// of 8, 16-byte aligned bases.  (pt, pl): rows and columns of zeros in front of the input.
-KB_API int kb200_depthwise(int mode, const void* x, const void* w, void* y, const void* dy, float* dw, int N, int H, int W, int C, int OH, int OW, int K, int S,
-                           int pt, int pl, cudaStream_t stream) {
+// Partial sums of a weight gradient: the first dimension of `partial` below.
+KB_API int kb200_depthwise_slabs(int N, int OH, int OW, int C, int K) {
+  return N <= 0 || OH <= 0 || OW <= 0 || C < 8 || K <= 0 ? 0 : (int)wgrad_grid(N, OH, OW, C, K).grid.x;
+}
+
+// mode 0: y = conv(x, w);  1: y = dx from x = dy;  2: dw (fp32) from x and dy, added to what dw holds where `accumulate`; partial: scratch, fp32
+// [kb200_depthwise_slabs, K, K, C].  x: [N, H, W, C], dy: [N, OH, OW, C], w: [K, K, C]; C a multiple of 8, 16-byte aligned bases.
+// (pt, pl): rows and columns of zeros in front of the input.
+KB_API int kb200_depthwise(int mode, const void* x, const void* w, void* y, const void* dy, float* dw, float* partial, int accumulate, int N, int H, int W, int C,
+                           int OH, int OW, int K, int S, int pt, int pl, cudaStream_t stream) {
   if (N <= 0 || H <= 0 || W <= 0 || C <= 0 || OH <= 0 || OW <= 0) return 0;
   if ((long long)N * H * W >= (1ll << 30) || (long long)N * OH * OW >= (1ll << 30)) {
     kb200_set_error("depthwise: more than 2^30 pixels");
@@ -309,9 +332,9 @@ KB_API int kb200_depthwise(int mode, const void* x, const void* w, void* y, cons
     kb200_set_error("depthwise: 3, 5 or 7 taps, stride 1 or 2, channels a multiple of 8, 16-byte aligned tensors");
     return -2;
   }
-  DwArgs a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, (const __nv_bfloat16*)dy, dw, N, H, W, C, OH, OW, pt, pl, 0};
+  DwArgs a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, (const __nv_bfloat16*)dy, partial, N, H, W, C, OH, OW, pt, pl, 0};
   const int rc = K == 3 ? dw_launch<3>(mode, a, S, stream) : K == 5 ? dw_launch<5>(mode, a, S, stream) : dw_launch<7>(mode, a, S, stream);
   if (rc != 0) return rc;
   KB_CHECK_LAUNCH("depthwise");
-  return 0;
+  return mode == 2 ? kb200_sum_slabs(partial, dw, kb200_depthwise_slabs(N, OH, OW, C, K), K * K * C, accumulate, stream) : 0;
 }

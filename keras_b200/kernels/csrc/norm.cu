@@ -602,6 +602,14 @@ __global__ void __launch_bounds__(256) act_bwd_kernel(const __nv_bfloat16* __res
   }
 }
 
+// out[c] = sum over the rows of partial [slabs, cols], added to what out holds where `accumulate`; a fixed order
+KB_API int kb200_sum_slabs(const float* partial, float* out, int slabs, int cols, int accumulate, cudaStream_t stream) {
+  if (cols <= 0) return 0;
+  norm_partial_reduce2_kernel<<<dim3((cols + 31) / 32, 1), 1024, 0, stream>>>(partial, out, nullptr, nullptr, slabs, cols, accumulate);
+  KB_CHECK_LAUNCH("sum_slabs");
+  return 0;
+}
+
 KB_API int kb200_colsum_slabs(long long rows, int cols, int dtype) {
   const int vn = dtype == 1 ? 8 : 4;
   const int col_blocks = (cols + 32 * vn - 1) / (32 * vn);

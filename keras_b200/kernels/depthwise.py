@@ -12,10 +12,14 @@ from keras_b200.kernels import shadow
 from keras_b200.kernels.conv import _target_param
 
 
-def _launch(mode, x, w, y, dy, dw, g):
+def _launch(mode, x, w, y, dy, dw, g, accumulate=True):
     N, H, W, C, OH, OW, K, S, pt, pl = g
     i, p = kops._i, kops._p
-    code = kops._lib().kb200_depthwise(i(mode), p(x), p(w), p(y), p(dy), p(dw), i(N), i(H), i(W), i(C), i(OH), i(OW), i(K), i(S), i(pt), i(pl), kops._stream())
+    lib, partial = kops._lib(), None
+    if mode == 2:
+        partial = torch.empty((lib.kb200_depthwise_slabs(i(N), i(OH), i(OW), i(C), i(K)), K * K * C), dtype=torch.float32, device=x.device)
+    code = lib.kb200_depthwise(i(mode), p(x), p(w), p(y), p(dy), p(dw), p(partial), i(1 if accumulate else 0), i(N), i(H), i(W), i(C), i(OH), i(OW), i(K),
+                               i(S), i(pt), i(pl), kops._stream())
     kops._check(code, "depthwise")
 
 
@@ -58,8 +62,8 @@ class DepthwiseFn(torch.autograd.Function):
             _launch(1, dy, _aligned(w), dx, None, None, g)
         if ctx.needs_input_grad[1]:
             slot = shadow.grad_slot(ctx.grad_target, w.shape)
-            buf = slot if slot is not None else torch.zeros(w.shape, dtype=torch.float32, device=dy.device)
-            _launch(2, _aligned(x), None, None, dy, buf, g)
+            buf = slot if slot is not None else torch.empty(w.shape, dtype=torch.float32, device=dy.device)
+            _launch(2, _aligned(x), None, None, dy, buf, g, accumulate=slot is not None)
             dw = buf.to(w.dtype) if slot is None else None  # already inside the parameter's gradient
         return dx, dw, None, None
 

@@ -492,6 +492,28 @@ def test_depthwise_convolution_and_gradients_against_64_bits(K, S, padding, N, H
     assert rel(y, want) < 2.0 ** -8 and rel(x.grad, xe.grad) < 2.0 ** -8 and rel(w.grad, we.grad) < 2.0 ** -8
 
 
+@pytest.mark.parametrize("K,S,N,H,C", [(3, 1, 64, 28, 192), (3, 2, 32, 57, 144), (5, 1, 16, 28, 8), (7, 2, 8, 30, 520), (3, 1, 40, 28, 64)])
+def test_depthwise_weight_gradient_repeats_and_adds(K, S, N, H, C):
+    from keras_b200.kernels import depthwise as dw
+
+    g = torch.Generator(device="cuda").manual_seed(C)
+    OH = -(-H // S)
+    geometry = (N, H, H, C, OH, OH, K, S) + (max((OH - 1) * S + K - H, 0) // 2,) * 2
+    x, dy = (torch.randn((N, n, n, C), generator=g, device="cuda").bfloat16() for n in (H, OH))
+    first, again = (torch.full((K, K, C, 1), float("nan"), device="cuda") for _ in range(2))
+    dw._launch(2, x, None, None, dy, first, geometry, accumulate=False)
+    for _ in range(8):
+        dw._launch(2, x, None, None, dy, again, geometry, accumulate=False)
+        assert torch.equal(first, again)
+    total = torch.ones((K, K, C, 1), device="cuda")
+    dw._launch(2, x, None, None, dy, total, geometry)
+    assert torch.equal(total, first + 1)
+    w = torch.zeros((K, K, C, 1), dtype=torch.double, device="cuda", requires_grad=True)
+    dw._composed(x.double(), w, geometry).backward(dy.double())
+    # sums of N * OH * OW products in fp32
+    assert ((first.double() - w.grad).norm() / w.grad.norm()).item() < 1e-5
+
+
 def test_depthwise_routes():
     import keras_b200 as keras
     from keras_b200.kernels import depthwise as dw
