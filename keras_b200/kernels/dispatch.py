@@ -69,16 +69,21 @@ def _i8_owner(t):
     return t if t._base is None else t._base
 
 
+def _i8_key(t):
+    # by stream too: what one stream is still making is not there yet for another, which makes its own
+    return t.data_ptr(), torch._C._cuda_getCurrentRawStream(t.device.index)
+
+
 def _i8_kept(cache, t):
     """What was made from ``t`` while the tensor that owns its memory lives and is unchanged; an address alone may be another's by now."""
-    entry = cache.get(t.data_ptr())
+    entry = cache.get(_i8_key(t))
     return entry[2] if entry is not None and entry[0]() is _i8_owner(t) and entry[1] == (t._version, t.stride()) else None
 
 
 def _i8_keep(cache, t, made):
     if len(cache) > 256:
         cache.clear()
-    cache[t.data_ptr()] = (weakref.ref(_i8_owner(t)), (t._version, t.stride()), made)
+    cache[_i8_key(t)] = (weakref.ref(_i8_owner(t)), (t._version, t.stride()), made)
 
 
 def _i8_operands(kernel, kernel_scale):

@@ -1082,6 +1082,31 @@ def test_int8_operands_are_not_taken_for_those_of_a_freed_kernel():
     raise AssertionError("no kernel took the place of another one")
 
 
+def test_int8_operands_of_two_streams():
+    """What is laid out for a kernel on one stream, behind other work, is not yet there for a second one."""
+    from keras_b200.kernels import dispatch
+
+    x = torch.randint(-127, 128, (64, 512), device="cuda", dtype=torch.int8)
+    kernel = torch.randint(-127, 128, (512, 1024), device="cuda", dtype=torch.int8)
+    one, scale = torch.ones((64, 1), device="cuda"), torch.rand(1024, device="cuda") + 0.5
+    want = (x.double() @ kernel.double()) / scale.double()
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    dispatch.int8_matmul(x, kernel.clone(), one, scale.clone(), out_dtype=torch.float32)  # all kernels are loaded
+    with torch.cuda.stream(first):
+        torch.cuda._sleep(1)
+        torch.full((1 << 22,), 77, device="cuda", dtype=torch.int8)  # leaves something else in the memory that is handed out next
+    torch.cuda.synchronize()
+    outs = []
+    for stream in (first, second):
+        with torch.cuda.stream(stream):
+            if stream is first:
+                torch.cuda._sleep(200_000_000)  # a tenth of a second
+            outs.append(dispatch.int8_matmul(x, kernel, one, scale, out_dtype=torch.float32))
+    torch.cuda.synchronize()
+    for out in outs:
+        assert torch.allclose(out.double(), want, rtol=1e-6, atol=1e-3)
+
+
 @pytest.mark.parametrize("n", [8, 4096, 8 * 148 * 16 * 256 * 2 + 8, 999])
 def test_copy_and_cast(n):
     from keras_b200.kernels import ops as kops
