@@ -20,6 +20,9 @@
 // 73 us (351 TFLOP/s), 2 x 4096 x 32/8 x 128 2060 -> 246 us (1115), 64 x 128 x 16 x 128 100 -> 32 us.  Two threads a row (576
 // threads, 96 registers) ran at 107 / 451 us: spills; 168 registers a thread without the hand-over at 82 / 269.
 //
+// Two tiles of rows in turn, rescaling only when it matters and a share of the exponentials as a polynomial are published ideas: FlashAttention-3
+// (Shah et al., 2024) and the descriptions of FlashAttention-4 (2025).  The code and its constants are this file's own.
+//
 // A mask (bytes, non-zero = attend) is turned into 128 bits a row with coalesced byte loads and ballots, so any stride and alignment
 // of its rows will do.  Masked scores become a large finite negative: a row with every key masked attends uniformly
 // (keras/src/backend/torch/nn.py:1539).
@@ -112,7 +115,8 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 
 // 2^x of two values on the FMA pipe, for the share of the exponentials that the special-function pipe has no time for.
 // x = n + f with n the nearest integer (the sum with 1.5 * 2^23 leaves n in the low bits), 2^f on [-1/2, 1/2] by a polynomial of
-// degree 5 fitted to the least relative error (2.1e-7, as the hardware's own approximation), n added to the exponent.  x is at
+// degree 5 with the least maximum relative error (a linear program over 4000 Chebyshev points gives its coefficients, rounded to float32;
+// 2.1e-7 in float32, as the hardware's own approximation), n added to the exponent.  x is at
 // most RESCALE_LOG2; below -126 the result is held at 2^-126, which is nothing beside a row sum of at least 2^-8.
 __device__ __forceinline__ void exp2_poly2(uint64_t x2, float& y0, float& y1) {
   float x0, x1;

@@ -134,8 +134,9 @@ __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { retu
 
 // Cumulative distribution function of the normal distribution, Phi(v) = erfc(-v / sqrt(2)) / 2, for the exact GELU and its derivative.
 // With a = |v| and t = 1 / (1 + 0.35 a):  Phi(-a) = t * 2^(p(t) - a^2 log2(e) / 2), where p is the polynomial of degree 7 that fits
-// log2(Phi(-a) e^(a^2/2) / t) on 0 <= a <= 14 with the least maximum error (5.6e-7 relative; 2.5e-6 for a < 6 in float32, where
-// the exponent's rounding is most of it).  Sixteen instructions, two of them on the special-function pipe; 1 + erf(v / sqrt(2))
+// log2(Phi(-a) e^(a^2/2) / t) on 0 <= a <= 14 with the least maximum error (a linear program over 6000 Chebyshev points gives its
+// coefficients; 6e-7 relative, in float32 9e-7 for a < 1 and 2.5e-6 for a < 6, where the exponent's rounding is most of it).  For results
+// that are rounded to bf16; those stored as float32 take erff where it is nearer (gemm_sm100.cuh).  Sixteen instructions, two of them on the special-function pipe; 1 + erf(v / sqrt(2))
 // takes twice as many and loses its relative accuracy for negative v.  [16384, 3072, 768] with gelu in the epilogue: 117 -> 94 us.
 __device__ __forceinline__ float normal_cdf(float v) {
   const float a = fabsf(v), t = __fdividef(1.f, fmaf(0.35f, a, 1.f)), x = a * 0.8493218002880191f;  // x^2 = a^2 log2(e) / 2

@@ -1,7 +1,7 @@
 // Matrices whose width is no multiple of 8 (a 50257-word vocabulary) against the GEMM's rows of 16-byte pitch: zero-padding a bf16
 // matrix, and adding a padded bf16 gradient to the fp32 matrix it belongs to; and the copy of a batch with its rounding.  Both are bound by their traffic; the library's kernels
 // for them fall back to scalar indexing because one side's rows start at odd addresses.
-// [768, 50257]: pad 116 (fill and copy) -> 41 us, add 164 -> 83 us; the traffic takes 23 and 58 us.
+// [768, 50257]: pad 109 (fill and copy) -> 33 us, add 148 -> 65 us; the traffic takes 23 and 58 us.
 #include "common.cuh"
 
 namespace {

@@ -90,7 +90,7 @@ def depthwise(x, kernel, strides, padding, data_format, dilation, variable=None)
         return None
     if sh == 1 and K == 3 and not (torch.is_grad_enabled() and (x.requires_grad or kernel.requires_grad)):
         # the forward pass alone: without a stride nothing is padded or re-laid, and the library's 3x3 kernel takes 0.86 of this one's
-        # time (28x28x192 31 us against 35; 5x5 67 / 61, 7x7 at 56x56x96 115 / 109); with gradients these kernels take 0.6 of its
+        # time (28x28x192 31 us against 35; 5x5 66 / 61, 7x7 at 56x56x96 115 / 109); with gradients these kernels take 0.6 of its
         return None
     target = _target_param(variable, kernel) if variable is not None and kernel.is_contiguous() else None
     return DepthwiseFn.apply(x, kernel, (N, H, W, C, OH, OW, K, sh, pt, pl), target)

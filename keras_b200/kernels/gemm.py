@@ -200,9 +200,10 @@ def _qualifies(x2, w):
         return False
     M, K = x2.shape
     N = w.shape[1]
-    # Rows may be any number: the copies clip them.  Below a tile of them the library's small-batch kernels are quicker (77 x 3072 x
-    # 768: 4 us against 10) where it has aligned ones; a width that is no multiple of 8 sends it to kernels of three generations ago
-    # (77 x 50257 x 768 100 us).
+    # Rows may be any number: the copies clip them.  Up to a tile of them the library's small-batch kernels take half of this one's time
+    # ([77, 3072, 768] 6.0 us against 13.2, [77, 768, 3072] 3.6 / 6.2, [77, 768, 50264] 12 / 20; 72 to 128 rows the same), and row counts that
+    # are no multiple of 8 go to them; multiples of 8 do not, a line that time did not draw.  A width that is no multiple of 8 would send
+    # the library to kernels of three generations ago ([77, 768, 50257] 100 us): those stay here.
     if K % 8 or (M % 8 and M < 128 and N % 8 == 0):
         return False
     if N % 8 and N < 256 and (N < 16 or M < 8192):
