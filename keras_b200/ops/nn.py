@@ -674,6 +674,12 @@ def _attention_mask_bias(mask, dtype):
     return torch.where(mask, torch.zeros((), dtype=dtype, device=mask.device), torch.full((), -0.7 * torch.finfo(dtype).max, dtype=dtype, device=mask.device))
 
 
+def _whole_rows(t, T, S):
+    """A mask or bias with every row and key of its own: the library's fused kernels read it as vectors along the keys, so a stride of zero
+    or one row's worth of memory there is not theirs to be given."""
+    return t.expand(torch.broadcast_shapes(t.shape, (T, S)))
+
+
 @op("nn")
 def dot_product_attention(query, key, value, bias=None, mask=None, scale=None, is_causal=False, flash_attention=None, attn_logits_soft_cap=None):
     """Inputs are ``[B, T, N, H]`` / ``[B, S, K, H]`` (K divides N: grouped-query)."""
@@ -719,14 +725,14 @@ def dot_product_attention(query, key, value, bias=None, mask=None, scale=None, i
         # probabilities from a log-sum that the negative has swallowed, take each for one.
         empty = ~attn_mask.any(dim=-1, keepdim=True)
         qh = torch.where(empty, torch.zeros((), dtype=d, device=q.device), qh)
-        attn_mask = attn_mask | empty
+        attn_mask = _whole_rows(attn_mask | empty, T, S)
     if bias is not None:
-        b = _t(bias).to(d)
+        b = _whole_rows(_t(bias).to(d), T, S)
         if attn_mask is not None:
             b = torch.where(empty, torch.zeros((), dtype=d, device=b.device), b) + _attention_mask_bias(attn_mask, d)
-        attn_mask = b
+        attn_mask = b.contiguous()
     elif attn_mask is not None:
-        attn_mask = _attention_mask_bias(attn_mask, d)
+        attn_mask = _attention_mask_bias(attn_mask, d).contiguous()
     out = F.scaled_dot_product_attention(qh, kh, vh, attn_mask=attn_mask, is_causal=is_causal and attn_mask is None, scale=scale, enable_gqa=(K != N))
     return out.transpose(1, 2)
 

@@ -261,6 +261,41 @@ def test_attention_of_rows_without_a_key_is_uniform_in_training_too(dtype, causa
     _uniform_rows(keras, dtype, causal, biased, "cuda")
 
 
+def _broadcast_masks(keras, dtype, device, T, S, H, D):
+    """Masks and biases of one column, one row or one head, with and without gradients, against 64 bits."""
+    g = torch.Generator(device=device).manual_seed(T * S)
+    q = torch.randn((3, T, H, D), generator=g, device=device).to(dtype)
+    k, v = (torch.randn((3, S, H, D), generator=g, device=device).to(dtype) for _ in range(2))
+    for shape in ((3, 1, T, 1), (3, 1, 1, S), (1, 1, T, 1), (T, 1), (1, 1, 1, 1), (3, H, 1, S)):
+        for kind in ("mask", "bias"):
+            t = torch.randn(shape, generator=g, device=device)
+            given = t > -0.5 if kind == "mask" else t.to(dtype)
+            s = torch.matmul(q.double().transpose(1, 2), k.double().permute(0, 2, 3, 1)) * D ** -0.5
+            if kind == "mask":
+                empty = ~given.expand(torch.broadcast_shapes(given.shape, (T, S))).any(-1, keepdim=True)
+                s = s.masked_fill(~given, -1e30).masked_fill(empty, 0.0)
+            else:
+                s = s + given.double()
+            want = torch.matmul(torch.softmax(s, -1), v.double().transpose(1, 2)).transpose(1, 2)
+            with torch.no_grad():
+                outs = [keras.ops.dot_product_attention(q, k, v, **{kind: given})]
+            args = [x.clone().requires_grad_(True) for x in (q, k, v)]
+            outs.append(keras.ops.dot_product_attention(*args, **{kind: given}))
+            outs[-1].backward(torch.ones_like(outs[-1]))
+            bound = {torch.bfloat16: 2.0 ** -6, torch.float16: 2.0 ** -9, torch.float32: 1e-5}[dtype]
+            for out in outs:
+                assert ((out.double() - want).norm() / want.norm()).item() < bound, (shape, kind)
+            assert all(a.grad.isfinite().all() for a in args)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("T,S,H,D", [(16, 12, 1, 32), (254, 284, 2, 64), (181, 181, 4, 32), (40, 64, 2, 40)])
+def test_attention_under_broadcast_masks_and_biases(dtype, T, S, H, D):
+    import keras_b200 as keras
+
+    _broadcast_masks(keras, dtype, "cuda", T, S, H, D)
+
+
 def test_attention_keeps_a_nan_to_the_rows_that_see_it():
     from keras_b200.kernels import attention
 

@@ -122,3 +122,21 @@ def test_attention_of_rows_without_a_key_is_uniform_and_has_its_gradients(causal
     from tests.test_gpu_hot_paths import _uniform_rows
 
     _uniform_rows(keras, torch.float32, causal, biased, "cpu")
+
+
+def test_attention_under_broadcast_masks_and_biases():
+    from tests.test_gpu_hot_paths import _broadcast_masks
+
+    for shape in ((16, 12, 1, 32), (7, 9, 2, 8)):
+        _broadcast_masks(keras, torch.float32, "cpu", *shape)
+
+
+def test_masks_and_biases_reach_the_library_whole(monkeypatch):
+    seen, plain = [], torch.nn.functional.scaled_dot_product_attention
+    monkeypatch.setattr(torch.nn.functional, "scaled_dot_product_attention", lambda *a, **k: seen.append(k["attn_mask"]) or plain(*a, **k))
+    q, k = torch.randn(2, 5, 3, 8), torch.randn(2, 7, 3, 8)
+    for t in (torch.ones(2, 1, 5, 1), torch.ones(1, 1, 1, 7), torch.ones(5, 1), torch.ones(7), torch.ones(2, 3, 5, 7)):
+        keras.ops.dot_product_attention(q, k, k, mask=t.bool())
+        keras.ops.dot_product_attention(q, k, k, bias=t)
+        keras.ops.dot_product_attention(q, k, k, mask=t.bool(), bias=torch.ones(1, 3, 5, 1))
+    assert len(seen) == 15 and all(tuple(m.shape[-2:]) == (5, 7) and m.is_contiguous() for m in seen)
