@@ -132,7 +132,7 @@ class ConvFn(torch.autograd.Function):
         N, H, W, Cin, Cout, Ho, Wo = g.N, g.H, g.W, g.Cin, g.Cout, g.Ho, g.Wo
         if dy.dtype != torch.bfloat16:
             dy = dy.to(torch.bfloat16)
-        dy = dy.contiguous()
+        dy = kops.aligned(dy)
         dx = dw = None
         one = g.R == 1 and g.S == 1
         if ctx.needs_input_grad[0]:

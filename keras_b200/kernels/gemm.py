@@ -154,8 +154,7 @@ class GemmFn(torch.autograd.Function):
         N, Np = ctx.n, w.shape[1]
         sums = bias_slot = None
         if ctx.act:
-            dy = dy.contiguous()
-            dy = dy if dy.data_ptr() % 16 == 0 else dy.clone()
+            dy = kops.aligned(dy)
             wanted = ctx.has_bias and ctx.needs_input_grad[2]
             bias_slot = shadow.grad_slot(ctx.bias_target, (N,)) if wanted else None
             dy, sums = kops.activation_backward(dy, pre, ctx.act, wanted, bias_slot.view(N) if bias_slot is not None else None)
@@ -171,7 +170,7 @@ class GemmFn(torch.autograd.Function):
                 wide_dy[:, N:].zero_()
                 dy = wide_dy
         elif not _ok_2d(dy):
-            dy = dy.contiguous()
+            dy = kops.aligned(dy)
         dx = dw = db = None
         if ctx.needs_input_grad[0]:
             dx = gemm(dy, w, 0, 0, M, K, N)  # the sum ends at N; below, the columns behind it stay columns of their own

@@ -85,13 +85,20 @@ def _check(code, what):
 
 
 # ------------------------------------------------------------------------------ max pooling
+def aligned(t):
+    """Contiguous and 16-byte aligned, as kernels that read whole vectors need it: a contiguous view may start anywhere (the gradient of a
+    concatenation of flattened tensors)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class FusedMaxPool2D(torch.autograd.Function):
     """Channels-last 2-D max pooling with the padding folded in (``pad_mode`` 1: zeros, 0: ignored)."""
 
     @staticmethod
     def forward(ctx, x, pool, strides, pads, out_hw, pad_mode):
         lib = _lib()
-        x = x.contiguous()
+        x = aligned(x)
         N, H, W, C = x.shape
         OH, OW = out_hw
         y = torch.empty((N, OH, OW, C), dtype=x.dtype, device=x.device)
@@ -107,7 +114,7 @@ class FusedMaxPool2D(torch.autograd.Function):
         lib = _lib()
         (idx,) = ctx.saved_tensors
         N, H, W, C, OH, OW, pool, strides, pads, dt = ctx.geom
-        dy = dy.contiguous()
+        dy = aligned(dy)
         dx = torch.empty((N, H, W, C), dtype=dy.dtype, device=dy.device)
         _check(lib.kb200_maxpool2d_bwd(_p(dy), _p(idx), _p(dx), _i(N), _i(H), _i(W), _i(C), _i(OH), _i(OW), _i(pool[0]), _i(pool[1]), _i(strides[0]),
                                        _i(strides[1]), _i(pads[0]), _i(pads[1]), _i(dt), _stream()), "maxpool_bwd")
@@ -121,7 +128,7 @@ class FusedAvgPool2D(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, pool, strides, pads, out_hw):
         lib = _lib()
-        x = x.contiguous()
+        x = aligned(x)
         N, H, W, C = x.shape
         OH, OW = out_hw
         y = torch.empty((N, OH, OW, C), dtype=x.dtype, device=x.device)
@@ -134,7 +141,7 @@ class FusedAvgPool2D(torch.autograd.Function):
     def backward(ctx, dy):
         lib = _lib()
         N, H, W, C, OH, OW, pool, strides, pads = ctx.geom
-        dy = dy.contiguous()
+        dy = aligned(dy)
         dx = torch.empty((N, H, W, C), dtype=dy.dtype, device=dy.device)
         _check(lib.kb200_avgpool2d_bwd(_p(dy), _p(dx), _i(N), _i(H), _i(W), _i(C), _i(OH), _i(OW), _i(pool[0]), _i(pool[1]), _i(strides[0]), _i(strides[1]),
                                        _i(pads[0]), _i(pads[1]), _i(_dt(dy)), _stream()), "avgpool_bwd")
@@ -147,7 +154,7 @@ class FusedGlobalAvgPool(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x):
         lib = _lib()
-        x = x.contiguous()
+        x = aligned(x)
         N, C = x.shape[0], x.shape[-1]
         P = x.numel() // (N * C)
         y = torch.empty((N, C), dtype=x.dtype, device=x.device)
@@ -163,7 +170,7 @@ class FusedGlobalAvgPool(torch.autograd.Function):
         P = 1
         for d in shape[1:-1]:
             P *= d
-        dy = dy.contiguous()
+        dy = aligned(dy)
         dx = torch.empty(shape, dtype=dy.dtype, device=dy.device)
         _check(lib.kb200_global_avgpool_bwd(_p(dy), _p(dx), _i(N), _i(P), _i(C), _i(_dt(dy)), _stream()), "global_avgpool_bwd")
         return dx
@@ -213,8 +220,7 @@ class FusedEmbedding(torch.autograd.Function):
         ids64 = ids.reshape(-1).to(torch.int64).contiguous()
         n = ids64.numel()
         src = table.detach()
-        if not src.is_contiguous():
-            src = src.contiguous()
+        src = aligned(src)
         out = torch.empty((n, D), dtype=out_dtype, device=table.device)
         _check(lib.kb200_embedding_fwd(_p(src), _p(ids64), _p(out), _ll(n), _i(D), _ll(V), _i(_dt(src)), _i(_dt(out)), _stream()), "embedding_fwd")
         ctx.save_for_backward(ids64)
@@ -233,7 +239,7 @@ class FusedEmbedding(torch.autograd.Function):
         V, D = ctx.table_shape
         if dout.dtype not in (torch.float32, torch.bfloat16):
             dout = dout.float()
-        dout = dout.reshape(-1, D).contiguous()
+        dout = aligned(dout.reshape(-1, D))
         slot = shadow.grad_slot(ctx.target, (V, D))
         acc = slot.view(V, D) if slot is not None else torch.zeros((V, D), dtype=torch.float32, device=dout.device)
         _check(lib.kb200_embedding_bwd(_p(dout), _p(ids64), _p(acc), _ll(ids64.numel()), _i(D), _ll(V), _i(_dt(dout)), _stream()), "embedding_bwd")
@@ -276,7 +282,7 @@ class FusedBatchNormAct(torch.autograd.Function):
         lib = _lib()
         C = x.shape[-1]
         M = x.numel() // C
-        x = x.contiguous()
+        x = aligned(x)
         dev = x.device
         stats = torch.empty(4 * C, dtype=torch.float32, device=dev)
         mean, invstd, scale, shift = stats[:C], stats[C:2 * C], stats[2 * C:3 * C], stats[3 * C:]
@@ -294,7 +300,7 @@ class FusedBatchNormAct(torch.autograd.Function):
             _check(lib.kb200_bn_stats(_p(x), _ll(M), _i(C), _i(dt), _p(sums), st), "bn_stats")
             _check(lib.kb200_bn_finalize(_p(sums), _p(gamma), _p(beta), _p(pre_bias), _p(moving_mean), _p(moving_var), _f(momentum), _f(eps), _ll(M), _i(C),
                                          _p(mean), _p(invstd), _p(scale), _p(shift), st), "bn_finalize")
-        res = residual.contiguous() if residual is not None else None
+        res = aligned(residual) if residual is not None else None
         bits = None
         if relu:
             bits = torch.empty(M * (C // (8 if dt == 1 else 4)), dtype=torch.uint8, device=dev)
@@ -321,7 +327,7 @@ class FusedBatchNormAct(torch.autograd.Function):
         x, bits, gamma, stats = ctx.saved_tensors
         M, C = ctx.dims
         mean, invstd = stats[:C], stats[C:2 * C]
-        dy = dy.contiguous()
+        dy = aligned(dy)
         dev = x.device
         sums = torch.empty(5 * C, dtype=torch.float32, device=dev)
         coef = sums[2 * C:]
@@ -355,12 +361,12 @@ def bn_inference(x, scale, shift, residual, relu, cap=None):
     lib = _lib()
     C = x.shape[-1]
     M = x.numel() // C
-    x = x.contiguous()
+    x = aligned(x)
     y = torch.empty_like(x)
     if cap is not None:
         _check(lib.kb200_bn_apply_cap(_p(x), _p(y), _vp(0), _p(scale), _p(shift), _ll(M), _i(C), _f(cap), _i(_dt(x)), _stream()), "bn_apply")
         return y
-    res = residual.contiguous() if residual is not None else None
+    res = aligned(residual) if residual is not None else None
     _check(lib.kb200_bn_apply(_p(x), _p(res), _p(y), _p(scale), _p(shift), _ll(M), _i(C), _i(1 if relu else 0), _i(_dt(x)), _stream()), "bn_apply")
     return y
 

@@ -1117,6 +1117,51 @@ def test_int8_operands_are_not_taken_for_those_of_a_freed_kernel():
     raise AssertionError("no kernel took the place of another one")
 
 
+def _anywhere(t):
+    """The same values in a contiguous tensor that starts one element behind a 16-byte line."""
+    return torch.cat([t.new_zeros(1), t.detach().reshape(-1)])[1:].reshape(t.shape)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_layers_take_tensors_and_gradients_that_start_anywhere(dtype):
+    """The gradient of a concatenation of flattened tensors is contiguous and starts where the one before ends."""
+    import keras_b200 as keras
+    from keras_b200.kernels import ops as kops
+
+    L = keras.layers
+    name = "float32" if dtype == torch.float32 else "mixed_bfloat16"
+    g = torch.Generator(device="cuda").manual_seed(3)
+    ones, zeros = torch.ones(64, device="cuda"), torch.zeros(64, device="cuda")
+
+    def norm(x, res=None, cap=None):
+        return kops.FusedBatchNormAct.apply(x, ones, zeros, res, zeros.clone(), ones.clone(), 0.9, 1e-3, True, None, None, None, cap)
+
+    calls = {"norm + relu": lambda x: norm(x), "norm + relu6": lambda x: norm(x, cap=6.0), "norm + sum": lambda x: norm(x, x)}
+    layers = {"max": L.MaxPooling2D(2), "average": L.AveragePooling2D(2), "global": L.GlobalAveragePooling2D(), "conv": L.Conv2D(64, 3), "dense": L.Dense(128),
+              "dense + gelu": L.Dense(128, activation="gelu"), "depthwise": L.DepthwiseConv2D(3, strides=2), "layer norm": L.LayerNormalization()}
+    for key, layer in layers.items():
+        layer.dtype_policy = keras.dtype_policies.get(name)
+        calls[key] = layer
+    for key, call in calls.items():
+        x = torch.randn((4, 16, 16, 64), generator=g, device="cuda").to(dtype)
+        results = []
+        for place in (lambda t: t, _anywhere):
+            xi = place(x).requires_grad_(True)
+            assert place is not _anywhere or xi.data_ptr() % 16
+            y = call(xi)
+            dy = torch.randn(y.shape, generator=torch.Generator(device="cuda").manual_seed(4), device="cuda").to(y.dtype)
+            (dx,) = torch.autograd.grad(y, xi, place(dy))
+            results.append((y.detach(), dx))
+        for a, b in zip(*results):
+            assert ((a.float() - b.float()).norm() / a.float().norm()).item() < 2.0 ** -7, key  # an unaligned one may run in the library
+    out = kops.bn_inference(_anywhere(x), ones, zeros, _anywhere(x), True)
+    assert torch.equal(out, torch.relu(x.float() * 1 + x.float()).to(dtype))
+    table, ids = torch.randn((33, 64), generator=g, device="cuda"), torch.randint(0, 33, (40,), generator=g, device="cuda")
+    rows = kops.FusedEmbedding.apply(_anywhere(table).requires_grad_(True), ids, torch.float32, None)
+    assert torch.equal(rows, table[ids])
+    rows.backward(_anywhere(torch.ones_like(rows)))
+
+
 def test_int8_operands_of_two_streams():
     """What is laid out for a kernel on one stream, behind other work, is not yet there for a second one."""
     from keras_b200.kernels import dispatch
