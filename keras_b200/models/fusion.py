@@ -295,6 +295,9 @@ def run_bn(layer, x, training, residual=None, relu=False, pre_bias=None, stats=N
         x, stats = x.to(td), None
     if residual is not None and residual.dtype != td and residual.dtype.is_floating_point:
         residual = residual.to(td)
+    if residual is not None and residual.shape != x.shape:  # the kernel adds element to element: a broadcast sum is made outside
+        out = run_bn(layer, x, training, pre_bias=pre_bias, stats=stats) + residual
+        return torch.relu(out) if relu else out
     bias_value = pre_bias._value if pre_bias is not None else None
     out = dispatch.batch_norm(layer, x, train, residual=residual, relu=relu, pre_bias=bias_value, conv_stats=stats, cap=cap)
     if out is not None:

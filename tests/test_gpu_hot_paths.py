@@ -764,6 +764,26 @@ def test_folded_chains_answer_as_their_layers_do(policy, training):
             assert torch.allclose(a, v.value, rtol=step, atol=step), name
 
 
+@pytest.mark.parametrize("rows", [(8, 1), (1, 8)])
+@pytest.mark.parametrize("training", [False, True])
+def test_a_sum_behind_a_norm_broadcasts(rows, training):
+    """Two inputs of declared equal shapes and different batches: the kernel's element by element sum would read behind the smaller one."""
+    import keras_b200 as keras
+
+    L = keras.layers
+    a, b = keras.Input((6, 6, 16)), keras.Input((6, 6, 16))
+    model = keras.Model([a, b], L.ReLU()(L.Add()([L.BatchNormalization()(L.Conv2D(16, 1)(a)), b])))
+    xa, xb = (torch.randn((n, 6, 6, 16), device="cuda") for n in rows)
+    conv, norm = (next(layer for layer in model.layers if isinstance(layer, t)) for t in (L.Conv2D, L.BatchNormalization))
+    state = [v.value.clone() for v in norm.weights]
+    with torch.no_grad():
+        got = model([xa, xb], training=training)
+        for v, s in zip(norm.weights, state):
+            v.assign(s)
+        want = torch.relu(norm(conv(xa), training=training) + xb)
+    assert got.shape == want.shape and torch.allclose(got, want, atol=1e-5, rtol=1e-5)
+
+
 @pytest.mark.parametrize("relu,res", [(True, True), (True, False), (False, False)])
 @pytest.mark.parametrize("rows,C", [(20011, 144), (15003, 192), (70001, 48), (3001, 960), (9001, 320), (2200, 1000), (600, 4096), (30, 24)])
 def test_batch_norm_at_channel_counts_that_are_no_power_of_two(rows, C, relu, res):
