@@ -715,11 +715,12 @@ def dot_product_attention(query, key, value, bias=None, mask=None, scale=None, i
         probs = torch.softmax(logits.float(), dim=-1).to(d)
         return torch.matmul(probs, vh).transpose(1, 2)
     attn_mask = None
-    if mask is not None:
-        attn_mask = _t(mask).to(torch.bool)
+    if mask is not None or (bias is not None and is_causal):  # the library takes a mask or a causal one, not both
         if is_causal:
-            attn_mask = attn_mask & torch.ones((T, S), dtype=torch.bool, device=q.device).tril()
-            is_causal = False
+            causal = torch.ones((T, S), dtype=torch.bool, device=q.device).tril()
+            attn_mask = causal if mask is None else _t(mask).to(torch.bool) & causal
+        else:
+            attn_mask = _t(mask).to(torch.bool)
         # A row with every position masked attends uniformly (keras/src/backend/torch/nn.py:1539): a query of zeros that sees them all.  Left to
         # the large negative below, the library's kernels overflow to zeros on the GPU, and their backward passes, which recompute the
         # probabilities from a log-sum that the negative has swallowed, take each for one.

@@ -140,3 +140,18 @@ def test_masks_and_biases_reach_the_library_whole(monkeypatch):
         keras.ops.dot_product_attention(q, k, k, bias=t)
         keras.ops.dot_product_attention(q, k, k, mask=t.bool(), bias=torch.ones(1, 3, 5, 1))
     assert len(seen) == 15 and all(tuple(m.shape[-2:]) == (5, 7) and m.is_contiguous() for m in seen)
+
+
+@pytest.mark.parametrize("masked", [False, True])
+def test_causal_attention_under_a_bias_stays_causal(masked):
+    g = torch.Generator().manual_seed(1)
+    q, k, v = (torch.randn((2, 6, 3, 8), generator=g) for _ in range(3))
+    bias = torch.randn((3, 6, 6), generator=g)
+    mask = torch.rand((2, 1, 6, 6), generator=g) < 0.6 if masked else None
+    if masked:
+        mask[..., 0] = True
+    seen = torch.ones((6, 6), dtype=torch.bool).tril() & (mask if masked else True)
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) * 8 ** -0.5 + bias.double()
+    want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s.masked_fill(~seen, float("-inf")), -1), v.double())
+    out = keras.ops.dot_product_attention(q, k, v, bias=bias, mask=mask, is_causal=True)
+    assert torch.allclose(out.double(), want, atol=1e-5)
