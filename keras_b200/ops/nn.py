@@ -725,15 +725,15 @@ def dot_product_attention(query, key, value, bias=None, mask=None, scale=None, i
         # the large negative below, the library's kernels overflow to zeros on the GPU, and their backward passes, which recompute the
         # probabilities from a log-sum that the negative has swallowed, take each for one.
         empty = ~attn_mask.any(dim=-1, keepdim=True)
-        qh = torch.where(empty, torch.zeros((), dtype=d, device=q.device), qh)
-        attn_mask = _whole_rows(attn_mask | empty, T, S)
+        zero = torch.zeros((), dtype=d, device=q.device)
+        qh = torch.where(empty, zero, qh)
+        lowest = torch.where(empty, zero, torch.full((), -0.7 * torch.finfo(d).max, dtype=d, device=q.device))
+        attn_mask = torch.where(_whole_rows(attn_mask, T, S), zero, lowest)
     if bias is not None:
         b = _whole_rows(_t(bias).to(d), T, S)
-        if attn_mask is not None:
-            b = torch.where(empty, torch.zeros((), dtype=d, device=b.device), b) + _attention_mask_bias(attn_mask, d)
-        attn_mask = b.contiguous()
-    elif attn_mask is not None:
-        attn_mask = _attention_mask_bias(attn_mask, d).contiguous()
+        attn_mask = b if attn_mask is None else torch.where(empty, zero, b) + attn_mask
+    if attn_mask is not None:
+        attn_mask = attn_mask.contiguous()
     out = F.scaled_dot_product_attention(qh, kh, vh, attn_mask=attn_mask, is_causal=is_causal and attn_mask is None, scale=scale, enable_gqa=(K != N))
     return out.transpose(1, 2)
 
