@@ -83,7 +83,8 @@ __device__ __forceinline__ float row_sum(float v, float* red, int row_in_block, 
 }
 
 template <typename T, int VPL, int NT, int WPR>
-__global__ void __launch_bounds__(NT) norm_fwd_warp_kernel(const T* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
+__global__ void __launch_bounds__(NT) norm_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ res, T* __restrict__ sum_out,
+                                                           const float* __restrict__ gamma, const float* __restrict__ beta,
                                                            T* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out,
                                                            long long rows, int D, float eps, int rms) {
   constexpr int VN = NVec<T>::N;
@@ -103,6 +104,23 @@ __global__ void __launch_bounds__(NT) norm_fwd_warp_kernel(const T* __restrict__
   for (int k = 0; k < VPL; ++k) {
     const int i = t + k * 32 * WPR;
     raw[k] = i < nvec ? __ldg(xr + i) : make_uint4(0, 0, 0, 0);
+  }
+  if (res != nullptr) {  // the row is a residual sum, rounded as the addition alone would leave it
+    const uint4* rr = reinterpret_cast<const uint4*>(res + row * D);
+    uint4 more[VPL];
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) more[k] = t + k * 32 * WPR < nvec ? __ldg(rr + t + k * 32 * WPR) : make_uint4(0, 0, 0, 0);
+    uint4* so = reinterpret_cast<uint4*>(sum_out + row * D);
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) {
+      float v[VN], m[VN];
+      nv_unpack<T>(raw[k], v);
+      nv_unpack<T>(more[k], m);
+#pragma unroll
+      for (int j = 0; j < VN; ++j) v[j] += m[j];
+      raw[k] = nv_pack<T>(v);
+      if (live && t + k * 32 * WPR < nvec) so[t + k * 32 * WPR] = raw[k];
+    }
   }
   float s = 0.f;
 #pragma unroll
@@ -127,7 +145,7 @@ __global__ void __launch_bounds__(NT) norm_fwd_warp_kernel(const T* __restrict__
   if (!live) return;
   if (t == 0) {
     if (mean_out) mean_out[row] = mean;
-    rstd_out[row] = rstd;
+    if (rstd_out) rstd_out[row] = rstd;
   }
   uint4* yr = reinterpret_cast<uint4*>(y + row * D);
 #pragma unroll
@@ -150,10 +168,14 @@ __global__ void __launch_bounds__(NT) norm_fwd_warp_kernel(const T* __restrict__
   }
 }
 
-template <typename T, int VPL, int NT, int WPR>
-__global__ void __launch_bounds__(NT) norm_bwd_warp_kernel(const T* __restrict__ dy, const T* __restrict__ x, const float* __restrict__ gamma,
-                                                           const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx,
-                                                           float* __restrict__ partial_dgamma, float* __restrict__ partial_dbeta,
+// Bound by loads in flight: a warp holds a row's two or three tensors and 16 sums a vector of its columns, and the fewer registers that
+// takes the more rows an SM has on their way.  MB blocks an SM of 128 threads, and vectors that divide the row (three a lane at 768
+// columns).  With the gradient of the sum's other reader added on the way: [16384, 768] bf16 30.5 + 10.7 us apart -> 36.7, [2664, 512]
+// 8.2 + 2.0 -> 7.1 (four blocks an SM at three vectors spill: 45.6).
+template <typename T, int VPL, int NT, int WPR, int MB = 1>
+__global__ void __launch_bounds__(NT, MB) norm_bwd_warp_kernel(const T* __restrict__ dy, const T* __restrict__ x, const float* __restrict__ gamma,
+                                                           const float* __restrict__ mean, const float* __restrict__ rstd, const T* __restrict__ dres,
+                                                           T* __restrict__ dx, float* __restrict__ partial_dgamma, float* __restrict__ partial_dbeta,
                                                            long long rows, int D, int rms) {
   constexpr int VN = NVec<T>::N;
   constexpr int RPB = NT / 32 / WPR;
@@ -230,6 +252,12 @@ __global__ void __launch_bounds__(NT) norm_bwd_warp_kernel(const T* __restrict__
             const float g = gamma ? gv[j] * dv[j] : dv[j];
             dv[j] = rs * (g - m1 - xhat * m2);
           }
+          if (dres != nullptr) {  // what reaches the normalised sum on its other way
+            float ov[VN];
+            nv_unpack<T>(__ldg(reinterpret_cast<const uint4*>(dres + row * D) + i), ov);
+#pragma unroll
+            for (int j = 0; j < VN; ++j) dv[j] += ov[j];
+          }
           dxr[i] = nv_pack<T>(dv);
         }
       }
@@ -290,16 +318,19 @@ __global__ void __launch_bounds__(1024) norm_partial_reduce2_kernel(const float*
 
 // rms != 0: RMSNorm (no mean subtraction, no beta)
 template <typename T>
-__global__ void __launch_bounds__(NORM_THREADS) norm_fwd_kernel(const T* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
+__global__ void __launch_bounds__(NORM_THREADS) norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ res, T* __restrict__ sum_out, const float* __restrict__ gamma,
+                                                                const float* __restrict__ beta,
                                                                 T* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int D,
                                                                 float eps, int rms) {
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const T* xr = x + row * D;
+  auto value = [&](int i) { return res != nullptr ? to_f32<T>(from_f32<T>(to_f32<T>(xr[i]) + to_f32<T>(res[row * D + i]))) : to_f32<T>(xr[i]); };
   T* yr = y + row * D;
   float s = 0.f, ss = 0.f;
   for (int i = threadIdx.x; i < D; i += NORM_THREADS) {
-    const float v = to_f32<T>(xr[i]);
+    const float v = value(i);
+    if (res != nullptr) sum_out[row * D + i] = from_f32<T>(v);
     s += v;
     ss += v * v;
   }
@@ -310,10 +341,10 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_fwd_kernel(const T* __restr
   const float rstd = rsqrtf(var + eps);
   if (threadIdx.x == 0) {
     if (mean_out) mean_out[row] = mean;
-    rstd_out[row] = rstd;
+    if (rstd_out) rstd_out[row] = rstd;
   }
   for (int i = threadIdx.x; i < D; i += NORM_THREADS) {
-    float v = (to_f32<T>(xr[i]) - mean) * rstd;
+    float v = (value(i) - mean) * rstd;
     if (gamma) v *= gamma[i];
     if (beta) v += beta[i];
     yr[i] = from_f32<T>(v);
@@ -323,8 +354,8 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_fwd_kernel(const T* __restr
 // Each block walks rows blockIdx.x, +gridDim.x, ...; thread t owns columns t, t+256, ... (<= MAXC per thread)
 template <typename T, int MAXC>
 __global__ void __launch_bounds__(NORM_THREADS) norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const float* __restrict__ gamma,
-                                                                const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx,
-                                                                float* __restrict__ partial_dgamma, float* __restrict__ partial_dbeta,
+                                                                const float* __restrict__ mean, const float* __restrict__ rstd, const T* __restrict__ dres,
+                                                                T* __restrict__ dx, float* __restrict__ partial_dgamma, float* __restrict__ partial_dbeta,
                                                                 long long rows, int D, int rms) {
   __shared__ float red[32];
   float dg[MAXC], db[MAXC];
@@ -360,7 +391,7 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_bwd_kernel(const T* __restr
         const float xhat = (to_f32<T>(xr[i]) - mu) * rs;
         const float d = to_f32<T>(dyr[i]);
         const float g = gamma ? gamma[i] * d : d;
-        dxr[i] = from_f32<T>(rs * (g - m1 - xhat * m2));
+        dxr[i] = from_f32<T>(rs * (g - m1 - xhat * m2) + (dres != nullptr ? to_f32<T>(dres[row * D + i]) : 0.f));
       }
     }
   }
@@ -382,24 +413,28 @@ __global__ void norm_partial_reduce_kernel(const float* __restrict__ partial, fl
   out[i] = accumulate ? out[i] + s : s;
 }
 
-KB_API int kb200_norm_fwd(const void* x, const float* gamma, const float* beta, void* y, float* mean, float* rstd, long long rows, int D, float eps,
-                          int rms, int dtype, cudaStream_t stream) {
+// y = norm(x), or norm(sum) with sum = x + res where `res` is given: a block of a transformer adds its branch and normalises the sum, and
+// the sum has another reader, the next addition; one pass writes both.  [16384, 768] bf16: 10.7 + 13.5 us apart, 16.6 together.
+// mean / rstd: null where nobody takes a gradient.
+KB_API int kb200_norm_fwd(const void* x, const void* res, void* sum, const float* gamma, const float* beta, void* y, float* mean, float* rstd, long long rows, int D,
+                          float eps, int rms, int dtype, cudaStream_t stream) {
   if (rows <= 0) return 0;
   {
     const int vn = dtype == 1 ? 8 : 4;
-    const bool aligned = ((((uintptr_t)x | (uintptr_t)y | (uintptr_t)gamma | (uintptr_t)beta) & 15) == 0) && D % vn == 0;
+    const bool aligned = ((((uintptr_t)x | (uintptr_t)res | (uintptr_t)sum | (uintptr_t)y | (uintptr_t)gamma | (uintptr_t)beta) & 15) == 0) && D % vn == 0;
     const int nvec = aligned ? D / vn : 0;
     // shapes: (threads, warps per row); up to 8 vectors per thread
 #define LAUNCH_FW(T, VPL, NT, WPR)                                                                                                                \
   do {                                                                                                                                            \
     constexpr int rpb = NT / 32 / WPR;                                                                                                            \
-    norm_fwd_warp_kernel<T, VPL, NT, WPR><<<(unsigned)((rows + rpb - 1) / rpb), NT, 0, stream>>>((const T*)x, gamma, beta, (T*)y, mean, rstd,     \
+    norm_fwd_warp_kernel<T, VPL, NT, WPR><<<(unsigned)((rows + rpb - 1) / rpb), NT, 0, stream>>>((const T*)x, (const T*)res, (T*)sum, gamma, beta, (T*)y, mean, rstd, \
                                                                                                   rows, D, eps, rms);                             \
   } while (0)
 #define PICK_FW(T)                                                   \
   do {                                                               \
     if (nvec <= 32) LAUNCH_FW(T, 1, 128, 1);                         \
     else if (nvec <= 64) LAUNCH_FW(T, 2, 128, 1);                    \
+    else if (nvec <= 96) LAUNCH_FW(T, 3, 128, 1);                    \
     else if (nvec <= 128) LAUNCH_FW(T, 4, 128, 1);                   \
     else if (nvec <= 256) LAUNCH_FW(T, 2, 128, 4);                   \
     else if (nvec <= 512) LAUNCH_FW(T, 4, 128, 4);                   \
@@ -416,9 +451,9 @@ KB_API int kb200_norm_fwd(const void* x, const float* gamma, const float* beta, 
 #undef LAUNCH_FW
   }
   if (dtype == 1)
-    norm_fwd_kernel<__nv_bfloat16><<<(unsigned)rows, NORM_THREADS, 0, stream>>>((const __nv_bfloat16*)x, gamma, beta, (__nv_bfloat16*)y, mean, rstd, D, eps, rms);
+    norm_fwd_kernel<__nv_bfloat16><<<(unsigned)rows, NORM_THREADS, 0, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (__nv_bfloat16*)sum, gamma, beta, (__nv_bfloat16*)y, mean, rstd, D, eps, rms);
   else
-    norm_fwd_kernel<float><<<(unsigned)rows, NORM_THREADS, 0, stream>>>((const float*)x, gamma, beta, (float*)y, mean, rstd, D, eps, rms);
+    norm_fwd_kernel<float><<<(unsigned)rows, NORM_THREADS, 0, stream>>>((const float*)x, (const float*)res, (float*)sum, gamma, beta, (float*)y, mean, rstd, D, eps, rms);
   KB_CHECK_LAUNCH("norm_fwd");
   return 0;
 }
@@ -429,29 +464,33 @@ KB_API int kb200_norm_bwd_blocks(long long rows) {
 }
 
 // partial_dgamma / partial_dbeta: scratch [kb200_norm_bwd_blocks(rows), D] fp32; accumulate != 0: dgamma and dbeta are added to
-KB_API int kb200_norm_bwd(const void* dy, const void* x, const float* gamma, const float* mean, const float* rstd, void* dx, float* partial_dgamma,
+// `dres`: a gradient of x from elsewhere that is added to dx (of a residual sum, whose other reader is the next addition), or null.
+KB_API int kb200_norm_bwd(const void* dy, const void* x, const float* gamma, const float* mean, const float* rstd, const void* dres, void* dx, float* partial_dgamma,
                           float* partial_dbeta, float* dgamma, float* dbeta, long long rows, int D, int rms, int dtype, int accumulate,
                           cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (D > NORM_THREADS * 32) { kb200_set_error("norm_bwd: D too large (max 8192)"); return -2; }
-  const int blocks = kb200_norm_bwd_blocks(rows);
+  int blocks = kb200_norm_bwd_blocks(rows);
   {
     const int vn = dtype == 1 ? 8 : 4;
-    const bool aligned = ((((uintptr_t)x | (uintptr_t)dy | (uintptr_t)dx | (uintptr_t)gamma) & 15) == 0) && D % vn == 0;
+    const bool aligned = ((((uintptr_t)x | (uintptr_t)dy | (uintptr_t)dx | (uintptr_t)dres | (uintptr_t)gamma) & 15) == 0) && D % vn == 0;
     const int nvec = aligned ? D / vn : 0;
-#define LAUNCH_BW(T, VPL, NT, WPR)                                                                                                                 \
+#define LAUNCH_BW(T, VPL, NT, WPR, ...)                                                                                                            \
   do {                                                                                                                                             \
     const size_t smem = (size_t)(NT / 32 / WPR) * D * sizeof(float);                                                                               \
-    norm_bwd_warp_kernel<T, VPL, NT, WPR><<<blocks, NT, smem, stream>>>((const T*)dy, (const T*)x, gamma, mean, rstd, (T*)dx, partial_dgamma,      \
+    norm_bwd_warp_kernel<T, VPL, NT, WPR, ##__VA_ARGS__><<<blocks, NT, smem, stream>>>((const T*)dy, (const T*)x, gamma, mean, rstd, (const T*)dres, (T*)dx, partial_dgamma,      \
                                                                          partial_dbeta, rows, D, rms);                                             \
   } while (0)
     // per-thread accumulators: 2 x VPL x (8 or 4) floats, so at most 4 vectors per thread for bf16 and 8 for fp32
     bool done = true;
     if (dtype == 1) {
+      const int resident = (nvec > 64 ? 3 : 4) * kb_sm_count();  // what runs at once below 1024 columns: a second, shorter wave would only add partial sums
+      if (nvec >= 1 && nvec <= 96 && blocks > resident) blocks = resident;
       if (nvec < 1) done = false;
-      else if (nvec <= 32) LAUNCH_BW(__nv_bfloat16, 1, 128, 1);
-      else if (nvec <= 64) LAUNCH_BW(__nv_bfloat16, 2, 128, 1);
-      else if (nvec <= 128) LAUNCH_BW(__nv_bfloat16, 4, 128, 1);
+      else if (nvec <= 32) LAUNCH_BW(__nv_bfloat16, 1, 128, 1, 4);
+      else if (nvec <= 64) LAUNCH_BW(__nv_bfloat16, 2, 128, 1, 4);
+      else if (nvec <= 96) LAUNCH_BW(__nv_bfloat16, 3, 128, 1, 3);
+      else if (nvec <= 128) LAUNCH_BW(__nv_bfloat16, 4, 128, 1, 3);
       else if (nvec <= 256) LAUNCH_BW(__nv_bfloat16, 2, 128, 4);
       else if (nvec <= 512) LAUNCH_BW(__nv_bfloat16, 4, 128, 4);
       else if (nvec <= 1024) LAUNCH_BW(__nv_bfloat16, 4, 256, 8);
@@ -480,7 +519,7 @@ KB_API int kb200_norm_bwd(const void* dy, const void* x, const float* gamma, con
   }
   const int per = (D + NORM_THREADS - 1) / NORM_THREADS;
 #define LAUNCH(T, MAXC)                                                                                                            \
-  norm_bwd_kernel<T, MAXC><<<blocks, NORM_THREADS, 0, stream>>>((const T*)dy, (const T*)x, gamma, mean, rstd, (T*)dx, partial_dgamma, \
+  norm_bwd_kernel<T, MAXC><<<blocks, NORM_THREADS, 0, stream>>>((const T*)dy, (const T*)x, gamma, mean, rstd, (const T*)dres, (T*)dx, partial_dgamma, \
                                                                  partial_dbeta, rows, D, rms)
   if (dtype == 1) {
     if (per <= 4) LAUNCH(__nv_bfloat16, 4);

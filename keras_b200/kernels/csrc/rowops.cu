@@ -6,6 +6,8 @@
 //   pooling      keras/src/backend/torch/nn.py:361-533 (transposes to channels-first and back around the library call)
 //   resize       keras/src/backend/torch/image.py (interpolate on a permuted view)
 // All arithmetic is fp32; tensors are bf16 or fp32 (uint8 also for resize).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
@@ -228,16 +230,18 @@ KB_API int kb200_softmax_bwd(const void* y, const void* dy, void* dx, long long 
 // ------------------------------------------------------------------------------------------------ embedding
 namespace {
 
-// out[r, :] = table[ids[r], :] converted to the output type; one thread per 8 output elements.  Ids outside [0, V) give zeros.
-template <typename TT, typename TO>
-__global__ void __launch_bounds__(RO_THREADS) embedding_fwd_kernel(const TT* __restrict__ table, const long long* __restrict__ ids, TO* __restrict__ out,
-                                                                   long long n, int D, long long V) {
+// out[r, :] = table[ids[r], :] converted to the output type; one thread per 8 output elements.  Ids outside [0, V) give zeros; with `wrap`
+// negative ids count from the end of the table.
+template <typename TT, typename TO, typename TI>
+__global__ void __launch_bounds__(RO_THREADS) embedding_fwd_kernel(const TT* __restrict__ table, const TI* __restrict__ ids, TO* __restrict__ out,
+                                                                   long long n, int D, long long V, int wrap) {
   const int vpr = D >> 3;  // vectors of 8 elements per row
   const long long total = n * vpr;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
     const long long r = idx / vpr;
     const int c = (int)(idx - r * vpr) << 3;
-    const long long id = ids[r];
+    long long id = ids[r];
+    if (wrap && id < 0) id += V;
     float v[8];
     if (id >= 0 && id < V) {
       const TT* src = table + id * D + c;
@@ -296,8 +300,9 @@ inline unsigned flat_grid(long long work_items) {
 
 }  // namespace
 
-// table: [V, D] fp32 (table_dtype 0) or bf16 (1); out: [n, D] fp32 or bf16; D a multiple of 8, pointers 16-byte aligned.
-KB_API int kb200_embedding_fwd(const void* table, const long long* ids, void* out, long long n, int D, long long V, int table_dtype, int out_dtype,
+// table: [V, D] fp32 (table_dtype 0) or bf16 (1); ids: int64, or int32 where ids32; out: [n, D] fp32 or bf16; D a multiple of 8, pointers
+// 16-byte aligned.  wrap: an id below zero counts from the end.
+KB_API int kb200_embedding_fwd(const void* table, const void* ids, void* out, long long n, int D, long long V, int table_dtype, int out_dtype, int ids32, int wrap,
                                cudaStream_t stream) {
   if (n <= 0 || D <= 0) return 0;
   if ((D & 7) || (((uintptr_t)table | (uintptr_t)out) & 15)) {
@@ -305,14 +310,16 @@ KB_API int kb200_embedding_fwd(const void* table, const long long* ids, void* ou
     return -2;
   }
   const unsigned grid = flat_grid(n * (D >> 3));
-  if (table_dtype == 1 && out_dtype == 1)
-    embedding_fwd_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, RO_THREADS, 0, stream>>>((const __nv_bfloat16*)table, ids, (__nv_bfloat16*)out, n, D, V);
-  else if (table_dtype == 0 && out_dtype == 1)
-    embedding_fwd_kernel<float, __nv_bfloat16><<<grid, RO_THREADS, 0, stream>>>((const float*)table, ids, (__nv_bfloat16*)out, n, D, V);
-  else if (table_dtype == 0 && out_dtype == 0)
-    embedding_fwd_kernel<float, float><<<grid, RO_THREADS, 0, stream>>>((const float*)table, ids, (float*)out, n, D, V);
-  else
-    embedding_fwd_kernel<__nv_bfloat16, float><<<grid, RO_THREADS, 0, stream>>>((const __nv_bfloat16*)table, ids, (float*)out, n, D, V);
+  auto run = [&](auto* t, auto* o) {
+    using TT = std::remove_const_t<std::remove_pointer_t<decltype(t)>>;
+    using TO = std::remove_pointer_t<decltype(o)>;
+    if (ids32) embedding_fwd_kernel<TT, TO, int><<<grid, RO_THREADS, 0, stream>>>(t, (const int*)ids, o, n, D, V, wrap);
+    else embedding_fwd_kernel<TT, TO, long long><<<grid, RO_THREADS, 0, stream>>>(t, (const long long*)ids, o, n, D, V, wrap);
+  };
+  if (table_dtype == 1 && out_dtype == 1) run((const __nv_bfloat16*)table, (__nv_bfloat16*)out);
+  else if (table_dtype == 0 && out_dtype == 1) run((const float*)table, (__nv_bfloat16*)out);
+  else if (table_dtype == 0 && out_dtype == 0) run((const float*)table, (float*)out);
+  else run((const __nv_bfloat16*)table, (float*)out);
   KB_CHECK_LAUNCH("embedding_fwd");
   return 0;
 }

@@ -222,7 +222,7 @@ class FusedEmbedding(torch.autograd.Function):
         src = table.detach()
         src = aligned(src)
         out = torch.empty((n, D), dtype=out_dtype, device=table.device)
-        _check(lib.kb200_embedding_fwd(_p(src), _p(ids64), _p(out), _ll(n), _i(D), _ll(V), _i(_dt(src)), _i(_dt(out)), _stream()), "embedding_fwd")
+        _check(lib.kb200_embedding_fwd(_p(src), _p(ids64), _p(out), _ll(n), _i(D), _ll(V), _i(_dt(src)), _i(_dt(out)), _i(0), _i(0), _stream()), "embedding_fwd")
         ctx.save_for_backward(ids64)
         ctx.table_shape, ctx.table_dtype, ctx.target = (V, D), table.dtype, target
         ctx.set_materialize_grads(False)
@@ -384,7 +384,7 @@ class FusedNorm(torch.autograd.Function):
         mean, rstd = stats[:rows], stats[rows:]
         g = gamma.float().contiguous() if gamma is not None else None
         b = beta.float().contiguous() if beta is not None else None
-        _check(lib.kb200_norm_fwd(_p(x), _p(g), _p(b), _p(y), _p(mean), _p(rstd), _ll(rows), _i(D), _f(eps), _i(1 if rms else 0), _i(_dt(x)), _stream()), "norm_fwd")
+        _check(lib.kb200_norm_fwd(_p(x), _vp(0), _vp(0), _p(g), _p(b), _p(y), _p(mean), _p(rstd), _ll(rows), _i(D), _f(eps), _i(1 if rms else 0), _i(_dt(x)), _stream()), "norm_fwd")
         ctx.save_for_backward(x, g, stats)
         ctx.rms = rms
         ctx.has_beta = beta is not None
@@ -413,18 +413,75 @@ class FusedNorm(torch.autograd.Function):
         slot_g = shadow.grad_slot(ctx.leaves[0], (D,)) if g is not None else None
         slot_b = shadow.grad_slot(ctx.leaves[1], (D,)) if ctx.has_beta else None
         if g is not None and slot_g is not None and (slot_b is not None or not ctx.has_beta):
-            _check(lib.kb200_norm_bwd(_p(dy), _p(x), _p(g), _p(mean), _p(rstd), _p(dx), _p(pdg), _p(pdb), _p(slot_g), _p(slot_b), _ll(rows), _i(D),
+            _check(lib.kb200_norm_bwd(_p(dy), _p(x), _p(g), _p(mean), _p(rstd), _vp(0), _p(dx), _p(pdg), _p(pdb), _p(slot_g), _p(slot_b), _ll(rows), _i(D),
                                       _i(1 if ctx.rms else 0), _i(_dt(x)), _i(1), _stream()), "norm_bwd")
             return dx, None, None, None, None
         dgamma = torch.empty(D, dtype=torch.float32, device=x.device) if g is not None else None
         dbeta = torch.empty(D, dtype=torch.float32, device=x.device) if ctx.has_beta else None
-        _check(lib.kb200_norm_bwd(_p(dy), _p(x), _p(g), _p(mean), _p(rstd), _p(dx), _p(pdg), _p(pdb), _p(dgamma), _p(dbeta), _ll(rows), _i(D),
+        _check(lib.kb200_norm_bwd(_p(dy), _p(x), _p(g), _p(mean), _p(rstd), _vp(0), _p(dx), _p(pdg), _p(pdb), _p(dgamma), _p(dbeta), _ll(rows), _i(D),
                                   _i(1 if ctx.rms else 0), _i(_dt(x)), _i(0), _stream()), "norm_bwd")
         if dgamma is not None and ctx.gamma_dtype != torch.float32:
             dgamma = dgamma.to(ctx.gamma_dtype)
         if dbeta is not None and ctx.beta_dtype != torch.float32:
             dbeta = dbeta.to(ctx.beta_dtype)
         return dx, dgamma, dbeta, None, None
+
+
+class FusedAddNorm(torch.autograd.Function):
+    """``(a + b, norm(a + b))``: a branch added to its residual stream and the sum normalised in one pass; backward the gradient that
+    reaches the sum by its other reader is added where the normalisation's is made."""
+
+    @staticmethod
+    def forward(ctx, a, b, gamma, beta, eps, rms):
+        D = a.shape[-1]
+        rows = a.numel() // D
+        total, y = torch.empty_like(a), torch.empty_like(a)
+        stats = torch.empty(2 * rows, dtype=torch.float32, device=a.device)
+        _check(_lib().kb200_norm_fwd(_p(a), _p(b), _p(total), _p(gamma), _p(beta), _p(y), _p(stats[:rows]), _p(stats[rows:]), _ll(rows), _i(D), _f(eps),
+                                     _i(1 if rms else 0), _i(_dt(a)), _stream()), "add_norm_fwd")
+        ctx.save_for_backward(total, gamma, beta, stats)
+        ctx.eps, ctx.rms = eps, rms
+        ctx.set_materialize_grads(False)
+        return total, y
+
+    @staticmethod
+    def backward(ctx, dtotal, dy):
+        total, gamma, beta, stats = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        if dy is None:
+            return dtotal, dtotal, None, None, None, None
+        if torch.is_grad_enabled():  # a gradient of this gradient is wanted: differentiate the normalisation from library operations
+            x = total.float()
+            if ctx.rms:
+                y = torch.nn.functional.rms_norm(x, x.shape[-1:], gamma, ctx.eps)
+            else:
+                y = torch.nn.functional.layer_norm(x, x.shape[-1:], gamma, beta, ctx.eps)
+            wanted = [total] + [t for t, n in ((gamma, need[2]), (beta, need[3])) if n]
+            grads = iter(torch.autograd.grad(y.to(total.dtype), wanted, dy, create_graph=True))
+            dx = next(grads)
+            dx = dx if dtotal is None else dx + dtotal
+            return dx, dx, next(grads) if need[2] else None, next(grads) if need[3] else None, None, None
+        lib = _lib()
+        D = total.shape[-1]
+        rows = total.numel() // D
+        dy = aligned(dy)
+        other = aligned(dtotal) if dtotal is not None else None
+        dx = torch.empty_like(total)
+        lib.kb200_norm_bwd_blocks.restype = ctypes.c_int
+        nb = lib.kb200_norm_bwd_blocks(_ll(rows))
+        partial = torch.empty((2, nb, D), dtype=torch.float32, device=total.device)
+        from keras_b200.kernels import shadow
+
+        params = [(gamma, need[2]), (beta, need[3])]
+        slots = [shadow.grad_slot(t, (D,)) if n else None for t, n in params]
+        in_place = all(s is not None for s, (_, n) in zip(slots, params) if n)
+        out = [s if in_place else torch.empty(D, dtype=torch.float32, device=total.device) if n else None for s, (_, n) in zip(slots, params)]
+        _check(lib.kb200_norm_bwd(_p(dy), _p(total), _p(gamma), _p(stats[:rows]), _p(stats[rows:]), _p(other), _p(dx), _p(partial[0]),
+                                  _p(partial[1] if need[3] else None), _p(out[0]), _p(out[1]), _ll(rows), _i(D), _i(1 if ctx.rms else 0), _i(_dt(total)),
+                                  _i(1 if in_place else 0), _stream()), "add_norm_bwd")
+        if in_place:
+            out = [None, None]
+        return dx, dx, out[0], out[1], None, None
 
 
 def column_sum(x, accumulate_into=None):

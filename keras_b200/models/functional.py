@@ -97,6 +97,11 @@ class Functional(Function, Model):
                 from keras_b200.models import fusion as fusion_mod
 
                 fusion = _FusionCtx(fusion_mod, training)
+                if not kwargs and (torch.is_grad_enabled() or not training):
+                    from keras_b200.models import direct
+
+                    if direct.usable(inputs[0]):
+                        fusion.direct = direct
         outputs = self._run_through_graph(inputs, operation_fn=lambda op: operation_fn(op, training=training, **kwargs), fusion=fusion)
         return unpack_singleton(outputs)
 
@@ -289,10 +294,10 @@ class Functional(Function, Model):
 
 
 class _FusionCtx:
-    __slots__ = ("mod", "training", "Deferred", "NoBias", "run_bn", "run_conv_nobias", "run_pool_padded", "Padded", "build_plan", "applicable", "relu_cap", "shared_cast")
+    __slots__ = ("mod", "training", "Deferred", "NoBias", "run_bn", "run_conv_nobias", "run_pool_padded", "Padded", "build_plan", "applicable", "relu_cap", "shared_cast", "direct", "recording")
 
     def __init__(self, mod, training):
-        self.mod, self.training = mod, training
+        self.mod, self.training, self.direct, self.recording = mod, training, None, torch.is_grad_enabled()
         self.Deferred, self.NoBias, self.run_bn, self.build_plan, self.applicable = mod.Deferred, mod.NoBias, mod.run_bn, mod.build_plan, mod.applicable
         self.relu_cap, self.shared_cast = mod.relu_cap, mod.shared_cast
         self.run_conv_nobias, self.run_pool_padded, self.Padded = mod.run_conv_nobias, mod.run_pool_padded, mod.Padded

@@ -133,6 +133,12 @@ class Function(Operation):
         merge = plan.get("merge_tensors", ())
         marked = set()
         casts = {}
+        direct, runs, joined, computed = fusion.direct, {}, {}, None
+        if direct is not None:
+            runs, joined = direct.plan_of(self, nodes)
+            computed = set()
+            if fusion.recording:
+                runs = {}
         if merge:
             import torch
 
@@ -150,6 +156,22 @@ class Function(Operation):
                             grad_merge.mark(env[id(t)])
             role = plan.get(id(node))
             outs = node.outputs
+            if role is None and computed is not None:
+                if id(node) in computed:
+                    continue
+                pair = joined.get(id(node))
+                if pair is not None:
+                    both = direct.add_norm(node.operation, pair[0].operation, [env[i] for i in pair[1]])
+                    if both is not None:
+                        env[id(outs[0])], env[id(pair[0].outputs[0])] = both
+                        computed.add(id(pair[0]))
+                        continue
+                run = runs.get(id(node))
+                if run is not None:
+                    result = run(env)
+                    if result is not None:
+                        env[id(outs[0])] = result
+                        continue
             if role == "pad_fold":
                 x = env[id(ins[0])]
                 if isinstance(x, fusion.Deferred):

@@ -35,3 +35,196 @@ def test_lstm_on_clusters_against_the_steps_in_64_bits(B, T, U, reverse, sequenc
         assert _rel(r, w) < 3e-6  # fp32 sums over U terms a step, a few steps deep
     for a, b, n in zip(mine, exact, wanted):
         assert not n or _rel(a.grad, b.grad) < 1e-5  # up to B * T terms in the weight gradient
+
+
+# ------------------------------------------------------------------------------------------------ products of inference
+@pytest.mark.parametrize("fp32", [True, False])
+@pytest.mark.parametrize("M,K,widths", [(1, 64, (64,)), (7, 72, (72,)), (77, 768, (1001,)), (128, 200, (264,)), (128, 3072, (64, 64, 128)), (33, 256, (1024, 256, 256)),
+                                        (129, 64, (64,)), (300, 200, (1001,)), (257, 768, (192, 64, 64)), (130, 512, (4099,))])
+def test_inference_products_read_weights_as_stored(M, K, widths, fp32):
+    """Up to 128 rows straight from the weight, above through one bf16 matrix; any width, one weight or three, every epilogue."""
+    from keras_b200.kernels import gemm
+    from keras_b200.models import direct
+
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    ws = [torch.randn(K, n, generator=g, device="cuda") * K ** -0.5 for n in widths]
+    bs = [torch.randn(n, generator=g, device="cuda") for n in widths]
+    ws = ws if fp32 else [w.bfloat16() for w in ws]
+    acts = {0: lambda t: t, 1: torch.relu, 3: torch.nn.functional.silu, 4: torch.nn.functional.gelu}
+    for act, fn in acts.items():
+        for biases in ([None] * len(ws), bs, [b.bfloat16() for b in bs]):
+            out = direct._product(x, ws, biases, act)
+            ref = torch.cat([x.double() @ w.bfloat16().double() + (0 if b is None else b.double()) for w, b in zip(ws, biases)], 1)
+            # exact products of bf16, summed in fp32, one rounding to bf16
+            assert _rel(out[:, :sum(widths)], fn(ref)) < 2.0 ** -8
+            if biases[0] is None:
+                assert not out[:, sum(widths):].float().any()
+            assert torch.equal(out, direct._product(x, ws, biases, act))
+    gemm.check_errors()
+
+
+def _models(keras):
+    L = keras.layers
+
+    def tokens(layer):
+        i = keras.Input((24,), dtype="int32")
+        return keras.Model(i, layer(i))
+
+    def decoder(i):
+        h = L.Embedding(301, 128)(i)
+        a = L.MultiHeadAttention(2, 64, use_bias=True)(L.LayerNormalization()(h), L.LayerNormalization()(h))
+        h = L.Add()([h, a])
+        n = L.LayerNormalization()(h)
+        n = L.MultiHeadAttention(2, 64, use_bias=False)(n, n, use_causal_mask=True)
+        h = L.Add()([h, n])
+        m = L.LayerNormalization(center=False)(h)
+        h = L.Add()([h, L.Dense(128)(L.Dense(256, activation="gelu")(m))])
+        return L.Dense(301)(L.LayerNormalization()(h))
+
+    def gated(i):
+        h = L.Embedding(301, 256)(i)
+        a = L.RMSNormalization()(h)
+        h = L.Add()([h, L.GroupedQueryAttention(64, 4, 2, use_bias=False)(a, a, use_causal_mask=True)])
+        m = L.RMSNormalization()(h)
+        m = L.Multiply()([L.Dense(512, activation="silu")(m), L.Dense(512, activation=lambda t: t * 2)(m)])
+        return L.Add()([h, L.Dense(256)(m)])
+
+    def padded(i):
+        h = L.Embedding(301, 128, mask_zero=True)(i)
+        for _ in range(2):
+            h = L.LayerNormalization()(L.Add()([h, L.MultiHeadAttention(2, 64)(h, h)]))
+            h = L.LayerNormalization()(L.Add()([h, L.Dense(128, activation="relu")(h)]))
+        return h
+
+    return {"decoder": tokens(decoder), "gated": tokens(gated), "padded": tokens(padded)}
+
+
+@pytest.mark.parametrize("policy", ["mixed_bfloat16", "bfloat16"])
+@pytest.mark.parametrize("batch", [1, 2, 40])
+def test_layers_called_directly_agree_with_their_own_calls(policy, batch, monkeypatch):
+    import keras_b200 as keras
+    from keras_b200.models import direct
+
+    keras.utils.set_random_seed(3)
+    keras.config.set_dtype_policy(policy)
+    try:
+        models = _models(keras)
+    finally:
+        keras.config.set_dtype_policy("float32")
+    ids = torch.randint(-1, 301, (batch, 24), device="cuda", dtype=torch.int32)
+    ids[:, 17:] = 0
+    for name, model in models.items():
+        with torch.no_grad():
+            model(ids)  # the first call is the layers' own
+            taken = []
+            for fn in ("_dense", "_attention", "add_norm", "_embedding"):
+                plain = getattr(direct, fn)
+                monkeypatch.setattr(direct, fn, lambda *a, _f=plain, _n=fn: (lambda r: (taken.append(_n) if r is not None else None, r)[1])(_f(*a)))
+            direct._PLANS.clear()
+            mine = model(ids)
+            monkeypatch.undo()
+            direct._PLANS.clear()
+            assert {"_dense", "_attention", "add_norm", "_embedding"} <= set(taken), (name, taken)
+            monkeypatch.setattr(direct, "usable", lambda x: False)
+            own = model(ids)
+            monkeypatch.undo()
+        assert mine.shape == own.shape and mine.dtype == own.dtype
+        # bf16 throughout, some ten roundings deep; the direct calls round parameters of norms and biases less often
+        assert _rel(mine.float(), own.double()) < 0.02, name
+        a, b = getattr(mine, "_keras_mask", None), getattr(own, "_keras_mask", None)
+        assert (a is None) == (b is None) and (a is None or torch.equal(a, b))
+
+
+def test_direct_calls_see_every_change_of_a_layer(monkeypatch):
+    import keras_b200 as keras
+    from keras_b200.models import direct
+
+    keras.utils.set_random_seed(4)
+    keras.config.set_dtype_policy("mixed_bfloat16")
+    try:
+        i = keras.Input((128,))
+        first, second = keras.layers.Dense(128, activation="relu"), keras.layers.Dense(64)
+        model = keras.Model(i, second(first(i)))
+    finally:
+        keras.config.set_dtype_policy("float32")
+    x = torch.randn(9, 128, device="cuda")
+
+    def both():
+        with torch.no_grad():
+            model(x)
+            mine = model(x)
+            monkeypatch.setattr(direct, "usable", lambda x: False)
+            own = model(x)
+            monkeypatch.undo()
+        assert _rel(mine.float(), own.double()) < 0.01 or not own.any()
+        return mine
+
+    seen = [both()]
+    first.activation = keras.activations.silu
+    seen.append(both())
+    first.activation = lambda t: t + 1
+    seen.append(both())
+    first.kernel.assign(first.kernel * 0.5)
+    seen.append(both())
+    first.kernel.value.data.mul_(2.0)  # past the version counter
+    seen.append(both())
+    first.call = lambda inputs, training=None: inputs * 0
+    seen.append(both())
+    del first.call
+    second.enable_lora(4)
+    second.lora_kernel_b.assign(torch.randn(4, 64, device="cuda"))
+    seen.append(both())
+    second.quantize("int8")
+    seen.append(both())
+    assert all(not torch.equal(a, b) for a, b in zip(seen, seen[1:]))
+    trained = keras.Model(i, first(i))
+    trained.compile(keras.optimizers.SGD(0.5), "mse")
+    trained.train_on_batch(x, torch.zeros(9, 128, device="cuda"))  # weights now have 16-bit shadows
+    with torch.no_grad():
+        mine = trained(x)
+        ref = torch.matmul(x.bfloat16().double(), first._kernel._value.bfloat16().double()) + first.bias._value.double() + 1
+    assert _rel(mine.float(), ref) < 0.01
+
+
+# ------------------------------------------------------------------------------------------------ residual sums with their normalisation
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,D", [(1, 8), (50, 100), (5, 200), (700, 256), (2664, 512), (1500, 768), (33, 776), (900, 1024), (77, 2048), (40, 4096), (9, 8192)])
+@pytest.mark.parametrize("rms", [False, True])
+def test_add_and_norm_in_one_pass(rows, D, dtype, rms):
+    from keras_b200.kernels import ops as kops
+
+    g = torch.Generator(device="cuda").manual_seed(D)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")  # noqa: E731
+    mine = [rnd(rows, D).to(dtype).requires_grad_(True), rnd(rows, D).to(dtype).requires_grad_(True), rnd(D).requires_grad_(True)]
+    mine.append(None if rms else rnd(D).requires_grad_(True))
+    up = (rnd(rows, D).to(dtype), rnd(rows, D).to(dtype))
+    total, y = kops.FusedAddNorm.apply(*mine, 1e-5, rms)
+    exact = [None if t is None else t.detach().double().requires_grad_(True) for t in mine]
+    s = exact[0] + exact[1]
+    s = s + (s.to(dtype).double() - s).detach()  # the sum is rounded to its type before it is normalised
+    n = torch.nn.functional.rms_norm(s, (D,), exact[2], 1e-5) if rms else torch.nn.functional.layer_norm(s, (D,), exact[2], exact[3], 1e-5)
+    assert torch.equal(total, mine[0] + mine[1])
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-6  # one rounding of each result; fp32 sums of at most 8192 values
+    assert _rel(y, n) < tol
+    for outs in ((0, 1), (1,), (0,)):  # either result may have no gradient
+        have = [t for t in mine if t is not None]
+        a = torch.autograd.grad([(total, y)[k] for k in outs], have, [up[k] for k in outs], retain_graph=True, allow_unused=True)
+        b = torch.autograd.grad([(s, n)[k] for k in outs], [t for t in exact if t is not None], [up[k].double() for k in outs], retain_graph=True, allow_unused=True)
+        for p, q in zip(a, b):
+            assert (p is None) == (q is None) and (p is None or _rel(p, q) < (tol if p.ndim > 1 else 1e-4 if dtype == torch.bfloat16 else 1e-5))
+
+
+def test_add_and_norm_second_derivatives():
+    from keras_b200.kernels import ops as kops
+
+    a, b = (torch.randn(6, 64, device="cuda", requires_grad=True) for _ in range(2))
+    gamma, beta = (torch.randn(64, device="cuda", requires_grad=True) for _ in range(2))
+    second = []
+    for f in (lambda: kops.FusedAddNorm.apply(a, b, gamma, beta, 1e-5, False),
+              lambda: (a + b, torch.nn.functional.layer_norm(a + b, (64,), gamma, beta, 1e-5))):
+        t, y = f()
+        (g,) = torch.autograd.grad((y ** 2).sum() + (t ** 3).sum(), a, create_graph=True)
+        second.append(torch.autograd.grad((g ** 2).sum(), [a, b, gamma]))
+    for p, q in zip(*second):
+        assert torch.allclose(p, q, rtol=1e-4, atol=1e-4 * q.abs().max().item())
