@@ -25,8 +25,7 @@ using namespace kbgemm;
 // takes six, or its loop waits for L2 (600 ns a 64-element K block with three: [2664, 512, 2048] 12.1 -> 10.7 us).
 template <int STAGES>
 __global__ void __launch_bounds__(THREADS, STAGES == 3 ? 2 : 1)
-gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                         const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
+gemm_bf16_tcgen05_kernel(const __grid_constant__ GroupMaps maps, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment is required by the 128-byte swizzle atoms
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -40,12 +39,17 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * STAGES + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_tiles = (p.N + BN - 1) / BN;
+  const int n_tiles = p.groups > 1 && !p.sum_k ? p.tile_end[p.groups - 1] : (p.N + BN - 1) / BN;
   const int m0 = (blockIdx.x / n_tiles) * BM;
-  const int n0 = (blockIdx.x % n_tiles) * BN;
-  const int k_blocks = (p.K + BK - 1) / BK;
+  int first_tile;
+  const int tile_group = group_of_tile(p, blockIdx.x % n_tiles, first_tile);
+  const int n0 = ((int)(blockIdx.x % n_tiles) - first_tile) * BN;
+  const int k_blocks = p.sum_k ? p.kb_end[p.groups - 1] : (p.K + BK - 1) / BK;
   auto load_block = [&](int kb) {
-    const int s = kb % STAGES, k0 = kb * BK;
+    int first_kb;
+    const int g = tile_group + group_of_block(p, kb, first_kb);
+    const CUtensorMap &map_a = maps.a[p.sum_k ? g : 0], &map_b = maps.b[g];
+    const int s = kb % STAGES, k0 = (kb - first_kb) * BK;
     const uint32_t sa = base + s * STAGE_BYTES, sb = sa + A_TILE_BYTES;
     mbar_expect_tx(full_bar(s), STAGE_BYTES);
     if (p.a_mn_major) {
@@ -64,9 +68,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   const int first_blocks = min(STAGES, k_blocks);  // loaded ahead of the barrier below, while TMEM is being allocated
 
   if (threadIdx.x == 0) {
-    prefetch_map(&map_a);
-    prefetch_map(&map_b);
-    prefetch_map(&map_c);
+    prefetch_map(&maps.a[0]);
+    prefetch_map(&maps.b[0]);
+    prefetch_map(&maps.c[0]);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
@@ -148,7 +152,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const int q = warp & 3;  // TMEM lane quarter this warp may access
       // every MMA of this CTA's only tile has completed, so the operand ring is free: stage 0 holds the staging buffers
       uint32_t stores = 0;
-      store_rows_tma(tmem_base + ((uint32_t)(q * 32) << 16), BN, n0, m0 + q * 32, base + (uint32_t)(warp - 2) * 8192u, stores, &map_c, p, lane);
+      store_rows_group(tmem_base + ((uint32_t)(q * 32) << 16), BN, n0, m0 + q * 32, base + (uint32_t)(warp - 2) * 8192u, stores, maps, tile_group, p, lane);
       if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // staging read out; the writes land before the grid ends
     }
   }
@@ -165,8 +169,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 // tensor memory (512 columns) split into two 256-column accumulators so that the epilogue of tile i
 // overlaps the main loop of tile i+1.  One CTA per SM; tiles are handed out round-robin in an order
 __global__ void __launch_bounds__(THREADS, 1)
-gemm_bf16_tcgen05_persistent(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                             const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
+gemm_bf16_tcgen05_persistent(const __grid_constant__ GroupMaps maps, const GemmParams p) {
   constexpr int BM = v2::BM, BN = v2::BN, BK = v2::BK, STAGES = v2::STAGES, STAGE_BYTES = v2::STAGE_BYTES, A_BYTES = v2::A_BYTES;
   constexpr uint32_t TMEM_COLS = v2::TMEM_COLS;
   extern __shared__ uint8_t smem_raw[];
@@ -184,17 +187,17 @@ gemm_bf16_tcgen05_persistent(const __grid_constant__ CUtensorMap map_a, const __
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * STAGES + 5);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m_tiles = (p.M + BM - 1) / BM, n_tiles = (p.N + BN - 1) / BN;
+  const int m_tiles = (p.M + BM - 1) / BM, n_tiles = p.groups > 1 && !p.sum_k ? p.tile_end[p.groups - 1] : (p.N + BN - 1) / BN;
   const int split = p.split_k > 1 ? p.split_k : 1;
   const int total_tiles = m_tiles * n_tiles * split;  // work units: (output tile, K slice)
   const int bk = (p.fp8 || p.int8) ? 2 * BK : BK;  // elements per 128-byte K block
-  const int k_blocks_all = (p.K + bk - 1) / bk;
+  const int k_blocks_all = p.sum_k ? p.kb_end[p.groups - 1] : (p.K + bk - 1) / bk;
   const int kb_per = split > 1 ? p.kb_per_split : k_blocks_all;
 
   if (threadIdx.x == 0) {
-    prefetch_map(&map_a);
-    prefetch_map(&map_b);
-    prefetch_map(&map_c);
+    prefetch_map(&maps.a[0]);
+    prefetch_map(&maps.b[0]);
+    prefetch_map(&maps.c[0]);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
@@ -222,8 +225,10 @@ gemm_bf16_tcgen05_persistent(const __grid_constant__ CUtensorMap map_a, const __
       uint32_t issued = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-        int m0, n0;
+        int m0, n0, first_tile, first_kb;
         tile_coords(t / split, m_tiles, n_tiles, m0, n0);
+        const int tile_group = group_of_tile(p, n0 / BN, first_tile);
+        n0 -= first_tile * BN;
         const int kb0 = (t % split) * kb_per, kb1 = min(kb0 + kb_per, k_blocks_all);
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
@@ -231,7 +236,9 @@ gemm_bf16_tcgen05_persistent(const __grid_constant__ CUtensorMap map_a, const __
           if (!ok) break;
           const uint32_t sa = base + s * STAGE_BYTES, sb = sa + A_BYTES;
           mbar_expect_tx(full_bar(s), STAGE_BYTES);
-          const int k0 = kb * bk;
+          const int g = tile_group + group_of_block(p, kb, first_kb);
+          const CUtensorMap &map_a = maps.a[p.sum_k ? g : 0], &map_b = maps.b[g];
+          const int k0 = (kb - first_kb) * bk;
           if (p.a_mn_major) {
             tma_load_2d(sa, &map_a, full_bar(s), m0, k0);
             tma_load_2d(sa + 8192, &map_a, full_bar(s), m0 + 64, k0);
@@ -313,14 +320,16 @@ gemm_bf16_tcgen05_persistent(const __grid_constant__ CUtensorMap map_a, const __
     uint32_t local = 0, stores = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++local) {
-      int m0, n0;
+      int m0, n0, first_tile;
       tile_coords(t / split, m_tiles, n_tiles, m0, n0);
+      const int tile_group = group_of_tile(p, n0 / BN, first_tile);
+      n0 -= first_tile * BN;
       const uint32_t acc = local & 1;
       ok = mbar_wait(acc_full_bar(acc), (local >> 1) & 1, abort_flag);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tmem_row = tmem_base + acc * (uint32_t)BN + ((uint32_t)(q * 32) << 16);
-      store_rows_tma(tmem_row, BN, n0, m0 + q * 32, my_stage, stores, &map_c, p, lane);
+      store_rows_group(tmem_row, BN, n0, m0 + q * 32, my_stage, stores, maps, tile_group, p, lane);
       // this warp has finished reading the accumulator: hand it back to the MMA issuer
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -409,8 +418,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
 }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(v3::PAIR_THREADS, 1)
-gemm_bf16_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                       const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
+gemm_bf16_tcgen05_pair(const __grid_constant__ GroupMaps maps, const GemmParams p) {
   constexpr int BM = v3::BM, BN = v3::BN, BK = v3::BK, STAGES = v3::STAGES, A_BYTES = v3::A_BYTES, STAGE_BYTES = v3::STAGE_BYTES;
   constexpr uint32_t TMEM_COLS = v3::TMEM_COLS;
   extern __shared__ uint8_t smem_raw[];
@@ -429,24 +437,26 @@ gemm_bf16_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_rank();
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-  const int m_tiles = (p.M + 2 * BM - 1) / (2 * BM), n_tiles = (p.N + BN - 1) / BN;
+  const int m_tiles = (p.M + 2 * BM - 1) / (2 * BM), n_tiles = p.groups > 1 && !p.sum_k ? p.tile_end[p.groups - 1] : (p.N + BN - 1) / BN;
   const int split = p.split_k > 1 ? p.split_k : 1;
   const int total_tiles = m_tiles * n_tiles * split;
-  const int k_blocks_all = (p.K + BK - 1) / BK;
+  const int k_blocks_all = p.sum_k ? p.kb_end[p.groups - 1] : (p.K + BK - 1) / BK;
   const int kb_per = split > 1 ? p.kb_per_split : k_blocks_all;
-  auto coords = [&](int t, int& m0, int& n0) {
+  auto coords = [&](int t, int& m0, int& n0, int& g) {
     const int per_group = v3::GROUP_M * n_tiles;
-    const int g = t / per_group, first_m = g * v3::GROUP_M;
+    const int patch = t / per_group, first_m = patch * v3::GROUP_M;
     const int rows = min(v3::GROUP_M, m_tiles - first_m);
-    const int r = t - g * per_group;
+    const int r = t - patch * per_group;
     m0 = (first_m + r % rows) * (2 * BM);
-    n0 = (r / rows) * BN;
+    int first_tile;
+    g = group_of_tile(p, r / rows, first_tile);
+    n0 = (r / rows - first_tile) * BN;
   };
 
   if (threadIdx.x == 0) {
-    prefetch_map(&map_a);
-    prefetch_map(&map_b);
-    prefetch_map(&map_c);
+    prefetch_map(&maps.a[0]);
+    prefetch_map(&maps.b[0]);
+    prefetch_map(&maps.c[0]);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
@@ -475,8 +485,8 @@ gemm_bf16_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_c
       uint32_t it = 0;
       bool ok = true;
       for (int t = pair; t < total_tiles && ok; t += pairs) {
-        int m0, n0;
-        coords(t / split, m0, n0);
+        int m0, n0, tile_group, first_kb;
+        coords(t / split, m0, n0, tile_group);
         m0 += rank * BM;
         n0 += rank * (BN / 2);
         const int kb0 = (t % split) * kb_per, kb1 = min(kb0 + kb_per, k_blocks_all);
@@ -489,7 +499,9 @@ gemm_bf16_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_c
           // before the announcement, which is its only arrival.
           if (rank == 0) mbar_expect_tx(full_bar(s), 2 * STAGE_BYTES);
           const uint32_t bar = map_to_rank(full_bar(s), 0);
-          const int k0 = kb * BK;
+          const int g = tile_group + group_of_block(p, kb, first_kb);
+          const CUtensorMap &map_a = maps.a[p.sum_k ? g : 0], &map_b = maps.b[g];
+          const int k0 = (kb - first_kb) * BK;
           if (p.a_mn_major) {
             tma_load_2d_pair(sa, &map_a, bar, m0, k0);
             tma_load_2d_pair(sa + 8192, &map_a, bar, m0 + 64, k0);
@@ -556,14 +568,14 @@ gemm_bf16_tcgen05_pair(const __grid_constant__ CUtensorMap map_a, const __grid_c
     uint32_t local = 0, stores = 0;
     bool ok = true;
     for (int t = pair; t < total_tiles && ok; t += pairs, ++local) {
-      int m0, n0;
-      coords(t / split, m0, n0);
+      int m0, n0, tile_group;
+      coords(t / split, m0, n0, tile_group);
       const uint32_t acc = local & 1;
       ok = mbar_wait_cluster(acc_full_bar(acc), (local >> 1) & 1, abort_flag);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tmem_row = tmem_base + acc * (uint32_t)BN + (uint32_t)(half * (BN / 2)) + ((uint32_t)(q * 32) << 16);
-      store_rows_tma(tmem_row, BN / 2, n0 + half * (BN / 2), m0 + rank * BM + q * 32, my_stage, stores, &map_c, p, lane);
+      store_rows_group(tmem_row, BN / 2, n0 + half * (BN / 2), m0 + rank * BM + q * 32, my_stage, stores, maps, tile_group, p, lane);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(map_to_rank(acc_empty_bar(acc), 0));
@@ -613,38 +625,75 @@ static int gemm_variant(int M, int N, int split_k, int sms) {
   return N > 128 && t1 >= sms / 2 ? GV_PERSISTENT : GV_TILE;
 }
 
-// `bias_bf16`: the bias holds bf16.
-KB_API int kb200_gemm_bf16_run(const void* a, const void* b, void* c, const void* bias, int M, int N, int K, long long lda, long long ldb,
-                               long long ldc, int a_mn_major, int b_mn_major, int act, int out_fp32, int bias_bf16, int split_k, int variant, int* err,
-                               cudaStream_t stream) {
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
+// One product of a launch (see GemmParams::groups).
+struct GemmOperands {
+  const void *a, *b;
+  void* c;
+  const void* bias;
+  int N, K;
+  long long lda, ldb, ldc;
+};
+
+static int gemm_launch(const GemmOperands* ops, int groups, int sum_k, int M, int a_mn_major, int b_mn_major, int act, int out_fp32, int bias_bf16, int split_k,
+                       int variant, int* err, cudaStream_t stream) {
   const int accumulate = split_k < 0 ? 1 : 0;
   if (split_k < 0) split_k = -split_k;
-  if ((split_k > 1 || accumulate) && (!out_fp32 || bias != nullptr || act != ACT_NONE)) {
-    kb200_set_error("gemm_bf16: split-K needs an fp32 output without bias or activation");
-    return -4;
+  long long columns = 0, k_blocks = 0;  // column tiles are counted per product below
+  for (int g = 0; g < groups; ++g) {
+    const GemmOperands& o = ops[g];
+    if ((split_k > 1 || accumulate) && (!out_fp32 || o.bias != nullptr || act != ACT_NONE)) {
+      kb200_set_error("gemm_bf16: split-K needs an fp32 output without bias or activation");
+      return -4;
+    }
+    if ((o.lda % 8) || (o.ldb % 8) || (((uintptr_t)o.a | (uintptr_t)o.b) & 15) || (((uintptr_t)o.c) & 15) || (o.ldc % (out_fp32 ? 4 : 8))) {
+      kb200_set_error("gemm_bf16: operands must be 16-byte aligned with pitches that are multiples of 8 elements");
+      return -2;
+    }
+    if (groups > 1 && (sum_k ? o.K % BK || o.N != ops[0].N : o.K != ops[0].K)) {
+      kb200_set_error("gemm_bf16: products side by side share K, summed ones share N and have K in whole blocks");
+      return -2;
+    }
+    columns += o.N;
+    k_blocks += (o.K + BK - 1) / BK;
   }
-  if ((lda % 8) || (ldb % 8) || (((uintptr_t)a | (uintptr_t)b) & 15) || (((uintptr_t)c) & 15) || (ldc % (out_fp32 ? 4 : 8))) {
-    kb200_set_error("gemm_bf16: operands must be 16-byte aligned with pitches that are multiples of 8 elements");
-    return -2;
-  }
-  CUtensorMap map_a, map_b, map_c;
+  if (sum_k || groups == 1) columns = ops[0].N;
+  if (!sum_k) k_blocks = (ops[0].K + BK - 1) / BK;
   const int sm_count = kb_sm_count();
   int kb_per_split = 0;
   if (split_k > 1) {
-    const int k_blocks = (K + BK - 1) / BK;
-    if (split_k > k_blocks) split_k = k_blocks;
-    kb_per_split = (k_blocks + split_k - 1) / split_k;
-    split_k = (k_blocks + kb_per_split - 1) / kb_per_split;  // every slice holds at least one K block
+    if (split_k > k_blocks) split_k = (int)k_blocks;
+    kb_per_split = (int)((k_blocks + split_k - 1) / split_k);
+    split_k = (int)((k_blocks + kb_per_split - 1) / kb_per_split);  // every slice holds at least one K block
   }
   if (split_k < 1) split_k = 1;
-  if (variant == GV_AUTO) variant = gemm_variant(M, N, split_k, sm_count);
+  if (variant == GV_AUTO) variant = gemm_variant(M, (int)(columns > 0x7fffffff ? 0x7fffffff : columns), split_k, sm_count);
   if (split_k > 1 && variant == GV_TILE) variant = GV_PERSISTENT;
+  const int tile_m = variant == GV_PAIR256 ? 256 : 128, tile_n = variant == GV_TILE ? 128 : 256;
   // rows of B's box: the N range one CTA loads
   const int bn = variant == GV_PERSISTENT ? 256 : 128;
-  bool ok = a_mn_major ? make_map(&map_a, a, M, K, lda, 64, BK) : make_map(&map_a, a, K, M, lda, BK, BM);
-  ok = ok && (b_mn_major ? make_map(&map_b, b, N, K, ldb, 64, BK) : make_map(&map_b, b, K, N, ldb, BK, bn));
-  ok = ok && make_map(&map_c, c, N, M, ldc, out_fp32 ? 32 : 64, 32, out_fp32 != 0);
+  GroupMaps maps;
+  GemmParams p{ops[0].c, bias_bf16 ? nullptr : (const float*)ops[0].bias, M, ops[0].N, ops[0].K, ops[0].ldc, a_mn_major, b_mn_major, act, out_fp32, err, split_k, kb_per_split};
+  p.accumulate = accumulate;
+  p.groups = groups;
+  p.sum_k = sum_k;
+  // with several products this only says which type the biases are
+  p.bias16 = bias_bf16 ? (const __nv_bfloat16*)(groups > 1 ? ops[0].a : ops[0].bias) : nullptr;
+  int tiles_n = 0, blocks = 0;
+  bool ok = true;
+  for (int g = 0; g < 3; ++g) {
+    if (g >= groups) {
+      maps.a[g] = maps.a[0], maps.b[g] = maps.b[0], maps.c[g] = maps.c[0];
+      continue;
+    }
+    const GemmOperands& o = ops[g];
+    ok = ok && (a_mn_major ? make_map(&maps.a[g], o.a, M, o.K, o.lda, 64, BK) : make_map(&maps.a[g], o.a, o.K, M, o.lda, BK, BM));
+    ok = ok && (b_mn_major ? make_map(&maps.b[g], o.b, o.N, o.K, o.ldb, 64, BK) : make_map(&maps.b[g], o.b, o.K, o.N, o.ldb, BK, bn));
+    ok = ok && make_map(&maps.c[g], o.c, o.N, M, o.ldc, out_fp32 ? 32 : 64, 32, out_fp32 != 0);
+    tiles_n += (o.N + tile_n - 1) / tile_n;
+    blocks += (o.K + BK - 1) / BK;
+    p.tile_end[g] = tiles_n, p.width[g] = o.N, p.kb_end[g] = blocks, p.bias_of[g] = o.bias;
+  }
+  if (sum_k) tiles_n = p.tile_end[0];
   if (!ok) {
     kb200_set_error("gemm_bf16: cuTensorMapEncodeTiled failed");
     return -3;
@@ -661,24 +710,51 @@ KB_API int kb200_gemm_bf16_run(const void* a, const void* b, void* c, const void
     kb200_set_error("gemm_bf16: cannot raise the shared-memory limit of the kernel on this device");
     return -3;
   }
-  GemmParams p{c, bias_bf16 ? nullptr : (const float*)bias, M, N, K, ldc, a_mn_major, b_mn_major, act, out_fp32, err, split_k, kb_per_split};
-  p.bias16 = bias_bf16 ? (const __nv_bfloat16*)bias : nullptr;
-  p.accumulate = accumulate;
-  const int tile_m = variant == GV_PAIR256 ? 256 : 128, tile_n = variant == GV_TILE ? 128 : 256;
-  const long long units = (long long)((M + tile_m - 1) / tile_m) * ((N + tile_n - 1) / tile_n) * split_k;
+  const long long units = (long long)((M + tile_m - 1) / tile_m) * tiles_n * split_k;
   if (variant == GV_TILE) {
     if (units <= sm_count)
-      gemm_bf16_tcgen05_kernel<LONG><<<(unsigned)units, THREADS, smem_long, stream>>>(map_a, map_b, map_c, p);
+      gemm_bf16_tcgen05_kernel<LONG><<<(unsigned)units, THREADS, smem_long, stream>>>(maps, p);
     else
-      gemm_bf16_tcgen05_kernel<STAGES><<<(unsigned)units, THREADS, smem_v1, stream>>>(map_a, map_b, map_c, p);
+      gemm_bf16_tcgen05_kernel<STAGES><<<(unsigned)units, THREADS, smem_v1, stream>>>(maps, p);
   } else if (variant == GV_PERSISTENT) {
-    gemm_bf16_tcgen05_persistent<<<(unsigned)(units < sm_count ? units : sm_count), THREADS, v2::SMEM_BYTES, stream>>>(map_a, map_b, map_c, p);
+    gemm_bf16_tcgen05_persistent<<<(unsigned)(units < sm_count ? units : sm_count), THREADS, v2::SMEM_BYTES, stream>>>(maps, p);
   } else {
     const int pairs = (int)(units < sm_count / 2 ? units : sm_count / 2);
-    gemm_bf16_tcgen05_pair<<<(unsigned)(2 * pairs), v3::PAIR_THREADS, v3::SMEM_BYTES, stream>>>(map_a, map_b, map_c, p);
+    gemm_bf16_tcgen05_pair<<<(unsigned)(2 * pairs), v3::PAIR_THREADS, v3::SMEM_BYTES, stream>>>(maps, p);
   }
   KB_CHECK_LAUNCH("gemm_bf16");
   return 0;
+}
+
+// `bias_bf16`: the bias holds bf16.
+KB_API int kb200_gemm_bf16_run(const void* a, const void* b, void* c, const void* bias, int M, int N, int K, long long lda, long long ldb,
+                               long long ldc, int a_mn_major, int b_mn_major, int act, int out_fp32, int bias_bf16, int split_k, int variant, int* err,
+                               cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const GemmOperands o{a, b, c, bias, N, K, lda, ldb, ldc};
+  return gemm_launch(&o, 1, 0, M, a_mn_major, b_mn_major, act, out_fp32, bias_bf16, split_k, variant, err, stream);
+}
+
+// Up to three products in one launch, the fields of GemmOperands one product after the other: pointers (a, b, c, bias), sizes (N, K) and
+// pitches (lda, ldb, ldc).  sum_k = 0: C_i = A B_i + bias_i, side by side; sum_k = 1: C = the sum of A_i B_i, added in fp32.  The projections
+// of an attention layer, their weight gradients, and the gradient of their common input.
+KB_API int kb200_gemm_group(const void* const* pointers, const int* sizes, const long long* pitches, int groups, int sum_k, int M, int a_mn_major, int b_mn_major,
+                            int out_fp32, int bias_bf16, int split_k, int variant, int* err, cudaStream_t stream) {
+  if (M <= 0) return 0;
+  GemmOperands o[3];
+  if (groups < 1 || groups > 3) {
+    kb200_set_error("gemm_group: one to three products");
+    return -2;
+  }
+  for (int g = 0; g < groups; ++g) {
+    o[g] = GemmOperands{pointers[4 * g], pointers[4 * g + 1], const_cast<void*>(pointers[4 * g + 2]), pointers[4 * g + 3], sizes[2 * g], sizes[2 * g + 1],
+                        pitches[3 * g], pitches[3 * g + 1], pitches[3 * g + 2]};
+    if (o[g].N <= 0 || o[g].K <= 0) {
+      kb200_set_error("gemm_group: empty product");
+      return -2;
+    }
+  }
+  return gemm_launch(o, groups, groups > 1 ? sum_k : 0, M, a_mn_major, b_mn_major, ACT_NONE, out_fp32, bias_bf16, split_k, variant, err, stream);
 }
 
 // C[M,N] = act(alpha * (A x B^T) + bias) with one-byte floating-point operands on kind::f8f6f4 tensor-core instructions.
@@ -692,7 +768,8 @@ KB_API int kb200_gemm_fp8(const void* a, const void* b, void* c, const float* bi
     kb200_set_error("gemm_fp8: operands must be 16-byte aligned with pitches that are multiples of 16 bytes; formats 0 (e4m3) or 1 (e5m2)");
     return -2;
   }
-  CUtensorMap map_a, map_b, map_c;
+  GroupMaps maps;
+  CUtensorMap &map_a = maps.a[0], &map_b = maps.b[0], &map_c = maps.c[0];
   bool ok = make_map_u8(&map_a, a, K, M, lda, 128, v2::BM) && make_map_u8(&map_b, b, K, N, ldb, 128, v2::BN);
   ok = ok && make_map(&map_c, c, N, M, ldc, out_fp32 ? 32 : 64, 32, out_fp32 != 0);
   if (!ok) {
@@ -707,7 +784,7 @@ KB_API int kb200_gemm_fp8(const void* a, const void* b, void* c, const float* bi
   const int sm_count = kb_sm_count();
   GemmParams p{c, bias, M, N, K, ldc, 0, 0, act, out_fp32, err, 1, 0, 1 + a_format + 2 * b_format, alpha};
   const long long tiles = (long long)((M + v2::BM - 1) / v2::BM) * ((N + v2::BN - 1) / v2::BN);
-  gemm_bf16_tcgen05_persistent<<<(unsigned)(tiles < sm_count ? tiles : sm_count), THREADS, v2::SMEM_BYTES, stream>>>(map_a, map_b, map_c, p);
+  gemm_bf16_tcgen05_persistent<<<(unsigned)(tiles < sm_count ? tiles : sm_count), THREADS, v2::SMEM_BYTES, stream>>>(maps, p);
   KB_CHECK_LAUNCH("gemm_fp8");
   return 0;
 }
@@ -721,7 +798,8 @@ KB_API int kb200_gemm_i8(const void* a, const void* b, void* c, const float* bia
     kb200_set_error("gemm_i8: operands must be 16-byte aligned with pitches that are multiples of 16 bytes");
     return -2;
   }
-  CUtensorMap map_a, map_b, map_c;
+  GroupMaps maps;
+  CUtensorMap &map_a = maps.a[0], &map_b = maps.b[0], &map_c = maps.c[0];
   bool ok = make_map_u8(&map_a, a, K, M, lda, 128, v2::BM) && make_map_u8(&map_b, b, K, N, ldb, 128, v2::BN);
   ok = ok && make_map(&map_c, c, N, M, ldc, out_fp32 ? 32 : 64, 32, out_fp32 != 0);
   if (!ok) {
@@ -736,7 +814,7 @@ KB_API int kb200_gemm_i8(const void* a, const void* b, void* c, const float* bia
   const int sm_count = kb_sm_count();
   GemmParams p{c, bias, M, N, K, ldc, 0, 0, act, out_fp32, err, 1, 0, 0, nullptr, 1, row_scale, col_scale};
   const long long tiles = (long long)((M + v2::BM - 1) / v2::BM) * ((N + v2::BN - 1) / v2::BN);
-  gemm_bf16_tcgen05_persistent<<<(unsigned)(tiles < sm_count ? tiles : sm_count), THREADS, v2::SMEM_BYTES, stream>>>(map_a, map_b, map_c, p);
+  gemm_bf16_tcgen05_persistent<<<(unsigned)(tiles < sm_count ? tiles : sm_count), THREADS, v2::SMEM_BYTES, stream>>>(maps, p);
   KB_CHECK_LAUNCH("gemm_i8");
   return 0;
 }

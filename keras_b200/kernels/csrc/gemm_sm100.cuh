@@ -40,6 +40,16 @@ struct GemmParams {
   const float* col_scale = nullptr;
   const __nv_bfloat16* bias16 = nullptr;  // a bias in bf16 (instead of `bias`): a layer's 16-bit read of it needs no cast
   int accumulate = 0;                // 1: add the fp32 tile into C (TMA reduce store) instead of overwriting it
+  // Several products in one launch (1: a single one), with operands of their own and everything else in common:
+  //   side by side (sum_k = 0): B and C differ, N is the widest; tile_end: end of each product's column tiles
+  //   summed (sum_k = 1): A and B differ, one C; kb_end: end of each product's K blocks, all K multiples of a block
+  int groups = 1, sum_k = 0;
+  int tile_end[3] = {0, 0, 0}, width[3] = {0, 0, 0}, kb_end[3] = {0, 0, 0};
+  const void* bias_of[3] = {nullptr, nullptr, nullptr};  // fp32, or bf16 where bias16 is set
+};
+
+struct GroupMaps {
+  CUtensorMap a[3], b[3], c[3];
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -158,6 +168,21 @@ __device__ __forceinline__ float apply_act(float v, int act) {
   }
 }
 
+// The same for the 32 values of a lane, the choice made once: a branch a value keeps them from overlapping (gelu at [16384, 3072, 768]: 99 us
+// against 190).
+template <bool PRECISE, int ACT>
+__device__ __forceinline__ void apply_act_to(float* v) {
+#pragma unroll
+  for (int j = 0; j < 32; ++j) v[j] = apply_act<PRECISE>(v[j], ACT);
+}
+template <bool PRECISE>
+__device__ __forceinline__ void apply_act32(float* v, int act) {
+  if (act == ACT_GELU_ERF) apply_act_to<PRECISE, ACT_GELU_ERF>(v);
+  else if (act == ACT_RELU) apply_act_to<PRECISE, ACT_RELU>(v);
+  else if (act == ACT_SILU) apply_act_to<PRECISE, ACT_SILU>(v);
+  else if (act == ACT_GELU_TANH) apply_act_to<PRECISE, ACT_GELU_TANH>(v);
+}
+
 // Epilogue of one 32-row slice of an accumulator tile (rows `row0`.., `ncols` columns from TMEM address `tmem_row`).
 // The warp converts 128 bytes of each row at a time (64 bf16 or 32 fp32 columns), writes them into a swizzled
 // 32 x 128 B staging buffer (`stage`: two such buffers, 1024-byte aligned) and lets the TMA engine store that box, so
@@ -165,7 +190,7 @@ __device__ __forceinline__ float apply_act(float v, int act) {
 // the boxes this warp has issued (selects the staging buffer).  Lane 0 must run `cp.async.bulk.wait_group.read 0` before
 // the CTA exits.
 __device__ __forceinline__ void store_rows_tma(uint32_t tmem_row, int ncols, int n0, int row0, uint32_t stage, uint32_t& stores,
-                                               const CUtensorMap* map_c, const GemmParams& p, int lane) {
+                                               const CUtensorMap* map_c, const GemmParams& p, int lane, int N, const float* bias, const __nv_bfloat16* bias16) {
   const int cols_per_chunk = p.out_fp32 ? 32 : 64;
   const int chunks = ncols / cols_per_chunk;
   const uint32_t sw = (uint32_t)(lane & 7);
@@ -174,7 +199,17 @@ __device__ __forceinline__ void store_rows_tma(uint32_t tmem_row, int ncols, int
 #pragma unroll 1
   for (int c = 0; c < chunks; ++c) {
     const int col0 = n0 + c * cols_per_chunk;
-    if (col0 >= p.N) break;
+    if (col0 >= N) break;
+    // bias of this lane's column (of either half), handed round with shuffles: one load a column instead of one a value and lane
+    float lane_bias[2] = {0.f, 0.f};
+    const bool biased = bias != nullptr || bias16 != nullptr;
+    if (bias != nullptr) {
+      lane_bias[0] = __ldg(bias + min(col0 + lane, N - 1));
+      if (!p.out_fp32) lane_bias[1] = __ldg(bias + min(col0 + 32 + lane, N - 1));
+    } else if (bias16 != nullptr) {
+      lane_bias[0] = __bfloat162float(bias16[min(col0 + lane, N - 1)]);
+      if (!p.out_fp32) lane_bias[1] = __bfloat162float(bias16[min(col0 + 32 + lane, N - 1)]);
+    }
     uint32_t r[64];
     tmem_ld32(tmem_row + (uint32_t)(c * cols_per_chunk), r);
     if (!p.out_fp32) tmem_ld32(tmem_row + (uint32_t)(c * cols_per_chunk + 32), r + 32);
@@ -189,19 +224,13 @@ __device__ __forceinline__ void store_rows_tma(uint32_t tmem_row, int ncols, int
       for (int j = 0; j < 32; ++j) v[j] = (p.int8 ? __int2float_rn((int)r[j]) : __uint_as_float(r[j])) * alpha;
       if (p.col_scale != nullptr) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] *= __ldg(p.col_scale + min(col0 + j, p.N - 1));
+        for (int j = 0; j < 32; ++j) v[j] *= __ldg(p.col_scale + min(col0 + j, N - 1));
       }
-      if (p.bias != nullptr) {
+      if (biased) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] += __ldg(p.bias + min(col0 + j, p.N - 1));
-      } else if (p.bias16 != nullptr) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] += __bfloat162float(p.bias16[min(col0 + j, p.N - 1)]);
+        for (int j = 0; j < 32; ++j) v[j] += __shfl_sync(0xffffffffu, lane_bias[0], j);
       }
-      if (p.act != ACT_NONE) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = apply_act<true>(v[j], p.act);
-      }
+      apply_act32<true>(v, p.act);
 #pragma unroll
       for (int u = 0; u < 8; ++u)
         asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(buf + (((uint32_t)u ^ sw) << 4)), "f"(v[u * 4]), "f"(v[u * 4 + 1]),
@@ -214,19 +243,13 @@ __device__ __forceinline__ void store_rows_tma(uint32_t tmem_row, int ncols, int
         for (int j = 0; j < 32; ++j) v[j] = (p.int8 ? __int2float_rn((int)r[h * 32 + j]) : __uint_as_float(r[h * 32 + j])) * alpha;
         if (p.col_scale != nullptr) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] *= __ldg(p.col_scale + min(col0 + h * 32 + j, p.N - 1));
+          for (int j = 0; j < 32; ++j) v[j] *= __ldg(p.col_scale + min(col0 + h * 32 + j, N - 1));
         }
-        if (p.bias != nullptr) {
+        if (biased) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] += __ldg(p.bias + min(col0 + h * 32 + j, p.N - 1));
-        } else if (p.bias16 != nullptr) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] += __bfloat162float(p.bias16[min(col0 + h * 32 + j, p.N - 1)]);
+          for (int j = 0; j < 32; ++j) v[j] += __shfl_sync(0xffffffffu, lane_bias[h], j);
         }
-        if (p.act != ACT_NONE) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = apply_act<false>(v[j], p.act);
-        }
+        apply_act32<false>(v, p.act);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const bf16x8 pk = pack8(v + u * 8);
@@ -253,6 +276,34 @@ __device__ __forceinline__ void store_rows_tma(uint32_t tmem_row, int ncols, int
     if (row0 < p.M) ++stores;
   }
 }
+__device__ __forceinline__ void store_rows_tma(uint32_t tmem_row, int ncols, int n0, int row0, uint32_t stage, uint32_t& stores,
+                                               const CUtensorMap* map_c, const GemmParams& p, int lane) {
+  store_rows_tma(tmem_row, ncols, n0, row0, stage, stores, map_c, p, lane, p.N, p.bias, p.bias16);
+}
+// the same for the tile's product of a group
+__device__ __forceinline__ void store_rows_group(uint32_t tmem_row, int ncols, int n0, int row0, uint32_t stage, uint32_t& stores, const GroupMaps& maps, int g,
+                                                 const GemmParams& p, int lane) {
+  const bool one = p.groups == 1;
+  const void* bias = one ? (p.bias16 != nullptr ? (const void*)p.bias16 : (const void*)p.bias) : p.bias_of[g];
+  store_rows_tma(tmem_row, ncols, n0, row0, stage, stores, &maps.c[g], p, lane, one ? p.N : p.width[g], p.bias16 != nullptr ? nullptr : (const float*)bias,
+                 p.bias16 != nullptr ? (const __nv_bfloat16*)bias : nullptr);
+}
+// product of a column tile, and the column tiles before it
+__device__ __forceinline__ int group_of_tile(const GemmParams& p, int nt, int& first) {
+  first = 0;
+  if (p.groups == 1 || p.sum_k) return 0;
+  const int g = nt >= p.tile_end[0] ? (p.groups > 2 && nt >= p.tile_end[1] ? 2 : 1) : 0;
+  if (g > 0) first = p.tile_end[g - 1];
+  return g;
+}
+// product of a K block, and the K blocks before it
+__device__ __forceinline__ int group_of_block(const GemmParams& p, int kb, int& first) {
+  first = 0;
+  if (!p.sum_k) return 0;
+  const int g = kb >= p.kb_end[0] ? (p.groups > 2 && kb >= p.kb_end[1] ? 2 : 1) : 0;
+  if (g > 0) first = p.kb_end[g - 1];
+  return g;
+}
 
 
 // that keeps the CTAs running at the same time on neighbouring tiles (8 row-tiles per group) for L2 reuse.
@@ -271,7 +322,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-__device__ __forceinline__ void tile_coords(int t, int m_tiles, int n_tiles, int& m0, int& n0) {
+__device__ __forceinline__ void tile_coords(int t, int m_tiles, int n_tiles, int& m0, int& n0) {  // n0: of a single product
   const int per_group = v2::GROUP_M * n_tiles;
   const int g = t / per_group;
   const int first_m = g * v2::GROUP_M;

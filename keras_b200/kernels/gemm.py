@@ -194,6 +194,93 @@ class GemmFn(torch.autograd.Function):
         return (dx, dw, db, None, None, None)[: len(ctx.needs_input_grad)]
 
 
+def group(products, M, a_mn, b_mn, sum_k, split_k=1, accumulate=False):
+    """One launch for up to three products, each ``(a, b, c, bias)``: side by side (``c`` of their own, one ``a``), or summed into the first
+    one's ``c``.  ``N`` and ``K`` are read from ``b`` as the major flag says.  ``accumulate``: added to what the float32 ``c`` hold."""
+    lib = kops._lib()
+    n = len(products)
+    a0, _, c0, bias0 = products[0]
+    pointers, sizes, pitches = (ctypes.c_void_p * (4 * n))(), (ctypes.c_int * (2 * n))(), (ctypes.c_longlong * (3 * n))()
+    for i, (a, b, c, bias) in enumerate(products):
+        c = c0 if sum_k else c
+        pointers[4 * i:4 * i + 4] = [a.data_ptr(), b.data_ptr(), c.data_ptr(), bias.data_ptr() if bias is not None else None]
+        sizes[2 * i:2 * i + 2] = [b.shape[1], b.shape[0]] if b_mn else [b.shape[0], b.shape[1]]
+        pitches[3 * i:3 * i + 3] = [a.stride(0), b.stride(0), c.stride(0)]
+    bias16 = any(p[3] is not None and p[3].dtype == torch.bfloat16 for p in products)
+    code = lib.kb200_gemm_group(pointers, sizes, pitches, kops._i(n), kops._i(1 if sum_k else 0), kops._i(M), kops._i(a_mn), kops._i(b_mn),
+                                kops._i(1 if c0.dtype == torch.float32 else 0), kops._i(1 if bias16 else 0), kops._i(-max(1, split_k) if accumulate else split_k),
+                                kops._i(0), kops._p(_err_flag(a0.device)), kops._stream())
+    kops._check(code, "gemm_group")
+
+
+class ProjectionsFn(torch.autograd.Function):
+    """``x @ w_i (+ bias_i)`` for the three projections of an attention layer: one launch forward, one for the gradient of ``x`` (a sum over
+    the three in fp32, where three results in bf16 were added afterwards) and one for the weights' gradients."""
+
+    @staticmethod
+    def forward(ctx, x, targets, w0, w1, w2, *biases):
+        ws = (w0, w1, w2)
+        M = x.shape[0]
+        outs = [torch.empty((M, w.shape[1]), dtype=torch.bfloat16, device=x.device) for w in ws]
+        group([(x, w, o, b) for w, o, b in zip(ws, outs, [b.detach() for b in biases] or [None] * 3)], M, 0, 1, False)
+        ctx.save_for_backward(x, *ws, *biases)
+        ctx.targets = targets  # the parameters behind weights and biases, where their gradients may be added in place
+        return tuple(outs)
+
+    @staticmethod
+    def backward(ctx, *dys):
+        x, *rest = ctx.saved_tensors
+        ws, biases = rest[:3], rest[3:]
+        need = ctx.needs_input_grad
+        if torch.is_grad_enabled():  # a gradient of this gradient is wanted: differentiate the same products from library operations
+            operands = [t for t, n in zip((x, *ws, *biases), (need[0], *need[2:])) if n]
+            outs = [torch.matmul(x, w) + (biases[i] if biases else 0) for i, w in enumerate(ws)]
+            grads = iter(torch.autograd.grad(outs, operands, dys, create_graph=True))
+            picked = [next(grads) if n else None for n in (need[0], *need[2:])]
+            return (picked[0], None, *picked[1:])
+        dys = [dy if _ok_2d(dy) else kops.aligned(dy) for dy in dys]
+        M, K = x.shape
+        dx = None
+        if need[0]:
+            dx = torch.empty((M, K), dtype=torch.bfloat16, device=x.device)
+            group([(dy, w, dx, None) for dy, w in zip(dys, ws)], M, 0, 0, True)
+        dws = [None] * 3
+        if any(need[2:5]):
+            slots = [shadow.grad_slot(t, w.shape) if n else None for t, w, n in zip(ctx.targets[:3], ws, need[2:5])]
+            if all(s is not None for s in slots):
+                split = split_k_for(K, sum(w.shape[1] for w in ws), M, x.device)
+                group([(x, dy, s.view(w.shape), None) for dy, w, s in zip(dys, ws, slots)], K, 1, 1, False, split_k=split, accumulate=True)
+            else:
+                for i, (dy, w, s) in enumerate(zip(dys, ws, slots)):
+                    if need[2 + i]:
+                        into = s.view(w.shape) if s is not None else None
+                        made = gemm(x, dy, 1, 1, K, w.shape[1], M, split_k=split_k_for(K, w.shape[1], M, x.device), accumulate_into=into)
+                        dws[i] = made if s is None else None
+        dbs = [None] * len(biases)
+        for i, b in enumerate(biases):
+            if need[5 + i]:
+                s = shadow.grad_slot(ctx.targets[3 + i], b.shape)
+                made = kops.column_sum(dys[i], accumulate_into=s.view(-1) if s is not None else None)
+                dbs[i] = made.to(b.dtype) if s is None else None
+        return (dx, None, *dws, *dbs)
+
+
+def projections(x, kernels, biases, weights):
+    """The three projections of ``x`` [..., K] by ``kernels`` (variables that read as ``weights``, [K, heads, size]) as [..., heads, size], or
+    ``None`` where their products do not fit one launch."""
+    K = x.shape[-1]
+    x2 = x.reshape(-1, K)
+    flat = [w.reshape(K, -1) for w in weights]
+    if K % 64 or any(w.shape[1] % 64 or not _qualifies(x2, w) for w in flat):
+        return None
+    bs = [b.value.reshape(-1) for b in biases]
+    if any(b.dtype != bs[0].dtype or b.dtype not in (torch.float32, torch.bfloat16) or not b.is_contiguous() for b in bs):
+        return None
+    targets = [_grad_target(k, w) for k, w in zip(kernels, weights)] + [_grad_target(v, b) for v, b in zip(biases, bs)]
+    outs = ProjectionsFn.apply(x2, targets, *flat, *bs)
+    return tuple(o.reshape(tuple(x.shape[:-1]) + tuple(w.shape[1:])) for o, w in zip(outs, weights))
+
+
 def _qualifies(x2, w):
     if not (_ok_2d(x2) and _ok_2d(w, any_width=True)):
         return False

@@ -50,6 +50,12 @@ def _attention_equations(rank, attn_axes):
     return dot, combine, len(product)
 
 
+def _joint_projections(layer, x):
+    from keras_b200.models import direct
+
+    return direct.joint_projections(layer, x)
+
+
 def _full_shape(rank, last):
     return [None] * (rank - len(last)) + list(last)
 
@@ -240,9 +246,13 @@ class MultiHeadAttention(Layer):
             projections = [self._query_dense, self._key_dense, self._value_dense] + ([self._gate_dense] if self._use_gate else [])
             tp = tensor_parallel.mark_attention(self, projections, self._output_dense)
         gate = self._gate_dense(query) if self._use_gate else None
-        q = self._query_dense(query)
-        k = self._key_dense(key)
-        v = self._value_dense(value)
+        joint = _joint_projections(self, query) if query is value and query is key and tp is None else None
+        if joint is not None:
+            q, k, v = joint
+        else:
+            q = self._query_dense(query)
+            k = self._key_dense(key)
+            v = self._value_dense(value)
         out = scores = None
         if padding_only:
             out = self._attend_padded(q, k, v, query_mask, value_mask, key_mask)
@@ -425,9 +435,13 @@ class GroupedQueryAttention(Layer):
             projections = [self._query_dense, self._key_dense, self._value_dense] + ([self._gate_dense] if self.use_gate else [])
             tp = tensor_parallel.mark_attention(self, projections, self._output_dense)
         gate = self._gate_dense(query) if self.use_gate else None
-        q = self._query_dense(query)
-        k = self._key_dense(key)
-        v = self._value_dense(value)
+        joint = _joint_projections(self, query) if query is value and query is key and tp is None else None
+        if joint is not None:
+            q, k, v = joint
+        else:
+            q = self._query_dense(query)
+            k = self._key_dense(key)
+            v = self._value_dense(value)
         out, scores = self._compute_attention(q, k, v, attention_mask=attention_mask, training=training)
         if gate is not None:
             out = ops.multiply(out, gate)

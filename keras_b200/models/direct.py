@@ -17,6 +17,7 @@ from keras_b200.core import global_state
 from keras_b200.core.keras_tensor import KerasTensor
 from keras_b200.core.variables import Variable, get_stateless_scope
 from keras_b200.kernels import attention as kattention
+from keras_b200.kernels import dispatch
 from keras_b200.kernels import gemm as kgemm
 from keras_b200.kernels import ops as kops
 from keras_b200.layers import layer as layer_module
@@ -367,6 +368,30 @@ def _attention(layer, x, causal, mask=None):
         return None
     out = _product(out.view(B, T, heads * size), [parts[3][0]], [parts[3][1]], 0)
     return None if out is None else _pass_mask(out[:, :parts[3][0].shape[2]].view(B, T, -1), mask)
+
+
+def joint_projections(layer, x):
+    """Query, key and value of a self-attention layer's call with gradients from one launch each way, or ``None``."""
+    d = layer.__dict__
+    if type(x) is not torch.Tensor or x.dtype != _BF16 or x.ndim != 3 or not torch.is_grad_enabled() or not dispatch.enabled(x) or not usable(x) or not _ordinary(layer):
+        return None
+    subs = [d["_query_dense"], d["_key_dense"], d["_value_dense"]]
+    for sub in subs:
+        s = sub.__dict__
+        if (type(sub) is not EinsumDense or not _ordinary(sub) or s["_input_spec"] is not None or s["lora_enabled"] or s["_gemm"] != (1, 2)
+                or not (s["activation"] is None or s["activation"] is activations.linear) or type(s.get("_kernel")) is not Variable
+                or s["_kernel"]._shard_slices is not None or s["_kernel"].shape[0] != x.shape[-1]):
+            return None
+    biases = [sub.__dict__["bias"] for sub in subs]
+    if all(b is None for b in biases):
+        biases = []
+    elif any(type(b) is not Variable or tuple(b.shape) != tuple(sub.__dict__["_kernel"].shape[1:]) for b, sub in zip(biases, subs)):
+        return None
+    kernels = [sub.__dict__["_kernel"] for sub in subs]
+    weights = [k.value for k in kernels]  # in the layer's type: its call has set the scope
+    if any(w.dtype != _BF16 or w.ndim != 3 for w in weights) or not (x.requires_grad or any(w.requires_grad for w in weights)):
+        return None
+    return kgemm.projections(x, kernels, biases, weights)
 
 
 def _sub_ordinary(layer):

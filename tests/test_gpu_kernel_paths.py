@@ -228,3 +228,76 @@ def test_add_and_norm_second_derivatives():
         second.append(torch.autograd.grad((g ** 2).sum(), [a, b, gamma]))
     for p, q in zip(*second):
         assert torch.allclose(p, q, rtol=1e-4, atol=1e-4 * q.abs().max().item())
+
+
+# ------------------------------------------------------------------------------------------------ several products in one launch
+@pytest.mark.parametrize("variant", [1, 2, 3])
+@pytest.mark.parametrize("M,K,widths", [(128, 64, (64, 64, 64)), (333, 192, (128, 64, 64)), (2664, 512, (512, 512, 512)), (300, 256, (1024, 256, 256)), (200, 64, (320, 72))])
+def test_grouped_products(variant, M, K, widths):
+    from keras_b200.kernels import gemm
+    from keras_b200.kernels import ops as kops
+
+    g = torch.Generator(device="cuda").manual_seed(M)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").bfloat16()  # noqa: E731
+    x, ws, dys = rnd(M, K), [rnd(K, n) for n in widths], [rnd(M, n) for n in widths]
+    bs = [torch.randn(n, generator=g, device="cuda") for n in widths]
+    real = kops._lib().kb200_gemm_group
+    plain, kops._lib().kb200_gemm_group = real, lambda *a: real(*a[:11], kops._i(variant), *a[12:])  # this kernel, whatever the rule says
+    try:
+        for biases in ([None] * len(ws), bs, [b.bfloat16() for b in bs]):
+            outs = [torch.empty(M, n, device="cuda", dtype=torch.bfloat16) for n in widths]
+            gemm.group([(x, w, o, b) for w, o, b in zip(ws, outs, biases)], M, 0, 1, False)
+            for w, o, b in zip(ws, outs, biases):
+                assert _rel(o, x.double() @ w.double() + (0 if b is None else b.double())) < 2.0 ** -8
+        for split in (1, 2):
+            if variant == 1 and split > 1:
+                continue
+            grads = [torch.full((K, n), 3.0, device="cuda") for n in widths]
+            gemm.group([(x, dy, d, None) for dy, d in zip(dys, grads)], K, 1, 1, False, split_k=split, accumulate=True)
+            for dy, d in zip(dys, grads):
+                assert _rel(d, 3.0 + x.double().t() @ dy.double()) < 2.0 ** -17
+        if all(n % 64 == 0 for n in widths):
+            dx = torch.empty(M, K, device="cuda", dtype=torch.bfloat16)
+            gemm.group([(dy, w, dx, None) for dy, w in zip(dys, ws)], M, 0, 0, True)
+            assert _rel(dx, sum(dy.double() @ w.double().t() for dy, w in zip(dys, ws))) < 2.0 ** -8
+    finally:
+        kops._lib().kb200_gemm_group = plain
+    gemm.check_errors()
+
+
+@pytest.mark.parametrize("grouped,bias", [(False, False), (False, True), (True, True)])
+def test_attention_layers_take_their_projections_together(grouped, bias, monkeypatch):
+    """The same outputs and gradients as three layers of their own, inside and outside an arena's backward pass."""
+    import keras_b200 as keras
+    from keras_b200.kernels import gemm
+
+    def step(joint):
+        keras.utils.set_random_seed(5)
+        keras.config.set_dtype_policy("mixed_bfloat16")
+        try:
+            i = keras.Input((96, 256))
+            layer = keras.layers.GroupedQueryAttention(64, 4, 2, use_bias=bias) if grouped else keras.layers.MultiHeadAttention(4, 64, use_bias=bias)
+            h = keras.layers.LayerNormalization()(keras.layers.Dense(256)(i))
+            model = keras.Model(i, keras.layers.Dense(8)(layer(h, h, use_causal_mask=True)))
+        finally:
+            keras.config.set_dtype_policy("float32")
+        if not joint:
+            monkeypatch.setattr(gemm, "projections", lambda *a: None)
+        used = []
+        plain = gemm.ProjectionsFn.apply
+        monkeypatch.setattr(gemm.ProjectionsFn, "apply", lambda *a: (used.append(1), plain(*a))[1])
+        x = torch.randn(4, 96, 256, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1), requires_grad=True)
+        model(x)
+        y = model(x)
+        grads = torch.autograd.grad((y.float() ** 2).sum(), [x] + [v.value for v in model.trainable_variables])
+        model.compile(keras.optimizers.SGD(0.1, momentum=0.9), "mse")
+        for _ in range(3):
+            model.train_on_batch(x.detach(), torch.zeros(4, 96, 8, device="cuda"))
+        monkeypatch.undo()
+        assert bool(used) == joint
+        return [y, *grads, *[v.value.detach().clone() for v in model.trainable_variables]]
+
+    for a, b in zip(step(True), step(False)):
+        # bf16 gradients; the input's is rounded once instead of three times.  A key's bias has none: what is there is rounding
+        assert _rel(a.float(), b.double()) < 0.02 or b.abs().max() < 1e-5
+    gemm.check_errors()
