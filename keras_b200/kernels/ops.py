@@ -519,6 +519,28 @@ def activation_backward(dy, z, act, want_sums=False, accumulate_into=None):
 
 
 # ----------------------------------------------------------------- softmax cross-entropy
+_EXPECTED = threading.local()
+
+
+class gradient_follows:
+    """Scope of a loss whose gradient is taken in the same step, unscaled.  ``upstream(rows)``, set inside it by the reduction that knows, is
+    the gradient that every row's loss will receive; ``FusedSoftmaxXent`` then computes the logits' gradient while it has the row."""
+
+    def __enter__(self):
+        _EXPECTED.on, _EXPECTED.upstream = True, None
+        return self
+
+    def __exit__(self, *exc):
+        _EXPECTED.on, _EXPECTED.upstream = False, None
+        return False
+
+
+def expect_upstream(fn):
+    """Called by a loss before its values are computed: ``fn(number of values)`` is the gradient of its result by each of them, or ``None``."""
+    if getattr(_EXPECTED, "on", False):
+        _EXPECTED.upstream = fn
+
+
 class FusedSoftmaxXent(torch.autograd.Function):
     """Per-row loss in float32 from logits of any float dtype.  Logits may be the leading columns of a wider buffer
     (rows with a uniform pitch, as a padded GEMM returns them); the gradient then has the same pitch and zeroed padding."""
@@ -535,10 +557,19 @@ class FusedSoftmaxXent(torch.autograd.Function):
         labels64 = labels.reshape(-1).to(torch.int64).contiguous()
         out = torch.empty(2 * rows, dtype=torch.float32, device=logits.device)
         loss, lse = out[:rows], out[rows:]
-        _check(lib.kb200_xent_fwd(_p(flat), _p(labels64), _p(loss), _p(lse), _ll(rows), _i(V), _ll(ld), _i(_dt(flat)), _stream()), "xent_fwd")
+        upstream = getattr(_EXPECTED, "upstream", None)
+        # the gradient made here, and the upstream gradient that it is for; the first backward pass takes it
+        ctx.made, ctx.made_for = None, 0.0
+        zero_to = ld if ld - V < 16 else V
+        if upstream is not None and ctx.needs_input_grad[0] and lib.kb200_xent_wide(_i(V)):
+            ctx.made, ctx.made_for = torch.empty((rows, ld), dtype=flat.dtype, device=flat.device), float(upstream(rows))
+            _check(lib.kb200_xent_fwd_grad(_p(flat), _p(labels64), _p(loss), _p(lse), _p(ctx.made), _f(ctx.made_for), _ll(rows), _i(V), _ll(ld), _i(zero_to),
+                                           _i(_dt(flat)), _stream()), "xent_fwd_grad")
+        else:
+            _check(lib.kb200_xent_fwd(_p(flat), _p(labels64), _p(loss), _p(lse), _ll(rows), _i(V), _ll(ld), _i(_dt(flat)), _stream()), "xent_fwd")
         ctx.save_for_backward(flat, labels64, lse)
         ctx.logits_shape = tuple(logits.shape)
-        ctx.ld = ld
+        ctx.ld, ctx.zero_to = ld, zero_to
         return loss.reshape(labels.shape)
 
     @staticmethod
@@ -548,10 +579,12 @@ class FusedSoftmaxXent(torch.autograd.Function):
         rows, V = flat.shape
         ld = ctx.ld
         dl = dloss.reshape(-1).float().contiguous()
-        buf = torch.empty((rows, ld), dtype=flat.dtype, device=flat.device)
-        zero_to = ld if ld - V < 16 else V
-        _check(lib.kb200_xent_bwd(_p(flat), _p(labels64), _p(lse), _p(dl), _p(buf), _ll(rows), _i(V), _ll(ld), _i(zero_to), _i(_dt(flat)), _stream()),
-               "xent_bwd")
+        buf, ctx.made = ctx.made, None
+        done = buf is not None
+        if not done:
+            buf = torch.empty((rows, ld), dtype=flat.dtype, device=flat.device)
+        _check(lib.kb200_xent_bwd(_p(flat), _p(labels64), _p(lse), _p(dl), _p(buf), _ll(rows), _i(V), _ll(ld), _i(ctx.zero_to), _i(1 if done else 0),
+                                  _f(ctx.made_for), _i(_dt(flat)), _stream()), "xent_bwd")
         dlogits = buf if ld == V else buf[:, :V]
         return dlogits.reshape(ctx.logits_shape), None
 

@@ -12,6 +12,7 @@ from keras_b200.core.dtypes import to_torch_dtype
 from keras_b200.core.export_registry import keras_export
 from keras_b200.core.naming import auto_name
 from keras_b200.core.tensor import convert_to_tensor
+from keras_b200.kernels import ops as kops
 from keras_b200.ops.operation import KerasSaveable
 
 
@@ -31,13 +32,23 @@ class Loss(KerasSaveable):
         """True when ``call`` computes in float32 from half-precision predictions by itself (no up-cast copy needed)."""
         return False
 
+    def _values_as_computed(self):
+        """True when ``call`` returns the values of a kernel that can make their gradient at once, and does nothing to them."""
+        return False
+
     def __call__(self, y_true, y_pred, sample_weight=None):
         in_mask = getattr(y_pred, "_keras_mask", None)
         td = to_torch_dtype(self.dtype)
         if not self._accepts_low_precision(y_pred):
             y_pred = tree.map_structure(lambda x: convert_to_tensor(x, dtype=td), y_pred)
         y_true = tree.map_structure(lambda x: _convert_true(x, td), y_true)
+        # what a kernel may rely on to make the gradient beside the loss (it checks): each value's share of an unweighted result
+        share = None
+        if sample_weight is None and in_mask is None and self._values_as_computed():
+            share = {"sum": lambda n: 1.0}.get(self.reduction, lambda n: 1.0 / n) if self.reduction not in (None, "none") else None
+        kops.expect_upstream(share)
         losses = self.call(y_true, y_pred)
+        kops.expect_upstream(None)
         out_mask = getattr(losses, "_keras_mask", None)
         if in_mask is not None and out_mask is not None:
             mask = in_mask & out_mask

@@ -39,6 +39,10 @@ class LossFunctionWrapper(Loss):
 
         return self.dtype == "float32" and dispatch.enabled(y_pred) and y_pred.shape[-1] >= 64
 
+    def _values_as_computed(self):
+        return (self.fn is sparse_categorical_crossentropy and type(self).call is LossFunctionWrapper.call
+                and self._fn_kwargs.get("from_logits") is True and self._fn_kwargs.get("ignore_class") is None)
+
     def call(self, y_true, y_pred):
         y_true_y_pred = tree.map_structure(squeeze_or_expand_to_same_rank, y_true, y_pred)
         y_true = tree.map_structure_up_to(y_true, lambda x: x[0], y_true_y_pred)

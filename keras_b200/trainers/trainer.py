@@ -12,6 +12,7 @@ forward → zero grads → loss → scale → backward → optimizer).  Differen
   wrapper, and metric state is reduced once per read as one packed buffer.
 """
 
+import contextlib
 import inspect
 import platform
 import warnings
@@ -26,6 +27,8 @@ from keras_b200.core.dtypes import standardize_dtype
 from keras_b200.core.export_registry import keras_export
 from keras_b200.core.keras_tensor import KerasTensor
 from keras_b200.core.tensor import convert_to_tensor, get_device
+from keras_b200.kernels import ops as kops
+from keras_b200.optimizers.base_optimizer import BaseOptimizer
 from keras_b200.trainers import data_adapters
 from keras_b200.trainers.compile_utils import CompileLoss, CompileMetrics
 from keras_b200.trainers.data_adapters import data_adapter_utils
@@ -268,7 +271,11 @@ class Trainer:
             y_pred = self(x, training=True)
         else:
             y_pred = self(x)
-        loss = self._compute_loss(x=x, y=y, y_pred=y_pred, sample_weight=sample_weight, training=True)
+        # alone on its device, with unweighted and unscaled losses, a step takes the gradient that its losses' reductions spread
+        plain = (self._parallel_engine is None and self.trainable_weights and self._compile_loss is not None and not self._compile_loss._user_loss_weights
+                 and (self.optimizer is None or (type(self.optimizer).scale_loss is BaseOptimizer.scale_loss and self.optimizer.loss_scale_factor is None)))
+        with kops.gradient_follows() if plain else contextlib.nullcontext():
+            loss = self._compute_loss(x=x, y=y, y_pred=y_pred, sample_weight=sample_weight, training=True)
         self._loss_tracker.update_state(loss, sample_weight=next(i for i in tree.flatten(x) if i is not None).shape[0])
         trainable_weights = self.trainable_weights
         if trainable_weights:

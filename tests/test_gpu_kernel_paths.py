@@ -301,3 +301,33 @@ def test_attention_layers_take_their_projections_together(grouped, bias, monkeyp
         # bf16 gradients; the input's is rounded once instead of three times.  A key's bias has none: what is there is rounding
         assert _rel(a.float(), b.double()) < 0.02 or b.abs().max() < 1e-5
     gemm.check_errors()
+
+
+# ------------------------------------------------------------------------------------------------ cross-entropy with its gradient
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,V,ld", [(3, 2049, 2056), (130, 5001, 5008), (65, 8009, 8016), (64, 50257, 50264)])
+def test_cross_entropy_that_makes_its_gradient_ahead(rows, V, ld, dtype):
+    from keras_b200.kernels import ops as kops
+
+    buf = (torch.randn(rows, ld, device="cuda") * 3).to(dtype)
+    buf[:, 3:17] = float("-inf")
+    labels = torch.randint(20, V, (rows,), device="cuda")
+    labels[1] = -1
+    expected = torch.full((rows,), 1.0 / rows, device="cuda")
+    other = expected.clone()
+    other[::3] *= 2
+    other[2] = float("nan")
+    results = []
+    for ahead in (True, False):
+        for upstream in (expected, other, torch.zeros_like(expected)):
+            logits = buf.clone()[:, :V].requires_grad_(True)
+            with kops.gradient_follows():
+                if ahead:
+                    kops.expect_upstream(lambda n: 1.0 / n)
+                loss = kops.FusedSoftmaxXent.apply(logits, labels)
+            first = torch.autograd.grad(loss, logits, upstream, retain_graph=True)[0].clone()
+            again = torch.autograd.grad(loss, logits, upstream)[0]  # a second pass has no gradient made ahead
+            assert torch.equal(first, again) or upstream is other and torch.equal(first.nan_to_num(), again.nan_to_num())
+            results.append((loss.detach(), first.nan_to_num()))
+    for (la, ga), (lb, gb) in zip(results[:3], results[3:]):
+        assert torch.equal(la, lb) and torch.equal(ga, gb)
