@@ -37,6 +37,12 @@ def matmul(a, b):
 def dense(x, kernel, bias, activation_name, kernel_shape=None, value=None):
     if not enabled(x):
         return None
+    if x.dtype == torch.float32:
+        if kernel_shape is not None or x.ndim < 2:
+            return None
+        from keras_b200.kernels import sgemm
+
+        return sgemm.dense(x, kernel, bias, activation_name)
     from keras_b200.kernels import gemm
 
     return gemm.dense(x, kernel, bias, activation_name, kernel_shape, value)

@@ -331,3 +331,40 @@ def test_cross_entropy_that_makes_its_gradient_ahead(rows, V, ld, dtype):
             results.append((loss.detach(), first.nan_to_num()))
     for (la, ga), (lb, gb) in zip(results[:3], results[3:]):
         assert torch.equal(la, lb) and torch.equal(ga, gb)
+
+
+# ------------------------------------------------------------------------------------------------ float32 products of few rows
+@pytest.mark.parametrize("M,K,N", [(1, 16, 1), (16, 17, 64), (77, 130, 33), (128, 784, 512), (128, 512, 10), (256, 500, 1000), (64, 64, 64), (65, 2048, 65)])
+@pytest.mark.parametrize("relu,bias", [(True, True), (False, False), (False, True)])
+def test_float32_dense_products(M, K, N, relu, bias):
+    from keras_b200.kernels import sgemm
+
+    g = torch.Generator(device="cuda").manual_seed(M)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")  # noqa: E731
+    mine = [rnd(M, K).requires_grad_(True), (rnd(K, N) * K ** -0.5).requires_grad_(True)] + ([rnd(N).requires_grad_(True)] if bias else [])
+    out = sgemm.DenseFn.apply(mine[0], mine[1], mine[2] if bias else None, None, None, relu)
+    exact = [t.detach().double().requires_grad_(True) for t in mine]
+    ref = exact[0] @ exact[1] + (exact[2] if bias else 0)
+    ref = ref * (out.detach() > 0) if relu else ref  # the rectifier as the fp32 sum decides it
+    up = rnd(M, N)
+    assert _rel(out, ref) < 2e-6 or not ref.any()  # fp32 products, sums of at most 2048 of them
+    for a, b in zip(torch.autograd.grad(out, mine, up), torch.autograd.grad(ref, exact, up.double())):
+        assert _rel(a, b) < 2e-6 or not b.any()
+
+
+def test_float32_dense_layer_keeps_nan_and_second_derivatives():
+    import keras_b200 as keras
+
+    layer = keras.layers.Dense(32, activation="relu")
+    x = torch.randn(8, 48, device="cuda", requires_grad=True)
+    y = layer(x)
+    assert "DenseFn" in str(type(y.grad_fn)) or any("DenseFn" in str(type(f[0])) for f in y.grad_fn.next_functions)
+    w, b = (v.value for v in layer.trainable_variables)
+    second = []
+    for out in (y, torch.relu(x @ w + b)):
+        (g,) = torch.autograd.grad((out ** 3).sum(), x, create_graph=True)
+        second.append(torch.autograd.grad((g ** 2).sum(), w)[0])
+    assert torch.allclose(second[0], second[1], rtol=1e-4, atol=1e-5 * second[1].abs().max().item())
+    bad = x.detach().clone()
+    bad[0, 0] = float("nan")
+    assert layer(bad)[0].isnan().all() and not layer(bad)[1:].isnan().any()
