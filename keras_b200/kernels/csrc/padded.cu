@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(THREADS) add_rows_kernel(const __nv_bfloat16* 
 }
 
 // A batch on its way into a recorded step: its copy and its bf16 rounding from one read.  [256, 56, 56, 256]: copy 251 us and cast 174 us
-// -> 349 us together; the 2.06 GB take 310.
+// -> 349 us together; the 2.06 GB take 310.  Where the step reads nothing but the rounding, the copy is left out (dst null): 180 us, 1.23 GB.
 __global__ void __launch_bounds__(THREADS) copy_cast_kernel(const float4* __restrict__ src, float4* __restrict__ dst, uint4* __restrict__ dst16, long long vecs) {
   constexpr int U = 2;
   const long long step = (long long)gridDim.x * THREADS;
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(THREADS) copy_cast_kernel(const float4* __rest
     for (int u = 0; u < U; ++u) {
       const long long v = v0 + u * step;
       if (v < vecs) {
-        dst[2 * v] = a[u][0], dst[2 * v + 1] = a[u][1];
+        if (dst != nullptr) dst[2 * v] = a[u][0], dst[2 * v + 1] = a[u][1];
         const float f[8] = {a[u][0].x, a[u][0].y, a[u][0].z, a[u][0].w, a[u][1].x, a[u][1].y, a[u][1].z, a[u][1].w};
         const bf16x8 h = pack8(f);
         dst16[v] = reinterpret_cast<const uint4&>(h);
@@ -90,7 +90,7 @@ KB_API int kb200_add_rows(const void* src, long long ld, float* dst, int rows, i
   return 0;
 }
 
-// dst = src and dst16 = its rounding to bf16: n values, a multiple of 8, all 16-byte aligned
+// dst = src (unless null) and dst16 = its rounding to bf16: n values, a multiple of 8, all 16-byte aligned
 KB_API int kb200_copy_cast(const void* src, void* dst, void* dst16, long long n, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (n % 8 || (((uintptr_t)src | (uintptr_t)dst | (uintptr_t)dst16) & 15)) {

@@ -690,14 +690,16 @@ def add_rows(dst, src):
 
 
 def copy_and_cast(src, dst, dst16):
-    """``dst.copy_(src)`` and ``dst16.copy_(src)`` (bf16) of one fp32 tensor, from one read of it where it is laid out for that."""
-    if (src.is_cuda and src.device == dst.device == dst16.device and src.dtype == dst.dtype == torch.float32 and dst16.dtype == torch.bfloat16
-            and src.is_contiguous() and dst.is_contiguous() and dst16.is_contiguous() and src.shape == dst.shape == dst16.shape
-            and src.numel() % 8 == 0 and not (src.data_ptr() | dst.data_ptr() | dst16.data_ptr()) % 16):
+    """``dst.copy_(src)`` and ``dst16.copy_(src)`` (bf16) of one fp32 tensor, from one read of it where it is laid out for that.  ``dst``:
+    ``None`` where only the rounding is wanted."""
+    made = (dst16,) if dst is None else (dst, dst16)
+    if (src.is_cuda and src.dtype == torch.float32 and dst16.dtype == torch.bfloat16 and (dst is None or dst.dtype == torch.float32) and src.is_contiguous()
+            and src.numel() % 8 == 0 and not src.data_ptr() % 16
+            and all(t.device == src.device and t.shape == src.shape and t.is_contiguous() and not t.data_ptr() % 16 for t in made)):
         _check(_lib().kb200_copy_cast(_p(src), _p(dst), _p(dst16), _ll(src.numel()), _stream()), "copy_cast")
     else:
-        dst.copy_(src, non_blocking=True)
-        dst16.copy_(dst)
+        for t in made:
+            t.copy_(src, non_blocking=True)
 
 
 def cast_f32_to_bf16(src, dst):

@@ -190,10 +190,27 @@ class GraphedTrainStep:
         self.launches_per_replay = kops.launch_count() - launches_before
         kops.add_launches(-self.launches_per_replay)
         self.graph, self.signature, self.static_leaves, self.input_casts = graph, sig, static, input_casts
+        self.rounded_only = {0} if 0 in input_casts and self._only_rounded(data) else set()
         self.out_structure, self.out_type = raw, type(logs)
         self.out_leaves, self.out_packed, self.out_packed_index = out_leaves, packed, packed_index
         # capture records the step without running it: this batch is the first replay
         return self._replay(leaves, copy_inputs=False)
+
+    def _only_rounded(self, data):
+        """Whether the recorded step reads its first leaf, the model's one input, through its rounding alone: a stock step of a stock graph
+        whose input goes to convolution blocks, each of which reads the rounding (``fusion.shared_cast``), and nowhere else."""
+        from keras_b200.models.functional import Functional
+        from keras_b200.trainers.trainer import Trainer
+
+        model = self.model
+        stock = [(Trainer, n) for n in ("train_step", "compute_loss", "compute_metrics", "_compute_loss")] + [(Functional, n) for n in ("call", "__call__")]
+        if not isinstance(model, Functional) or any(n in vars(model) or getattr(type(model), n) is not getattr(c, n) for c, n in stock):
+            return False
+        if not isinstance(data, (tuple, list)) or not isinstance(data[0], torch.Tensor) or len(model._inputs) != 1 or model._fusion_plan is None:
+            return False
+        entry = model._inputs[0]
+        readers = [n for n in model._ordered_nodes() if any(t is entry for t in n.input_tensors)]
+        return bool(readers) and all(model._fusion_plan.get(id(n)) == "conv_fold_bias" for n in readers) and all(t is not entry for t in model._outputs)
 
     def _resync_host_state(self):
         """Recording a step runs its Python side (the optimizer's host mirror of the iteration counter moved) but not its
@@ -206,7 +223,7 @@ class GraphedTrainStep:
         if copy_inputs:
             for i, (dst, src) in enumerate(zip(self.static_leaves, leaves)):
                 if i in self.input_casts:
-                    kops.copy_and_cast(src, dst, self.input_casts[i])
+                    kops.copy_and_cast(src, None if i in self.rounded_only else dst, self.input_casts[i])
                 elif isinstance(dst, torch.Tensor):
                     dst.copy_(src, non_blocking=True)
         else:

@@ -368,3 +368,33 @@ def test_float32_dense_layer_keeps_nan_and_second_derivatives():
     bad = x.detach().clone()
     bad[0, 0] = float("nan")
     assert layer(bad)[0].isnan().all() and not layer(bad)[1:].isnan().any()
+
+
+# ------------------------------------------------------------------------------------------------ a recorded step that reads a rounded batch
+@pytest.mark.parametrize("other_reader", [False, True])
+def test_recorded_step_copies_what_it_reads(other_reader):
+    """New batches reach a step whose input only convolutions read, and one whose input something else reads too."""
+    import keras_b200 as keras
+
+    def run(graph):
+        keras.utils.set_random_seed(6)
+        keras.config.set_dtype_policy("mixed_bfloat16")
+        try:
+            i = keras.Input((12, 12, 16))
+            h = keras.layers.ReLU()(keras.layers.BatchNormalization()(keras.layers.Conv2D(32, 1, use_bias=False)(i)))
+            out = keras.layers.Dense(4)(keras.layers.GlobalAveragePooling2D()(h))
+            if other_reader:
+                out = keras.layers.Add()([out, keras.layers.Dense(4)(keras.layers.GlobalAveragePooling2D()(i))])
+            model = keras.Model(i, out)
+        finally:
+            keras.config.set_dtype_policy("float32")
+        model.compile(keras.optimizers.SGD(0.05), keras.losses.SparseCategoricalCrossentropy(from_logits=True), jit_compile="auto" if graph else False)
+        losses = []
+        for k in range(7):
+            g = torch.Generator(device="cuda").manual_seed(k)
+            x = torch.randn(64, 12, 12, 16, generator=g, device="cuda")
+            losses.append(float(model.train_on_batch(x, torch.randint(0, 4, (64,), generator=g, device="cuda"))))
+        return losses, getattr(model, "_graph_step", None)
+
+    recorded, eager = run(True)[0], run(False)[0]
+    assert max(abs(a - b) for a, b in zip(recorded, eager)) < 2e-2, (recorded, eager)
