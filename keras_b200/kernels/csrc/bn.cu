@@ -5,11 +5,12 @@
 // by: one statistics pass (per-channel sum / sum of squares, fp32 accumulation, E[x^2]-E[x]^2
 // variance as the reference), a C-sized finalize (scale/shift, moving statistics update) and one
 // apply pass y = relu(x*scale + shift + residual) with bf16 or fp32 I/O.  Backward is one
-// reduction pass, a C-sized coefficient kernel and one apply pass dx = A*dy' + B*x + C.
+// reduction pass and one apply pass dx = a*dy' + b*x + c (bn.cuh).
 //
 // All passes are HBM-bound.  Work split: a thread owns one 16-byte channel vector for the whole
 // kernel (its per-channel coefficients live in registers, no index arithmetic per element) and
 // walks rows with four independent 16-byte loads in flight per tensor.
+#include "bn.cuh"
 #include "common.cuh"
 
 template <typename T>
@@ -33,7 +34,7 @@ struct Vec<float> {
 
 // bn_stream.cu: the two-input passes on a shared-memory ring fed by bulk copies (bf16); returns 1 when it does not apply
 int kb200_bn_stream_launch(int mode, const void* in0, const void* in1, const unsigned char* bits_in, void* out0, void* out1, unsigned char* bits_out,
-                           const float* p0, const float* p1, const float* p2, float* sums, long long M, int C, int relu, cudaStream_t stream);
+                           const float* p0, const float* p1, const BnCoef* coef, float* sums, long long M, int C, int relu, cudaStream_t stream);
 
 template <typename T>
 struct IsBf16 { static constexpr bool value = false; };
@@ -212,9 +213,10 @@ __device__ __forceinline__ float bn_variance(float v) { return v < 0.f ? 0.f : v
 __global__ void bn_finalize_kernel(const float* __restrict__ sums, const float* __restrict__ gamma, const float* __restrict__ beta,
                                    const float* __restrict__ pre_bias, float* __restrict__ moving_mean, float* __restrict__ moving_var,
                                    float momentum, float eps, float inv_m, int C, float* __restrict__ mean_out, float* __restrict__ invstd_out,
-                                   float* __restrict__ scale_out, float* __restrict__ shift_out) {
+                                   float* __restrict__ scale_out, float* __restrict__ shift_out, float* __restrict__ zero) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
+  if (zero != nullptr) zero[c] = zero[C + c] = 0.f;
   const float mean = sums[c] * inv_m;
   const float var = bn_variance(sums[C + c] * inv_m - mean * mean);
   const float invstd = rsqrtf(var + eps);
@@ -235,7 +237,7 @@ __global__ void bn_finalize_partials_kernel(const float* __restrict__ partials, 
                                             const float* __restrict__ gamma, const float* __restrict__ beta, const float* __restrict__ pre_bias,
                                             float* __restrict__ moving_mean, float* __restrict__ moving_var, float momentum, float eps, float inv_m,
                                             int C, float* __restrict__ mean_out, float* __restrict__ invstd_out, float* __restrict__ scale_out,
-                                            float* __restrict__ shift_out) {
+                                            float* __restrict__ shift_out, float* __restrict__ zero) {
   const int lane = threadIdx.x & 31;
   const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (c >= C) return;
@@ -251,6 +253,7 @@ __global__ void bn_finalize_partials_kernel(const float* __restrict__ partials, 
   s = warp_sum(s);
   q = warp_sum(q);
   if (lane != 0) return;
+  if (zero != nullptr) zero[c] = zero[C + c] = 0.f;
   const float mean = s * inv_m;
   const float var = bn_variance(q * inv_m - mean * mean);
   const float invstd = rsqrtf(var + eps);
@@ -264,31 +267,14 @@ __global__ void bn_finalize_partials_kernel(const float* __restrict__ partials, 
   if (moving_var) moving_var[c] = moving_var[c] * momentum + var * (1.f - momentum);
 }
 
-// Backward coefficients: dx = A*dy' + B*x + Cc
-// dgamma_acc / dbeta_acc (optional): persistent gradient storage of gamma and beta; the sums are added there as well
-__global__ void bn_bwd_coeff_kernel(const float* __restrict__ sums, const float* __restrict__ gamma, const float* __restrict__ mean,
-                                    const float* __restrict__ invstd, float inv_m, int C, float* __restrict__ coef, float* __restrict__ dgamma_acc,
-                                    float* __restrict__ dbeta_acc) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  if (dgamma_acc != nullptr) dgamma_acc[c] += sums[C + c];
-  if (dbeta_acc != nullptr) dbeta_acc[c] += sums[c];
-  const float g = gamma ? gamma[c] : 1.f, is = invstd[c], mu = mean[c];
-  const float s1 = sums[c] * inv_m, s2 = sums[C + c] * inv_m;
-  const float a = g * is;
-  coef[c] = a;
-  coef[C + c] = -a * is * s2;
-  coef[2 * C + c] = a * (mu * is * s2 - s1);
-}
-
 // MODE 0: y  = relu?(x*p0 + p1 (+ res)), bits = !(y <= 0)     (p0 = scale, p1 = shift)
-// MODE 1: dx = p0*dy' + p1*x + p2, dres = dy'                 (in0 = dy, in1 = x, mask from bits or y)
+// MODE 1: dx = a*dy' + b*x + c, dres = dy'                     (in0 = dy, in1 = x, mask from bits or y; a, b, c of bn_coefficients)
 // U rows in flight per thread: 4, or 8 for the forward pass without a residual input (one stream of loads only)
 template <typename T, int MODE, int U = BN_U>
 __global__ void __launch_bounds__(BN_THREADS, 2) bn_apply_kernel(const T* __restrict__ in0, const T* __restrict__ in1, const T* __restrict__ ymask,
                                                              unsigned char* __restrict__ bits, T* __restrict__ out0, T* __restrict__ out1,
                                                              const float* __restrict__ p0, const float* __restrict__ p1,
-                                                             const float* __restrict__ p2, long long M, int C, int cx, int relu,
+                                                             const BnCoef q, long long M, int C, int cx, int relu,
                                                              float cap = INFINITY) {
   constexpr int V = Vec<T>::N;
   const bool capped = cap < INFINITY;
@@ -302,9 +288,14 @@ __global__ void __launch_bounds__(BN_THREADS, 2) bn_apply_kernel(const T* __rest
   float a[V], b[V], cc[V];
 #pragma unroll
   for (int k = 0; k < V; ++k) {
-    a[k] = p0[c0 + k];
-    b[k] = p1[c0 + k];
-    cc[k] = (MODE == 1) ? p2[c0 + k] : 0.f;
+    if (MODE == 1) {
+      bn_coefficients(q, C, c0 + k, a[k], b[k], cc[k]);
+      if (blockIdx.x == 0 && ty == 0) bn_keep_sums(q, C, c0 + k);
+    } else {
+      a[k] = p0[c0 + k];
+      b[k] = p1[c0 + k];
+      cc[k] = 0.f;
+    }
   }
   const long long step = (long long)gridDim.x * ry * U;
   for (long long r0 = (long long)blockIdx.x * ry * U + ty; r0 < M; r0 += step) {
@@ -370,11 +361,11 @@ static inline int ilog2(int v) {
 
 template <typename T>
 static int bn_reduce_launch(int mode, const void* x, const void* dy, const void* y, const unsigned char* bits, const float* mean,
-                            const float* invstd, long long M, int C, float* sums, cudaStream_t stream) {
+                            const float* invstd, long long M, int C, float* sums, cudaStream_t stream, bool zeroed = false) {
   constexpr int V = Vec<T>::N;
   constexpr int U0 = 8;
   if (C % V != 0) { kb200_set_error("bn: C must be a multiple of the vector width"); return -2; }
-  cudaMemsetAsync(sums, 0, sizeof(float) * 2 * C, stream);
+  if (!zeroed) cudaMemsetAsync(sums, 0, sizeof(float) * 2 * C, stream);
   if (mode == 0) {
     static const int resident = bn_resident_blocks(bn_reduce_kernel<T, 0, U0>);
     const BnGeom g = bn_geom(M, C / V, resident, U0);
@@ -400,11 +391,12 @@ KB_API int kb200_bn_stats(const void* x, long long M, int C, int dtype, float* s
                     : bn_reduce_launch<float>(0, x, nullptr, nullptr, nullptr, nullptr, nullptr, M, C, sums, stream);
 }
 
+// zero (both entries): 2 C floats to be cleared for the backward reduction that follows, or null.
 KB_API int kb200_bn_finalize(const float* sums, const float* gamma, const float* beta, const float* pre_bias, float* moving_mean,
                              float* moving_var, float momentum, float eps, long long M, int C, float* mean_out, float* invstd_out,
-                             float* scale_out, float* shift_out, cudaStream_t stream) {
+                             float* scale_out, float* shift_out, float* zero, cudaStream_t stream) {
   bn_finalize_kernel<<<(C + 127) / 128, 128, 0, stream>>>(sums, gamma, beta, pre_bias, moving_mean, moving_var, momentum, eps, 1.f / (float)M, C,
-                                                          mean_out, invstd_out, scale_out, shift_out);
+                                                          mean_out, invstd_out, scale_out, shift_out, zero);
   KB_CHECK_LAUNCH("bn_finalize");
   return 0;
 }
@@ -413,13 +405,13 @@ KB_API int kb200_bn_finalize(const float* sums, const float* gamma, const float*
 // the plan values that kb200_conv_igemm reported, `ld` the row pitch of `partials`.
 KB_API int kb200_bn_finalize_partials(const float* partials, int grid, int n_tiles, int bn, int ld, const float* gamma, const float* beta,
                                       const float* pre_bias, float* moving_mean, float* moving_var, float momentum, float eps, long long M, int C,
-                                      float* mean_out, float* invstd_out, float* scale_out, float* shift_out, cudaStream_t stream) {
+                                      float* mean_out, float* invstd_out, float* scale_out, float* shift_out, float* zero, cudaStream_t stream) {
   if (grid <= 0 || n_tiles <= 0 || bn <= 0 || C > n_tiles * bn || ld < n_tiles * bn) {
     kb200_set_error("bn_finalize_partials: inconsistent plan");
     return -2;
   }
   bn_finalize_partials_kernel<<<(C + 3) / 4, 128, 0, stream>>>(partials, grid, n_tiles, bn, ld, gamma, beta, pre_bias, moving_mean, moving_var, momentum,
-                                                                eps, 1.f / (float)M, C, mean_out, invstd_out, scale_out, shift_out);
+                                                                eps, 1.f / (float)M, C, mean_out, invstd_out, scale_out, shift_out, zero);
   KB_CHECK_LAUNCH("bn_finalize_partials");
   return 0;
 }
@@ -433,7 +425,7 @@ static int bn_apply_launch(const void* x, const void* res, void* y, unsigned cha
   if (res == nullptr) {
     static const int resident8 = bn_resident_blocks(bn_apply_kernel<T, 0, 8>);
     const BnGeom g8 = bn_geom_apply(M, C / V, resident8, 8);
-    bn_apply_kernel<T, 0, 8><<<dim3(g8.gx, g8.gy), BN_THREADS, 0, stream>>>((const T*)x, nullptr, nullptr, bits, (T*)y, nullptr, scale, shift, nullptr,
+    bn_apply_kernel<T, 0, 8><<<dim3(g8.gx, g8.gy), BN_THREADS, 0, stream>>>((const T*)x, nullptr, nullptr, bits, (T*)y, nullptr, scale, shift, BnCoef{},
                                                                            M, C, g8.cx, relu, cap);
     KB_CHECK_LAUNCH("bn_apply");
     return 0;
@@ -445,7 +437,7 @@ static int bn_apply_launch(const void* x, const void* res, void* y, unsigned cha
   static const int resident = bn_resident_blocks(bn_apply_kernel<T, 0>);
   const BnGeom g = bn_geom_apply(M, C / V, resident, BN_U);
   bn_apply_kernel<T, 0><<<dim3(g.gx, g.gy), BN_THREADS, 0, stream>>>((const T*)x, (const T*)res, nullptr, bits, (T*)y, nullptr, scale, shift,
-                                                                    nullptr, M, C, g.cx, relu);
+                                                                    BnCoef{}, M, C, g.cx, relu);
   KB_CHECK_LAUNCH("bn_apply");
   return 0;
 }
@@ -479,55 +471,54 @@ KB_API int kb200_bn_bwd_reduce(const void* dy, const void* x, const void* y, con
 }
 
 template <typename T>
-static int bn_bwd_apply_launch(const void* dy, const void* x, const void* y, const unsigned char* bits, const float* coef, void* dx, void* dres,
+static int bn_bwd_apply_launch(const void* dy, const void* x, const void* y, const unsigned char* bits, const BnCoef& q, void* dx, void* dres,
                                long long M, int C, cudaStream_t stream) {
   constexpr int V = Vec<T>::N;
   if (IsBf16<T>::value && y == nullptr) {
-    const int rc = kb200_bn_stream_launch(2, dy, x, bits, dx, dres, nullptr, coef, coef + C, coef + 2 * C, nullptr, M, C, 0, stream);
+    const int rc = kb200_bn_stream_launch(2, dy, x, bits, dx, dres, nullptr, nullptr, nullptr, &q, nullptr, M, C, 0, stream);
     if (rc <= 0) return rc;
   }
   static const int resident = bn_resident_blocks(bn_apply_kernel<T, 1>);
   const BnGeom g = bn_geom_apply(M, C / V, resident, BN_U);
   bn_apply_kernel<T, 1><<<dim3(g.gx, g.gy), BN_THREADS, 0, stream>>>((const T*)dy, (const T*)x, (const T*)y, const_cast<unsigned char*>(bits),
-                                                                    (T*)dx, (T*)dres, coef, coef + C, coef + 2 * C, M, C, g.cx, 0);
+                                                                    (T*)dx, (T*)dres, nullptr, nullptr, q, M, C, g.cx, 0);
   KB_CHECK_LAUNCH("bn_bwd_apply");
   return 0;
 }
 
 static int bn_bwd_apply_any(const void* dy, const void* x, const void* y, const unsigned char* bits, const float* mean, const float* invstd,
-                            const float* gamma, const float* sums, float* coef, void* dx, void* dres, long long M, int C, int dtype,
+                            const float* gamma, const float* sums, void* dx, void* dres, long long M, int C, int dtype,
                             cudaStream_t stream, float* dgamma_acc = nullptr, float* dbeta_acc = nullptr) {
   const int V = dtype == 1 ? 8 : 4;
   if (C % V != 0) { kb200_set_error("bn: C must be a multiple of the vector width"); return -2; }
-  bn_bwd_coeff_kernel<<<(C + 127) / 128, 128, 0, stream>>>(sums, gamma, mean, invstd, 1.f / (float)M, C, coef, dgamma_acc, dbeta_acc);
-  KB_CHECK_LAUNCH("bn_bwd_coeff");
-  return dtype == 1 ? bn_bwd_apply_launch<__nv_bfloat16>(dy, x, y, bits, coef, dx, dres, M, C, stream)
-                    : bn_bwd_apply_launch<float>(dy, x, y, bits, coef, dx, dres, M, C, stream);
+  const BnCoef q{sums, gamma, mean, invstd, 1.f / (float)M, dgamma_acc, dbeta_acc};
+  return dtype == 1 ? bn_bwd_apply_launch<__nv_bfloat16>(dy, x, y, bits, q, dx, dres, M, C, stream)
+                    : bn_bwd_apply_launch<float>(dy, x, y, bits, q, dx, dres, M, C, stream);
 }
 
-// coef: scratch of 3*C floats (written here)
+// coef: not used any more (the passes work the coefficients out for themselves); may be null
 KB_API int kb200_bn_bwd_apply(const void* dy, const void* x, const void* y, const float* mean, const float* invstd, const float* gamma,
-                              const float* sums, float* coef, void* dx, void* dres, long long M, int C, int dtype, cudaStream_t stream) {
-  return bn_bwd_apply_any(dy, x, y, nullptr, mean, invstd, gamma, sums, coef, dx, dres, M, C, dtype, stream);
+                              const float* sums, float* /*coef*/, void* dx, void* dres, long long M, int C, int dtype, cudaStream_t stream) {
+  return bn_bwd_apply_any(dy, x, y, nullptr, mean, invstd, gamma, sums, dx, dres, M, C, dtype, stream);
 }
 
-// Backward with the ReLU mask taken from the bit mask of kb200_bn_apply_mask (bits may be null: no ReLU).
+// Backward with the ReLU mask taken from the bit mask of kb200_bn_apply_mask (bits may be null: no ReLU).  zeroed: the caller has cleared sums.
 KB_API int kb200_bn_bwd_reduce_mask(const void* dy, const void* x, const unsigned char* bits, const float* mean, const float* invstd, long long M,
-                                    int C, int dtype, float* sums, cudaStream_t stream) {
-  return dtype == 1 ? bn_reduce_launch<__nv_bfloat16>(1, x, dy, nullptr, bits, mean, invstd, M, C, sums, stream)
-                    : bn_reduce_launch<float>(1, x, dy, nullptr, bits, mean, invstd, M, C, sums, stream);
+                                    int C, int dtype, float* sums, int zeroed, cudaStream_t stream) {
+  return dtype == 1 ? bn_reduce_launch<__nv_bfloat16>(1, x, dy, nullptr, bits, mean, invstd, M, C, sums, stream, zeroed != 0)
+                    : bn_reduce_launch<float>(1, x, dy, nullptr, bits, mean, invstd, M, C, sums, stream, zeroed != 0);
 }
 
 KB_API int kb200_bn_bwd_apply_mask(const void* dy, const void* x, const unsigned char* bits, const float* mean, const float* invstd,
-                                   const float* gamma, const float* sums, float* coef, void* dx, void* dres, long long M, int C, int dtype,
+                                   const float* gamma, const float* sums, float* /*coef*/, void* dx, void* dres, long long M, int C, int dtype,
                                    cudaStream_t stream) {
-  return bn_bwd_apply_any(dy, x, nullptr, bits, mean, invstd, gamma, sums, coef, dx, dres, M, C, dtype, stream);
+  return bn_bwd_apply_any(dy, x, nullptr, bits, mean, invstd, gamma, sums, dx, dres, M, C, dtype, stream);
 }
 
 // As kb200_bn_bwd_apply_mask; in addition the gradients of gamma and beta are ADDED into dgamma_acc / dbeta_acc (fp32 [C],
 // either may be null): persistent gradient storage, so that no separate accumulation kernel runs.
 KB_API int kb200_bn_bwd_apply_mask_acc(const void* dy, const void* x, const unsigned char* bits, const float* mean, const float* invstd,
-                                       const float* gamma, const float* sums, float* coef, void* dx, void* dres, float* dgamma_acc,
+                                       const float* gamma, const float* sums, float* /*coef*/, void* dx, void* dres, float* dgamma_acc,
                                        float* dbeta_acc, long long M, int C, int dtype, cudaStream_t stream) {
-  return bn_bwd_apply_any(dy, x, nullptr, bits, mean, invstd, gamma, sums, coef, dx, dres, M, C, dtype, stream, dgamma_acc, dbeta_acc);
+  return bn_bwd_apply_any(dy, x, nullptr, bits, mean, invstd, gamma, sums, dx, dres, M, C, dtype, stream, dgamma_acc, dbeta_acc);
 }

@@ -11,6 +11,7 @@
 //
 // Every mbarrier wait is bounded; a wait that runs out raises a device flag (kb200_bn_stream_status) and the block
 // leaves its loops.  Formulas as bn.cu (keras/src/backend/torch/nn.py:1020-1092 for the forward definition).
+#include "bn.cuh"
 #include "common.cuh"
 
 namespace {
@@ -32,7 +33,7 @@ struct BsParams {
   unsigned char* bits_out;
   const float* p0;
   const float* p1;
-  const float* p2;
+  BnCoef coef;
   float* sums;
   long long M;
   long long tiles;
@@ -97,7 +98,7 @@ __device__ __forceinline__ uint4 bs_pack8(const float* f) {
 
 // MODE 0: y = relu?(in0*p0 + p1 + in1), bits_out = !(y <= 0)                         in0 = x, in1 = residual
 // MODE 1: sums[c] += sum d, sums[C + c] += p1[c] * sum d*(in1 - p0[c]),  d = mask ? in0 : 0   in0 = dy, in1 = x, p0 = mean, p1 = invstd
-// MODE 2: out0 = p0*d + p1*in1 + p2, out1 = d (optional)                             in0 = dy, in1 = x
+// MODE 2: out0 = a*d + b*in1 + c, out1 = d (optional)                                in0 = dy, in1 = x; a, b, c of bn_coefficients
 template <int MODE>
 __global__ void __launch_bounds__(BS_THREADS, 1) bn_stream_kernel(const BsParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -148,9 +149,14 @@ __global__ void __launch_bounds__(BS_THREADS, 1) bn_stream_kernel(const BsParams
   float a[8], b[8], cc[8], sa[8], sb[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
-    a[k] = p.p0[c0 + k];
-    b[k] = (MODE == 1) ? 0.f : p.p1[c0 + k];
-    cc[k] = (MODE == 2) ? p.p2[c0 + k] : 0.f;
+    if (MODE == 2) {
+      bn_coefficients(p.coef, p.C, c0 + k, a[k], b[k], cc[k]);
+      if (blockIdx.x == 0 && rl == 0) bn_keep_sums(p.coef, p.C, c0 + k);
+    } else {
+      a[k] = p.p0[c0 + k];
+      b[k] = (MODE == 1) ? 0.f : p.p1[c0 + k];
+      cc[k] = 0.f;
+    }
     sa[k] = 0.f;
     sb[k] = 0.f;
   }
@@ -282,7 +288,7 @@ int bs_set_attr(size_t smem) {
 // Returns 1 when the streaming kernel does not apply (the caller then uses the register kernels), 0 when it was
 // launched, a negative code on a launch error.  mode as bn_stream_kernel.  bf16 only.
 int kb200_bn_stream_launch(int mode, const void* in0, const void* in1, const unsigned char* bits_in, void* out0, void* out1, unsigned char* bits_out,
-                           const float* p0, const float* p1, const float* p2, float* sums, long long M, int C, int relu, cudaStream_t stream) {
+                           const float* p0, const float* p1, const BnCoef* coef, float* sums, long long M, int C, int relu, cudaStream_t stream) {
   if (!bs_enabled() || in0 == nullptr || in1 == nullptr || C % 8 != 0) return 1;
   const int cvecs = C / 8;
   if (cvecs < 1 || cvecs > BS_CONSUMERS) return 1;
@@ -300,7 +306,7 @@ int kb200_bn_stream_launch(int mode, const void* in0, const void* in1, const uns
   p.bits_out = bits_out;
   p.p0 = p0;
   p.p1 = p1;
-  p.p2 = p2;
+  p.coef = coef != nullptr ? *coef : BnCoef{};
   p.sums = sums;
   p.M = M;
   p.C = C;

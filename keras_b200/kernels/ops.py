@@ -284,8 +284,9 @@ class FusedBatchNormAct(torch.autograd.Function):
         M = x.numel() // C
         x = aligned(x)
         dev = x.device
-        stats = torch.empty(4 * C, dtype=torch.float32, device=dev)
-        mean, invstd, scale, shift = stats[:C], stats[C:2 * C], stats[2 * C:3 * C], stats[3 * C:]
+        # behind the statistics the sums of the backward pass: what finalises the statistics clears them, without a launch of its own
+        stats = torch.empty(6 * C, dtype=torch.float32, device=dev)
+        mean, invstd, scale, shift, zero = stats[:C], stats[C:2 * C], stats[2 * C:3 * C], stats[3 * C:4 * C], stats[4 * C:]
         y = torch.empty_like(x)
         st = _stream()
         dt = _dt(x)
@@ -294,12 +295,12 @@ class FusedBatchNormAct(torch.autograd.Function):
             cs = conv_stats
             _check(lib.kb200_bn_finalize_partials(_p(cs.partials), _i(cs.grid), _i(cs.n_tiles), _i(cs.bn), _i(cs.ld), _p(gamma), _p(beta), _p(pre_bias),
                                                   _p(moving_mean), _p(moving_var), _f(momentum), _f(eps), _ll(M), _i(C), _p(mean), _p(invstd), _p(scale),
-                                                  _p(shift), st), "bn_finalize_partials")
+                                                  _p(shift), _p(zero), st), "bn_finalize_partials")
         else:
             sums = torch.empty(2 * C, dtype=torch.float32, device=dev)
             _check(lib.kb200_bn_stats(_p(x), _ll(M), _i(C), _i(dt), _p(sums), st), "bn_stats")
             _check(lib.kb200_bn_finalize(_p(sums), _p(gamma), _p(beta), _p(pre_bias), _p(moving_mean), _p(moving_var), _f(momentum), _f(eps), _ll(M), _i(C),
-                                         _p(mean), _p(invstd), _p(scale), _p(shift), st), "bn_finalize")
+                                         _p(mean), _p(invstd), _p(scale), _p(shift), _p(zero), st), "bn_finalize")
         res = aligned(residual) if residual is not None else None
         bits = None
         if relu:
@@ -319,6 +320,7 @@ class FusedBatchNormAct(torch.autograd.Function):
         ctx.merge = merge if residual is not None else None  # grad_merge.MergeSlot of the residual activation
         ctx.res_shape = tuple(residual.shape) if residual is not None else None
         ctx.dims = (M, C)
+        ctx.cleared = True
         return y
 
     @staticmethod
@@ -329,17 +331,19 @@ class FusedBatchNormAct(torch.autograd.Function):
         mean, invstd = stats[:C], stats[C:2 * C]
         dy = aligned(dy)
         dev = x.device
-        sums = torch.empty(5 * C, dtype=torch.float32, device=dev)
-        coef = sums[2 * C:]
+        from keras_b200.kernels import shadow
+
+        slot_g, slot_b = shadow.grad_slot(ctx.leaves[0], (C,)), shadow.grad_slot(ctx.leaves[1], (C,))
+        # sums that become gradients of their own need storage of their own, and a second pass finds the first one's
+        cleared = ctx.cleared and slot_b is not None and (gamma is None or slot_g is not None)
+        sums = stats[4 * C:] if cleared else torch.empty(2 * C, dtype=torch.float32, device=dev)
+        ctx.cleared = ctx.cleared and not cleared
         dx = torch.empty_like(x)
         dres = torch.empty_like(x) if ctx.has_res else None
         st = _stream()
         dt = _dt(x)
-        _check(lib.kb200_bn_bwd_reduce_mask(_p(dy), _p(x), _p(bits), _p(mean), _p(invstd), _ll(M), _i(C), _i(dt), _p(sums), st), "bn_bwd_reduce")
-        from keras_b200.kernels import shadow
-
-        slot_g, slot_b = shadow.grad_slot(ctx.leaves[0], (C,)), shadow.grad_slot(ctx.leaves[1], (C,))
-        _check(lib.kb200_bn_bwd_apply_mask_acc(_p(dy), _p(x), _p(bits), _p(mean), _p(invstd), _p(gamma), _p(sums), _p(coef), _p(dx), _p(dres),
+        _check(lib.kb200_bn_bwd_reduce_mask(_p(dy), _p(x), _p(bits), _p(mean), _p(invstd), _ll(M), _i(C), _i(dt), _p(sums), _i(1 if cleared else 0), st), "bn_bwd_reduce")
+        _check(lib.kb200_bn_bwd_apply_mask_acc(_p(dy), _p(x), _p(bits), _p(mean), _p(invstd), _p(gamma), _p(sums), _vp(0), _p(dx), _p(dres),
                                                _p(slot_g), _p(slot_b), _ll(M), _i(C), _i(dt), st), "bn_bwd_apply")
         dgamma = sums[C:2 * C] if gamma is not None and slot_g is None else None
         dbeta = sums[:C] if slot_b is None else None

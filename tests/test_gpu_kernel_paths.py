@@ -398,3 +398,44 @@ def test_recorded_step_copies_what_it_reads(other_reader):
 
     recorded, eager = run(True)[0], run(False)[0]
     assert max(abs(a - b) for a, b in zip(recorded, eager)) < 2e-2, (recorded, eager)
+
+
+# ------------------------------------------------------------------------------------------------ BatchNorm sums
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", [(2, 3, 3, 8), (4, 9, 9, 96), (24, 18, 18, 384), (32, 32, 32, 256)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_batch_norm_backward_twice_and_into_the_arena(shape, dtype, residual):
+    """The sums that the forward pass clears serve one backward pass; another one, and gradients of their own, have theirs."""
+    from keras_b200.kernels import ops as kops
+    from keras_b200.kernels import shadow
+
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")  # noqa: E731
+    C = shape[-1]
+    x, r = rnd(*shape).to(dtype).requires_grad_(True), (rnd(*shape).to(dtype).requires_grad_(True) if residual else None)
+    gamma, beta = (1 + 0.1 * rnd(C)).requires_grad_(True), rnd(C).requires_grad_(True)
+    up = rnd(*shape).to(dtype)
+
+    def forward():
+        return kops.FusedBatchNormAct.apply(x, gamma, beta, r, torch.zeros(C, device="cuda"), torch.ones(C, device="cuda"), 0.9, 1e-3, True)
+
+    inputs = [t for t in (x, gamma, beta, r) if t is not None]
+    y = forward()
+    own = [torch.autograd.grad(y, inputs, up, retain_graph=True) for _ in range(2)]  # of one forward pass: another's mean may turn a rectifier over
+    gamma.grad, beta.grad = torch.full((C,), 2.0, device="cuda"), torch.full((C,), -1.0, device="cuda")
+    rest = [t for t in (x, r) if t is not None]
+    with shadow.arena_backward():
+        arena = [torch.autograd.grad(y, rest, up, retain_graph=k == 0) for k in range(2)]
+    tol = 2e-5 if dtype == torch.float32 else 2.0 ** -7  # sums of up to 32768 products in fp32, added in any order; one rounding of dx
+    for k in range(2):
+        for a, b in zip([own[k][0]] + list(own[k][3:]), own[0][:1] + own[0][3:]):
+            assert _rel(a, b.double()) < tol
+        assert _rel(own[k][1], own[0][1].double()) < 1e-5 and _rel(own[k][2], own[0][2].double()) < 1e-5
+        for a, b in zip(arena[k], own[0][:1] + own[0][3:]):
+            assert _rel(a, b.double()) < tol
+    assert _rel(gamma.grad - 2.0, 2 * own[0][1].double()) < 1e-4 and _rel(beta.grad + 1.0, 2 * own[0][2].double()) < 1e-4
+    ex = [t.detach().double().requires_grad_(True) for t in inputs]
+    flat = ex[0].reshape(-1, C)
+    z = torch.nn.functional.batch_norm(flat, None, None, ex[1], ex[2], True, 0.0, 1e-3).reshape(shape) + (ex[3] if residual else 0)
+    for a, b in zip(own[0], torch.autograd.grad(z * (y.detach() > 0), ex, up.double())):
+        assert _rel(a, b) < (1e-4 if dtype == torch.float32 else 2.0 ** -6)
