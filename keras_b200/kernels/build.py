@@ -26,7 +26,7 @@ NVCC_FLAGS = [
 ]
 
 # Sources whose float32 results stand next to the library's own float32 math: exact division and full-accuracy functions.
-PRECISE = {"lstm.cu", "sgemm.cu"}
+PRECISE = {"lstm.cu", "sgemm.cu", "xent_classes.cu", "metrics.cu"}
 
 
 def _flags(src):

@@ -1,63 +1,14 @@
 // Fused softmax cross-entropy over large vocabularies: logits[rows, V] (bf16 or fp32) and integer
 // labels -> per-row loss and log-sum-exp (forward); dlogits = (softmax - onehot) * dloss (backward).
 // Replaces log_softmax + nll_loss (keras/src/backend/torch/nn.py:936-982) and their fp32 upcast copies.
-#include "common.cuh"
+#define XE_EXP __expf
+#include "xent_rows.cuh"
 
 constexpr int XE_THREADS = 512;
 
 // `ld` is the row pitch in elements (>= V).  When rows start 16-byte aligned (`vec` = 1: base pointer aligned and the pitch a
 // multiple of 16 bytes) the body is read and written as 16-byte vectors; the tail and unaligned inputs use scalar accesses.
 // Backward also zeroes the columns [V, Vz) of each row: a padded logits buffer gets a gradient that a padded GEMM can consume.
-template <typename T>
-struct XeVec {
-  static constexpr int N = 16 / sizeof(T);
-};
-
-template <typename T>
-__device__ __forceinline__ void xe_load(const T* p, float* v) {
-  const uint4 raw = *reinterpret_cast<const uint4*>(p);
-  if constexpr (sizeof(T) == 2) {
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 f = __bfloat1622float2(h[j]);
-      v[2 * j] = f.x;
-      v[2 * j + 1] = f.y;
-    }
-  } else {
-    const float* f = reinterpret_cast<const float*>(&raw);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = f[j];
-  }
-}
-
-template <typename T>
-__device__ __forceinline__ void xe_store(T* p, const float* v) {
-  uint4 raw;
-  if constexpr (sizeof(T) == 2) {
-    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&raw);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-  } else {
-    float* f = reinterpret_cast<float*>(&raw);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) f[j] = v[j];
-  }
-  *reinterpret_cast<uint4*>(p) = raw;
-}
-
-// The running maximum starts at the lowest finite value, not at -inf: a masked class (-inf) then adds exp(-inf) = 0 from the first on, and
-// needs no test of its own (one in this loop cost [16384, 50257] fp32 520 -> 1176 us).
-constexpr float XE_LOWEST = -3.402823466e38f;
-__device__ __forceinline__ void xe_online(float v, float& m, float& s) {
-  if (v > m) {
-    s = s * __expf(m - v) + 1.f;
-    m = v;
-  } else {
-    s += __expf(v - m);
-  }
-}
-
 template <typename T>
 __global__ void __launch_bounds__(XE_THREADS) xent_fwd_kernel(const T* __restrict__ logits, const long long* __restrict__ labels,
                                                               float* __restrict__ loss, float* __restrict__ lse_out, int V, long long ld, int vec) {
@@ -163,11 +114,11 @@ __global__ void __launch_bounds__(XE_THREADS) xent_fwd_grad_kernel(const T* __re
 
 template <typename T>
 __global__ void __launch_bounds__(XE_THREADS) xent_bwd_kernel(const T* __restrict__ logits, const long long* __restrict__ labels,
-                                                              const float* __restrict__ lse, const float* __restrict__ dloss, T* __restrict__ dlogits,
+                                                              const float* __restrict__ lse, const float* __restrict__ dloss, int ds, T* __restrict__ dlogits,
                                                               int V, long long ld, int Vz, int vec) {
   const long long row = blockIdx.x;
   const long long t = labels[row];
-  xe_row_gradient<T>(logits + row * ld, dlogits + row * ld, lse[row], t, t >= 0 && t < V ? dloss[row] : 0.f, V, Vz, vec);
+  xe_row_gradient<T>(logits + row * ld, dlogits + row * ld, lse[row], t, t >= 0 && t < V ? dloss[row * ds] : 0.f, V, Vz, vec);
 }
 
 // The rows hold the gradient for an upstream gradient of g0: those that another one reaches are computed again.  XE_CHECKED rows a block,
@@ -175,7 +126,7 @@ __global__ void __launch_bounds__(XE_THREADS) xent_bwd_kernel(const T* __restric
 constexpr int XE_CHECKED = 64;
 template <typename T>
 __global__ void __launch_bounds__(XE_THREADS) xent_bwd_check_kernel(const T* __restrict__ logits, const long long* __restrict__ labels,
-                                                                    const float* __restrict__ lse, const float* __restrict__ dloss, T* __restrict__ dlogits,
+                                                                    const float* __restrict__ lse, const float* __restrict__ dloss, int ds, T* __restrict__ dlogits,
                                                                     long long rows, int V, long long ld, int Vz, int vec, float g0) {
   __shared__ unsigned char again[XE_CHECKED];
   const long long first = (long long)blockIdx.x * XE_CHECKED;
@@ -184,7 +135,7 @@ __global__ void __launch_bounds__(XE_THREADS) xent_bwd_check_kernel(const T* __r
     const long long row = first + threadIdx.x;
     if (row < rows) {
       const long long t = labels[row];
-      any = t >= 0 && t < V && dloss[row] != g0;  // a NaN differs
+      any = t >= 0 && t < V && dloss[row * ds] != g0;  // a NaN differs
     }
     again[threadIdx.x] = (unsigned char)any;
   }
@@ -192,123 +143,23 @@ __global__ void __launch_bounds__(XE_THREADS) xent_bwd_check_kernel(const T* __r
   for (int i = 0; i < XE_CHECKED; ++i) {
     if (!again[i]) continue;
     const long long row = first + i;
-    xe_row_gradient<T>(logits + row * ld, dlogits + row * ld, lse[row], labels[row], dloss[row], V, Vz, vec);
+    xe_row_gradient<T>(logits + row * ld, dlogits + row * ld, lse[row], labels[row], dloss[row * ds], V, Vz, vec);
   }
 }
 
-// Narrow rows (at most XE_NARROW columns: classifiers, per-pixel labels).  A CTA per row leaves most of its 512 threads without a
-// column and pays two block-wide reductions for a row of a few hundred bytes; here G lanes of a warp share a row, so a warp
-// holds 32 / G rows and the reductions are shuffles.  Bound by the logits' traffic.  [200704, 64] bf16 (25.7 MB of logits):
-// forward 569 -> 9 us, backward 321 -> 13 us.
-constexpr int XE_NARROW = 2048;  // 8 vectors a lane at G = 32; beyond it a CTA per row has work for all of its warps
-
-template <typename T, int G>
-__global__ void __launch_bounds__(256) xent_narrow_fwd_kernel(const T* __restrict__ logits, const long long* __restrict__ labels,
-                                                              float* __restrict__ loss, float* __restrict__ lse_out, long long rows, int V, long long ld,
-                                                              int vec) {
-  constexpr int VN = XeVec<T>::N;
-  const int gl = threadIdx.x & (G - 1);
-  const long long row = (long long)blockIdx.x * (256 / G) + threadIdx.x / G;
-  const bool live = row < rows;  // no early exit: every lane takes part in the shuffles
-  const T* l = logits + (live ? row : 0) * ld;
-  const int n = live ? V : 0;
-  const int body = vec ? (n / VN) * VN : 0;
-  float m = XE_LOWEST, s = 0.f;
-  for (int i = gl * VN; i < body; i += G * VN) {
-    float v[VN];
-    xe_load<T>(l + i, v);
-    float vm = v[0];
-#pragma unroll
-    for (int j = 1; j < VN; ++j) vm = fmaxf(vm, v[j]);
-    if (vm > m) {
-      s *= __expf(m - vm);
-      m = vm;
-    }
-#pragma unroll
-    for (int j = 0; j < VN; ++j) s += __expf(v[j] - m);
-  }
-  for (int i = body + gl; i < n; i += G) xe_online(to_f32<T>(l[i]), m, s);
-  float gm = m;
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) gm = fmaxf(gm, __shfl_xor_sync(0xffffffffu, gm, o));
-  s *= __expf(m - gm);
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (live && gl == 0) {
-    const float lse = gm + logf(s);
-    const long long t = labels[row];
-    lse_out[row] = lse;
-    loss[row] = (t >= 0 && t < V) ? lse - to_f32<T>(l[t]) : 0.f;
-  }
-}
-
-template <typename T, int G>
-__global__ void __launch_bounds__(256) xent_narrow_bwd_kernel(const T* __restrict__ logits, const long long* __restrict__ labels,
-                                                              const float* __restrict__ lse, const float* __restrict__ dloss, T* __restrict__ dlogits,
-                                                              long long rows, int V, long long ld, int Vz, int vec) {
-  constexpr int VN = XeVec<T>::N;
-  const int gl = threadIdx.x & (G - 1);
-  const long long row = (long long)blockIdx.x * (256 / G) + threadIdx.x / G;
-  if (row >= rows) return;
-  const T* l = logits + row * ld;
-  T* d = dlogits + row * ld;
-  const float r_lse = lse[row];
-  const long long t = labels[row];
-  const float g = (t >= 0 && t < V) ? dloss[row] : 0.f;
-  const int body = vec ? (V / VN) * VN : 0;
-  for (int i = gl * VN; i < body; i += G * VN) {
-    float v[VN];
-    xe_load<T>(l + i, v);
-#pragma unroll
-    for (int j = 0; j < VN; ++j) {
-      float p = __expf(v[j] - r_lse);
-      if (i + j == t) p -= 1.f;
-      v[j] = p * g;
-    }
-    xe_store<T>(d + i, v);
-  }
-  for (int i = body + gl; i < Vz; i += G) {
-    float p = 0.f;
-    if (i < V) {
-      p = __expf(to_f32<T>(l[i]) - r_lse);
-      if (i == t) p -= 1.f;
-    }
-    d[i] = from_f32<T>(p * g);
-  }
-}
-
-// Lanes a row: enough that each has one vector (or, on the scalar path, a handful of elements), never more than a warp.
-static int xe_lanes(int V, int vec, int vn) {
-  const int items = vec ? (V + vn - 1) / vn : (V + 3) / 4;
-  return items <= 4 ? 4 : items <= 8 ? 8 : items <= 16 ? 16 : 32;
-}
-
-template <typename T>
-static void xe_narrow_fwd(const T* logits, const long long* labels, float* loss, float* lse, long long rows, int V, long long ld, int vec, cudaStream_t st) {
-  const int g = xe_lanes(V, vec, XeVec<T>::N);
-  const unsigned grid = (unsigned)((rows * g + 255) / 256);
-  if (g == 4) xent_narrow_fwd_kernel<T, 4><<<grid, 256, 0, st>>>(logits, labels, loss, lse, rows, V, ld, vec);
-  else if (g == 8) xent_narrow_fwd_kernel<T, 8><<<grid, 256, 0, st>>>(logits, labels, loss, lse, rows, V, ld, vec);
-  else if (g == 16) xent_narrow_fwd_kernel<T, 16><<<grid, 256, 0, st>>>(logits, labels, loss, lse, rows, V, ld, vec);
-  else xent_narrow_fwd_kernel<T, 32><<<grid, 256, 0, st>>>(logits, labels, loss, lse, rows, V, ld, vec);
-}
-
-template <typename T>
-static void xe_narrow_bwd(const T* logits, const long long* labels, const float* lse, const float* dloss, T* dlogits, long long rows, int V, long long ld,
-                          int Vz, int vec, cudaStream_t st) {
-  const int g = xe_lanes(V, vec, XeVec<T>::N);
-  const unsigned grid = (unsigned)((rows * g + 255) / 256);
-  if (g == 4) xent_narrow_bwd_kernel<T, 4><<<grid, 256, 0, st>>>(logits, labels, lse, dloss, dlogits, rows, V, ld, Vz, vec);
-  else if (g == 8) xent_narrow_bwd_kernel<T, 8><<<grid, 256, 0, st>>>(logits, labels, lse, dloss, dlogits, rows, V, ld, Vz, vec);
-  else if (g == 16) xent_narrow_bwd_kernel<T, 16><<<grid, 256, 0, st>>>(logits, labels, lse, dloss, dlogits, rows, V, ld, Vz, vec);
-  else xent_narrow_bwd_kernel<T, 32><<<grid, 256, 0, st>>>(logits, labels, lse, dloss, dlogits, rows, V, ld, Vz, vec);
-}
+// xent_classes.cu
+constexpr int XE_FEW = 64;
+int kb200_xent_classes_fwd(const void* logits, const long long* labels, float* loss, float* lse, long long rows, int V, long long ld, int vec, int dtype,
+                           cudaStream_t stream);
+int kb200_xent_classes_bwd(const void* logits, const long long* labels, const float* lse, const float* dloss, int dloss_stride, void* dlogits, long long rows, int V,
+                           long long ld, int zero_to, int vec, int dtype, cudaStream_t stream);
 
 KB_API int kb200_xent_fwd(const void* logits, const long long* labels, float* loss, float* lse, long long rows, int V, long long ld, int dtype,
                           cudaStream_t stream) {
   if (rows <= 0) return 0;
   const int esize = dtype == 1 ? 2 : 4;
   const int vec = (((uintptr_t)logits & 15) == 0 && (ld * esize) % 16 == 0) ? 1 : 0;
+  if (V < XE_FEW && rows * 32 < (1ll << 38)) return kb200_xent_classes_fwd(logits, labels, loss, lse, rows, V, ld, vec, dtype, stream);
   if (V <= XE_NARROW && rows * 32 < (1ll << 38)) {
     if (dtype == 1) xe_narrow_fwd<__nv_bfloat16>((const __nv_bfloat16*)logits, labels, loss, lse, rows, V, ld, vec, stream);
     else xe_narrow_fwd<float>((const float*)logits, labels, loss, lse, rows, V, ld, vec, stream);
@@ -340,30 +191,32 @@ KB_API int kb200_xent_fwd_grad(const void* logits, const long long* labels, floa
 }
 
 // `zero_to` (V <= zero_to <= ld): columns [V, zero_to) of every dlogits row are written as zeros.  done: dlogits come from
-// kb200_xent_fwd_grad with this g0.
-KB_API int kb200_xent_bwd(const void* logits, const long long* labels, const float* lse, const float* dloss, void* dlogits, long long rows, int V,
+// kb200_xent_fwd_grad with this g0.  dloss_stride: 1, or 0 where every row has the one upstream gradient.
+KB_API int kb200_xent_bwd(const void* logits, const long long* labels, const float* lse, const float* dloss, int dloss_stride, void* dlogits, long long rows, int V,
                           long long ld, int zero_to, int done, float g0, int dtype, cudaStream_t stream) {
   if (rows <= 0) return 0;
   const int esize = dtype == 1 ? 2 : 4;
   const int vec = ((((uintptr_t)logits | (uintptr_t)dlogits) & 15) == 0 && (ld * esize) % 16 == 0) ? 1 : 0;
   if (zero_to < V) zero_to = V;
+  if (V < XE_FEW && !done && rows * 32 < (1ll << 38))
+    return kb200_xent_classes_bwd(logits, labels, lse, dloss, dloss_stride, dlogits, rows, V, ld, zero_to, vec, dtype, stream);
   if (done) {
     const unsigned grid = (unsigned)((rows + XE_CHECKED - 1) / XE_CHECKED);
     if (dtype == 1)
-      xent_bwd_check_kernel<__nv_bfloat16><<<grid, XE_THREADS, 0, stream>>>((const __nv_bfloat16*)logits, labels, lse, dloss, (__nv_bfloat16*)dlogits, rows, V, ld,
+      xent_bwd_check_kernel<__nv_bfloat16><<<grid, XE_THREADS, 0, stream>>>((const __nv_bfloat16*)logits, labels, lse, dloss, dloss_stride, (__nv_bfloat16*)dlogits, rows, V, ld,
                                                                               zero_to, vec, g0);
     else
-      xent_bwd_check_kernel<float><<<grid, XE_THREADS, 0, stream>>>((const float*)logits, labels, lse, dloss, (float*)dlogits, rows, V, ld, zero_to, vec, g0);
+      xent_bwd_check_kernel<float><<<grid, XE_THREADS, 0, stream>>>((const float*)logits, labels, lse, dloss, dloss_stride, (float*)dlogits, rows, V, ld, zero_to, vec, g0);
   } else if (V <= XE_NARROW && rows * 32 < (1ll << 38)) {
     if (dtype == 1)
-      xe_narrow_bwd<__nv_bfloat16>((const __nv_bfloat16*)logits, labels, lse, dloss, (__nv_bfloat16*)dlogits, rows, V, ld, zero_to, vec, stream);
+      xe_narrow_bwd<__nv_bfloat16>((const __nv_bfloat16*)logits, labels, lse, dloss, dloss_stride, (__nv_bfloat16*)dlogits, rows, V, ld, zero_to, vec, stream);
     else
-      xe_narrow_bwd<float>((const float*)logits, labels, lse, dloss, (float*)dlogits, rows, V, ld, zero_to, vec, stream);
+      xe_narrow_bwd<float>((const float*)logits, labels, lse, dloss, dloss_stride, (float*)dlogits, rows, V, ld, zero_to, vec, stream);
   } else if (dtype == 1)
-    xent_bwd_kernel<__nv_bfloat16><<<(unsigned)rows, XE_THREADS, 0, stream>>>((const __nv_bfloat16*)logits, labels, lse, dloss, (__nv_bfloat16*)dlogits, V,
+    xent_bwd_kernel<__nv_bfloat16><<<(unsigned)rows, XE_THREADS, 0, stream>>>((const __nv_bfloat16*)logits, labels, lse, dloss, dloss_stride, (__nv_bfloat16*)dlogits, V,
                                                                                 ld, zero_to, vec);
   else
-    xent_bwd_kernel<float><<<(unsigned)rows, XE_THREADS, 0, stream>>>((const float*)logits, labels, lse, dloss, (float*)dlogits, V, ld, zero_to, vec);
+    xent_bwd_kernel<float><<<(unsigned)rows, XE_THREADS, 0, stream>>>((const float*)logits, labels, lse, dloss, dloss_stride, (float*)dlogits, V, ld, zero_to, vec);
   KB_CHECK_LAUNCH("xent_bwd");
   return 0;
 }

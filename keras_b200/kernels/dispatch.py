@@ -344,9 +344,15 @@ def resize(x, out_hw, interpolation):
 def softmax_cross_entropy(logits, labels):
     if not enabled(logits) or logits.dtype not in _FLOAT_IO or logits.numel() == 0:
         return None
-    if logits.shape[-1] < 64:
+    if logits.shape[-1] < 2:
         return None
     return _ops().FusedSoftmaxXent.apply(logits, labels)
+
+
+def running_mean(total, count, value=None):
+    """The kernels of a running mean held in ``total`` and ``count``, or ``None``."""
+    ops = _ops()
+    return ops if enabled(total) and ops.running_mean(total, count, value) else None
 
 
 def flash_attention(q, k, v, mask, scale, is_causal, row_mask=None):

@@ -582,12 +582,14 @@ class FusedSoftmaxXent(torch.autograd.Function):
         flat, labels64, lse = ctx.saved_tensors
         rows, V = flat.shape
         ld = ctx.ld
-        dl = dloss.reshape(-1).float().contiguous()
+        # the gradient of a plain mean is one number, seen by every row
+        spread = dloss.dtype == torch.float32 and dloss.numel() > 0 and not any(dloss.stride())
+        dl = dloss if spread else dloss.reshape(-1).float().contiguous()
         buf, ctx.made = ctx.made, None
         done = buf is not None
         if not done:
             buf = torch.empty((rows, ld), dtype=flat.dtype, device=flat.device)
-        _check(lib.kb200_xent_bwd(_p(flat), _p(labels64), _p(lse), _p(dl), _p(buf), _ll(rows), _i(V), _ll(ld), _i(ctx.zero_to), _i(1 if done else 0),
+        _check(lib.kb200_xent_bwd(_p(flat), _p(labels64), _p(lse), _p(dl), _i(0 if spread else 1), _p(buf), _ll(rows), _i(V), _ll(ld), _i(ctx.zero_to), _i(1 if done else 0),
                                   _f(ctx.made_for), _i(_dt(flat)), _stream()), "xent_bwd")
         dlogits = buf if ld == V else buf[:, :V]
         return dlogits.reshape(ctx.logits_shape), None
@@ -691,6 +693,27 @@ def add_rows(dst, src):
         _check(_lib().kb200_add_rows(_p(src), _ll(src.stride(0)), _p(dst), _i(src.shape[0]), _i(src.shape[1]), _stream()), "add_rows")
         return dst
     return dst.add_(src)
+
+
+def running_mean(total, count, value=None):
+    """Whether the running-mean kernels take these single numbers: float32 on one CUDA device."""
+    tensors = (total, count) if value is None else (total, count, value)
+    return all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.dtype == torch.float32 and t.ndim == 0 and t.device == total.device
+               for t in tensors)
+
+
+def mean_update(total, count, value, weight):
+    _check(_lib().kb200_mean_update(_p(total), _p(count), _p(value), _f(weight), _stream()), "mean_update")
+
+
+def mean_result(total, count):
+    out = torch.empty((), dtype=torch.float32, device=total.device)
+    _check(_lib().kb200_mean_result(_p(total), _p(count), _p(out), _stream()), "mean_result")
+    return out
+
+
+def mean_clear(total, count):
+    _check(_lib().kb200_mean_clear(_p(total), _p(count), _stream()), "mean_clear")
 
 
 def copy_and_cast(src, dst, dst16):

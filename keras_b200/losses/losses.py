@@ -37,7 +37,7 @@ class LossFunctionWrapper(Loss):
             return False
         from keras_b200.kernels import dispatch
 
-        return self.dtype == "float32" and dispatch.enabled(y_pred) and y_pred.shape[-1] >= 64
+        return self.dtype == "float32" and dispatch.enabled(y_pred) and y_pred.shape[-1] >= 2
 
     def _values_as_computed(self):
         return (self.fn is sparse_categorical_crossentropy and type(self).call is LossFunctionWrapper.call

@@ -5,7 +5,9 @@ import torch
 from keras_b200 import initializers, losses
 from keras_b200.core.dtypes import to_torch_dtype
 from keras_b200.core.export_registry import keras_export
+from keras_b200.core.scopes import get_stateless_scope
 from keras_b200.core.tensor import convert_to_tensor
+from keras_b200.kernels import dispatch
 from keras_b200.losses.loss import squeeze_or_expand_to_same_rank
 from keras_b200.metrics.metric import Metric
 
@@ -61,6 +63,10 @@ class Mean(Metric):
             # fast path used by the loss tracker: scalar loss weighted by the batch size
             with torch.no_grad():
                 v = values.detach().to(self.total._torch_dtype)
+                kernels = dispatch.running_mean(self.total._value, self.count._value, v)
+                if kernels is not None:
+                    kernels.mean_update(self.total._value, self.count._value, v, float(sample_weight))
+                    return
                 self.total._value.add_(v * sample_weight)
                 self.count._value.add_(sample_weight)
             return
@@ -77,11 +83,18 @@ class Mean(Metric):
         self.count.assign_add(num_samples)
 
     def reset_state(self):
+        kernels = dispatch.running_mean(self.total._value, self.count._value) if get_stateless_scope() is None else None
+        if kernels is not None:
+            kernels.mean_clear(self.total._value, self.count._value)
+            return
         self.total.assign(0)
         self.count.assign(0)
 
     def result(self):
         total, count = self.total.value, self.count.value
+        kernels = dispatch.running_mean(total, count)
+        if kernels is not None:
+            return kernels.mean_result(total, count)
         return torch.where(count == 0, torch.zeros_like(total), total / torch.where(count == 0, torch.ones_like(count), count))
 
 

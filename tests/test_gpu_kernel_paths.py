@@ -400,7 +400,51 @@ def test_recorded_step_copies_what_it_reads(other_reader):
     assert max(abs(a - b) for a, b in zip(recorded, eager)) < 2e-2, (recorded, eager)
 
 
-# ------------------------------------------------------------------------------------------------ BatchNorm sums
+# ------------------------------------------------------------------------------------------------ few classes, running means, BatchNorm sums
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,V,ld", [(1, 2, 2), (128, 10, 10), (777, 37, 40), (513, 21, 24), (65, 63, 63), (33, 8, 8)])
+@pytest.mark.parametrize("spread", [True, False])
+def test_cross_entropy_of_few_classes(rows, V, ld, dtype, spread):
+    from keras_b200.kernels import ops as kops
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    buf = (torch.randn(rows, ld, generator=g, device="cuda") * 4).to(dtype)
+    logits = buf[:, :V].requires_grad_(True)
+    if V > 9:
+        with torch.no_grad():
+            logits[0, 1], logits[0, 2] = float("-inf"), torch.finfo(dtype).min
+    labels = torch.randint(3 if V > 9 else 0, V, (rows,), generator=g, device="cuda")
+    ref_in = logits.detach().double().requires_grad_(True)
+    loss, ref = kops.FusedSoftmaxXent.apply(logits, labels), torch.nn.functional.cross_entropy(ref_in, labels, reduction="none")
+    up = torch.rand((), device="cuda").expand(rows) if spread else torch.rand(rows, device="cuda")
+    a, = torch.autograd.grad(loss, logits, up)
+    b, = torch.autograd.grad(ref, ref_in, up.double())
+    # fp32 sums of at most 63 exponentials in full accuracy on the exact inputs; the gradient is rounded once to its type
+    assert torch.allclose(loss.double(), ref, atol=2e-6, rtol=5e-7)
+    # a probability is exp(v - lse), whose argument of up to 32 is rounded at 2^-20; next to the label it is one less
+    assert torch.allclose(a.double(), b, atol=2.0 ** -20, rtol=2.0 ** -19 if dtype == torch.float32 else 2.0 ** -8)
+
+
+def test_running_means_round_as_their_operations():
+    import keras_b200 as keras
+
+    mean = keras.metrics.Mean()
+    total, count = torch.zeros((), device="cuda"), torch.zeros((), device="cuda")
+    assert float(mean.result()) == 0.0
+    for k, w in enumerate((3, 64, 0.1, 7)):
+        value = torch.randn((), device="cuda", generator=torch.Generator(device="cuda").manual_seed(k))
+        mean.update_state(value, sample_weight=w)
+        total, count = total + value * w, count + w
+        assert torch.equal(mean.result(), total / count) and mean.result().device.type == "cuda"
+    mean.reset_state()
+    assert float(mean.total.value) == float(mean.count.value) == float(mean.result()) == 0.0
+    mean.update_state(torch.tensor([1.0, 3.0], device="cuda"))
+    assert float(mean.result()) == 2.0
+    mean.reset_state()
+    mean.update_state(torch.tensor(float("nan"), device="cuda"), sample_weight=2)
+    assert torch.isnan(mean.result())
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("shape", [(2, 3, 3, 8), (4, 9, 9, 96), (24, 18, 18, 384), (32, 32, 32, 256)])
 @pytest.mark.parametrize("residual", [False, True])
