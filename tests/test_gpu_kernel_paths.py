@@ -483,3 +483,19 @@ def test_batch_norm_backward_twice_and_into_the_arena(shape, dtype, residual):
     z = torch.nn.functional.batch_norm(flat, None, None, ex[1], ex[2], True, 0.0, 1e-3).reshape(shape) + (ex[3] if residual else 0)
     for a, b in zip(own[0], torch.autograd.grad(z * (y.detach() > 0), ex, up.double())):
         assert _rel(a, b) < (1e-4 if dtype == torch.float32 else 2.0 ** -6)
+
+
+# ------------------------------------------------------------------------------------------------ slices of K, gradients in place
+@pytest.mark.parametrize("M,K,N", [(128, 64, 4096), (130, 256, 8009), (2664, 512, 8009), (4096, 512, 8009), (300, 768, 12000), (2664, 512, 512), (512, 384, 384)])
+def test_dense_gradients_in_slices(M, K, N):
+    from keras_b200.kernels import gemm
+
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16().requires_grad_(True)
+    w = (torch.randn(K, N, generator=g, device="cuda") * K ** -0.5).bfloat16().requires_grad_(True)
+    up = torch.randn(M, N, generator=g, device="cuda").bfloat16()
+    dx, dw = torch.autograd.grad(gemm.GemmFn.apply(x, w, None, None, None), (x, w), up)
+    # exact products of bf16, fp32 sums in any order, one rounding to bf16
+    assert _rel(dx, up.double() @ w.detach().double().t()) < 2.0 ** -8
+    assert _rel(dw, x.detach().double().t() @ up.double()) < 2.0 ** -8
+    gemm.check_errors()
