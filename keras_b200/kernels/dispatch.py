@@ -329,6 +329,8 @@ def embedding(variable, table, ids, out_dtype):
     from keras_b200.kernels import gemm
 
     target = gemm._grad_target(variable, table) if variable is not None else None
+    if target is None and variable is not None and table is variable._value and table.requires_grad:
+        target = table  # the float32 parameter itself: the layer reads its table as it is stored
     return _ops().FusedEmbedding.apply(table, ids, out_dtype, target)
 
 

@@ -499,3 +499,25 @@ def test_dense_gradients_in_slices(M, K, N):
     assert _rel(dx, up.double() @ w.detach().double().t()) < 2.0 ** -8
     assert _rel(dw, x.detach().double().t() @ up.double()) < 2.0 ** -8
     gemm.check_errors()
+
+
+def test_embedding_gradient_goes_into_the_arena():
+    import keras_b200 as keras
+    from keras_b200.kernels import shadow
+
+    keras.config.set_dtype_policy("mixed_bfloat16")
+    try:
+        layer = keras.layers.Embedding(50, 64)
+        layer.build((None, 7))
+    finally:
+        keras.config.set_dtype_policy("float32")
+    ids = torch.randint(-3, 50, (9, 7), device="cuda", dtype=torch.int32)
+    table = layer._embeddings._value
+    up = torch.randn(9, 7, 64, device="cuda").bfloat16()
+    want = torch.zeros(50, 64, device="cuda").index_add_(0, ids.long().reshape(-1) % 50, up.float().reshape(-1, 64))
+    (own,) = torch.autograd.grad(layer(ids), table, up)
+    table.grad = torch.full_like(table, 2.0)
+    y = layer(ids)
+    with shadow.arena_backward():
+        y.backward(up)
+    assert _rel(own, want.double()) < 1e-6 and _rel(table.grad - 2.0, want.double()) < 1e-5
