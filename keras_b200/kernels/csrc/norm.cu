@@ -170,8 +170,8 @@ __global__ void __launch_bounds__(NT) norm_fwd_warp_kernel(const T* __restrict__
 
 // Bound by loads in flight: a warp holds a row's two or three tensors and 16 sums a vector of its columns, and the fewer registers that
 // takes the more rows an SM has on their way.  MB blocks an SM of 128 threads, and vectors that divide the row (three a lane at 768
-// columns).  With the gradient of the sum's other reader added on the way: [16384, 768] bf16 30.5 + 10.7 us apart -> 36.7, [2664, 512]
-// 8.2 + 2.0 -> 7.1 (four blocks an SM at three vectors spill: 45.6).
+// columns).  With the gradient of the sum's other reader added on the way: [16384, 768] bf16 30.5 + 10.7 us apart -> 30.3, [2664, 512]
+// 8.2 + 2.0 -> 6.9 (four blocks an SM at three vectors spill, 45.6; the other gradient loaded behind the sums, 36.7).
 template <typename T, int VPL, int NT, int WPR, int MB = 1>
 __global__ void __launch_bounds__(NT, MB) norm_bwd_warp_kernel(const T* __restrict__ dy, const T* __restrict__ x, const float* __restrict__ gamma,
                                                            const float* __restrict__ mean, const float* __restrict__ rstd, const T* __restrict__ dres,
@@ -204,12 +204,15 @@ __global__ void __launch_bounds__(NT, MB) norm_bwd_warp_kernel(const T* __restri
     if (!live) row = rows - 1;
     const uint4* xr = reinterpret_cast<const uint4*>(x + row * D);
     const uint4* dyr = reinterpret_cast<const uint4*>(dy + row * D);
-    uint4 xraw[VPL], draw[VPL];
+    // the other gradient too where registers allow: behind the sums its latency would stand alone
+    constexpr bool EARLY = sizeof(T) == 2 && VPL <= 3;
+    uint4 xraw[VPL], draw[VPL], oraw[EARLY ? VPL : 1];
 #pragma unroll
     for (int k = 0; k < VPL; ++k) {
       const int i = t + k * 32 * WPR;
       xraw[k] = i < nvec ? __ldg(xr + i) : make_uint4(0, 0, 0, 0);
       draw[k] = i < nvec ? __ldg(dyr + i) : make_uint4(0, 0, 0, 0);
+      if (EARLY && dres != nullptr && i < nvec) oraw[EARLY ? k : 0] = __ldg(reinterpret_cast<const uint4*>(dres + row * D) + i);
     }
     const float mu = rms ? 0.f : mean[row];
     const float rs = rstd[row];
@@ -254,7 +257,7 @@ __global__ void __launch_bounds__(NT, MB) norm_bwd_warp_kernel(const T* __restri
           }
           if (dres != nullptr) {  // what reaches the normalised sum on its other way
             float ov[VN];
-            nv_unpack<T>(__ldg(reinterpret_cast<const uint4*>(dres + row * D) + i), ov);
+            nv_unpack<T>(EARLY ? oraw[EARLY ? k : 0] : __ldg(reinterpret_cast<const uint4*>(dres + row * D) + i), ov);
 #pragma unroll
             for (int j = 0; j < VN; ++j) dv[j] += ov[j];
           }
