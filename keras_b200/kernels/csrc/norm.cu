@@ -688,6 +688,39 @@ KB_API int kb200_colsum(const void* x, long long ld, long long rows, int cols, f
 
 // dz = dy * act'(z) on contiguous bf16 [rows, cols] (cols a multiple of 8, 16-byte aligned bases), act: 1 relu, 3 silu, 4 gelu (erf).
 // With partial (scratch as for kb200_colsum) the column sums of dz go to out, or are added to it (accumulate).
+// y = gelu(z), exact, bf16: the activation behind a product whose input the backward pass needs as it was.  Bound by its traffic: four
+// vectors a thread in flight, and a normal distribution function of sixteen instructions.  [16384, 3072] 63 -> 39 us; 201 MB take 31.
+__global__ void __launch_bounds__(256) gelu_fwd_kernel(const uint4* __restrict__ z, uint4* __restrict__ y, long long vecs) {
+  constexpr int U = 4;
+  const long long first = (long long)blockIdx.x * 256 * U + threadIdx.x;
+  uint4 raw[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (first + u * 256 < vecs) raw[u] = __ldg(z + first + u * 256);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (first + u * 256 < vecs) {
+      float v[8];
+      nv_unpack<__nv_bfloat16>(raw[u], v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] *= normal_cdf(v[j]);
+      y[first + u * 256] = nv_pack<__nv_bfloat16>(v);
+    }
+  }
+}
+
+// n values, a multiple of 8, 16-byte aligned
+KB_API int kb200_gelu_fwd(const void* z, void* y, long long n, cudaStream_t stream) {
+  if (n <= 0) return 0;
+  if (n % 8 || (((uintptr_t)z | (uintptr_t)y) & 15) || n / 8192 > 0x7ffffff0ll) {
+    kb200_set_error("gelu_fwd: values in multiples of 8, 16-byte aligned");
+    return -2;
+  }
+  gelu_fwd_kernel<<<(unsigned)((n + 8191) / 8192), 256, 0, stream>>>((const uint4*)z, (uint4*)y, n / 8);
+  KB_CHECK_LAUNCH("gelu_fwd");
+  return 0;
+}
+
 KB_API int kb200_act_bwd(const void* dy, const void* z, void* dz, long long rows, int cols, int act, float* partial, float* out, int accumulate,
                          cudaStream_t stream) {
   if (rows <= 0 || cols <= 0) return 0;

@@ -152,7 +152,7 @@ class GemmFn(torch.autograd.Function):
                 b = torch.nn.functional.pad(b, (0, Np - N))
         out, pre = gemm(x, wide, 0, 1, M, Np, K, bias=b), None
         if act:
-            pre, out = out, _ACT_FN[act](out)
+            pre, out = out, kops.gelu(out) if act == 4 else _ACT_FN[act](out)
         ctx.save_for_backward(x, w, bias, pre, wide if Np != N else None)
         ctx.act = act
         ctx.has_bias = bias is not None

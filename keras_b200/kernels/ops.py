@@ -507,6 +507,13 @@ def column_sum(x, accumulate_into=None):
     return out
 
 
+def gelu(z):
+    """The exact GELU of a contiguous bf16 tensor whose size is a multiple of 8."""
+    y = torch.empty_like(z)
+    _check(_lib().kb200_gelu_fwd(_p(z), _p(y), _ll(z.numel()), _stream()), "gelu_fwd")
+    return y
+
+
 def activation_backward(dy, z, act, want_sums=False, accumulate_into=None):
     """``(dy * act'(z), its column sums or None)`` for contiguous bf16 matrices, in one pass; ``act`` as the GEMM numbers it."""
     lib = _lib()

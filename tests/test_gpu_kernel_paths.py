@@ -521,3 +521,14 @@ def test_embedding_gradient_goes_into_the_arena():
     with shadow.arena_backward():
         y.backward(up)
     assert _rel(own, want.double()) < 1e-6 and _rel(table.grad - 2.0, want.double()) < 1e-5
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 1024), (1000, 264), (2664, 2048)])
+def test_gelu_of_a_matrix(rows, cols):
+    from keras_b200.kernels import ops as kops
+
+    z = (torch.randn(rows, cols, device="cuda") * 4).bfloat16()
+    z[0, :4] = torch.tensor([float("inf"), float("-inf"), float("nan"), 0.0])
+    y, want = kops.gelu(z), z.double() * torch.special.erfc(z.double() * -(0.5 ** 0.5)) / 2  # without the cancellation of 1 + erf
+    assert torch.equal(y[0, :4].isnan(), want[0, :4].isnan()) and y[0, 0] == float("inf") and y[0, 3] == 0
+    assert torch.allclose(y.double(), want, rtol=2.0 ** -8, atol=1e-36, equal_nan=True)  # one rounding; the distribution function within 2.5e-6
