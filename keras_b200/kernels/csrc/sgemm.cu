@@ -201,6 +201,172 @@ int launch(const SgemmParams& p, long long tiles, cudaStream_t stream) {
   KB_CHECK_LAUNCH("sgemm");
   return 0;
 }
+
+// Weight gradients of layers that see many rows: C[M, N] = A^T B for A [K, M] and B [K, N] of K rows, and B's column sums beside it.
+//
+// Both operands lie in memory as the FMA loop wants them, k by k, so tiles go to shared memory by asynchronous copies alone and a thread
+// forms 8 x 8 sums from four 16-byte reads a k.  K is cut into so many slices that the CTAs fill the chip once; the slices' sums go
+// to a workspace (at most 20 MB, mostly met again in L2) and are added in their order by a second launch, which also adds to the gradient
+// where it is kept.  Bound by the FMA rate: 256 x 1024 over 6400 rows is 1.68 G products, 46 us at 128 a cycle
+// and SM; 77 us with the sums (the library's product 102 and sums 16), 32 x 1024 17 us (51).  The loop runs at 70 % of that rate with 8 x 8
+// sums a thread and 16 warps an SM, as it does with 16 x 8 and 8 warps.
+constexpr int WN = 128, WK = 16, W_STAGES = 3;
+constexpr int w_places(int wm) { return wm == 32 ? 6 : 4; }  // CTAs an SM: shared memory of 31 KB each, and 128 registers a thread
+
+struct WgradParams {
+  const float* a;
+  const float* b;
+  float* part;  // [slices, M + 1, pitch]: a slice's sums, its column sums in the last row
+  int M, N, K, slices, k_per, m_tiles, pitch;
+  long long lda, ldb;
+  int a_vec, b_vec;  // every row starts on a 16-byte line and holds a multiple of four values
+};
+
+__device__ __forceinline__ void copy_async16(uint32_t to, const float* from, bool real) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from), "r"(real ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_async4(uint32_t to, const float* from, bool real) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(from), "r"(real ? 4 : 0) : "memory");
+}
+
+// WK rows of an operand from row k0, W columns of them from column c0; zeros beyond k_end and beyond its `cols` columns
+template <int W, int T>
+__device__ __forceinline__ void copy_tile(float* tile, const float* p, long long ld, int cols, int c0, int k0, int k_end, int vec, int tid) {
+  const uint32_t to = (uint32_t)__cvta_generic_to_shared(tile);
+  if (vec) {
+#pragma unroll
+    for (int v = tid; v < WK * W / 4; v += T) {
+      const int k = v / (W / 4), c = v % (W / 4) * 4;
+      const bool real = k0 + k < k_end && c0 + c < cols;
+      copy_async16(to + v * 16, real ? p + (size_t)(k0 + k) * ld + c0 + c : p, real);
+    }
+  } else {
+    for (int v = tid; v < WK * W; v += T) {
+      const int k = v / W, c = v % W;
+      const bool real = k0 + k < k_end && c0 + c < cols;
+      copy_async4(to + v * 4, real ? p + (size_t)(k0 + k) * ld + c0 + c : p, real);
+    }
+  }
+}
+
+// A warp has 32 x 64 of a tile, a thread rows {0, 16} + 4 and columns {0, 32} + 4 of it: a warp's reads are 64 and 128 consecutive bytes
+template <int WM>
+__global__ void __launch_bounds__(WM * 2, w_places(WM)) wgrad_kernel(const WgradParams p) {
+  constexpr int T = WM * 2;
+  __shared__ __align__(16) float as[W_STAGES][WK][WM], bs[W_STAGES][WK][WN];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int slice = blockIdx.x % p.slices, tile = blockIdx.x / p.slices;
+  const int m0 = tile % p.m_tiles * WM, n0 = tile / p.m_tiles * WN;
+  const int k_begin = slice * p.k_per, k_end = min(p.K, k_begin + p.k_per), blocks = (k_end - k_begin + WK - 1) / WK;
+  const int rm = (warp >> 1) * 32 + (lane >> 3) * 4, rn = (warp & 1) * 64 + (lane & 7) * 4;
+  auto fetch = [&](int i) {
+    if (i < blocks) {
+      copy_tile<WM, T>(&as[i % W_STAGES][0][0], p.a, p.lda, p.M, m0, k_begin + i * WK, k_end, p.a_vec, tid);
+      copy_tile<WN, T>(&bs[i % W_STAGES][0][0], p.b, p.ldb, p.N, n0, k_begin + i * WK, k_end, p.b_vec, tid);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float2 acc[8][4] = {};  // pairs of columns: two products an instruction, so that the reads of shared memory find issue slots
+  float sums[WN / T] = {};
+#pragma unroll
+  for (int i = 0; i < W_STAGES - 1; ++i) fetch(i);
+  for (int i = 0; i < blocks; ++i) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(W_STAGES - 2) : "memory");
+    __syncthreads();  // block i is in shared memory, and every thread is done with block i - 1, whose place is filled next
+    fetch(i + W_STAGES - 1);
+    const float(*x)[WM] = as[i % W_STAGES];
+    const float(*y)[WN] = bs[i % W_STAGES];
+#pragma unroll
+    for (int k = 0; k < WK; ++k) {
+      float u[8];
+      float2 v[4];
+      *reinterpret_cast<float4*>(u) = *reinterpret_cast<const float4*>(&x[k][rm]);
+      *reinterpret_cast<float4*>(u + 4) = *reinterpret_cast<const float4*>(&x[k][rm + 16]);
+      *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(&y[k][rn]);
+      *reinterpret_cast<float4*>(v + 2) = *reinterpret_cast<const float4*>(&y[k][rn + 32]);
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[r][c] = __ffma2_rn(make_float2(u[r], u[r]), v[c], acc[r][c]);
+    }
+    if (m0 == 0) {
+#pragma unroll
+      for (int c = 0; c < WN / T; ++c)
+#pragma unroll
+        for (int k = 0; k < WK; ++k) sums[c] += y[k][c * T + tid];
+    }
+  }
+  float* out = p.part + (size_t)slice * (p.M + 1) * p.pitch;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const int m = m0 + rm + (r & 3) + (r >> 2) * 16;
+    if (m >= p.M) continue;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (n0 + rn + h * 32 < p.pitch)
+        *reinterpret_cast<float4*>(out + (size_t)m * p.pitch + n0 + rn + h * 32) = make_float4(acc[r][h * 2].x, acc[r][h * 2].y, acc[r][h * 2 + 1].x, acc[r][h * 2 + 1].y);
+  }
+  if (m0 == 0) {
+#pragma unroll
+    for (int c = 0; c < WN / T; ++c)
+      if (n0 + c * T + tid < p.pitch) out[(size_t)p.M * p.pitch + n0 + c * T + tid] = sums[c];
+  }
+}
+
+// c (+)= the slices' sums, db (+)= those of the last row (db null: left out).  A CTA has 32 quads of columns, its eight warps every eighth
+// slice, summed in a fixed order.
+__global__ void __launch_bounds__(256) wgrad_sum_kernel(const float* __restrict__ part, float* __restrict__ c, float* __restrict__ db, int M, int N, int pitch, int slices,
+                                                        int add, int add_db) {
+  __shared__ float4 warps[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quads = pitch / 4, at = blockIdx.x * 32 + lane;
+  const bool real = at < (M + (db != nullptr ? 1 : 0)) * quads;
+  const float4* s = reinterpret_cast<const float4*>(part) + at;
+  const size_t step = (size_t)(M + 1) * quads;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (real) {
+#pragma unroll 4
+    for (int i = warp; i < slices; i += 8) {
+      const float4 q = s[i * step];
+      v.x += q.x, v.y += q.y, v.z += q.z, v.w += q.w;
+    }
+  }
+  warps[warp][lane] = v;
+  __syncthreads();
+  if (warp != 0 || !real) return;
+  const int row = at / quads, col = at % quads * 4;
+  float* out = row < M ? c + (size_t)row * N + col : db + col;
+  const bool more = row < M ? add : add_db;
+  float old[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) old[j] = more && col + j < N ? out[j] : 0.f;
+#pragma unroll
+  for (int w = 1; w < 8; ++w) v.x += warps[w][lane].x, v.y += warps[w][lane].y, v.z += warps[w][lane].z, v.w += warps[w][lane].w;
+  const float t[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (col + j < N) out[j] = old[j] + t[j];
+}
+
+int wgrad_rows(int M) { return M <= 32 ? 32 : 64; }
+
+// Slices of K, their length a multiple of a block: the cheapest by the CTAs an SM has in turn (33 ns a row of K and full tile; fewer than
+// three full CTAs an SM leave the FMA pipes waiting) and by the workspace that is written and read again, among those that run at once.
+int wgrad_slices(int M, int N, int K, int* k_per) {
+  const int wm = wgrad_rows(M), sms = kb_sm_count(), full = 64 / wm;
+  const long long tiles = (long long)((M + wm - 1) / wm) * ((N + WN - 1) / WN);
+  int best = 1;
+  double least = 1e300;
+  for (long long s = 1; s == 1 || (s * tiles <= (long long)sms * w_places(wm) && s <= K / (2 * WK)); ++s) {
+    const int rows = (int)(((K + s - 1) / s + WK - 1) / WK * WK);
+    if (s > 1 && (long long)rows * (s - 1) >= K) continue;  // no rows for the last
+    const long long turn = (s * tiles + sms - 1) / sms;
+    const double alone = turn * 1. / full, idle = alone >= 4 ? 1.0 : alone >= 3 ? 1.07 : alone >= 2 ? 1.25 : alone >= 1 ? 2.2 : 2.2 / alone;
+    const double ns = turn * (rows + 2. * WK) * 33. / full * idle + s * (M + 1.) * N * 8. / 4000.;
+    if (ns < least) least = ns, best = (int)s;
+  }
+  *k_per = (int)(((K + best - 1) / best + WK - 1) / WK * WK);
+  return (K + *k_per - 1) / *k_per;
+}
 }  // namespace
 
 // C[M, N] = act(op(A) op(B) + bias) in float32.  a_rows: A is [M, K], else [K, M]; b_rows: B is [N, K], else [K, N] (not with A as [K, M]);
@@ -233,5 +399,39 @@ KB_API int kb200_relu_bwd(const float* dy, const float* out, float* dz, float* d
   if (M <= 0 || N <= 0) return 0;
   relu_bwd_kernel<<<(unsigned)((N + 31) / 32), 256, 0, stream>>>(dy, out, dz, db, M, N, accumulate);
   KB_CHECK_LAUNCH("relu_bwd");
+  return 0;
+}
+
+// Slices that kb200_sgemm_wgrad cuts K into: its workspace holds slices * (M + 1) * (N rounded up to 4) floats, 16-byte aligned.
+KB_API int kb200_sgemm_wgrad_slices(int M, int N, int K) {
+  int k_per;
+  return M <= 0 || N <= 0 || K <= 0 ? 0 : wgrad_slices(M, N, K, &k_per);
+}
+
+// c [M, N] (+)= A^T B and db [N] (+)= B's column sums (db null: left out); A [K, M] and B [K, N] of row pitches lda and ldb, c contiguous.
+KB_API int kb200_sgemm_wgrad(const float* a, const float* b, float* part, float* c, float* db, int M, int N, int K, long long lda, long long ldb, int add, int add_db,
+                             cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || lda < M || ldb < N || ((uintptr_t)part & 15)) {
+    kb200_set_error("sgemm_wgrad: an empty product, rows that overlap, or a workspace off its 16-byte line");
+    return -2;
+  }
+  WgradParams p{a, b, part, M, N, K, 0, 0, 0, (N + 3) / 4 * 4, lda, ldb, 0, 0};
+  p.slices = wgrad_slices(M, N, K, &p.k_per);
+  auto lines = [](const float* q, long long ld, int cols) { return ((uintptr_t)q & 15) == 0 && ld % 4 == 0 && cols % 4 == 0 ? 1 : 0; };
+  p.a_vec = lines(a, lda, M), p.b_vec = lines(b, ldb, N);
+  const int wm = wgrad_rows(M);
+  p.m_tiles = (M + wm - 1) / wm;
+  const long long ctas = (long long)p.m_tiles * ((N + WN - 1) / WN) * p.slices, quads = (long long)(M + 1) * (p.pitch / 4);
+  if (ctas > 0x7fffffffll || quads > 0x7fffff00ll) {
+    kb200_set_error("sgemm_wgrad: too many tiles for one launch");
+    return -2;
+  }
+  if (wm == 32)
+    wgrad_kernel<32><<<(unsigned)ctas, 64, 0, stream>>>(p);
+  else
+    wgrad_kernel<64><<<(unsigned)ctas, 128, 0, stream>>>(p);
+  KB_CHECK_LAUNCH("sgemm_wgrad");
+  wgrad_sum_kernel<<<(unsigned)((quads + 31) / 32), 256, 0, stream>>>(part, c, db, M, N, p.pitch, p.slices, add, add_db);
+  KB_CHECK_LAUNCH("sgemm_wgrad sums");
   return 0;
 }

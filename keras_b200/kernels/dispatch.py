@@ -375,10 +375,10 @@ def lstm_takes(sequences, initial_state, cell):
     return klstm.takes(sequences, initial_state, cell)
 
 
-def lstm(xz, bias, h0, c0, recurrent_kernel, reverse, want_sequence):
+def lstm(sequences, cell, initial_state, reverse, want_sequence):
     from keras_b200.kernels import lstm as klstm
 
-    return klstm.run(xz, bias, h0, c0, recurrent_kernel, reverse, want_sequence)
+    return klstm.layer(sequences, cell, initial_state[0], initial_state[1], reverse, want_sequence)
 
 
 # ---------------------------------------------------------------------------- optimizers

@@ -1,7 +1,7 @@
 """Front-end of the whole-sequence LSTM kernels (``csrc/lstm.cu``).
 
 ``run`` takes the projected inputs of all time steps and returns the outputs, the last state and the last cell state of a stock
-LSTM layer (keras/src/layers/rnn/lstm.py:240-300) from one launch; its backward pass is one launch and two products.
+LSTM layer (keras/src/layers/rnn/lstm.py:240-300) from one launch; its backward pass is one launch and the weight gradients.
 """
 
 import ctypes
@@ -9,6 +9,7 @@ import ctypes
 import torch
 
 from keras_b200.kernels import ops as kops
+from keras_b200.kernels import sgemm
 from keras_b200.kernels.gemm import _err_flag
 
 _i = ctypes.c_int
@@ -65,9 +66,48 @@ def _aligned(t):
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
+class Project(torch.autograd.Function):
+    """``x @ W`` of every time step, its weight gradient by the kernel for products over many rows."""
+
+    @staticmethod
+    def forward(ctx, x, W, target):
+        ctx.save_for_backward(x, W)
+        ctx.target = target
+        return torch.matmul(x, W)
+
+    @staticmethod
+    def backward(ctx, dxz):
+        x, W = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        if torch.is_grad_enabled():  # a gradient of this gradient is wanted: differentiate the library's product
+            grads = iter(torch.autograd.grad(torch.matmul(x, W), [t for t, n in zip((x, W), need) if n], dxz, create_graph=True))
+            return tuple(next(grads) if n else None for n in need[:2]) + (None,)
+        rows, dz = x.reshape(-1, x.shape[-1]), dxz.reshape(-1, dxz.shape[-1]).contiguous()
+        dW = None
+        if need[1]:
+            if sgemm.takes_weight_gradient(rows.shape[0], rows.shape[1], dz.shape[1], False):
+                dW, _ = sgemm.weight_gradient(rows.contiguous(), dz, ctx.target)
+            else:
+                dW = torch.matmul(rows.t(), dz)
+        return torch.matmul(dxz, W.t()) if need[0] else None, dW, None
+
+
+def _target(variable, tensor):
+    """The parameter itself where a kernel may add its gradient in place, else ``None``."""
+    return tensor if getattr(variable, "_value", None) is tensor and tensor.requires_grad else None
+
+
+def project(sequences, kernel):
+    """The projected inputs of all time steps, for operands that ``takes`` has let through."""
+    W = kernel.value if hasattr(kernel, "value") else kernel
+    if torch.is_grad_enabled() and W.requires_grad and W.ndim == 2 and W.shape[0] == sequences.shape[-1] and not torch.is_autocast_enabled("cuda"):
+        return Project.apply(sequences, W, _target(kernel, W))
+    return torch.matmul(sequences, W)
+
+
 class LstmSequence(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, xz, bias, h0, c0, R, reverse, want_sequence, recording):
+    def forward(ctx, xz, bias, h0, c0, R, reverse, want_sequence, recording, bias_target=None, R_target=None):
         B, T = xz.shape[0], xz.shape[1]
         U = R.shape[0]
         x, h, c, r = _aligned(xz), _aligned(h0), _aligned(c0), _aligned(R)
@@ -80,7 +120,7 @@ class LstmSequence(torch.autograd.Function):
         gates, cs = (empty(T, B, 4 * U), empty(T, B, U)) if grad else (None, None)
         _launch(0, x, b, h, c, r, hprev, out, hT, cT, gates, cs, None, None, None, None, None, None, reverse)
         ctx.save_for_backward(xz, bias, h0, c0, R, hprev, gates, cs)
-        ctx.reverse = reverse
+        ctx.reverse, ctx.targets = reverse, (bias_target, R_target)
         ctx.set_materialize_grads(False)
         return out, hT, cT
 
@@ -88,14 +128,14 @@ class LstmSequence(torch.autograd.Function):
     def backward(ctx, dout, dhT, dcT):
         xz, bias, h0, c0, R, hprev, gates, cs = ctx.saved_tensors
         if dout is None and dhT is None and dcT is None:
-            return (None,) * 8
+            return (None,) * 10
         if torch.is_grad_enabled():  # a gradient of this gradient is wanted: differentiate the composed operations
             inputs = [xz, bias, h0, c0, R]
             wanted = [t for t, need in zip(inputs, ctx.needs_input_grad) if need]
             results = _composed(xz, bias, h0, c0, R, ctx.reverse)
             pairs = [(r, g) for r, g in zip(results, (dout, dhT, dcT)) if g is not None]
             grads = iter(torch.autograd.grad([r for r, _ in pairs], wanted, [g for _, g in pairs], create_graph=True, allow_unused=True))
-            return tuple(next(grads) if need else None for need in ctx.needs_input_grad[:5]) + (None,) * 3
+            return tuple(next(grads) if need else None for need in ctx.needs_input_grad[:5]) + (None,) * 5
         B, T, U = hprev.shape
         need = ctx.needs_input_grad
         dout, dhT, dcT = (g.contiguous() if g is not None else None for g in (dout, dhT, dcT))
@@ -105,11 +145,20 @@ class LstmSequence(torch.autograd.Function):
         _launch(1, xz, None, None, c0.detach().contiguous(), R.detach().contiguous(), None, None, None, None, gates, cs, dout, dhT, dcT, dz, dh0, dc0,
                 ctx.reverse)
         flat = dz.view(B * T, 4 * U)
-        dR = torch.matmul(hprev.view(B * T, U).t(), flat) if need[4] else None
-        db = flat.sum(0) if need[1] else None
-        return dz if need[0] else None, db, dh0, dc0 if need[3] else None, dR, None, None, None
+        if need[4] and sgemm.takes_weight_gradient(B * T, U, 4 * U, need[1]):
+            dR, db = sgemm.weight_gradient(hprev.view(B * T, U), flat, ctx.targets[1], ctx.targets[0], sums=need[1])
+        else:
+            dR = torch.matmul(hprev.view(B * T, U).t(), flat) if need[4] else None
+            db = flat.sum(0) if need[1] else None
+        return (dz if need[0] else None, db, dh0, dc0 if need[3] else None, dR) + (None,) * 5
 
 
-def run(xz, bias, h0, c0, R, reverse, want_sequence):
-    """``(outputs [B, T, U] in processing order or None, last h, last c)``."""
-    return LstmSequence.apply(xz, bias, h0, c0, R, bool(reverse), bool(want_sequence), torch.is_grad_enabled())
+def run(xz, bias, h0, c0, R, reverse, want_sequence, bias_target=None, R_target=None):
+    """``(outputs [B, T, U] in processing order or None, last h, last c)``; targets as ``_target`` finds them."""
+    return LstmSequence.apply(xz, bias, h0, c0, R, bool(reverse), bool(want_sequence), torch.is_grad_enabled(), bias_target, R_target)
+
+
+def layer(sequences, cell, h0, c0, reverse, want_sequence):
+    """``run`` on the inputs of a stock cell that ``takes`` has let through."""
+    (bias, R), xz = [(v.value if hasattr(v, "value") else v) for v in (cell.bias, cell.recurrent_kernel)], project(sequences, cell.kernel)
+    return run(xz, bias, h0, c0, R, reverse, want_sequence, _target(cell.bias, bias), _target(cell.recurrent_kernel, R))

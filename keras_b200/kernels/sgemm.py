@@ -23,6 +23,35 @@ def product(a, b, a_rows, b_rows, M, N, K, bias=None, relu=False, into=None):
     return out
 
 
+def weight_gradient(a, b, target=None, bias_target=None, sums=False):
+    """``(a^T b, column sums of b or None)`` of ``a [K, M]`` and ``b [K, N]``, float32 with unit column strides.  What could be added to
+    its target's kept gradient comes back as ``None``."""
+    (K, M), N = a.shape, b.shape[1]
+    lib, p = kops._lib(), kops._p
+    empty = lambda *shape: torch.empty(shape, dtype=torch.float32, device=b.device)  # noqa: E731
+    slot = shadow.grad_slot(target, (M, N))
+    db_slot = shadow.grad_slot(bias_target, (N,)) if sums else None
+    c = empty(M, N) if slot is None else slot
+    db = (empty(N) if db_slot is None else db_slot) if sums else None
+    part = empty(lib.kb200_sgemm_wgrad_slices(_i(M), _i(N), _i(K)) * (M + 1) * ((N + 3) // 4 * 4))
+    kops._check(lib.kb200_sgemm_wgrad(p(a), p(b), p(part), p(c), p(db), _i(M), _i(N), _i(K), _ll(a.stride(0)), _ll(b.stride(0)), _i(0 if slot is None else 1),
+                                      _i(0 if db_slot is None else 1), kops._stream()), "sgemm_wgrad")
+    return c if slot is None else None, db if db_slot is None else None
+
+
+def takes_weight_gradient(K, M, N, sums):
+    """Whether ``weight_gradient`` is the quicker one, against the library's product and, with ``sums``, its column sums (us):
+
+    with sums     6400 rows, 256 x 1024 118 -> 77; 128 rows, 256 x 1024 9.1 -> 7.6; beyond, 2000 rows, 512 x 2048 92 -> 107
+    without       6400 rows, 32 x 1024 51 -> 17; few rows, 512 of 256 x 1024 11.3 -> 12.9; one column, 102400 of 1 x 400 45 -> 95
+    many rows     102400 of 256 x 1024 with sums 1164 -> 1086, without 1066 -> 1086, and 1168 -> 1277 where 250 columns are copied singly"""
+    if not 0 < M <= 256 or N <= 0 or K <= 0 or torch.backends.cuda.matmul.allow_tf32:
+        return False
+    if K > 32768 and M > 128 and (M % 4 or not sums):
+        return False
+    return sums or (K >= 1024 and M >= 8)
+
+
 class DenseFn(torch.autograd.Function):
     """``relu?(x @ w + bias)``; ``w_target`` / ``bias_target``: the parameters themselves where their gradients may be added in place."""
 

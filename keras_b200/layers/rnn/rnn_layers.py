@@ -677,9 +677,7 @@ class LSTM(_CellRNN):
             return None
         if not dispatch.lstm_takes(sequences, initial_state, cell):
             return None
-        bias = cell.bias.value if cell.bias is not None else None
-        outputs, h, c = dispatch.lstm(ops.matmul(sequences, cell.kernel), bias, initial_state[0], initial_state[1], cell.recurrent_kernel.value,
-                                      self.go_backwards, self.return_sequences)
+        outputs, h, c = dispatch.lstm(sequences, cell, initial_state, self.go_backwards, self.return_sequences)
         return h, outputs if self.return_sequences else h.unsqueeze(1), [h, c]
 
     def call(self, sequences, initial_state=None, mask=None, training=False):

@@ -37,6 +37,61 @@ def test_lstm_on_clusters_against_the_steps_in_64_bits(B, T, U, reverse, sequenc
         assert not n or _rel(a.grad, b.grad) < 1e-5  # up to B * T terms in the weight gradient
 
 
+# ------------------------------------------------------------------------------------------------ weight gradients over many rows
+# the edges of a tile (32, 64 rows, 128 columns) and of a block of K (16), one slice and many, rows that are copied value by value
+@pytest.mark.parametrize("K,M,N", [(1, 1, 1), (15, 3, 5), (16, 32, 128), (17, 33, 129), (33, 31, 127), (200, 64, 256), (1030, 65, 132), (3000, 250, 1000), (6400, 256, 1024),
+                                   (40000, 8, 48)])
+@pytest.mark.parametrize("kept", [False, True])
+def test_weight_gradient_of_many_rows(K, M, N, kept):
+    from keras_b200.kernels import sgemm, shadow
+
+    g = torch.Generator(device="cuda").manual_seed(K + M)
+    a = torch.randn((K, M + 4), generator=g, device="cuda")[:, :M]  # a row pitch of its own
+    b = torch.randn((K, N), generator=g, device="cuda")
+    if kept:
+        targets = [torch.nn.Parameter(torch.zeros(s, device="cuda")) for s in ((M, N), (N,))]
+        for t in targets:
+            t.grad = torch.ones_like(t)
+        with shadow.arena_backward():
+            assert sgemm.weight_gradient(a, b, *targets, sums=True) == (None, None)
+        w, s = (t.grad for t in targets)
+    else:
+        w, s = sgemm.weight_gradient(a, b, sums=True)
+        assert torch.equal(w, sgemm.weight_gradient(a, b)[0])
+    # any order of K products and sums errs by K + 2 roundings of 2^-24 of the sum of magnitudes at most
+    bound, old = (K + 2) * 2.0 ** -24, 1.0 if kept else 0.0
+    assert ((w.double() - old - a.double().t() @ b.double()).abs() <= bound * (a.double().abs().t() @ b.double().abs() + old)).all()
+    assert ((s.double() - old - b.double().sum(0)).abs() <= bound * (b.double().abs().sum(0) + old)).all()
+
+
+@pytest.mark.parametrize("F", [4, 24])  # the library's product, this package's
+def test_lstm_layer_weight_gradients_in_place_and_twice(F):
+    import keras_b200 as keras
+    from keras_b200.kernels import lstm, shadow
+
+    keras.utils.set_random_seed(0)
+    layer = keras.layers.LSTM(20, return_sequences=True)
+    x = torch.randn(128, 9, F, device="cuda")
+    up = torch.randn(128, 9, 20, device="cuda")
+    layer(x)
+    weights = [v._value for v in layer.trainable_variables]
+    exact = [w.detach().double().requires_grad_(True) for w in weights]
+    zero = torch.zeros(128, 20, device="cuda", dtype=torch.float64)
+    want = torch.autograd.grad((lstm._composed(x.double() @ exact[0], exact[2], zero, zero, exact[1], False)[0] * up).sum(), exact)
+    grads = torch.autograd.grad((layer(x) * up).sum(), weights)
+    for w in weights:
+        w.grad = torch.zeros_like(w)
+    with shadow.arena_backward():
+        (layer(x) * up).sum().backward()
+    for w, mine, ref in zip(weights, grads, want):
+        assert _rel(mine, ref) < 1e-5 and _rel(w.grad, ref) < 1e-5  # up to 1152 terms each
+        w.grad = None
+    twice = torch.autograd.grad((layer(x) * up).sum(), weights, create_graph=True)
+    for mine, ref in zip(twice, want):
+        assert _rel(mine.detach(), ref) < 1e-5
+    assert all(torch.isfinite(t).all() for t in torch.autograd.grad(sum((t ** 2).sum() for t in twice), weights))
+
+
 # ------------------------------------------------------------------------------------------------ products of inference
 @pytest.mark.parametrize("fp32", [True, False])
 @pytest.mark.parametrize("M,K,widths", [(1, 64, (64,)), (7, 72, (72,)), (77, 768, (1001,)), (128, 200, (264,)), (128, 3072, (64, 64, 128)), (33, 256, (1024, 256, 256)),
