@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(256) place_weight_kernel(const T* __restrict__
   const int v = (int)(i - r * vecs);
   const T* s = src + r * N + (long long)v * 8;
   float f[8];
-  if (vec && sizeof(T) == 4) {
+  if (vec && sizeof(T) == 4 && v * 8 < N) {
     const float4 lo = *reinterpret_cast<const float4*>(s), hi = v * 8 + 4 < N ? *reinterpret_cast<const float4*>(s + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
     f[0] = lo.x, f[1] = lo.y, f[2] = lo.z, f[3] = lo.w, f[4] = hi.x, f[5] = hi.y, f[6] = hi.z, f[7] = hi.w;
   } else {
@@ -327,8 +327,9 @@ KB_API int kb200_dense_direct(int M) { return M <= rw::BM ? 1 : 0; }
 
 // C[M, ldo] (bf16, contiguous rows) = act(A x [W0 W1 W2] + bias): A bf16 [M, K], pitch lda; W_i [K, n_i] contiguous, all float32 (w_fp32) or
 // bf16; biases per weight, float32 or (bias16) bf16, null where there is none.  More than one weight: widths that are multiples of 64.
-// ldo: the sum of the widths up to the next multiple of 8; the columns behind it hold zeros.  scratch: where kb200_dense_direct says 0, a bf16
-// matrix [K, ldo] and ldo floats behind it, or null if there is one bf16 weight whose width is a multiple of 8.
+// ldo: the sum of the widths up to the next multiple of 8, or of 64 for one odd width of many rows; the columns behind it hold zeros.
+// scratch: where kb200_dense_direct says 0, a bf16 matrix [K, ldo] and ldo floats behind it, or null if there is one bf16 weight whose width
+// is a multiple of 8.
 KB_API int kb200_dense_infer(const void* a, const void* w0, const void* w1, const void* w2, const void* b0, const void* b1, const void* b2, int n0, int n1, int n2,
                              void* out, void* scratch, int M, int K, long long lda, long long ldo, int w_fp32, int bias16, int act, int* err, cudaStream_t stream) {
   if (M <= 0 || K <= 0 || n0 <= 0) return 0;
@@ -337,7 +338,9 @@ KB_API int kb200_dense_infer(const void* a, const void* w0, const void* w1, cons
   const int n[MAX_WEIGHTS] = {n0, n1, n2};
   const int count = n2 > 0 ? 3 : n1 > 0 ? 2 : 1, total = n0 + n1 + n2;
   const bool has_bias = b0 != nullptr || b1 != nullptr || b2 != nullptr;
-  if ((lda % 8) || (K % 8) || ldo != (total + 7) / 8 * 8 || (((uintptr_t)a | (uintptr_t)out | (uintptr_t)scratch) & 15) ||
+  // one odd width in whole 128-byte lines (a matrix of its own then)
+  const bool wider = M > rw::BM && count == 1 && n0 % 8 && ldo == (total + 63ll) / 64 * 64;
+  if ((lda % 8) || (K % 8) || !(ldo == (total + 7) / 8 * 8 || wider) || (((uintptr_t)a | (uintptr_t)out | (uintptr_t)scratch) & 15) ||
       (count > 1 && ((n0 % 64) || (n1 % 64) || (n2 % 64) || bias16)) || (bias16 && n0 % 8)) {
     kb200_set_error("dense_infer: 16-byte aligned operands, pitches in multiples of 8, several weights only in multiples of 64 columns with float32 biases, odd widths with float32 ones");
     return -2;
@@ -373,7 +376,7 @@ KB_API int kb200_dense_infer(const void* a, const void* w0, const void* w1, cons
   float* bias = (float*)(matrix + (size_t)K * ldo);
   const bool place_bias = has_bias && (count > 1 || n0 % 8) && !bias16;
   for (int i = 0, at = 0; i < count; at += n[i], ++i) {
-    const int vecs = (n[i] + 7) / 8;
+    const int vecs = count == 1 ? (int)(ldo / 8) : (n[i] + 7) / 8;
     const long long grid = ((long long)K * vecs + 255) / 256;
     if (grid > 0x7fffffffll) {
       kb200_set_error("dense_infer: weight too large for one launch");

@@ -571,7 +571,7 @@ class FusedSoftmaxXent(torch.autograd.Function):
         upstream = getattr(_EXPECTED, "upstream", None)
         # the gradient made here, and the upstream gradient that it is for; the first backward pass takes it
         ctx.made, ctx.made_for = None, 0.0
-        zero_to = ld if ld - V < 16 else V
+        zero_to = ld if ld - V < 64 else V
         if upstream is not None and ctx.needs_input_grad[0] and lib.kb200_xent_wide(_i(V)):
             ctx.made, ctx.made_for = torch.empty((rows, ld), dtype=flat.dtype, device=flat.device), float(upstream(rows))
             _check(lib.kb200_xent_fwd_grad(_p(flat), _p(labels64), _p(loss), _p(lse), _p(ctx.made), _f(ctx.made_for), _ll(rows), _i(V), _ll(ld), _i(zero_to),

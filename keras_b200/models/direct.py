@@ -74,7 +74,7 @@ _DENSE = [_V] * 7 + [_I] * 3 + [_V] * 2 + [_I] * 2 + [_L] * 2 + [_I] * 3 + [_V] 
 
 
 def _product(x, weights, biases, act):
-    """``act(x @ [w0 w1 w2] + bias)`` of contiguous matrices of one type, as rows of a pitch that is a multiple of 8; ``None`` where the
+    """``act(x @ [w0 w1 w2] + bias)`` of contiguous matrices of one type, as rows of a pitch that is a multiple of 8 (``gemm.padded_width`` above 128 rows); ``None`` where the
     kernels do not take it."""
     K = x.shape[-1]
     widths = [w.numel() // K for w in weights]
@@ -97,7 +97,7 @@ def _product(x, weights, biases, act):
             biases, bias16 = [b if b is None else b.float() for b in biases], False
     if len(weights) > 1 and any(n % 64 for n in widths):
         return None
-    pitch = (N + 7) // 8 * 8
+    pitch = kgemm.padded_width(N) if M > 128 else (N + 7) // 8 * 8
     out = torch.empty((M, pitch), dtype=_BF16, device=x.device)
     scratch = None
     if M > 128 and (fp32 or len(weights) > 1 or N % 8):

@@ -37,6 +37,35 @@ def test_lstm_on_clusters_against_the_steps_in_64_bits(B, T, U, reverse, sequenc
         assert not n or _rel(a.grad, b.grad) < 1e-5  # up to B * T terms in the weight gradient
 
 
+# ------------------------------------------------------------------------------------------------ products of odd width
+# the last width in multiples of 8, the first and the fullest in multiples of 64, one that is a multiple of 8
+@pytest.mark.parametrize("N,pitch", [(1023, 1024), (1025, 1088), (1087, 1088), (1032, 1032), (8009, 8064)])
+def test_odd_widths_are_computed_in_whole_lines(N, pitch):
+    from keras_b200.kernels import gemm
+    from keras_b200.kernels import ops as kops
+
+    g = torch.Generator(device="cuda").manual_seed(N)
+    M, K = 300, 128
+    x = torch.randn((M, K), generator=g, device="cuda").bfloat16().requires_grad_(True)
+    w = (torch.randn((K, N), generator=g, device="cuda") * K ** -0.5).bfloat16().requires_grad_(True)
+    b = torch.randn(N, generator=g, device="cuda").requires_grad_(True)
+    labels = torch.randint(0, N, (M,), generator=g, device="cuda")
+    y = gemm.GemmFn.apply(x, w, b)
+    assert gemm.padded_width(N) == pitch and y.shape == (M, N) and y.stride() == (pitch, 1)
+    seen = []
+    y.register_hook(seen.append)
+    kops.FusedSoftmaxXent.apply(y, labels).sum().backward()
+    gemm.check_errors()
+    assert seen[0].stride() == (pitch, 1) and not seen[0].as_strided((M, pitch), (pitch, 1))[:, N:].any()
+    exact = [t.detach().double().requires_grad_(True) for t in (x, w, b)]
+    want = exact[0] @ exact[1] + exact[2]
+    torch.nn.functional.cross_entropy(want, labels, reduction="sum").backward()
+    # logits rounded to bf16 (2^-9 of values up to 5), and their gradient with them
+    assert _rel(y.detach(), want.detach()) < 2.0 ** -8
+    for got, ref in zip((x, w, b), exact):
+        assert _rel(got.grad, ref.grad) < 2.0 ** -6
+
+
 # ------------------------------------------------------------------------------------------------ weight gradients over many rows
 # the edges of a tile (32, 64 rows, 128 columns) and of a block of K (16), one slice and many, rows that are copied value by value
 @pytest.mark.parametrize("K,M,N", [(1, 1, 1), (15, 3, 5), (16, 32, 128), (17, 33, 129), (33, 31, 127), (200, 64, 256), (1030, 65, 132), (3000, 250, 1000), (6400, 256, 1024),
