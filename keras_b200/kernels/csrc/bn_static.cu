@@ -11,8 +11,8 @@ extern "C" int kb200_bn_bwd_reduce(const void* dy, const void* x, const void* y,
 extern "C" int kb200_bn_bwd_apply(const void* dy, const void* x, const void* y, const float* mean, const float* invstd, const float* gamma,
                                   const float* sums, float* coef, void* dx, void* dres, long long M, int C, int dtype, cudaStream_t stream);
 
-// [0, 2C): per-channel sums (must be zero when the reduction starts); [2C, 5C): dx coefficients.
-static __device__ __align__(256) float g_bn_static_scratch[5 * KB200_BN_STATIC_MAX_C];
+// [0, 2C): per-channel sums (must be zero when the reduction starts).
+static __device__ __align__(256) float g_bn_static_scratch[2 * KB200_BN_STATIC_MAX_C];
 
 namespace {
 constexpr int kMaxDevices = 64;
@@ -57,10 +57,9 @@ KB_API int kb200_bn_bwd_static(const void* dy, const void* x, const void* y, con
   float* scratch = nullptr;
   if (scratch_for_current_device(&scratch) != 0) return -1;
   float* sums = scratch;
-  float* coef = scratch + 2 * (size_t)C;
   int rc = kb200_bn_bwd_reduce(dy, x, y, mean, invstd, M, C, dtype, sums, stream);  // clears sums[0:2C] on `stream` first
   if (rc != 0) return rc;
-  rc = kb200_bn_bwd_apply(dy, x, y, mean, invstd, gamma, sums, coef, dx, dres, M, C, dtype, stream);
+  rc = kb200_bn_bwd_apply(dy, x, y, mean, invstd, gamma, sums, nullptr, dx, dres, M, C, dtype, stream);
   if (rc != 0) return rc;
   cudaError_t e = cudaSuccess;
   if (dbeta != nullptr) e = cudaMemcpyAsync(dbeta, sums, sizeof(float) * C, cudaMemcpyDeviceToDevice, stream);

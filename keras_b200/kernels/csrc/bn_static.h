@@ -3,13 +3,12 @@
 // This entry point has no counterpart in the reference (keras-team/keras has no C ABI and leaves
 // all temporaries to its backend's allocator).  It exists for callers of libkb200.so that are not
 // allowed to allocate: a C or C++ serving/runtime process that links the library without torch
-// (so there is no caching allocator to hand out the 5*C-float temporary), and processes that have
+// (so there is no caching allocator to hand out the 2*C-float temporary), and processes that have
 // already handed all free HBM to their own pools, where cudaMalloc can fail and, like cudaFree,
 // stalls every stream of the device while it runs.
 //
-// The temporary that kb200_bn_bwd_reduce / kb200_bn_bwd_apply take from the caller (2*C sums and
-// 3*C coefficients, fp32) lives in a file-scope `static __device__` array of
-// KB200_BN_STATIC_MAX_C * 5 floats (80 KiB) instead.  The host asks for its address once per
+// The temporary that kb200_bn_bwd_reduce / kb200_bn_bwd_apply take from the caller (2*C sums, fp32)
+// lives in a file-scope `static __device__` array of KB200_BN_STATIC_MAX_C * 2 floats (32 KiB) instead.  The host asks for its address once per
 // device (cudaGetSymbolAddress, with that device current) and hands the pointer to the kernels.
 //
 // Rules for callers
@@ -20,8 +19,7 @@
 //    so that later calls only enqueue work on `stream`.
 //  * Every call on a device shares the one array.  The first 2*C floats must be zero when the
 //    reduction starts; the call clears them itself on `stream` (cudaMemsetAsync), so callers need
-//    not.  The remaining 3*C floats are fully written before they are read.  Stale values beyond
-//    5*C from an earlier, wider call are never read.
+//    not.  Stale values beyond 2*C from an earlier, wider call are never read.
 //  * Two calls that can run at the same time on one device (different streams with no ordering
 //    between them, or two host threads) race on the array and give wrong gradients.  Order them
 //    on one stream or with events.
