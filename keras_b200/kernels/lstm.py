@@ -94,7 +94,7 @@ class Project(torch.autograd.Function):
 
 def _target(variable, tensor):
     """The parameter itself where a kernel may add its gradient in place, else ``None``."""
-    return tensor if getattr(variable, "_value", None) is tensor and tensor.requires_grad else None
+    return tensor if tensor is not None and getattr(variable, "_value", None) is tensor and tensor.requires_grad else None
 
 
 def project(sequences, kernel):

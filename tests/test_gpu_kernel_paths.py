@@ -93,20 +93,20 @@ def test_weight_gradient_of_many_rows(K, M, N, kept):
     assert ((s.double() - old - b.double().sum(0)).abs() <= bound * (b.double().abs().sum(0) + old)).all()
 
 
-@pytest.mark.parametrize("F", [4, 24])  # the library's product, this package's
-def test_lstm_layer_weight_gradients_in_place_and_twice(F):
+@pytest.mark.parametrize("F,bias", [(4, True), (24, True), (24, False)])  # the library's product, this package's
+def test_lstm_layer_weight_gradients_in_place_and_twice(F, bias):
     import keras_b200 as keras
     from keras_b200.kernels import lstm, shadow
 
     keras.utils.set_random_seed(0)
-    layer = keras.layers.LSTM(20, return_sequences=True)
+    layer = keras.layers.LSTM(20, return_sequences=True, use_bias=bias)
     x = torch.randn(128, 9, F, device="cuda")
     up = torch.randn(128, 9, 20, device="cuda")
     layer(x)
     weights = [v._value for v in layer.trainable_variables]
     exact = [w.detach().double().requires_grad_(True) for w in weights]
     zero = torch.zeros(128, 20, device="cuda", dtype=torch.float64)
-    want = torch.autograd.grad((lstm._composed(x.double() @ exact[0], exact[2], zero, zero, exact[1], False)[0] * up).sum(), exact)
+    want = torch.autograd.grad((lstm._composed(x.double() @ exact[0], exact[2] if bias else None, zero, zero, exact[1], False)[0] * up).sum(), exact)
     grads = torch.autograd.grad((layer(x) * up).sum(), weights)
     for w in weights:
         w.grad = torch.zeros_like(w)
