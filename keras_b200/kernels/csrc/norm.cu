@@ -686,8 +686,6 @@ KB_API int kb200_colsum(const void* x, long long ld, long long rows, int cols, f
   return 0;
 }
 
-// dz = dy * act'(z) on contiguous bf16 [rows, cols] (cols a multiple of 8, 16-byte aligned bases), act: 1 relu, 3 silu, 4 gelu (erf).
-// With partial (scratch as for kb200_colsum) the column sums of dz go to out, or are added to it (accumulate).
 // y = gelu(z), exact, bf16: the activation behind a product whose input the backward pass needs as it was.  Bound by its traffic: four
 // vectors a thread in flight, and a normal distribution function of sixteen instructions.  [16384, 3072] 63 -> 39 us; 201 MB take 31.
 __global__ void __launch_bounds__(256) gelu_fwd_kernel(const uint4* __restrict__ z, uint4* __restrict__ y, long long vecs) {
@@ -721,6 +719,8 @@ KB_API int kb200_gelu_fwd(const void* z, void* y, long long n, cudaStream_t stre
   return 0;
 }
 
+// dz = dy * act'(z) on contiguous bf16 [rows, cols] (cols a multiple of 8, 16-byte aligned bases), act: 1 relu, 3 silu, 4 gelu (erf).
+// With partial (scratch as for kb200_colsum) the column sums of dz go to out, or are added to it (accumulate).
 KB_API int kb200_act_bwd(const void* dy, const void* z, void* dz, long long rows, int cols, int act, float* partial, float* out, int accumulate,
                          cudaStream_t stream) {
   if (rows <= 0 || cols <= 0) return 0;
