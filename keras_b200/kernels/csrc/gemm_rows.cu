@@ -3,10 +3,11 @@
 // Inference on a handful of tokens reads every weight once and does little else: the bound is the weights' bytes.  A float32 weight used
 // to be read, written as bf16 by a cast of its own and read again by the library's product; here its tiles go through registers,
 // where they are rounded, straight into the swizzled operand layout in shared memory, and no copy of the weight exists.  A CTA has 64
-// columns; where those are few the K range is shared by the CTAs of a cluster, whose sums are added in the order of their ranks through distributed
-// shared memory, so results do not depend on timing.  Three CTAs an SM keep some 48 KB of weights in flight.
+// columns and walks the whole of K, three CTAs an SM with some 48 KB of weights in flight, so it takes a weight of many columns: a
+// vocabulary.  CTAs that share K would have narrower ones run as quickly, but their sums round otherwise than those of the layers' own calls,
+// which run along K, and a first call would differ from a second one.
 //
-// Every wait is bounded: on expiry the kernel records a code in *err, and the CTAs of a cluster leave together.
+// Every wait is bounded: on expiry the kernel records a code in *err and returns.
 #include "gemm_sm100.cuh"
 
 namespace {
@@ -30,9 +31,9 @@ struct RowsParams {
   int vec[MAX_WEIGHTS];           // rows of this weight start on 16-byte lines
   int weights;
   void* out;
-  int M, K, slices, kb_per;
+  int M, K;
   long long ldo;
-  int act, bias16;
+  int act, bias16, apart;
   int* err;
 };
 struct WView {  // the weight of a tile
@@ -126,10 +127,10 @@ __global__ void __launch_bounds__(rw::THREADS, 3) gemm_rows_kernel(const __grid_
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + rw::STAGES * rw::STAGE + 8 * (2 * rw::STAGES + 1));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int slice = blockIdx.x % p.slices, n0 = (blockIdx.x / p.slices) * rw::BN;
+  const int n0 = blockIdx.x * rw::BN;
   const int which = p.weights > 2 && n0 >= p.start[2] ? 2 : p.weights > 1 && n0 >= p.start[1] ? 1 : 0;
   const WView wv{p.w[which], p.width[which], n0 - p.start[which], p.K, p.vec[which]};
-  const int kb_all = (p.K + rw::BK - 1) / rw::BK, kb0 = slice * p.kb_per, blocks = min(p.kb_per, kb_all - kb0);  // at least one
+  const int blocks = (p.K + rw::BK - 1) / rw::BK;
 
   if (tid == rw::LOADERS) {
     prefetch_map(&map_a);
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(rw::THREADS, 3) gemm_rows_kernel(const __grid_
         ok = rows_wait(empty(s), ((b / rw::STAGES) & 1) ^ 1, abort_flag);
         if (!ok) break;
         mbar_expect_tx(full(s), rw::A_BYTES);
-        tma_load_2d(base + s * rw::STAGE, &map_a, full(s), (kb0 + b) * rw::BK, 0);
+        tma_load_2d(base + s * rw::STAGE, &map_a, full(s), b * rw::BK, 0);
         issued = b + 1;
       }
       if (!ok) {
@@ -194,11 +195,11 @@ __global__ void __launch_bounds__(rw::THREADS, 3) gemm_rows_kernel(const __grid_
   } else {
     bool ok = true;
     WTile<T> tile;
-    tile.load(wv, kb0 * rw::BK, tid);
+    tile.load(wv, 0, tid);
     for (int b = 0; b < blocks && ok; ++b) {
       const int s = b % rw::STAGES;
       WTile<T> next;
-      if (b + 1 < blocks) next.load(wv, (kb0 + b + 1) * rw::BK, tid);
+      if (b + 1 < blocks) next.load(wv, (b + 1) * rw::BK, tid);
       ok = rows_wait(empty(s), ((b / rw::STAGES) & 1) ^ 1, abort_flag);
       if (!ok) break;
       tile.store(base + s * rw::STAGE + rw::A_BYTES, wv.vec, tid);
@@ -227,45 +228,25 @@ __global__ void __launch_bounds__(rw::THREADS, 3) gemm_rows_kernel(const __grid_
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
-  if (p.slices > 1) {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-  }
-  // Rows of the result: those of this CTA's share, eight columns a thread
-  const int share = (p.M + p.slices - 1) / p.slices, r0 = slice * share, r1 = min(p.M, r0 + share);
+  // Rows of the result, eight columns a thread
   const void* bias = p.bias[which];
   const int width = min(rw::BN, (int)p.ldo - n0);  // columns of the output's rows, their padding included
-  for (int i = r0 * 8 + tid; i < r1 * 8; i += rw::THREADS) {
+  for (int i = tid; i < p.M * 8; i += rw::THREADS) {
     const int row = i >> 3, c = (i & 7) * 8;
     if (c >= width) continue;
-    const uint32_t at = base + (uint32_t)((row * rw::SUM_PITCH + c) * 4);
-    float v[8] = {};
-    for (int s = 0; s < p.slices; ++s) {
-      uint32_t peer = at;
-      if (p.slices > 1) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(s));
-      float f[8];
-      if (p.slices > 1) {
-        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]) : "r"(peer) : "memory");
-        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "r"(peer + 16) : "memory");
-      } else {
-        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]) : "r"(peer) : "memory");
-        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "r"(peer + 16) : "memory");
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = s == 0 ? f[j] : v[j] + f[j];
-    }
+    const float* sum = reinterpret_cast<const float*>(base_ptr) + (size_t)row * rw::SUM_PITCH + c;
+    const float4 lo = *reinterpret_cast<const float4*>(sum), hi = *reinterpret_cast<const float4*>(sum + 4);
+    float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int n = wv.n0 + c + j;
-      if (bias != nullptr && n < wv.N) v[j] += p.bias16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(bias)[n]) : reinterpret_cast<const float*>(bias)[n];
+      if (p.apart) v[j] = __bfloat162float(__float2bfloat16(v[j]));
+      if (bias != nullptr && n < wv.N)  // in the layer's type, as the layer itself reads it
+        v[j] += __bfloat162float(p.bias16 ? reinterpret_cast<const __nv_bfloat16*>(bias)[n] : __float2bfloat16(reinterpret_cast<const float*>(bias)[n]));
       v[j] = apply_act<false>(v[j], p.act);
     }
     const bf16x8 pk = pack8(v);
     *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)row * p.ldo + n0 + c) = *reinterpret_cast<const uint4*>(&pk);
-  }
-  if (p.slices > 1) {  // the peers still read these sums
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
 }
 
@@ -276,38 +257,42 @@ int launch_rows(const CUtensorMap& map_a, const RowsParams& p, int n_tiles, cuda
     kb200_set_error("gemm_rows: cannot raise the shared-memory limit of the kernel on this device");
     return -3;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(n_tiles * p.slices));
-  cfg.blockDim = dim3(rw::THREADS);
-  cfg.dynamicSmemBytes = rw::SMEM;
-  cfg.stream = stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)p.slices;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, gemm_rows_kernel<T>, map_a, p);
+  gemm_rows_kernel<T><<<(unsigned)n_tiles, rw::THREADS, rw::SMEM, stream>>>(map_a, p);
   KB_CHECK_LAUNCH("gemm_rows");
   return 0;
 }
 
-// A weight for the GEMM of many rows: W [K, N] float32 or bf16 of any width into columns [at, at + pad) of a bf16 matrix, zeros behind
-// N.  Bound by its traffic: [768, 50257] float32, 231 MB: 44 us; a cast and a padding pass of its own took 24 + 31.
+// Weights for the GEMM of many rows: W_i [K, N_i] float32 or bf16 of any width into columns [start, start + 8 vecs) of a bf16 matrix, zeros
+// behind N_i, and their biases rounded to bf16 beside it.  Bound by its traffic: [768, 50257] float32, 231 MB: 44 us; a cast and a padding
+// pass of its own took 24 + 31.
+struct PlaceParams {
+  const void* w[MAX_WEIGHTS];
+  const float* bias[MAX_WEIGHTS];
+  int start[MAX_WEIGHTS], width[MAX_WEIGHTS], vecs[MAX_WEIGHTS];
+  long long end[MAX_WEIGHTS];  // blocks up to the end of this weight
+  int vec[MAX_WEIGHTS];
+  int rows;
+  __nv_bfloat16* dst;
+  float* bias_out;
+  long long ldd;
+};
 template <typename T>
-__global__ void __launch_bounds__(256) place_weight_kernel(const T* __restrict__ src, __nv_bfloat16* __restrict__ dst, int rows, int N, int vecs, long long ldd, int vec,
-                                                           const float* __restrict__ bias, float* __restrict__ bias_out) {
-  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (bias_out != nullptr && i < vecs) {
+__global__ void __launch_bounds__(256) place_weight_kernel(const PlaceParams p) {
+  const int which = blockIdx.x < p.end[0] ? 0 : blockIdx.x < p.end[1] ? 1 : 2;
+  const int N = p.width[which], vecs = p.vecs[which];
+  const long long i = ((long long)blockIdx.x - (which > 0 ? p.end[which - 1] : 0)) * 256 + threadIdx.x;
+  if (p.bias_out != nullptr && i < vecs) {
+    const float* bias = p.bias[which];
+    float* to = p.bias_out + p.start[which] + i * 8;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) bias_out[i * 8 + j] = bias != nullptr && i * 8 + j < N ? bias[i * 8 + j] : 0.f;
+    for (int j = 0; j < 8; ++j) to[j] = bias != nullptr && i * 8 + j < N ? __bfloat162float(__float2bfloat16(bias[i * 8 + j])) : 0.f;
   }
   const long long r = i / vecs;
-  if (r >= rows) return;
+  if (r >= p.rows) return;
   const int v = (int)(i - r * vecs);
-  const T* s = src + r * N + (long long)v * 8;
+  const T* s = reinterpret_cast<const T*>(p.w[which]) + r * N + (long long)v * 8;
   float f[8];
-  if (vec && sizeof(T) == 4 && v * 8 < N) {
+  if (p.vec[which] && sizeof(T) == 4 && v * 8 < N) {
     const float4 lo = *reinterpret_cast<const float4*>(s), hi = v * 8 + 4 < N ? *reinterpret_cast<const float4*>(s + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
     f[0] = lo.x, f[1] = lo.y, f[2] = lo.z, f[3] = lo.w, f[4] = hi.x, f[5] = hi.y, f[6] = hi.z, f[7] = hi.w;
   } else {
@@ -315,23 +300,61 @@ __global__ void __launch_bounds__(256) place_weight_kernel(const T* __restrict__
     for (int j = 0; j < 8; ++j) f[j] = v * 8 + j < N ? to_f32<T>(s[j]) : 0.f;
   }
   const bf16x8 pk = pack8(f);
-  *reinterpret_cast<uint4*>(dst + r * ldd + (long long)v * 8) = *reinterpret_cast<const uint4*>(&pk);
+  *reinterpret_cast<uint4*>(p.dst + r * p.ldd + p.start[which] + (long long)v * 8) = *reinterpret_cast<const uint4*>(&pk);
+}
+
+// Up to three weights side by side and their biases behind one another; false: too large for a launch.
+bool place(const void* const* w, const void* const* b, const int* n, int count, __nv_bfloat16* matrix, float* bias, int K, long long ld, int w_fp32, cudaStream_t stream) {
+  PlaceParams p{};
+  long long blocks = 0;
+  for (int i = 0, at = 0; i < MAX_WEIGHTS; at += n[i], ++i) {
+    if (i < count) {
+      p.w[i] = w[i], p.bias[i] = (const float*)b[i], p.start[i] = at, p.width[i] = n[i];
+      p.vecs[i] = count == 1 ? (int)(ld / 8) : (n[i] + 7) / 8;
+      p.vec[i] = ((uintptr_t)w[i] & 15) == 0 && n[i] % 4 == 0;
+      blocks += ((long long)K * p.vecs[i] + 255) / 256;
+    }
+    p.end[i] = blocks;
+  }
+  if (blocks > 0x7fffffffll) return false;
+  p.rows = K, p.dst = matrix, p.bias_out = bias, p.ldd = ld;
+  if (w_fp32) place_weight_kernel<float><<<(unsigned)blocks, 256, 0, stream>>>(p);
+  else place_weight_kernel<__nv_bfloat16><<<(unsigned)blocks, 256, 0, stream>>>(p);
+  return true;
+}
+
+// out = relu?(out + bias) on contiguous bf16 rows of `ld` columns, a multiple of 8; the bias in bf16 or float32, its first `n` columns
+__global__ void __launch_bounds__(256) bias_rows_kernel(uint4* __restrict__ out, const void* __restrict__ bias, long long vecs, int per_row, int n, int bias16, int relu) {
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= vecs) return;
+  const int c = (int)(i % per_row) * 8;
+  const uint4 raw = out[i];
+  const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&raw);
+  float v[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    v[j] = __bfloat162float(h[j]);
+    if (bias != nullptr && c + j < n) v[j] += bias16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(bias)[c + j]) : reinterpret_cast<const float*>(bias)[c + j];
+    if (relu) v[j] = v[j] <= 0.f ? 0.f : v[j];  // a NaN stays one
+  }
+  const bf16x8 pk = pack8(v);
+  out[i] = *reinterpret_cast<const uint4*>(&pk);
 }
 }  // namespace
 
 KB_API int kb200_gemm_bf16_run(const void* a, const void* b, void* c, const void* bias, int M, int N, int K, long long lda, long long ldb, long long ldc,
                                int a_mn_major, int b_mn_major, int act, int out_fp32, int bias_bf16, int split_k, int variant, int* err, cudaStream_t stream);
 
-// Whether a product of this many rows reads its weights as they are (no scratch matrix).
-KB_API int kb200_dense_direct(int M) { return M <= rw::BM ? 1 : 0; }
-
 // C[M, ldo] (bf16, contiguous rows) = act(A x [W0 W1 W2] + bias): A bf16 [M, K], pitch lda; W_i [K, n_i] contiguous, all float32 (w_fp32) or
-// bf16; biases per weight, float32 or (bias16) bf16, null where there is none.  More than one weight: widths that are multiples of 64.
-// ldo: the sum of the widths up to the next multiple of 8, or of 64 for one odd width of many rows; the columns behind it hold zeros.
-// scratch: where kb200_dense_direct says 0, a bf16 matrix [K, ldo] and ldo floats behind it, or null if there is one bf16 weight whose width
-// is a multiple of 8.
+// bf16; biases per weight, float32 (rounded to bf16 as they are read) or (bias16) bf16, null where there is none.  More than one weight:
+// widths that are multiples of 64.  ldo: the sum of the widths up to the next multiple of 8, or of 64 for one odd width; the columns behind it
+// hold act(0).
+// rows: by the kernel for few rows (M <= 128), which needs no scratch.  apart: the product is rounded before the bias, as two operations would
+// leave it (act: none or relu).  scratch: a bf16 matrix [K, ldo] and ldo floats behind it, or null if
+// there is one bf16 weight whose width is a multiple of 8, without a bias in float32.
 KB_API int kb200_dense_infer(const void* a, const void* w0, const void* w1, const void* w2, const void* b0, const void* b1, const void* b2, int n0, int n1, int n2,
-                             void* out, void* scratch, int M, int K, long long lda, long long ldo, int w_fp32, int bias16, int act, int* err, cudaStream_t stream) {
+                             void* out, void* scratch, int M, int K, long long lda, long long ldo, int w_fp32, int bias16, int act, int rows, int apart, int* err,
+                             cudaStream_t stream) {
   if (M <= 0 || K <= 0 || n0 <= 0) return 0;
   const void* w[MAX_WEIGHTS] = {w0, w1, w2};
   const void* b[MAX_WEIGHTS] = {b0, b1, b2};
@@ -339,56 +362,50 @@ KB_API int kb200_dense_infer(const void* a, const void* w0, const void* w1, cons
   const int count = n2 > 0 ? 3 : n1 > 0 ? 2 : 1, total = n0 + n1 + n2;
   const bool has_bias = b0 != nullptr || b1 != nullptr || b2 != nullptr;
   // one odd width in whole 128-byte lines (a matrix of its own then)
-  const bool wider = M > rw::BM && count == 1 && n0 % 8 && ldo == (total + 63ll) / 64 * 64;
-  if ((lda % 8) || (K % 8) || !(ldo == (total + 7) / 8 * 8 || wider) || (((uintptr_t)a | (uintptr_t)out | (uintptr_t)scratch) & 15) ||
+  const bool wider = !rows && count == 1 && n0 % 8 && ldo == (total + 63ll) / 64 * 64;
+  if ((lda % 8) || (K % 8) || (rows && M > rw::BM) || (apart && act != ACT_NONE && act != ACT_RELU) || !(ldo == (total + 7) / 8 * 8 || wider) || (((uintptr_t)a | (uintptr_t)out | (uintptr_t)scratch) & 15) ||
       (count > 1 && ((n0 % 64) || (n1 % 64) || (n2 % 64) || bias16)) || (bias16 && n0 % 8)) {
     kb200_set_error("dense_infer: 16-byte aligned operands, pitches in multiples of 8, several weights only in multiples of 64 columns with float32 biases, odd widths with float32 ones");
     return -2;
   }
-  if (M <= rw::BM) {
+  if (rows) {
     CUtensorMap map_a;
     if (!make_map(&map_a, a, K, M, lda, rw::BK, rw::BM)) {
       kb200_set_error("dense_infer: cuTensorMapEncodeTiled failed");
       return -3;
     }
-    const int n_tiles = (total + rw::BN - 1) / rw::BN, kb = (K + rw::BK - 1) / rw::BK;
-    // K shared by up to eight CTAs while that leaves each two blocks or more and all of them run at once, three an SM
-    int slices = 1;
-    while (slices < 8 && (long long)n_tiles * (slices + 1) <= 3ll * kb_sm_count() && kb / (slices + 1) >= 2) ++slices;
-    const int kb_per = (kb + slices - 1) / slices;
-    slices = (kb + kb_per - 1) / kb_per;
     RowsParams p{};
     for (int i = 0, at = 0; i < count; at += n[i], ++i) {
       p.w[i] = w[i], p.bias[i] = b[i], p.start[i] = at, p.width[i] = n[i];
       p.vec[i] = ((uintptr_t)w[i] & 15) == 0 && n[i] % (w_fp32 ? 4 : 8) == 0;
     }
-    p.weights = count, p.out = out, p.M = M, p.K = K, p.slices = slices, p.kb_per = kb_per, p.ldo = ldo, p.act = act, p.bias16 = bias16, p.err = err;
+    p.weights = count, p.out = out, p.M = M, p.K = K, p.ldo = ldo, p.act = act, p.bias16 = bias16, p.apart = apart, p.err = err;
+    const int n_tiles = (total + rw::BN - 1) / rw::BN;
     return w_fp32 ? launch_rows<float>(map_a, p, n_tiles, stream) : launch_rows<__nv_bfloat16>(map_a, p, n_tiles, stream);
   }
-  if (scratch == nullptr) {
-    if (w_fp32 || count > 1 || n0 % 8) {
-      kb200_set_error("dense_infer: these weights need a scratch matrix");
-      return -2;
-    }
-    return kb200_gemm_bf16_run(a, w0, out, b0, M, n0, K, lda, n0, ldo, 0, 1, act, 0, bias16, 1, 0, err, stream);
-  }
-  __nv_bfloat16* matrix = (__nv_bfloat16*)scratch;
-  float* bias = (float*)(matrix + (size_t)K * ldo);
-  const bool place_bias = has_bias && (count > 1 || n0 % 8) && !bias16;
-  for (int i = 0, at = 0; i < count; at += n[i], ++i) {
-    const int vecs = count == 1 ? (int)(ldo / 8) : (n[i] + 7) / 8;
-    const long long grid = ((long long)K * vecs + 255) / 256;
-    if (grid > 0x7fffffffll) {
+  const __nv_bfloat16* matrix = (const __nv_bfloat16*)w0;
+  const void* bias = b0;
+  if (scratch != nullptr) {
+    __nv_bfloat16* to = (__nv_bfloat16*)scratch;
+    float* placed = has_bias && !bias16 ? (float*)(to + (size_t)K * ldo) : nullptr;
+    if (!place(w, b, n, count, to, placed, K, ldo, w_fp32, stream)) {
       kb200_set_error("dense_infer: weight too large for one launch");
       return -2;
     }
-    const int vec = ((uintptr_t)w[i] & 15) == 0 && n[i] % 4 == 0;
-    float* to = place_bias ? bias + at : nullptr;
-    if (w_fp32)
-      place_weight_kernel<float><<<(unsigned)grid, 256, 0, stream>>>((const float*)w[i], matrix + at, K, n[i], vecs, ldo, vec, (const float*)b[i], to);
-    else
-      place_weight_kernel<__nv_bfloat16><<<(unsigned)grid, 256, 0, stream>>>((const __nv_bfloat16*)w[i], matrix + at, K, n[i], vecs, ldo, 0, (const float*)b[i], to);
+    KB_CHECK_LAUNCH("place_weight");
+    matrix = to, bias = bias16 ? b0 : placed;
+  } else if (w_fp32 || count > 1 || n0 % 8 || (has_bias && !bias16)) {
+    kb200_set_error("dense_infer: these weights need a scratch matrix");
+    return -2;
   }
-  KB_CHECK_LAUNCH("place_weight");
-  return kb200_gemm_bf16_run(a, matrix, out, place_bias ? bias : b0, M, (int)ldo, K, lda, ldo, ldo, 0, 1, act, 0, place_bias ? 0 : bias16, 1, 0, err, stream);
+  const int rc = kb200_gemm_bf16_run(a, matrix, out, apart ? nullptr : bias, M, (int)ldo, K, lda, ldo, ldo, 0, 1, apart ? ACT_NONE : act, 0, bias16, 1, 0, err, stream);
+  if (rc != 0 || !apart || (!has_bias && act == ACT_NONE)) return rc;
+  const long long vecs = (long long)M * (ldo / 8);
+  if (vecs / 256 > 0x7ffffff0ll) {
+    kb200_set_error("dense_infer: result too large for one launch");
+    return -2;
+  }
+  bias_rows_kernel<<<(unsigned)((vecs + 255) / 256), 256, 0, stream>>>((uint4*)out, has_bias ? bias : nullptr, vecs, (int)(ldo / 8), total, bias16, act == ACT_RELU);
+  KB_CHECK_LAUNCH("bias_rows");
+  return 0;
 }

@@ -86,7 +86,7 @@ template <typename T, int VPL, int NT, int WPR>
 __global__ void __launch_bounds__(NT) norm_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ res, T* __restrict__ sum_out,
                                                            const float* __restrict__ gamma, const float* __restrict__ beta,
                                                            T* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out,
-                                                           long long rows, int D, float eps, int rms) {
+                                                           long long rows, int D, float eps, int rms, int narrow) {
   constexpr int VN = NVec<T>::N;
   constexpr int RPB = NT / 32 / WPR;  // rows per block
   __shared__ float red[2 * RPB * WPR];
@@ -159,8 +159,8 @@ __global__ void __launch_bounds__(NT) norm_fwd_warp_kernel(const T* __restrict__
 #pragma unroll
       for (int j = 0; j < VN; ++j) {
         float o = (v[j] - mean) * rstd;
-        if (gamma) o *= gv[j];
-        if (beta) o += bv[j];
+        if (gamma) o *= narrow ? to_f32<T>(from_f32<T>(gv[j])) : gv[j];
+        if (beta) o += narrow ? to_f32<T>(from_f32<T>(bv[j])) : bv[j];
         v[j] = o;
       }
       yr[i] = nv_pack<T>(v);
@@ -324,7 +324,7 @@ template <typename T>
 __global__ void __launch_bounds__(NORM_THREADS) norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ res, T* __restrict__ sum_out, const float* __restrict__ gamma,
                                                                 const float* __restrict__ beta,
                                                                 T* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int D,
-                                                                float eps, int rms) {
+                                                                float eps, int rms, int narrow) {
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const T* xr = x + row * D;
@@ -348,8 +348,8 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_fwd_kernel(const T* __restr
   }
   for (int i = threadIdx.x; i < D; i += NORM_THREADS) {
     float v = (value(i) - mean) * rstd;
-    if (gamma) v *= gamma[i];
-    if (beta) v += beta[i];
+    if (gamma) v *= narrow ? to_f32<T>(from_f32<T>(gamma[i])) : gamma[i];
+    if (beta) v += narrow ? to_f32<T>(from_f32<T>(beta[i])) : beta[i];
     yr[i] = from_f32<T>(v);
   }
 }
@@ -418,9 +418,9 @@ __global__ void norm_partial_reduce_kernel(const float* __restrict__ partial, fl
 
 // y = norm(x), or norm(sum) with sum = x + res where `res` is given: a block of a transformer adds its branch and normalises the sum, and
 // the sum has another reader, the next addition; one pass writes both.  [16384, 768] bf16: 10.7 + 13.5 us apart, 16.6 together.
-// mean / rstd: null where nobody takes a gradient.
+// mean / rstd: null where nobody takes a gradient.  narrow: gamma and beta are rounded to the type of the rows as they are read.
 KB_API int kb200_norm_fwd(const void* x, const void* res, void* sum, const float* gamma, const float* beta, void* y, float* mean, float* rstd, long long rows, int D,
-                          float eps, int rms, int dtype, cudaStream_t stream) {
+                          float eps, int rms, int narrow, int dtype, cudaStream_t stream) {
   if (rows <= 0) return 0;
   {
     const int vn = dtype == 1 ? 8 : 4;
@@ -431,7 +431,7 @@ KB_API int kb200_norm_fwd(const void* x, const void* res, void* sum, const float
   do {                                                                                                                                            \
     constexpr int rpb = NT / 32 / WPR;                                                                                                            \
     norm_fwd_warp_kernel<T, VPL, NT, WPR><<<(unsigned)((rows + rpb - 1) / rpb), NT, 0, stream>>>((const T*)x, (const T*)res, (T*)sum, gamma, beta, (T*)y, mean, rstd, \
-                                                                                                  rows, D, eps, rms);                             \
+                                                                                                  rows, D, eps, rms, narrow);                     \
   } while (0)
 #define PICK_FW(T)                                                   \
   do {                                                               \
@@ -454,9 +454,9 @@ KB_API int kb200_norm_fwd(const void* x, const void* res, void* sum, const float
 #undef LAUNCH_FW
   }
   if (dtype == 1)
-    norm_fwd_kernel<__nv_bfloat16><<<(unsigned)rows, NORM_THREADS, 0, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (__nv_bfloat16*)sum, gamma, beta, (__nv_bfloat16*)y, mean, rstd, D, eps, rms);
+    norm_fwd_kernel<__nv_bfloat16><<<(unsigned)rows, NORM_THREADS, 0, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (__nv_bfloat16*)sum, gamma, beta, (__nv_bfloat16*)y, mean, rstd, D, eps, rms, narrow);
   else
-    norm_fwd_kernel<float><<<(unsigned)rows, NORM_THREADS, 0, stream>>>((const float*)x, (const float*)res, (float*)sum, gamma, beta, (float*)y, mean, rstd, D, eps, rms);
+    norm_fwd_kernel<float><<<(unsigned)rows, NORM_THREADS, 0, stream>>>((const float*)x, (const float*)res, (float*)sum, gamma, beta, (float*)y, mean, rstd, D, eps, rms, narrow);
   KB_CHECK_LAUNCH("norm_fwd");
   return 0;
 }

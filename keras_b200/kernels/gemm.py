@@ -311,7 +311,11 @@ def _qualifies(x2, w):
     if not (_ok_2d(x2) and _ok_2d(w, any_width=True)):
         return False
     M, K = x2.shape
-    N = w.shape[1]
+    return takes(M, w.shape[1], K)
+
+
+def takes(M, N, K):
+    """Whether products of this size run here: the others are the library's."""
     # Rows may be any number: the copies clip them.  Up to a tile of them the library's small-batch kernels take half of this one's time
     # ([77, 3072, 768] 6.0 us against 13.2, [77, 768, 3072] 3.6 / 6.2, [77, 768, 50264] 12 / 20; 72 to 128 rows the same), and row counts that
     # are no multiple of 8 go to them; multiples of 8 do not, a line that time did not draw.  A width that is no multiple of 8 would send

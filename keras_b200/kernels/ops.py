@@ -388,7 +388,8 @@ class FusedNorm(torch.autograd.Function):
         mean, rstd = stats[:rows], stats[rows:]
         g = gamma.float().contiguous() if gamma is not None else None
         b = beta.float().contiguous() if beta is not None else None
-        _check(lib.kb200_norm_fwd(_p(x), _vp(0), _vp(0), _p(g), _p(b), _p(y), _p(mean), _p(rstd), _ll(rows), _i(D), _f(eps), _i(1 if rms else 0), _i(_dt(x)), _stream()), "norm_fwd")
+        _check(lib.kb200_norm_fwd(_p(x), _vp(0), _vp(0), _p(g), _p(b), _p(y), _p(mean), _p(rstd), _ll(rows), _i(D), _f(eps), _i(1 if rms else 0), _i(0), _i(_dt(x)),
+                                     _stream()), "norm_fwd")
         ctx.save_for_backward(x, g, stats)
         ctx.rms = rms
         ctx.has_beta = beta is not None
@@ -442,7 +443,7 @@ class FusedAddNorm(torch.autograd.Function):
         total, y = torch.empty_like(a), torch.empty_like(a)
         stats = torch.empty(2 * rows, dtype=torch.float32, device=a.device)
         _check(_lib().kb200_norm_fwd(_p(a), _p(b), _p(total), _p(gamma), _p(beta), _p(y), _p(stats[:rows]), _p(stats[rows:]), _ll(rows), _i(D), _f(eps),
-                                     _i(1 if rms else 0), _i(_dt(a)), _stream()), "add_norm_fwd")
+                                     _i(1 if rms else 0), _i(0), _i(_dt(a)), _stream()), "add_norm_fwd")
         ctx.save_for_backward(total, gamma, beta, stats)
         ctx.eps, ctx.rms = eps, rms
         ctx.set_materialize_grads(False)

@@ -70,58 +70,76 @@ def _function(name, argtypes):
 
 
 _V, _I, _L = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
-_DENSE = [_V] * 7 + [_I] * 3 + [_V] * 2 + [_I] * 2 + [_L] * 2 + [_I] * 3 + [_V] * 2
+_DENSE = [_V] * 7 + [_I] * 3 + [_V] * 2 + [_I] * 2 + [_L] * 2 + [_I] * 5 + [_V] * 2
+_ACTIVATION = {3: torch.nn.functional.silu, 4: torch.nn.functional.gelu}
 
 
-def _product(x, weights, biases, act):
-    """``act(x @ [w0 w1 w2] + bias)`` of contiguous matrices of one type, as rows of a pitch that is a multiple of 8 (``gemm.padded_width`` above 128 rows); ``None`` where the
-    kernels do not take it."""
+def _product(x, weights, biases, act, as_layers=False):
+    """``act(x @ [w0 w1 w2] + bias)`` of contiguous matrices of one type, as rows of a pitch that is a multiple of 8; ``None`` where the kernels do not
+    take it.  ``as_layers``: with every bit of the layers' own calls, which see a layer's first call and whatever is not taken here: the
+    products that those leave to the library (whose sums run along K as these do) are rounded before the bias and the activation."""
     K = x.shape[-1]
-    widths = [w.numel() // K for w in weights]
-    M, N = x.numel() // K if K else 0, sum(widths)
-    fp32 = weights[0].dtype == _F32
+    if len(weights) == 1:
+        widths = (weights[0].numel() // K,) if K else (0,)
+        N = widths[0]
+    else:
+        widths = [w.numel() // K for w in weights] if K else [0]
+        N = sum(widths)
+        if any(n % 64 for n in widths) or any(w.dtype != weights[0].dtype for w in weights):
+            return None
+    M, fp32 = x.numel() // K if K else 0, weights[0].dtype == _F32
     # fewer than 64 columns of either operand: below a box of the copies, and nothing to gain
     if (M == 0 or K < 64 or K % 8 or N < 64 or not x.is_contiguous() or x.data_ptr() % 16 or M * N >= 1 << 40 or M >= 1 << 31
-            or any(w.dtype != weights[0].dtype or not w.is_contiguous() or w.data_ptr() % 16 and not M <= 128 for w in weights)
             or N % 8 and N < 256):  # few classes: the library's result is contiguous
         return None
-    bias16 = False
-    if any(b is not None for b in biases):
-        kinds = {b.dtype for b in biases if b is not None}
-        if len(kinds) > 1 or not all(b is None or b.is_contiguous() for b in biases):
+    # Few rows: weights as they are stored.  A CTA has 64 columns and walks all of K, at a microsecond a block of 64: with three CTAs for every second
+    # SM that is the weights' traffic ([77, 4096, 14336] 80 us, a weight placed and multiplied 82), with fewer up to 1024 of K a wait that costs no more
+    # than the launch it saves ([77, 768, 768] 14 and 9 us); [77, 3072, 768] 48 and 19.
+    rows = M <= 128 and (K <= 1024 or N > 96 * kgemm._sm_count(x.device))
+    plain, bias16, apart, w, b = not fp32 and len(weights) == 1 and N % 8 == 0, False, False, [0, 0, 0], [0, 0, 0]  # plain: a matrix as the products read it
+    for i, t in enumerate(weights):
+        w[i] = t.data_ptr()
+        if not t.is_contiguous() or not rows and w[i] % 16:
             return None
-        if not kinds <= {_F32, _BF16}:
+    biased = any(t is not None for t in biases)
+    if as_layers:
+        own = [kgemm.takes(M, n, K) for n in widths]
+        apart = (biased or act > 1) and not own[0]
+        if any(own) != all(own) and (biased or act > 1) or apart and N % 8:
+            return None
+    if biased:
+        kinds = {t.dtype for t in biases if t is not None}
+        if len(kinds) > 1 or not kinds <= {_F32, _BF16} or not all(t is None or t.is_contiguous() for t in biases):
             return None
         bias16 = kinds == {_BF16}
-        if bias16 and (len(weights) > 1 or N % 8):  # these are placed beside one another, in float32
-            biases, bias16 = [b if b is None else b.float() for b in biases], False
-    if len(weights) > 1 and any(n % 64 for n in widths):
-        return None
-    pitch = kgemm.padded_width(N) if M > 128 else (N + 7) // 8 * 8
+        if plain and not bias16:  # a bias is read in the layer's type wherever it is read
+            biases, bias16 = [biases[0].to(_BF16)], True
+        elif bias16 and (len(weights) > 1 or N % 8):  # these are placed beside one another, in float32
+            biases, bias16 = [t if t is None else t.float() for t in biases], False
+        for i, t in enumerate(biases):
+            b[i] = t.data_ptr() if t is not None else 0
+    n = (*widths, 0, 0)[:3]
+    pitch = (N + 7) // 8 * 8 if rows else kgemm.padded_width(N)
     out = torch.empty((M, pitch), dtype=_BF16, device=x.device)
-    scratch = None
-    if M > 128 and (fp32 or len(weights) > 1 or N % 8):
-        scratch = torch.empty(K * pitch + 2 * pitch, dtype=_BF16, device=x.device)
-    w = [t.data_ptr() for t in weights] + [0] * (3 - len(weights))
-    b = [t.data_ptr() if t is not None else 0 for t in biases] + [0] * (3 - len(biases))
-    n = widths + [0] * (3 - len(widths))
+    scratch = None if rows or plain else torch.empty(K * pitch + 2 * pitch, dtype=_BF16, device=x.device)
     code = _function("kb200_dense_infer", _DENSE)(x.data_ptr(), *w, *b, *n, out.data_ptr(), scratch.data_ptr() if scratch is not None else None, M, K, K, pitch,
-                                                  1 if fp32 else 0, 1 if bias16 else 0, act, kgemm._err_flag(x.device).data_ptr(), kops._stream())
+                                                  1 if fp32 else 0, 1 if bias16 else 0, 0 if apart and act > 1 else act, 1 if rows else 0, 1 if apart else 0,
+                                                  kgemm._err_flag(x.device).data_ptr(), kops._stream())
     kops._check(code, "dense_infer")
-    return out
+    return _ACTIVATION[act](out) if apart and act > 1 else out
 
 
-_NORM = [_V] * 8 + [_L, _I, ctypes.c_float, _I, _I, _V]
+_NORM = [_V] * 8 + [_L, _I, ctypes.c_float, _I, _I, _I, _V]
 
 
-def _normalise(x, residual, gamma, beta, eps, rms):
+def _normalise(x, residual, gamma, beta, eps, rms, narrow):
     """``(norm(x + residual), x + residual)`` over the last axis of contiguous bf16 tensors."""
     D = x.shape[-1]
     y = torch.empty_like(x)
     total = torch.empty_like(x) if residual is not None else None
     code = _function("kb200_norm_fwd", _NORM)(x.data_ptr(), residual.data_ptr() if residual is not None else None, total.data_ptr() if total is not None else None,
                                               gamma.data_ptr() if gamma is not None else None, beta.data_ptr() if beta is not None else None, y.data_ptr(), None, None,
-                                              x.numel() // D, D, eps, 1 if rms else 0, 1, kops._stream())
+                                              x.numel() // D, D, eps, 1 if rms else 0, 1 if narrow else 0, 1, kops._stream())
     kops._check(code, "norm_fwd")
     return y, total
 
@@ -195,7 +213,7 @@ def _dense(layer, x):
     parts = _matrix_layer(layer) if x is not None else None
     if parts is None or parts[0].ndim != 2 or parts[0].shape[0] != x.shape[-1] or x.ndim < 2:
         return None
-    out = _product(x, [parts[0]], [parts[1]], parts[2])
+    out = _product(x, [parts[0]], [parts[1]], parts[2], True)
     if out is None:
         return None
     n = parts[0].shape[1]
@@ -205,7 +223,7 @@ def _dense(layer, x):
 
 
 def _norm_parts(layer, x):
-    """``(gamma, beta, epsilon, rms)`` of a normalisation over the last axis, or ``None``."""
+    """``(gamma, beta, epsilon, rms, narrow)`` of a normalisation over the last axis, or ``None``; ``narrow``: its float32 parameters are read in bf16."""
     d = layer.__dict__
     if not _ordinary(layer) or x.ndim < 1 or not 0 < x.shape[-1] <= 8192 or x.numel() == 0 or not x.is_contiguous() or x.data_ptr() % 16:
         return None
@@ -218,7 +236,7 @@ def _norm_parts(layer, x):
     else:
         rms = bool(d["rms_scaling"])
         gamma, beta = d["gamma"] if d["scale"] or rms else None, d["beta"] if d["center"] and not rms else None
-    out = []
+    out, narrow = [], False
     for v in (gamma, beta):
         t = v
         if v is not None:
@@ -229,8 +247,9 @@ def _norm_parts(layer, x):
                 t = t.float()
             if t.dtype != _F32 or not t.is_contiguous() or t.data_ptr() % 16:
                 return None
+            narrow = narrow or v._autocast and d["autocast"]  # of one layer all or none: a parameter in bf16 stays what it is
         out.append(t)
-    return out[0], out[1], d["epsilon"], rms
+    return out[0], out[1], d["epsilon"], rms, narrow
 
 
 def _carries_mask(layer):
@@ -288,7 +307,7 @@ def add_norm(add, norm, inputs):
     if torch.is_grad_enabled():
         if type(norm) is not LayerNormalization:  # its parameters are float32 leaves; those of RMSNormalization are read in the layer's type
             return None
-        total, y = kops.FusedAddNorm.apply(a, b, *how)
+        total, y = kops.FusedAddNorm.apply(a, b, *how[:4])
     else:
         y, total = _normalise(a, b, *how)
     return _pass_mask(total, mask), _pass_mask(y, mask)
@@ -354,7 +373,7 @@ def _attention(layer, x, causal, mask=None):
         return None
     if kattention.os.environ.get("KERAS_B200_FLASH_ATTENTION", "inference") == "0":
         return None
-    qkv = _product(x, [p[0] for p in parts[:3]], [p[1] for p in parts[:3]], 0)
+    qkv = _product(x, [p[0] for p in parts[:3]], [p[1] for p in parts[:3]], 0, True)
     if qkv is None:
         return None
     B, T = x.shape[:2]
@@ -366,7 +385,7 @@ def _attention(layer, x, causal, mask=None):
         out = kattention.flash_attention(q, k, v, None, scale, causal)
     if out is None:
         return None
-    out = _product(out.view(B, T, heads * size), [parts[3][0]], [parts[3][1]], 0)
+    out = _product(out.view(B, T, heads * size), [parts[3][0]], [parts[3][1]], 0, True)
     return None if out is None else _pass_mask(out[:, :parts[3][0].shape[2]].view(B, T, -1), mask)
 
 

@@ -220,6 +220,47 @@ def test_layers_called_directly_agree_with_their_own_calls(policy, batch, monkey
         assert (a is None) == (b is None) and (a is None or torch.equal(a, b))
 
 
+@pytest.mark.parametrize("policy", ["mixed_bfloat16", "bfloat16"])
+@pytest.mark.parametrize("batch", [1, 2, 5, 40])
+def test_a_second_call_repeats_the_first_bit_for_bit(policy, batch):
+    """The first call of a model is its layers' own, the next are made directly."""
+    import keras_b200 as keras
+
+    keras.utils.set_random_seed(3)
+    keras.config.set_dtype_policy(policy)
+    try:
+        models = _models(keras)
+    finally:
+        keras.config.set_dtype_policy("float32")
+    g = torch.Generator(device="cuda").manual_seed(batch)
+    ids = torch.randint(0, 301, (batch, 24), device="cuda", dtype=torch.int32, generator=g)
+    for name, model in models.items():
+        for v in model.trainable_variables:
+            v.assign(v.value.float() + 0.3 * torch.randn(tuple(v.shape), device="cuda", generator=g))
+        with torch.no_grad():
+            assert torch.equal(model(ids), model(ids)), name
+
+
+@pytest.mark.parametrize("policy", ["mixed_bfloat16", "bfloat16"])
+@pytest.mark.parametrize("M,K,N", [(1, 768, 768), (77, 768, 3072), (77, 3072, 768), (64, 512, 1024), (13, 64, 64), (128, 264, 15000), (7, 72, 14336), (77, 64, 14337),
+                                   (8, 128, 304), (200, 64, 64), (300, 256, 1001), (130, 2048, 520)])
+@pytest.mark.parametrize("activation,bias", [(None, False), (None, True), ("relu", True), ("gelu", True), ("silu", False), ("silu", True)])
+def test_dense_called_directly_has_the_bits_of_its_own_call(policy, M, K, N, activation, bias):
+    """Both sides of every rule: the library's products and this package's, few rows and many, wide and narrow."""
+    import keras_b200 as keras
+    from keras_b200.models import direct
+
+    layer = keras.layers.Dense(N, activation=activation, use_bias=bias, dtype=policy)
+    layer.build((None, K))
+    if bias:
+        layer.bias.assign(torch.randn(N, device="cuda"))
+    x = torch.randn(M, K, device="cuda").bfloat16()
+    with torch.no_grad():
+        own = layer(x)
+        taken = direct._dense(layer, x)
+    assert taken is not None and torch.equal(own, taken)
+
+
 def test_direct_calls_see_every_change_of_a_layer(monkeypatch):
     import keras_b200 as keras
     from keras_b200.models import direct
