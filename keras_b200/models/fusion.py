@@ -204,19 +204,25 @@ def run_pool_padded(layer, x, pairs):
 
 class RecordedInputs(threading.local):
     """The batch of a step that is being recorded in this thread.  Its cast to bf16 is left to whoever copies a batch in, which reads
-    it anyway: ``casts`` maps the place of a batch tensor to the bf16 tensor that the recorded step reads."""
+    it anyway: ``casts`` maps the place of a batch tensor to the bf16 tensor that the recorded step reads; ``read``: the places of those that
+    a convolution was given as they are, or casts otherwise."""
 
     def __init__(self):
         self.end()
 
     def begin(self, leaves):
         self._leaves = [(leaf, leaf._version) if isinstance(leaf, torch.Tensor) else None for leaf in leaves]
-        self.casts = {}
+        self.casts, self.read = {}, set()
 
     def end(self):
-        casts = getattr(self, "casts", None)
-        self._leaves, self.casts = (), {}
-        return casts
+        made = getattr(self, "casts", None), getattr(self, "read", None)
+        self._leaves, self.casts, self.read = (), {}, set()
+        return made
+
+    def given(self, x):
+        """``x`` itself goes to a reader."""
+        self.read.update(i for i, entry in enumerate(self._leaves) if entry is not None and entry[0] is x)
+        return x
 
     def cast(self, x, dtype):
         for i, entry in enumerate(self._leaves):
@@ -235,14 +241,14 @@ def shared_cast(layer, x, casts):
     projected shortcut: [256, 56, 56, 256] in float32 is 185 us a cast).  Only where no gradient flows back, which would
     otherwise be summed in the narrow type; ``casts`` lives for one pass."""
     if not isinstance(x, torch.Tensor) or x.requires_grad or not x.dtype.is_floating_point:
-        return x
+        return recorded_inputs.given(x)
     td = layer._compute_torch_dtype()
     if x.dtype == td or not td.is_floating_point or (x.dtype == torch.float32 and x.shape[-1] % 8):
-        return x  # an fp32 input with few channels is cast inside the patch kernel
+        return recorded_inputs.given(x)  # an fp32 input with few channels is cast inside the patch kernel
     kept = casts.get((id(x), td))
     if kept is None or kept[0] is not x:
         recorded = recorded_inputs.cast(x, td)
-        kept = casts[(id(x), td)] = (x, x.to(td) if recorded is None else recorded)
+        kept = casts[(id(x), td)] = (x, recorded_inputs.given(x).to(td) if recorded is None else recorded)
     return kept[1]
 
 

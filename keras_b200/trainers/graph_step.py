@@ -182,7 +182,7 @@ class GraphedTrainStep:
             self._resync_host_state()
             torch.cuda.empty_cache()  # what the side-stream steps cached is of no use to the eager steps on the main stream
             return model.train_step(data)
-        input_casts = fusion.recorded_inputs.end()
+        input_casts, read = fusion.recorded_inputs.end()
         seed_generator.end_capture()
         self._resync_host_state()
         torch.cuda.empty_cache()      # the graph owns its pool; the warm-up's cached blocks go back to the device
@@ -190,15 +190,15 @@ class GraphedTrainStep:
         self.launches_per_replay = kops.launch_count() - launches_before
         kops.add_launches(-self.launches_per_replay)
         self.graph, self.signature, self.static_leaves, self.input_casts = graph, sig, static, input_casts
-        self.rounded_only = {0} if 0 in input_casts and self._only_rounded(data) else set()
+        self.rounded_only = {0} if 0 in input_casts and 0 not in read and self._only_to_convolutions(data) else set()
         self.out_structure, self.out_type = raw, type(logs)
         self.out_leaves, self.out_packed, self.out_packed_index = out_leaves, packed, packed_index
         # capture records the step without running it: this batch is the first replay
         return self._replay(leaves, copy_inputs=False)
 
-    def _only_rounded(self, data):
-        """Whether the recorded step reads its first leaf, the model's one input, through its rounding alone: a stock step of a stock graph
-        whose input goes to convolution blocks, each of which reads the rounding (``fusion.shared_cast``), and nowhere else."""
+    def _only_to_convolutions(self, data):
+        """Whether the recorded step reads its first leaf, the model's one input, in convolution blocks alone: a stock step of a stock graph
+        whose input goes nowhere else.  What each of them was given, the leaf or its rounding, ``fusion.shared_cast`` has noted."""
         from keras_b200.models.functional import Functional
         from keras_b200.trainers.trainer import Trainer
 

@@ -496,33 +496,44 @@ def test_float32_dense_layer_keeps_nan_and_second_derivatives():
 
 
 # ------------------------------------------------------------------------------------------------ a recorded step that reads a rounded batch
-@pytest.mark.parametrize("other_reader", [False, True])
-def test_recorded_step_copies_what_it_reads(other_reader):
-    """New batches reach a step whose input only convolutions read, and one whose input something else reads too."""
+@pytest.mark.parametrize("reader", [None, "dense", "mixed_float16", "mixed_bfloat16"])
+def test_recorded_step_copies_what_it_reads(reader):
+    """New batches reach a step whose input only convolutions read in bf16, and one whose input something else reads too.  Each batch has offsets of its
+    own, so that a branch that kept the recorded one would take its steps in other directions."""
     import keras_b200 as keras
 
     def run(graph):
+        L = keras.layers
         keras.utils.set_random_seed(6)
         keras.config.set_dtype_policy("mixed_bfloat16")
+
+        def branch(i, dtype=None):
+            return L.GlobalAveragePooling2D()(L.ReLU()(L.BatchNormalization(dtype=dtype)(L.Conv2D(32, 1, use_bias=False, dtype=dtype)(i))))
+
         try:
             i = keras.Input((12, 12, 16))
-            h = keras.layers.ReLU()(keras.layers.BatchNormalization()(keras.layers.Conv2D(32, 1, use_bias=False)(i)))
-            out = keras.layers.Dense(4)(keras.layers.GlobalAveragePooling2D()(h))
-            if other_reader:
-                out = keras.layers.Add()([out, keras.layers.Dense(4)(keras.layers.GlobalAveragePooling2D()(i))])
-            model = keras.Model(i, out)
+            parts = [branch(i)]
+            if reader:
+                parts.append(L.GlobalAveragePooling2D()(i) if reader == "dense" else branch(i, reader))
+            model = keras.Model(i, L.Dense(4)(L.Concatenate()(parts) if reader else parts[0]))
         finally:
             keras.config.set_dtype_policy("float32")
         model.compile(keras.optimizers.SGD(0.05), keras.losses.SparseCategoricalCrossentropy(from_logits=True), jit_compile="auto" if graph else False)
-        losses = []
-        for k in range(7):
+        before = [v.value.detach().clone() for v in model.trainable_variables]
+        for k in range(9):
             g = torch.Generator(device="cuda").manual_seed(k)
-            x = torch.randn(64, 12, 12, 16, generator=g, device="cuda")
-            losses.append(float(model.train_on_batch(x, torch.randint(0, 4, (64,), generator=g, device="cuda"))))
-        return losses, getattr(model, "_graph_step", None)
+            y = torch.randint(0, 4, (64,), generator=g, device="cuda")
+            x = torch.randn(64, 12, 12, 16, generator=g, device="cuda") + 2 * torch.randn(4, 16, generator=g, device="cuda")[y][:, None, None]
+            model.train_on_batch(x, y)
+        return model, [v.value.detach() - b for v, b in zip(model.trainable_variables, before)]
 
-    recorded, eager = run(True)[0], run(False)[0]
-    assert max(abs(a - b) for a, b in zip(recorded, eager)) < 2e-2, (recorded, eager)
+    (model, recorded), (_, eager) = run(True), run(False)
+    step = model._graphed_step
+    assert step is not None and step.replays >= 4, getattr(step, "disabled", None)
+    assert step.rounded_only == ({0} if reader in (None, "mixed_bfloat16") else set())
+    # the distance that each weight went: gradients in bf16, a hundredth apart in two runs
+    for a, b in zip(recorded, eager):
+        assert _rel(a, b.double()) < 0.1, [_rel(p, q.double()) for p, q in zip(recorded, eager)]
 
 
 # ------------------------------------------------------------------------------------------------ few classes, running means, BatchNorm sums

@@ -179,3 +179,24 @@ def test_only_stock_chains_are_planned_for_fused_kernels():
     assert sorted(map(str, roles(lambda x: L.ReLU()(L.Add()([norm(x), x]))))) == ["consume_add_relu", "defer_bn", "identity"]
     assert sorted(map(str, roles(lambda x: L.ReLU(6.0)(L.Add()([norm(x), x]))))) == ["None", "consume_add", "defer_bn"]
     assert set(roles(lambda x: L.Add(dtype="bfloat16")([norm(x), x]))) == {None}  # casts stand between them
+
+
+def test_recorded_inputs_note_who_reads_the_batch_itself():
+    """A convolution of another type than bf16 is given the batch, or a cast of it, and not the rounding that is made beside the copy."""
+    from keras_b200.models import fusion
+
+    def read(*dtypes, channels=8):
+        x = torch.zeros(2, 4, 4, channels)
+        fusion.recorded_inputs.begin([x, torch.zeros(2)])
+        fusion.recorded_inputs.cast = lambda t, dtype: t.to(dtype) if t is x and dtype == torch.bfloat16 else None  # as for a batch on a GPU
+        try:
+            casts = {}
+            for dtype in dtypes:
+                fusion.shared_cast(keras.layers.Conv2D(4, 1, dtype=dtype), x, casts)
+        finally:
+            del fusion.recorded_inputs.cast
+            made = fusion.recorded_inputs.end()[1]
+        return made
+
+    assert read("bfloat16") == read("mixed_bfloat16", "bfloat16") == set()
+    assert read("bfloat16", "float32") == read("float16", "bfloat16") == read("bfloat16", channels=3) == {0}
