@@ -213,10 +213,14 @@ class RecordedInputs(threading.local):
     def begin(self, leaves):
         self._leaves = [(leaf, leaf._version) if isinstance(leaf, torch.Tensor) else None for leaf in leaves]
         self.casts, self.read = {}, set()
+        # Made before the recording: what is allocated during one may lie where an earlier kernel of the graph keeps something of its own,
+        # which a replay writes there after the cast.
+        self._room = [torch.empty_like(leaf, dtype=torch.bfloat16) if isinstance(leaf, torch.Tensor) and leaf.is_cuda and leaf.dtype == torch.float32 else None
+                      for leaf in leaves]
 
     def end(self):
         made = getattr(self, "casts", None), getattr(self, "read", None)
-        self._leaves, self.casts, self.read = (), {}, set()
+        self._leaves, self._room, self.casts, self.read = (), (), {}, set()
         return made
 
     def given(self, x):
@@ -226,10 +230,8 @@ class RecordedInputs(threading.local):
 
     def cast(self, x, dtype):
         for i, entry in enumerate(self._leaves):
-            if entry is not None and entry[0] is x and entry[1] == x._version and x.is_cuda and x.dtype == torch.float32 and dtype == torch.bfloat16:
-                if i not in self.casts:
-                    self.casts[i] = torch.empty_like(x, dtype=dtype)
-                return self.casts[i]
+            if entry is not None and entry[0] is x and entry[1] == x._version and self._room[i] is not None and dtype == torch.bfloat16:
+                return self.casts.setdefault(i, self._room[i])
         return None
 
 

@@ -496,7 +496,7 @@ def test_float32_dense_layer_keeps_nan_and_second_derivatives():
 
 
 # ------------------------------------------------------------------------------------------------ a recorded step that reads a rounded batch
-@pytest.mark.parametrize("reader", [None, "dense", "mixed_float16", "mixed_bfloat16"])
+@pytest.mark.parametrize("reader", [None, "dense", "float32", "mixed_float16", "mixed_bfloat16"])
 def test_recorded_step_copies_what_it_reads(reader):
     """New batches reach a step whose input only convolutions read in bf16, and one whose input something else reads too.  Each batch has offsets of its
     own, so that a branch that kept the recorded one would take its steps in other directions."""
