@@ -579,16 +579,23 @@ class FusedSoftmaxXent(torch.autograd.Function):
                                            _i(_dt(flat)), _stream()), "xent_fwd_grad")
         else:
             _check(lib.kb200_xent_fwd(_p(flat), _p(labels64), _p(loss), _p(lse), _ll(rows), _i(V), _ll(ld), _i(_dt(flat)), _stream()), "xent_fwd")
-        ctx.save_for_backward(flat, labels64, lse)
-        ctx.logits_shape = tuple(logits.shape)
+        # the input itself, for a gradient of the gradient; its rows again only where they were copied
+        ctx.save_for_backward(logits, flat if flat.data_ptr() != logits.data_ptr() else None, labels64, lse)
         ctx.ld, ctx.zero_to = ld, zero_to
         return loss.reshape(labels.shape)
 
     @staticmethod
     def backward(ctx, dloss):
         lib = _lib()
-        flat, labels64, lse = ctx.saved_tensors
-        rows, V = flat.shape
+        logits, flat, labels64, lse = ctx.saved_tensors
+        V = logits.shape[-1]
+        rows = logits.numel() // V
+        if torch.is_grad_enabled():  # a gradient of this gradient is wanted: differentiate the same loss from library operations
+            x = logits.reshape(rows, V).float()
+            picked = x.gather(1, labels64.clamp(0, V - 1)[:, None])[:, 0]
+            values = torch.where((labels64 >= 0) & (labels64 < V), torch.logsumexp(x, 1) - picked, 0.0)
+            return torch.autograd.grad(values, logits, dloss.reshape(-1).float(), create_graph=True)[0], None
+        flat = logits.reshape(rows, V) if flat is None else flat
         ld = ctx.ld
         # the gradient of a plain mean is one number, seen by every row
         spread = dloss.dtype == torch.float32 and dloss.numel() > 0 and not any(dloss.stride())
@@ -600,7 +607,7 @@ class FusedSoftmaxXent(torch.autograd.Function):
         _check(lib.kb200_xent_bwd(_p(flat), _p(labels64), _p(lse), _p(dl), _i(0 if spread else 1), _p(buf), _ll(rows), _i(V), _ll(ld), _i(ctx.zero_to), _i(1 if done else 0),
                                   _f(ctx.made_for), _i(_dt(flat)), _stream()), "xent_bwd")
         dlogits = buf if ld == V else buf[:, :V]
-        return dlogits.reshape(ctx.logits_shape), None
+        return dlogits.reshape(logits.shape), None
 
 
 # ------------------------------------------------------------------------ fused optimizers

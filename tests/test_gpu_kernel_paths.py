@@ -561,6 +561,35 @@ def test_cross_entropy_of_few_classes(rows, V, ld, dtype, spread):
     assert torch.allclose(a.double(), b, atol=2.0 ** -20, rtol=2.0 ** -19 if dtype == torch.float32 else 2.0 ** -8)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("V,ld", [(2, 2), (10, 10), (37, 40), (63, 63), (64, 64), (300, 304), (2049, 2056)])
+@pytest.mark.parametrize("layout", ["rows", "columns", "expected"])
+def test_cross_entropy_second_derivatives(V, ld, dtype, layout):
+    """Rows with a pitch, rows that have to be copied, and a gradient that was made ahead."""
+    import contextlib
+
+    from keras_b200.kernels import ops as kops
+
+    g = torch.Generator(device="cuda").manual_seed(V)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").to(dtype)  # noqa: E731
+    logits = (rnd(V, 6).t() if layout == "columns" else rnd(6, ld)[:, :V]).requires_grad_(True)
+    labels = torch.randint(0, V, (6,), generator=g, device="cuda")
+    up = torch.rand(6, generator=g, device="cuda").requires_grad_(True)
+    with kops.gradient_follows() if layout == "expected" else contextlib.nullcontext():
+        kops.expect_upstream(lambda n: 1.0 / n)
+        loss = kops.FusedSoftmaxXent.apply(logits, labels)
+    exact = [t.detach().double().requires_grad_(True) for t in (logits, up)]
+    want = torch.nn.functional.cross_entropy(exact[0], labels, reduction="none")
+    probe = rnd(6, V)
+    both = []
+    for value, z, u in ((loss, logits, up), (want, *exact)):
+        (first,) = torch.autograd.grad((value * u).sum(), z, create_graph=True)
+        both.append((first, *torch.autograd.grad((first * probe.to(first.dtype)).sum(), (z, u))))
+    # three chains of fp32 operations, rounded to the type of the logits where they leave for them and back
+    for a, b in zip(*both):
+        assert _rel(a.detach(), b.detach()) < (1e-5 if dtype == torch.float32 else 2.0 ** -6)
+
+
 def test_running_means_round_as_their_operations():
     import keras_b200 as keras
 
