@@ -176,12 +176,14 @@ _load_user_config()
 
 _forward_ad = torch.autograd.forward_ad
 _in_function_transform = torch._C._are_functorch_transforms_active
+_tracing_state = torch._C._get_tracing_state
+_exporting = torch.compiler.is_exporting
 
 
 def fused_kernels_enabled():
-    """False when ``KERAS_B200_DISABLE_FUSED_KERNELS=1``, and inside the transforms of ``torch.func`` and forward-mode derivatives, which
-    kernels that work on raw pointers cannot take part in: every op then runs its library path."""
-    if _forward_ad._current_level >= 0 or _in_function_transform():
+    """False when ``KERAS_B200_DISABLE_FUSED_KERNELS=1``, and inside the transforms of ``torch.func``, forward-mode derivatives, ``torch.jit.trace`` and
+    ``torch.export``, which kernels that work on raw pointers cannot take part in: every op then runs its library path."""
+    if _forward_ad._current_level >= 0 or _in_function_transform() or _tracing_state() is not None or _exporting():
         return False
     return os.environ.get("KERAS_B200_DISABLE_FUSED_KERNELS", "0") != "1"
 

@@ -101,7 +101,8 @@ def dense(x, kernel, bias, activation_name):
     """``(output, activation_applied)`` or ``None``; ``kernel`` and ``bias`` are the layer's variables."""
     from keras_b200.core.variables import Variable
 
-    if type(kernel) is not Variable or kernel._shard_slices is not None or not (bias is None or type(bias) is Variable):
+    # the type before any size: a traced batch has none yet
+    if type(x) not in (torch.Tensor, torch.nn.Parameter) or type(kernel) is not Variable or kernel._shard_slices is not None or not (bias is None or type(bias) is Variable):
         return None
     w, b = kernel.value, None if bias is None else bias.value
     lead = x.shape[:-1]

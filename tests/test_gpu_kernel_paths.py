@@ -495,6 +495,31 @@ def test_float32_dense_layer_keeps_nan_and_second_derivatives():
     assert layer(bad)[0].isnan().all() and not layer(bad)[1:].isnan().any()
 
 
+@pytest.mark.parametrize("policy", ["float32", "mixed_bfloat16"])
+def test_exported_and_traced_layers_take_any_batch(policy, tmp_path):
+    import keras_b200 as keras
+
+    keras.config.set_dtype_policy(policy)
+    try:
+        i = keras.Input((48,))
+        layer = keras.layers.Dense(256, activation="relu")
+        model = keras.Model(i, keras.layers.Dense(64)(layer(i)))
+    finally:
+        keras.config.set_dtype_policy("float32")
+    tol = 1e-5 if policy == "float32" else 2e-2  # fp32 sums of 256; two roundings to bf16 a layer
+    x = torch.randn(300, 48, device="cuda")
+    want = model(x).detach()
+    model.export(str(tmp_path / "m"), format="torch_export", verbose=False)
+    program = torch.export.load(str(tmp_path / "m" / "serve.pt2")).module()
+    with torch.no_grad():
+        for v in layer.trainable_variables:  # a trace holds weights as constants
+            v._value.requires_grad_(False)
+        traced = torch.jit.trace(layer.call, x[:2], check_trace=False)
+        for n in (2, 3, 300):
+            assert _rel(program(x[:n]).float(), want[:n].double()) < tol, n
+            assert _rel(traced(x[:n]).float(), layer.call(x[:n]).double()) < tol, n
+
+
 # ------------------------------------------------------------------------------------------------ a recorded step that reads a rounded batch
 @pytest.mark.parametrize("reader", [None, "dense", "float32", "mixed_float16", "mixed_bfloat16"])
 def test_recorded_step_copies_what_it_reads(reader):
