@@ -15,8 +15,12 @@ from keras_b200.core import config
 _FLOAT_IO = (torch.float32, torch.bfloat16)
 
 
+_current_device = torch._C._cuda_getDevice if hasattr(torch._C, "_cuda_getDevice") else lambda: -1
+
+
 def enabled(t):
-    return isinstance(t, torch.Tensor) and t.is_cuda and config.fused_kernels_enabled()
+    """Launches go to the current device and its stream: a tensor of another one is left to the library."""
+    return isinstance(t, torch.Tensor) and t.is_cuda and t.get_device() == _current_device() and config.fused_kernels_enabled()
 
 
 def _ops():
@@ -311,7 +315,7 @@ def softmax(x, mask=None, masked_add=0.0, log=False):
     """softmax / log-softmax over the last axis in the input's dtype (fp32 arithmetic), or ``None``."""
     if not enabled(x) or x.dtype not in _FLOAT_IO or x.ndim < 1 or x.numel() == 0 or x.shape[-1] > (1 << 24):
         return None
-    if mask is not None and not (isinstance(mask, torch.Tensor) and mask.is_cuda):
+    if mask is not None and not (isinstance(mask, torch.Tensor) and mask.device == x.device):
         return None
     return _ops().FusedSoftmax.apply(x, mask, float(masked_add), bool(log))
 
@@ -320,7 +324,7 @@ def embedding(variable, table, ids, out_dtype):
     """``table[ids]`` cast to ``out_dtype`` in one gather kernel, with a scatter-add gradient, or ``None``.
 
     ``variable`` is the ``Variable`` the table was read from (or ``None``)."""
-    if not enabled(table) or not isinstance(ids, torch.Tensor) or not ids.is_cuda or table.ndim != 2 or table.dtype not in _FLOAT_IO:
+    if not enabled(table) or not isinstance(ids, torch.Tensor) or ids.device != table.device or table.ndim != 2 or table.dtype not in _FLOAT_IO:
         return None
     if out_dtype not in _FLOAT_IO or table.shape[1] % 8 or ids.dtype not in (torch.int32, torch.int64) or ids.numel() == 0:
         return None
@@ -346,7 +350,7 @@ def resize(x, out_hw, interpolation):
 def softmax_cross_entropy(logits, labels):
     if not enabled(logits) or logits.dtype not in _FLOAT_IO or logits.numel() == 0:
         return None
-    if logits.shape[-1] < 2:
+    if logits.shape[-1] < 2 or labels.device != logits.device:
         return None
     return _ops().FusedSoftmaxXent.apply(logits, labels)
 

@@ -300,7 +300,7 @@ def projections(x, kernels, biases, weights):
     if K % 64 or any(w.shape[1] % 64 or not _qualifies(x2, w) for w in flat):
         return None
     bs = [b.value.reshape(-1) for b in biases]
-    if any(b.dtype != bs[0].dtype or b.dtype not in (torch.float32, torch.bfloat16) or not b.is_contiguous() for b in bs):
+    if any(b.device != x.device or b.dtype != bs[0].dtype or b.dtype not in (torch.float32, torch.bfloat16) or not b.is_contiguous() for b in bs):
         return None
     targets = [_grad_target(k, w) for k, w in zip(kernels, weights)] + [_grad_target(v, b) for v, b in zip(biases, bs)]
     outs = ProjectionsFn.apply(x2, targets, *flat, *bs)
@@ -308,7 +308,7 @@ def projections(x, kernels, biases, weights):
 
 
 def _qualifies(x2, w):
-    if not (_ok_2d(x2) and _ok_2d(w, any_width=True)):
+    if not (_ok_2d(x2) and _ok_2d(w, any_width=True)) or w.device != x2.device:
         return False
     M, K = x2.shape
     return takes(M, w.shape[1], K)
@@ -363,6 +363,8 @@ def dense(x, kernel, bias, activation_name, kernel_shape=None, value=None):
     if not _qualifies(x2, w):
         return None
     b = bias.value if isinstance(bias, Variable) else bias
+    if b is not None and b.device != x.device:
+        return None
     needs_grad = torch.is_grad_enabled() and (x2.requires_grad or w.requires_grad or (b is not None and b.requires_grad))
     if not needs_grad:
         name = {"gelu": "gelu_erf"}.get(activation_name, activation_name)

@@ -108,9 +108,9 @@ def dense(x, kernel, bias, activation_name):
     lead = x.shape[:-1]
     M = x.numel() // x.shape[-1] if x.shape[-1] else 0
     # Few rows and little work: the tiles are few and the split of K is what counts; beyond, the library's larger tiles are as quick or quicker.
-    if not _matrix(w) or not 0 < M <= 256 or w.shape[0] != x.shape[-1] or w.shape[0] < 16 or w.shape[1] == 0 or M * w.numel() > 1 << 27:
+    if not _matrix(w) or w.device != x.device or not 0 < M <= 256 or w.shape[0] != x.shape[-1] or w.shape[0] < 16 or w.shape[1] == 0 or M * w.numel() > 1 << 27:
         return None
-    if torch.backends.cuda.matmul.allow_tf32 or (b is not None and (b.dtype != torch.float32 or not b.is_cuda or not b.is_contiguous())):
+    if torch.backends.cuda.matmul.allow_tf32 or (b is not None and (b.dtype != torch.float32 or b.device != x.device or not b.is_contiguous())):
         return None
     x2 = x.reshape(M, w.shape[0])
     if not _matrix(x2):

@@ -99,7 +99,7 @@ def _product(x, weights, biases, act, as_layers=False):
     plain, bias16, apart, w, b = not fp32 and len(weights) == 1 and N % 8 == 0, False, False, [0, 0, 0], [0, 0, 0]  # plain: a matrix as the products read it
     for i, t in enumerate(weights):
         w[i] = t.data_ptr()
-        if not t.is_contiguous() or not rows and w[i] % 16:
+        if t.device != x.device or not t.is_contiguous() or not rows and w[i] % 16:
             return None
     biased = any(t is not None for t in biases)
     if as_layers:
@@ -109,7 +109,7 @@ def _product(x, weights, biases, act, as_layers=False):
             return None
     if biased:
         kinds = {t.dtype for t in biases if t is not None}
-        if len(kinds) > 1 or not kinds <= {_F32, _BF16} or not all(t is None or t.is_contiguous() for t in biases):
+        if len(kinds) > 1 or not kinds <= {_F32, _BF16} or not all(t is None or t.is_contiguous() and t.device == x.device for t in biases):
             return None
         bias16 = kinds == {_BF16}
         if plain and not bias16:  # a bias is read in the layer's type wherever it is read
@@ -156,7 +156,7 @@ def _ordinary(layer):
 
 def _input(layer, x):
     """The input in the layer's type where its shape has passed the layer's checks before, else ``None``."""
-    if type(x) is not torch.Tensor or not x.is_cuda:
+    if type(x) is not torch.Tensor or not x.is_cuda or x.get_device() != dispatch._current_device():
         return None
     if x.dtype != _BF16:
         if not x.dtype.is_floating_point or not layer.__dict__["autocast"] or not layer.__dict__["_convert_input_args"]:
@@ -241,7 +241,7 @@ def _norm_parts(layer, x):
         t = v
         if v is not None:
             t = v._value if type(v) is Variable and v._shard_slices is None else None
-            if t is None or not t.is_cuda or t.ndim != 1 or t.shape[0] != x.shape[-1]:
+            if t is None or t.device != x.device or t.ndim != 1 or t.shape[0] != x.shape[-1]:
                 return None
             if t.dtype == _BF16 and not torch.is_grad_enabled():
                 t = t.float()
@@ -271,7 +271,7 @@ def _merge_inputs(layer, inputs):
     if not _ordinary(layer) or not d["autocast"] or d["_reshape_required"] or d["_input_spec"] is not None or len(inputs) != 2:
         return None
     a, b = inputs
-    if type(a) is not torch.Tensor or type(b) is not torch.Tensor or a.dtype != _BF16 or b.dtype != _BF16 or a.shape != b.shape or not a.is_cuda or not b.is_cuda:
+    if type(a) is not torch.Tensor or type(b) is not torch.Tensor or a.dtype != _BF16 or b.dtype != _BF16 or a.shape != b.shape or not a.is_cuda or b.device != a.device:
         return None
     m, n = getattr(a, "_keras_mask", None), getattr(b, "_keras_mask", None)
     if m is None or n is None:
@@ -318,12 +318,12 @@ _EMBED = [_V] * 3 + [_L, _I, _L] + [_I] * 4 + [_V]
 
 def _embedding(layer, ids):
     d = layer.__dict__
-    if not _ordinary(layer) or d["lora_enabled"] or d["_input_spec"] is not None or type(ids) is not torch.Tensor or not ids.is_cuda:
+    if not _ordinary(layer) or d["lora_enabled"] or d["_input_spec"] is not None or type(ids) is not torch.Tensor or not ids.is_cuda or ids.get_device() != dispatch._current_device():
         return None
     if ids.dtype not in (torch.int32, torch.int64) or getattr(ids, "_keras_mask", None) is not None or ids.numel() == 0:
         return None
     table = _stored(d.get("_embeddings"))
-    if table is None or table.ndim != 2 or table.shape[1] % 8 or not table.is_contiguous() or table.data_ptr() % 16 or not ids.is_contiguous():
+    if table is None or table.device != ids.device or table.ndim != 2 or table.shape[1] % 8 or not table.is_contiguous() or table.data_ptr() % 16 or not ids.is_contiguous():
         return None
     V, D = table.shape
     out = torch.empty(ids.shape + (D,), dtype=_BF16, device=ids.device)

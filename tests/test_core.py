@@ -119,3 +119,19 @@ def test_the_kernels_switch_is_read_from_the_environment_in_force(monkeypatch):
             assert config.fused_kernels_enabled() is on
         monkeypatch.delitem(os.environ, "KERAS_B200_DISABLE_FUSED_KERNELS")
         assert config.fused_kernels_enabled()
+
+
+def test_kernels_take_tensors_of_the_current_device_alone(monkeypatch):
+    """Launches go to the current device; what lies on another one is the library's."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from keras_b200.kernels import dispatch
+
+    with FakeTensorMode():
+        tensors = [torch.empty(2, 8, device=f"cuda:{i}") for i in range(2)]
+        labels = [torch.zeros(2, dtype=torch.long, device=f"cuda:{i}") for i in range(2)]
+    for current in range(2):
+        monkeypatch.setattr(dispatch, "_current_device", lambda: current)
+        assert [dispatch.enabled(t) for t in tensors] == [current == 0, current == 1]
+        assert dispatch.softmax_cross_entropy(tensors[current], labels[1 - current]) is None
+        assert dispatch.dense(tensors[1 - current], None, None, None) is None

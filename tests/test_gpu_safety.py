@@ -175,3 +175,30 @@ def test_order_independent_kernels_return_the_same_bits_twice():
     first, second = once(), once()
     for u, v in zip(first, second):
         assert torch.equal(u, v)
+
+
+def test_operands_of_two_devices_are_refused_as_before():
+    """Weights, labels or ids on the host reach no kernel: the library raises, or the call is left to it."""
+    import keras_b200 as keras
+    from keras_b200.kernels import dispatch, gemm, sgemm
+    from keras_b200.models import direct
+
+    x = torch.randn(64, 128, device="cuda")
+    layer = keras.layers.Dense(256)
+    layer.build((None, 128))
+    for v in layer.variables:
+        v._value.data = v._value.data.cpu()
+    with pytest.raises(RuntimeError):
+        layer(x)
+    w, b = (v._value.detach() for v in layer.variables)
+    layer.kernel._value.data = w.cuda()
+    assert sgemm.dense(x, layer._kernel, layer.bias, None) is None
+    x16, w16 = x.bfloat16(), w.bfloat16()
+    assert gemm.dense(x16, w16, None, None) is None and gemm.matmul(x16, w16) is None and gemm.dense(x16, w16.cuda(), b, None) is None
+    assert direct._product(x16, [w], [None], 0) is None and direct._product(x16, [w.cuda()], [b], 0) is None
+    with pytest.raises(RuntimeError):
+        keras.ops.sparse_categorical_crossentropy(torch.zeros(64, dtype=torch.long), x[:, :10], from_logits=True)
+    assert dispatch.softmax_cross_entropy(x, torch.zeros(64, dtype=torch.long)) is None
+    assert dispatch.embedding(None, x, torch.zeros(3, dtype=torch.long), torch.float32) is None
+    one = torch.ones((), device="cuda")
+    assert dispatch.running_mean(one, one.cpu()) is None and dispatch.running_mean(one, one, one.cpu()) is None
