@@ -36,14 +36,19 @@ _slot_observer = None
 
 def set_slot_observer(fn):
     """``fn(param)`` is called whenever ``grad_slot`` hands out a parameter's gradient storage, that is, just before a kernel
-    adds a contribution to it (the data-parallel engine counts these to know when a gradient is complete).  ``None`` clears."""
+    adds a contribution to it (the data-parallel engine counts these to know when a gradient is complete, and those that autograd
+    accumulates by a hook of its own on every parameter).  ``None`` clears."""
     global _slot_observer
     _slot_observer = fn
 
 
 def grad_slot(param, shape=None):
-    """``param.grad`` when a kernel may accumulate into it: inside ``arena_backward``, fp32, contiguous, 16-byte aligned."""
-    if _arena_backward_depth <= 0 or param is None:
+    """``param.grad`` when a kernel may accumulate into it: inside ``arena_backward``, fp32, contiguous, 16-byte aligned, and nobody but the observer
+    below has hooks on the parameter, which are to see its gradient."""
+    if _arena_backward_depth <= 0 or param is None or param._backward_hooks:
+        return None
+    after = param._post_accumulate_grad_hooks
+    if after and len(after) > (1 if _slot_observer is not None else 0):
         return None
     g = param.grad
     if g is None or g.dtype != torch.float32 or g.requires_grad or not g.is_contiguous() or g.data_ptr() % 16:

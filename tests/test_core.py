@@ -135,3 +135,33 @@ def test_kernels_take_tensors_of_the_current_device_alone(monkeypatch):
         assert [dispatch.enabled(t) for t in tensors] == [current == 0, current == 1]
         assert dispatch.softmax_cross_entropy(tensors[current], labels[1 - current]) is None
         assert dispatch.dense(tensors[1 - current], None, None, None) is None
+
+
+def test_hooks_on_a_parameter_see_its_gradient():
+    """A kernel that adds its gradient in place sends none through autograd: not for parameters with hooks."""
+    from keras_b200.kernels import shadow
+
+    def parameter():
+        p = torch.nn.Parameter(torch.zeros(4))
+        p.grad = torch.zeros(4)
+        return p
+
+    def has_slot(p):
+        return shadow.grad_slot(p, (4,)) is not None
+
+    plain, hooked, after, observed = (parameter() for _ in range(4))
+    handle = hooked.register_hook(lambda g: None)
+    after.register_post_accumulate_grad_hook(lambda q: None)
+    observed.register_post_accumulate_grad_hook(lambda q: None)
+    assert not has_slot(plain)
+    with shadow.arena_backward():
+        assert has_slot(plain) and not has_slot(hooked) and not has_slot(after)
+        handle.remove()
+        assert has_slot(hooked)
+        shadow.set_slot_observer(lambda q: None)
+        try:
+            assert has_slot(observed) and has_slot(plain)
+            observed.register_post_accumulate_grad_hook(lambda q: None)
+            assert not has_slot(observed)
+        finally:
+            shadow.set_slot_observer(None)

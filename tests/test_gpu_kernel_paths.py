@@ -722,3 +722,35 @@ def test_gelu_of_a_matrix(rows, cols):
     y, want = kops.gelu(z), z.double() * torch.special.erfc(z.double() * -(0.5 ** 0.5)) / 2  # without the cancellation of 1 + erf
     assert torch.equal(y[0, :4].isnan(), want[0, :4].isnan()) and y[0, 0] == float("inf") and y[0, 3] == 0
     assert torch.allclose(y.double(), want, rtol=2.0 ** -8, atol=1e-36, equal_nan=True)  # one rounding; the distribution function within 2.5e-6
+
+
+@pytest.mark.parametrize("policy", ["float32", "mixed_bfloat16"])
+def test_gradient_hooks_see_the_gradients_of_a_training_step(policy):
+    import keras_b200 as keras
+
+    def steps(hooked):
+        L = keras.layers
+        keras.utils.set_random_seed(8)
+        keras.config.set_dtype_policy(policy)
+        try:
+            i = keras.Input((40,), dtype="int32")
+            h = L.Embedding(30, 32)(i)
+            h = L.LSTM(16)(h) if policy == "float32" else L.GlobalAveragePooling1D()(L.LayerNormalization()(h))
+            model = keras.Model(i, L.Dense(64)(L.Dense(64, activation="relu")(h)))
+        finally:
+            keras.config.set_dtype_policy("float32")
+        model.compile(keras.optimizers.SGD(0.1), keras.losses.SparseCategoricalCrossentropy(from_logits=True), run_eagerly=True)
+        seen = {}
+        if hooked:
+            for v in model.trainable_variables:
+                v._value.register_hook(lambda g, _p=v.path: seen.setdefault(_p, []).append(None if g is None else g.detach().clone()))
+        g = torch.Generator(device="cuda").manual_seed(1)
+        for _ in range(4):
+            model.train_on_batch(torch.randint(0, 30, (64, 40), generator=g, device="cuda", dtype=torch.int32), torch.randint(0, 64, (64,), generator=g, device="cuda"))
+        return model, seen
+
+    model, seen = steps(True)
+    assert set(seen) == {v.path for v in model.trainable_variables}
+    assert all(len(gs) == 4 and all(g is not None and g.any() for g in gs) for gs in seen.values()), {p: [g is not None for g in gs] for p, gs in seen.items()}
+    for a, b in zip(model.trainable_variables, steps(False)[0].trainable_variables):
+        assert _rel(a.value, b.value.detach().double()) < (1e-5 if policy == "float32" else 1e-2)  # gradients in fp32 either way; rounded to bf16 on their way to a hook
