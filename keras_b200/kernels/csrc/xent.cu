@@ -150,16 +150,18 @@ __global__ void __launch_bounds__(XE_THREADS) xent_bwd_check_kernel(const T* __r
 // xent_classes.cu
 constexpr int XE_FEW = 64;
 int kb200_xent_classes_fwd(const void* logits, const long long* labels, float* loss, float* lse, long long rows, int V, long long ld, int vec, int dtype,
-                           cudaStream_t stream);
+                           int* outside, cudaStream_t stream);
 int kb200_xent_classes_bwd(const void* logits, const long long* labels, const float* lse, const float* dloss, int dloss_stride, void* dlogits, long long rows, int V,
                            long long ld, int zero_to, int vec, int dtype, cudaStream_t stream);
 
-KB_API int kb200_xent_fwd(const void* logits, const long long* labels, float* loss, float* lse, long long rows, int V, long long ld, int dtype,
+// outside: an int in host memory that the kernel can write, set where fewer than 64 classes meet a label that is none of them (nor the ignored
+// -100); or null.
+KB_API int kb200_xent_fwd(const void* logits, const long long* labels, float* loss, float* lse, long long rows, int V, long long ld, int dtype, int* outside,
                           cudaStream_t stream) {
   if (rows <= 0) return 0;
   const int esize = dtype == 1 ? 2 : 4;
   const int vec = (((uintptr_t)logits & 15) == 0 && (ld * esize) % 16 == 0) ? 1 : 0;
-  if (V < XE_FEW && rows * 32 < (1ll << 38)) return kb200_xent_classes_fwd(logits, labels, loss, lse, rows, V, ld, vec, dtype, stream);
+  if (V < XE_FEW && rows * 32 < (1ll << 38)) return kb200_xent_classes_fwd(logits, labels, loss, lse, rows, V, ld, vec, dtype, outside, stream);
   if (V <= XE_NARROW && rows * 32 < (1ll << 38)) {
     if (dtype == 1) xe_narrow_fwd<__nv_bfloat16>((const __nv_bfloat16*)logits, labels, loss, lse, rows, V, ld, vec, stream);
     else xe_narrow_fwd<float>((const float*)logits, labels, loss, lse, rows, V, ld, vec, stream);

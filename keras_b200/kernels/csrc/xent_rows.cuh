@@ -45,6 +45,11 @@ __device__ __forceinline__ void xe_store(T* p, const float* v) {
 // The running maximum starts at the lowest finite value, not at -inf: a masked class (-inf) then adds exp(-inf) = 0 from the first on, and
 // needs no test of its own (one in this loop cost [16384, 50257] fp32 520 -> 1176 us).
 constexpr float XE_LOWEST = -3.402823466e38f;
+
+// Labels outside the classes.  A vocabulary's are ignored: loss and gradient zero.  A classifier's (`strict`) are mistakes, but for the -100 that the
+// library's loss ignores: both are NaN, and the host is told through `outside` (in its memory; may be null).
+constexpr long long XE_IGNORED = -100;
+__device__ __forceinline__ bool xe_mistaken(long long t, int V, int strict) { return strict && (t < 0 || t >= V) && t != XE_IGNORED; }
 __device__ __forceinline__ void xe_online(float v, float& m, float& s) {
   if (v > m) {
     s = s * XE_EXP(m - v) + 1.f;
@@ -63,7 +68,7 @@ constexpr int XE_NARROW = 2048;  // 8 vectors a lane at G = 32; beyond it a CTA 
 template <typename T, int G>
 __global__ void __launch_bounds__(256) xent_narrow_fwd_kernel(const T* __restrict__ logits, const long long* __restrict__ labels,
                                                               float* __restrict__ loss, float* __restrict__ lse_out, long long rows, int V, long long ld,
-                                                              int vec) {
+                                                              int vec, int strict, int* outside) {
   constexpr int VN = XeVec<T>::N;
   const int gl = threadIdx.x & (G - 1);
   const long long row = (long long)blockIdx.x * (256 / G) + threadIdx.x / G;
@@ -95,15 +100,17 @@ __global__ void __launch_bounds__(256) xent_narrow_fwd_kernel(const T* __restric
   if (live && gl == 0) {
     const float lse = gm + logf(s);
     const long long t = labels[row];
+    const bool mistaken = xe_mistaken(t, V, strict);
     lse_out[row] = lse;
-    loss[row] = (t >= 0 && t < V) ? lse - to_f32<T>(l[t]) : 0.f;
+    loss[row] = (t >= 0 && t < V) ? lse - to_f32<T>(l[t]) : mistaken ? NAN : 0.f;
+    if (mistaken && outside != nullptr) *reinterpret_cast<volatile int*>(outside) = 1;
   }
 }
 
 template <typename T, int G>
 __global__ void __launch_bounds__(256) xent_narrow_bwd_kernel(const T* __restrict__ logits, const long long* __restrict__ labels,
                                                               const float* __restrict__ lse, const float* __restrict__ dloss, int ds, T* __restrict__ dlogits,
-                                                              long long rows, int V, long long ld, int Vz, int vec) {
+                                                              long long rows, int V, long long ld, int Vz, int vec, int strict) {
   constexpr int VN = XeVec<T>::N;
   const int gl = threadIdx.x & (G - 1);
   const long long row = (long long)blockIdx.x * (256 / G) + threadIdx.x / G;
@@ -112,7 +119,7 @@ __global__ void __launch_bounds__(256) xent_narrow_bwd_kernel(const T* __restric
   T* d = dlogits + row * ld;
   const float r_lse = lse[row];
   const long long t = labels[row];
-  const float g = (t >= 0 && t < V) ? dloss[row * ds] : 0.f;
+  const float g = (t >= 0 && t < V) ? dloss[row * ds] : xe_mistaken(t, V, strict) ? NAN : 0.f;
   const int body = vec ? (V / VN) * VN : 0;
   for (int i = gl * VN; i < body; i += G * VN) {
     float v[VN];
@@ -142,23 +149,24 @@ static int xe_lanes(int V, int vec, int vn) {
 }
 
 template <typename T>
-static void xe_narrow_fwd(const T* logits, const long long* labels, float* loss, float* lse, long long rows, int V, long long ld, int vec, cudaStream_t st) {
+static void xe_narrow_fwd(const T* logits, const long long* labels, float* loss, float* lse, long long rows, int V, long long ld, int vec, cudaStream_t st,
+                          int strict = 0, int* outside = nullptr) {
   const int g = xe_lanes(V, vec, XeVec<T>::N);
   const unsigned grid = (unsigned)((rows * g + 255) / 256);
-  if (g == 4) xent_narrow_fwd_kernel<T, 4><<<grid, 256, 0, st>>>(logits, labels, loss, lse, rows, V, ld, vec);
-  else if (g == 8) xent_narrow_fwd_kernel<T, 8><<<grid, 256, 0, st>>>(logits, labels, loss, lse, rows, V, ld, vec);
-  else if (g == 16) xent_narrow_fwd_kernel<T, 16><<<grid, 256, 0, st>>>(logits, labels, loss, lse, rows, V, ld, vec);
-  else xent_narrow_fwd_kernel<T, 32><<<grid, 256, 0, st>>>(logits, labels, loss, lse, rows, V, ld, vec);
+  if (g == 4) xent_narrow_fwd_kernel<T, 4><<<grid, 256, 0, st>>>(logits, labels, loss, lse, rows, V, ld, vec, strict, outside);
+  else if (g == 8) xent_narrow_fwd_kernel<T, 8><<<grid, 256, 0, st>>>(logits, labels, loss, lse, rows, V, ld, vec, strict, outside);
+  else if (g == 16) xent_narrow_fwd_kernel<T, 16><<<grid, 256, 0, st>>>(logits, labels, loss, lse, rows, V, ld, vec, strict, outside);
+  else xent_narrow_fwd_kernel<T, 32><<<grid, 256, 0, st>>>(logits, labels, loss, lse, rows, V, ld, vec, strict, outside);
 }
 
 template <typename T>
 static void xe_narrow_bwd(const T* logits, const long long* labels, const float* lse, const float* dloss, int ds, T* dlogits, long long rows, int V, long long ld,
-                          int Vz, int vec, cudaStream_t st) {
+                          int Vz, int vec, cudaStream_t st, int strict = 0) {
   const int g = xe_lanes(V, vec, XeVec<T>::N);
   const unsigned grid = (unsigned)((rows * g + 255) / 256);
-  if (g == 4) xent_narrow_bwd_kernel<T, 4><<<grid, 256, 0, st>>>(logits, labels, lse, dloss, ds, dlogits, rows, V, ld, Vz, vec);
-  else if (g == 8) xent_narrow_bwd_kernel<T, 8><<<grid, 256, 0, st>>>(logits, labels, lse, dloss, ds, dlogits, rows, V, ld, Vz, vec);
-  else if (g == 16) xent_narrow_bwd_kernel<T, 16><<<grid, 256, 0, st>>>(logits, labels, lse, dloss, ds, dlogits, rows, V, ld, Vz, vec);
-  else xent_narrow_bwd_kernel<T, 32><<<grid, 256, 0, st>>>(logits, labels, lse, dloss, ds, dlogits, rows, V, ld, Vz, vec);
+  if (g == 4) xent_narrow_bwd_kernel<T, 4><<<grid, 256, 0, st>>>(logits, labels, lse, dloss, ds, dlogits, rows, V, ld, Vz, vec, strict);
+  else if (g == 8) xent_narrow_bwd_kernel<T, 8><<<grid, 256, 0, st>>>(logits, labels, lse, dloss, ds, dlogits, rows, V, ld, Vz, vec, strict);
+  else if (g == 16) xent_narrow_bwd_kernel<T, 16><<<grid, 256, 0, st>>>(logits, labels, lse, dloss, ds, dlogits, rows, V, ld, Vz, vec, strict);
+  else xent_narrow_bwd_kernel<T, 32><<<grid, 256, 0, st>>>(logits, labels, lse, dloss, ds, dlogits, rows, V, ld, Vz, vec, strict);
 }
 }  // namespace

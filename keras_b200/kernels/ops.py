@@ -553,6 +553,27 @@ def expect_upstream(fn):
         _EXPECTED.upstream = fn
 
 
+_OUTSIDE = []
+
+
+def _outside_flag():
+    """The address of the flag that the kernels for a handful of classes raise: host memory, which is read for nothing once a step is done."""
+    if not _OUTSIDE:
+        if torch.cuda.is_current_stream_capturing():
+            return _vp(0)  # no allocation now; the loss is NaN all the same
+        flag = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+        _OUTSIDE.extend((flag.numpy(), flag))
+    return _p(_OUTSIDE[1])
+
+
+def check_labels():
+    """Raise if a loss that has been computed met a label that is none of its classes (fewer than 64: a vocabulary's are ignored).  Does not
+    synchronise: called where results have been read."""
+    if _OUTSIDE and _OUTSIDE[0][0]:
+        _OUTSIDE[0][0] = 0
+        raise ValueError("sparse_categorical_crossentropy met a label outside [0, number of classes): the loss and the gradients of that step are NaN.")
+
+
 class FusedSoftmaxXent(torch.autograd.Function):
     """Per-row loss in float32 from logits of any float dtype.  Logits may be the leading columns of a wider buffer
     (rows with a uniform pitch, as a padded GEMM returns them); the gradient then has the same pitch and zeroed padding."""
@@ -560,6 +581,7 @@ class FusedSoftmaxXent(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits, labels):
         lib = _lib()
+        check_labels()
         V = logits.shape[-1]
         rows = logits.numel() // V
         flat = logits.reshape(rows, V)  # a view whenever the leading dimensions collapse
@@ -578,7 +600,7 @@ class FusedSoftmaxXent(torch.autograd.Function):
             _check(lib.kb200_xent_fwd_grad(_p(flat), _p(labels64), _p(loss), _p(lse), _p(ctx.made), _f(ctx.made_for), _ll(rows), _i(V), _ll(ld), _i(zero_to),
                                            _i(_dt(flat)), _stream()), "xent_fwd_grad")
         else:
-            _check(lib.kb200_xent_fwd(_p(flat), _p(labels64), _p(loss), _p(lse), _ll(rows), _i(V), _ll(ld), _i(_dt(flat)), _stream()), "xent_fwd")
+            _check(lib.kb200_xent_fwd(_p(flat), _p(labels64), _p(loss), _p(lse), _ll(rows), _i(V), _ll(ld), _i(_dt(flat)), _outside_flag(), _stream()), "xent_fwd")
         # the input itself, for a gradient of the gradient; its rows again only where they were copied
         ctx.save_for_backward(logits, flat if flat.data_ptr() != logits.data_ptr() else None, labels64, lse)
         ctx.ld, ctx.zero_to = ld, zero_to

@@ -602,9 +602,8 @@ class Trainer:
 
             kgemm.check_errors()
             kattention.check_errors()
-            from keras_b200.kernels import ops as kops
-
             kops.check_stream_kernels()
+            kops.check_labels()
 
     def train_on_batch(self, x, y=None, sample_weight=None, class_weight=None, return_dict=False):
         self._assert_compile_called("train_on_batch")
@@ -618,6 +617,7 @@ class Trainer:
         self.reset_metrics()
         logs = self.train_function([data])
         logs = pythonify_logs(logs)
+        kops.check_labels()
         if return_dict:
             return logs
         return self._flatten_metrics_in_order(logs)
@@ -629,6 +629,7 @@ class Trainer:
         self.make_test_function()
         self.reset_metrics()
         logs = pythonify_logs(self.test_function([data]))
+        kops.check_labels()
         if return_dict:
             return logs
         return self._flatten_metrics_in_order(logs)

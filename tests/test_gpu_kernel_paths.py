@@ -587,6 +587,45 @@ def test_cross_entropy_of_few_classes(rows, V, ld, dtype, spread):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("V", [2, 10, 63])
+@pytest.mark.parametrize("bad", [-1, -101, 1 << 40, None])
+def test_a_label_that_is_no_class_is_refused(V, dtype, bad):
+    """NaN in its row and an error at the next look; -100 is ignored, as by the library."""
+    from keras_b200.kernels import ops as kops
+
+    logits = torch.randn(5, V, device="cuda").to(dtype).requires_grad_(True)
+    labels = torch.tensor([0, -100, V if bad is None else bad, V - 1, 1], device="cuda")
+    loss = kops.FusedSoftmaxXent.apply(logits, labels)
+    (grad,) = torch.autograd.grad(loss, logits, torch.ones(5, device="cuda"))
+    assert loss.isnan().tolist() == [False, False, True, False, False] and grad[2].isnan().all() and not grad[[0, 1, 3, 4]].isnan().any()
+    assert loss[1] == 0 and not grad[1].any()
+    with pytest.raises(ValueError, match="label outside"):
+        kops.check_labels()
+    kops.check_labels()
+    kops.FusedSoftmaxXent.apply(logits, labels.clamp(0, V - 1))
+    torch.cuda.synchronize()
+    kops.check_labels()
+
+
+@pytest.mark.parametrize("recorded", [True, False])
+def test_training_on_a_label_that_is_no_class_raises(recorded):
+    import keras_b200 as keras
+
+    model = keras.Sequential([keras.Input((8,)), keras.layers.Dense(5)])
+    model.compile("sgd", keras.losses.SparseCategoricalCrossentropy(from_logits=True), jit_compile="auto" if recorded else False)
+    x, y = torch.randn(16, 8, device="cuda"), torch.arange(16, device="cuda") % 5
+    for _ in range(6):
+        model.train_on_batch(x, y)
+    assert not recorded or model._graphed_step.replays
+    with pytest.raises(ValueError, match="label outside"):
+        model.train_on_batch(x, y + 1)
+    with pytest.raises(ValueError, match="label outside"):
+        model.test_on_batch(x, y + 1)
+    with pytest.raises(ValueError, match="label outside"):
+        model.fit(x, y + 1, batch_size=16, epochs=1, verbose=0)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("V,ld", [(2, 2), (10, 10), (37, 40), (63, 63), (64, 64), (300, 304), (2049, 2056)])
 @pytest.mark.parametrize("layout", ["rows", "columns", "expected"])
 def test_cross_entropy_second_derivatives(V, ld, dtype, layout):
