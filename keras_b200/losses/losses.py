@@ -10,6 +10,7 @@ from keras_b200.core import config
 from keras_b200.core.export_registry import keras_export
 from keras_b200.core.tensor import convert_to_tensor
 from keras_b200.losses.loss import Loss, squeeze_or_expand_to_same_rank
+from keras_b200.ops.nn import sparse_cross_entropy_values
 
 _EPS = config.epsilon
 
@@ -33,7 +34,7 @@ class LossFunctionWrapper(Loss):
         if self.fn is not sparse_categorical_crossentropy or not isinstance(y_pred, torch.Tensor) or y_pred.dtype != torch.bfloat16:
             return False
         kw = self._fn_kwargs
-        if not kw.get("from_logits") or kw.get("ignore_class") is not None or kw.get("axis", -1) not in (-1, y_pred.ndim - 1):
+        if type(self).call is not LossFunctionWrapper.call or not kw.get("from_logits") or kw.get("ignore_class") is not None or kw.get("axis", -1) not in (-1, y_pred.ndim - 1):
             return False
         from keras_b200.kernels import dispatch
 
@@ -47,6 +48,8 @@ class LossFunctionWrapper(Loss):
         y_true_y_pred = tree.map_structure(squeeze_or_expand_to_same_rank, y_true, y_pred)
         y_true = tree.map_structure_up_to(y_true, lambda x: x[0], y_true_y_pred)
         y_pred = tree.map_structure_up_to(y_pred, lambda x: x[1], y_true_y_pred)
+        if self._accepts_low_precision(y_pred):
+            return sparse_cross_entropy_values(y_true, y_pred, True, keep_float32=True)
         return self.fn(y_true, y_pred, **self._fn_kwargs)
 
     def get_config(self):

@@ -506,6 +506,11 @@ def categorical_crossentropy(target, output, from_logits=False, axis=-1):
 
 @op("nn")
 def sparse_categorical_crossentropy(target, output, from_logits=False, axis=-1):
+    return sparse_cross_entropy_values(target, output, from_logits, axis)
+
+
+def sparse_cross_entropy_values(target, output, from_logits=False, axis=-1, keep_float32=False):
+    """``sparse_categorical_crossentropy`` of tensors; ``keep_float32``: of 16-bit logits too."""
     target, output = _loss_pair(target, output)
     target = target.long()
     if target.ndim == output.ndim and target.shape[-1] == 1:
@@ -521,11 +526,12 @@ def sparse_categorical_crossentropy(target, output, from_logits=False, axis=-1):
         output = torch.movedim(output, axis, -1)
     if from_logits:
         fused = dispatch.softmax_cross_entropy(output, target)
-        if fused is not None:
-            return fused
+        if fused is not None:  # in float32, which the values of a classifier leave as the library's do
+            return fused if output.shape[-1] >= 64 or keep_float32 else fused.to(output.dtype)
         flat = output.reshape(-1, output.shape[-1])
         loss = F.cross_entropy(flat.float() if flat.dtype in (torch.float16, torch.bfloat16) else flat, target.reshape(-1), reduction="none")
-        return loss.reshape(target.shape).to(output.dtype)
+        loss = loss.reshape(target.shape)
+        return loss if keep_float32 else loss.to(output.dtype)
     output = output / torch.sum(output, dim=-1, keepdim=True)
     eps = config.epsilon()
     logp = torch.log(torch.clip(output, eps, 1.0 - eps))

@@ -654,6 +654,29 @@ def test_cross_entropy_second_derivatives(V, ld, dtype, layout):
         assert _rel(a.detach(), b.detach()) < (1e-5 if dtype == torch.float32 else 2.0 ** -6)
 
 
+@pytest.mark.parametrize("V", [2, 37, 63])
+def test_cross_entropy_of_few_classes_in_the_type_of_its_logits(V):
+    """The op's values have it, rounded once; a loss object's are float32 whatever it is given, and a subclass is given float32."""
+    import keras_b200 as keras
+
+    class Own(keras.losses.SparseCategoricalCrossentropy):
+        def call(self, y_true, y_pred):
+            seen.append(y_pred.dtype)
+            return super().call(y_true, y_pred)
+
+    seen = []
+    logits, labels = torch.randn(65, V, device="cuda").bfloat16(), torch.randint(0, V, (65,), device="cuda")
+    want = torch.nn.functional.cross_entropy(logits.double(), labels, reduction="none")
+    for fn in (keras.ops.sparse_categorical_crossentropy, keras.losses.sparse_categorical_crossentropy):
+        values = fn(labels, logits, from_logits=True)
+        assert values.dtype == torch.bfloat16 and torch.allclose(values.double(), want, rtol=2.0 ** -8, atol=1e-6)
+        assert fn(labels, logits.float(), from_logits=True).dtype == torch.float32
+    for kind in (keras.losses.SparseCategoricalCrossentropy, Own):
+        loss = kind(from_logits=True, reduction=None)(labels, logits)
+        assert loss.dtype == torch.float32 and torch.allclose(loss.double(), want, rtol=5e-7, atol=2e-6)
+    assert seen == [torch.float32]
+
+
 def test_running_means_round_as_their_operations():
     import keras_b200 as keras
 
