@@ -24,8 +24,8 @@ def _groups(batch, units):
 
 
 def takes(sequences, initial_state, cell):
-    """float32 tensors on one device, a batch and a width that the launch holds."""
-    if not _plain(sequences) or sequences.ndim != 3 or sequences.shape[0] == 0 or sequences.shape[1] == 0 or len(initial_state) != 2:
+    """float32 tensors on one device, a batch and a width that the launch holds; no ``torch.autocast``, whose products are 16-bit."""
+    if torch.is_autocast_enabled("cuda") or not _plain(sequences) or sequences.ndim != 3 or sequences.shape[0] == 0 or sequences.shape[1] == 0 or len(initial_state) != 2:
         return False
     weights = [cell.kernel, cell.recurrent_kernel] + ([cell.bias] if cell.bias is not None else [])
     if any(getattr(w, "_shard_slices", None) is not None for w in weights):
@@ -100,7 +100,7 @@ def _target(variable, tensor):
 def project(sequences, kernel):
     """The projected inputs of all time steps, for operands that ``takes`` has let through."""
     W = kernel.value if hasattr(kernel, "value") else kernel
-    if torch.is_grad_enabled() and W.requires_grad and W.ndim == 2 and W.shape[0] == sequences.shape[-1] and not torch.is_autocast_enabled("cuda"):
+    if torch.is_grad_enabled() and W.requires_grad and W.ndim == 2 and W.shape[0] == sequences.shape[-1]:
         return Project.apply(sequences, W, _target(kernel, W))
     return torch.matmul(sequences, W)
 

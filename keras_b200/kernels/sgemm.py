@@ -1,7 +1,7 @@
 """Front-end of the float32 products of few rows (``csrc/sgemm.cu``): dense layers under the float32 policy.
 
 A product, its bias and its rectifier are one launch; backward the rectifier's derivative and the bias gradient are one, and the weight
-gradient is added where it is kept.  Larger layers, and any where the caller allows TF32, stay with the library.
+gradient is added where it is kept.  Larger layers, and any where the caller allows TF32 or is inside ``torch.autocast``, stay with the library.
 """
 
 import ctypes
@@ -110,7 +110,7 @@ def dense(x, kernel, bias, activation_name):
     # Few rows and little work: the tiles are few and the split of K is what counts; beyond, the library's larger tiles are as quick or quicker.
     if not _matrix(w) or w.device != x.device or not 0 < M <= 256 or w.shape[0] != x.shape[-1] or w.shape[0] < 16 or w.shape[1] == 0 or M * w.numel() > 1 << 27:
         return None
-    if torch.backends.cuda.matmul.allow_tf32 or (b is not None and (b.dtype != torch.float32 or b.device != x.device or not b.is_contiguous())):
+    if torch.backends.cuda.matmul.allow_tf32 or torch.is_autocast_enabled("cuda") or (b is not None and (b.dtype != torch.float32 or b.device != x.device or not b.is_contiguous())):
         return None
     x2 = x.reshape(M, w.shape[0])
     if not _matrix(x2):

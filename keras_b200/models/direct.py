@@ -52,7 +52,7 @@ def usable(x):
             and not layer_module._NVTX_RANGES and get_stateless_scope() is None
             and all(global_state.get_global_attribute(a) is None for a in _ATTRIBUTES)
             and not torch._C._len_torch_function_stack() and not torch._C._len_torch_dispatch_stack()
-            and not torch.compiler.is_compiling() and torch._C._get_tracing_state() is None
+            and not torch.is_autocast_enabled("cuda") and not torch.compiler.is_compiling() and torch._C._get_tracing_state() is None
             and all(getattr(c, m) is f for (c, m), f in zip(_METHODS, _STOCK)))
 
 

@@ -520,6 +520,36 @@ def test_exported_and_traced_layers_take_any_batch(policy, tmp_path):
             assert _rel(traced(x[:n]).float(), layer.call(x[:n]).double()) < tol, n
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_autocast_reaches_layers_of_any_batch(dtype):
+    """The products of a float32 layer are the library's, in the type that the caller asked for, on both sides of the rules for kernels."""
+    import keras_b200 as keras
+
+    dense, lstm = keras.layers.Dense(64, activation="relu"), keras.layers.LSTM(16)
+    x = torch.randn(300, 12, 48, device="cuda")
+    want = dense(x[:, 0]), lstm(x)
+    with torch.autocast("cuda", dtype=dtype):
+        for n in (8, 300):
+            for layer, inputs, ref in ((dense, x[:n, 0], want[0]), (lstm, x[:n], want[1])):
+                # one product in 16 bits a step, twelve steps that forget
+                assert 1e-5 < _rel(layer(inputs).float(), ref[:n].detach().double()) < 2.0 ** -6
+
+
+def test_models_in_16_bits_under_autocast_repeat_themselves():
+    import keras_b200 as keras
+
+    keras.config.set_dtype_policy("mixed_bfloat16")
+    try:
+        i = keras.Input((64,))
+        model = keras.Model(i, keras.layers.Dense(64)(keras.layers.Dense(64, activation="gelu")(i)))
+    finally:
+        keras.config.set_dtype_policy("float32")
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.float16):
+        x = torch.randn(9, 64, device="cuda")
+        first, second = model(x), model(x)
+    assert first.dtype == second.dtype and torch.equal(first, second)
+
+
 # ------------------------------------------------------------------------------------------------ a recorded step that reads a rounded batch
 @pytest.mark.parametrize("reader", [None, "dense", "float32", "mixed_float16", "mixed_bfloat16"])
 def test_recorded_step_copies_what_it_reads(reader):
