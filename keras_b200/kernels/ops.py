@@ -733,8 +733,11 @@ def add_rows(dst, src):
 
 
 def running_mean(total, count, value=None):
-    """Whether the running-mean kernels take these single numbers: float32 on one CUDA device."""
+    """Whether the running-mean kernels take these single numbers: float32 on one CUDA device, of which nobody takes a gradient (a metric may be
+    computed from numbers of a caller's own)."""
     tensors = (total, count) if value is None else (total, count, value)
+    if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
+        return False
     return all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.dtype == torch.float32 and t.ndim == 0 and t.device == total.device
                for t in tensors)
 

@@ -727,6 +727,15 @@ def test_running_means_round_as_their_operations():
     assert torch.isnan(mean.result())
 
 
+def test_a_running_mean_of_given_numbers_has_gradients():
+    import keras_b200 as keras
+
+    mean = keras.metrics.Mean()
+    total, count = (torch.tensor(v, device="cuda", requires_grad=True) for v in (3.0, 2.0))
+    grads = torch.autograd.grad(mean.stateless_result([total, count]), (total, count))
+    assert [float(g) for g in grads] == [0.5, -0.75]
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("shape", [(2, 3, 3, 8), (4, 9, 9, 96), (24, 18, 18, 384), (32, 32, 32, 256)])
 @pytest.mark.parametrize("residual", [False, True])
