@@ -39,6 +39,7 @@ struct GemmParams {
   const float* row_scale = nullptr;  // [M] and [N] factors applied to the accumulator (int8 de-quantisation)
   const float* col_scale = nullptr;
   const __nv_bfloat16* bias16 = nullptr;  // a bias in bf16 (instead of `bias`): a layer's 16-bit read of it needs no cast
+  int slice_rows = 0;                // with split_k > 1: rows from one slice's result to the next (multiples of 32); 0: they are added up in C
   int accumulate = 0;                // 1: add the fp32 tile into C (TMA reduce store) instead of overwriting it
   // Several products in one launch (1: a single one), with operands of their own and everything else in common:
   //   side by side (sum_k = 0): B and C differ, N is the widest; tile_end: end of each product's column tiles
@@ -188,9 +189,9 @@ __device__ __forceinline__ void apply_act32(float* v, int act) {
 // 32 x 128 B staging buffer (`stage`: two such buffers, 1024-byte aligned) and lets the TMA engine store that box, so
 // global memory sees full 128-byte lines and rows/columns beyond M/N are clipped by the tensor map.  `stores` counts
 // the boxes this warp has issued (selects the staging buffer).  Lane 0 must run `cp.async.bulk.wait_group.read 0` before
-// the CTA exits.
+// the CTA exits.  `down`: rows that the result lies further down in C.
 __device__ __forceinline__ void store_rows_tma(uint32_t tmem_row, int ncols, int n0, int row0, uint32_t stage, uint32_t& stores,
-                                               const CUtensorMap* map_c, const GemmParams& p, int lane, int N, const float* bias, const __nv_bfloat16* bias16) {
+                                               const CUtensorMap* map_c, const GemmParams& p, int lane, int N, const float* bias, const __nv_bfloat16* bias16, int down = 0) {
   const int cols_per_chunk = p.out_fp32 ? 32 : 64;
   const int chunks = ncols / cols_per_chunk;
   const uint32_t sw = (uint32_t)(lane & 7);
@@ -262,12 +263,12 @@ __device__ __forceinline__ void store_rows_tma(uint32_t tmem_row, int ncols, int
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if (lane == 0 && row0 < p.M) {
-      if (p.split_k > 1 || p.accumulate) {
+      if ((p.split_k > 1 && p.slice_rows == 0) || p.accumulate) {
         asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map_c),
-                     "r"(stage + (stores & 1u) * 4096u), "r"(col0), "r"(row0) : "memory");
+                     "r"(stage + (stores & 1u) * 4096u), "r"(col0), "r"(row0 + down) : "memory");
       } else {
         asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map_c),
-                     "r"(stage + (stores & 1u) * 4096u), "r"(col0), "r"(row0) : "memory");
+                     "r"(stage + (stores & 1u) * 4096u), "r"(col0), "r"(row0 + down) : "memory");
       }
       asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     }
@@ -282,11 +283,11 @@ __device__ __forceinline__ void store_rows_tma(uint32_t tmem_row, int ncols, int
 }
 // the same for the tile's product of a group
 __device__ __forceinline__ void store_rows_group(uint32_t tmem_row, int ncols, int n0, int row0, uint32_t stage, uint32_t& stores, const GroupMaps& maps, int g,
-                                                 const GemmParams& p, int lane) {
+                                                 const GemmParams& p, int lane, int slice) {
   const bool one = p.groups == 1;
   const void* bias = one ? (p.bias16 != nullptr ? (const void*)p.bias16 : (const void*)p.bias) : p.bias_of[g];
   store_rows_tma(tmem_row, ncols, n0, row0, stage, stores, &maps.c[g], p, lane, one ? p.N : p.width[g], p.bias16 != nullptr ? nullptr : (const float*)bias,
-                 p.bias16 != nullptr ? (const __nv_bfloat16*)bias : nullptr);
+                 p.bias16 != nullptr ? (const __nv_bfloat16*)bias : nullptr, slice * p.slice_rows);
 }
 // product of a column tile, and the column tiles before it
 __device__ __forceinline__ int group_of_tile(const GemmParams& p, int nt, int& first) {

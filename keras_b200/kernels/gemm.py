@@ -59,11 +59,14 @@ def _sm_count(device):
 
 
 def split_k_for(M, N, K, device):
-    """K slices for an accumulated product (weight gradients: small M x N, K = tokens): those with the least waves x (K blocks + 10), the ten
-    for a unit's start and for adding its tile.  Against the time of 1 to 20 slices at eleven sizes it finds the best within 4 %:
-    [768, 2304, 16384] 55.2 -> 46.8 us in five slices (two, which fill a wave to three quarters, before), [512, 512, 2664] 10.1 -> 8.8."""
+    """K slices for an accumulated product (weight gradients: small M x N, K = tokens), which add their tiles as they come; so only where there
+    is much to gain, and the other products repeat bit for bit.  Those with the least waves x (K blocks + 10), the ten for a unit's start and
+    for adding its tile.  Against the time of 1 to 20 slices at eleven sizes it finds the best within 4 %: [768, 2304, 16384] 55.2 -> 46.8 us in five
+    slices (two, which fill a wave to three quarters, before), [512, 512, 2664] 10.1 -> 8.8."""
     sms = _sm_count(device)
     one, pair, blocks = -(-M // 128) * -(-N // 256), -(-M // 256) * -(-N // 256), -(-K // 64)
+    if one * 2 > sms or K < 2048:
+        return 1
     best, slices = None, 1
     for s in range(1, min(16, blocks // 3) + 1):
         per = -(-blocks // s)
@@ -79,11 +82,26 @@ def split_k_for(M, N, K, device):
 
 
 def input_gradient_slices(M, K, N, device):
-    """K slices for dX[M, K] = dY[M, N] W^T, whose result is bf16: a few tiles that each walk a vocabulary are worth a float32 sum that is cleared
-    and rounded ([2664, 512, 8009] 37.8 -> 28.9 us, [300, 768, 50257] 492 -> 56; [4096, 512, 8009] 38.3 and 39.8)."""
+    """K slices for dX[M, K] = dY[M, N] W^T, whose result is bf16: a few tiles that each walk a vocabulary are worth float32 results of their own and
+    a pass that adds them, in order ([2664, 512, 8009] 37.8 -> 28.9 us, [300, 768, 50257] 492 -> 56; [4096, 512, 8009] 38.3 and 39.8)."""
     tiles = -(-M // 128) * -(-K // 256)
     slices = min(_sm_count(device) // tiles, N // 512, 16)
     return slices if N >= 4096 and slices >= 3 else 1
+
+
+def input_gradient(dy, w, M, K, N):
+    """``dy @ w^T``, the sum over ``N`` columns, in bf16; the same bits every time."""
+    slices = input_gradient_slices(M, K, N, dy.device)
+    if slices == 1 or K % 8:
+        return gemm(dy, w, 0, 0, M, K, N)
+    lib = kops._lib()
+    lib.kb200_gemm_slices_floats.restype = ctypes.c_longlong
+    part = torch.empty(lib.kb200_gemm_slices_floats(kops._i(M), kops._i(K), kops._i(slices)), dtype=torch.float32, device=dy.device)
+    out = torch.empty((M, K), dtype=torch.bfloat16, device=dy.device)
+    code = lib.kb200_gemm_bf16_slices(kops._p(dy), kops._p(w), kops._p(out), kops._p(part), kops._i(M), kops._i(K), kops._i(N), kops._ll(dy.stride(0)), kops._ll(w.stride(0)),
+                                      kops._i(0), kops._i(0), kops._i(slices), kops._p(_err_flag(dy.device)), kops._stream())
+    kops._check(code, "gemm_bf16_slices")
+    return out
 
 
 def gemm(a, b, a_mn, b_mn, M, N, K, bias=None, act=0, out_dtype=torch.bfloat16, split_k=1, accumulate_into=None):
@@ -199,7 +217,7 @@ class GemmFn(torch.autograd.Function):
             dy = kops.aligned(dy)
         dx = dw = db = None
         if ctx.needs_input_grad[0]:
-            dx = gemm(dy, w, 0, 0, M, K, N, split_k=input_gradient_slices(M, K, N, x.device))  # the sum ends at N; below, the columns behind it stay columns of their own
+            dx = input_gradient(dy, w, M, K, N)  # the sum ends at N; below, the columns behind it stay columns of their own
         if ctx.needs_input_grad[1]:
             split = split_k_for(K, Np, M, x.device)
             g = shadow.grad_slot(ctx.grad_target, (K, N)) if Np == N and N % 4 == 0 else None

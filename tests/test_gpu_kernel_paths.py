@@ -792,6 +792,26 @@ def test_dense_gradients_in_slices(M, K, N):
     gemm.check_errors()
 
 
+@pytest.mark.parametrize("M,K,N", [(128, 64, 4096), (130, 256, 8009), (2664, 512, 8009), (300, 768, 12000), (31, 72, 5000), (1900, 512, 512), (1024, 1024, 3072),
+                                   (2047, 768, 2304), (5000, 2048, 2560)])
+def test_dense_gradients_repeat_bit_for_bit(M, K, N):
+    """Slices of a vocabulary are added in order; weight gradients over fewer than 2048 rows, or whose tiles fill half of the chip, are one slice."""
+    from keras_b200.kernels import gemm
+
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16().requires_grad_(True)
+    w = (torch.randn(K, N, generator=g, device="cuda") * K ** -0.5).bfloat16().requires_grad_(True)
+    up = torch.randn(M, N, generator=g, device="cuda").bfloat16()
+    y = gemm.GemmFn.apply(x, w, None, None, None)
+    first = torch.autograd.grad(y, (x, w), up, retain_graph=True)
+    assert _rel(first[0], up.double() @ w.detach().double().t()) < 2.0 ** -8  # exact products, fp32 sums, one rounding
+    for _ in range(5):
+        again = torch.autograd.grad(y, (x, w), up, retain_graph=True)
+        assert torch.equal(first[0], again[0])
+        assert M >= 2048 and K * N < 1 << 21 or torch.equal(first[1], again[1])
+    gemm.check_errors()
+
+
 def test_embedding_gradient_goes_into_the_arena():
     import keras_b200 as keras
     from keras_b200.kernels import shadow
