@@ -62,13 +62,14 @@ def split_k_for(M, N, K, device):
     """K slices for an accumulated product (weight gradients: small M x N, K = tokens), which add their tiles as they come; so only where there
     is much to gain, and the other products repeat bit for bit.  Those with the least waves x (K blocks + 10), the ten for a unit's start and
     for adding its tile.  Against the time of 1 to 20 slices at eleven sizes it finds the best within 4 %: [768, 2304, 16384] 55.2 -> 46.8 us in five
-    slices (two, which fill a wave to three quarters, before), [512, 512, 2664] 10.1 -> 8.8."""
+    slices (two, which fill a wave to three quarters, before), [512, 512, 2664] 10.1 -> 8.8.  Few tiles over very many rows take all SMs: cold,
+    [512, 64, 200704] 58 us in 37 slices and 86 in 16, [32, 24, 100352] 17 in 143 and 44."""
     sms = _sm_count(device)
     one, pair, blocks = -(-M // 128) * -(-N // 256), -(-M // 256) * -(-N // 256), -(-K // 64)
     if one * 2 > sms or K < 2048:
         return 1
     best, slices = None, 1
-    for s in range(1, min(16, blocks // 3) + 1):
+    for s in range(1, min(max(16, sms // one), blocks // 3) + 1):
         per = -(-blocks // s)
         if per * (s - 1) >= blocks:
             continue  # fewer slices hold as much

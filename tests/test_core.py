@@ -165,3 +165,15 @@ def test_hooks_on_a_parameter_see_its_gradient():
             assert not has_slot(observed)
         finally:
             shadow.set_slot_observer(None)
+
+
+def test_slices_of_tall_weight_gradients_fill_the_chip(monkeypatch):
+    """Few tiles over very many rows: one slice a streaming multiprocessor, or as many as K has blocks for."""
+    from keras_b200.kernels import gemm
+
+    monkeypatch.setattr(gemm, "_sm_count", lambda device: 148)
+    for M, N, K, tiles in ((512, 64, 200704, 4), (160, 96, 100352, 2), (32, 24, 100352, 1), (1024, 64, 30000, 8), (256, 128, 8192, 2)):
+        slices = gemm.split_k_for(M, N, K, None)
+        assert 0.8 * min(148, K // 256) <= slices * tiles <= 148, (M, N, K, slices)
+    for M, N, K in ((512, 512, 2047), (2048, 2560, 5000), (64, 64, 100)):
+        assert gemm.split_k_for(M, N, K, None) == 1
