@@ -155,7 +155,7 @@ def _ordinary(layer):
 
 
 def _input(layer, x):
-    """The input in the layer's type where its shape has passed the layer's checks before, else ``None``."""
+    """The input in the layer's type where its shape passes the layer's checks, else ``None``."""
     if type(x) is not torch.Tensor or not x.is_cuda or x.get_device() != dispatch._current_device():
         return None
     if x.dtype != _BF16:
@@ -166,8 +166,14 @@ def _input(layer, x):
         if mask is not None:
             return None  # the ordinary call knows whether the mask outlives the cast
     spec = layer.__dict__["_input_spec"]
-    if spec is not None and layer.__dict__.get("_spec_checked") != (id(spec), x.shape, x.dtype):
-        return None
+    if spec is not None:
+        seen = (id(spec), x.shape, x.dtype)
+        if layer.__dict__.get("_spec_checked") != seen:
+            try:
+                layer_module.assert_input_compatibility(spec, x, layer.name)
+            except Exception:
+                return None  # the ordinary call raises it
+            layer.__dict__["_spec_checked"] = seen
     return x
 
 

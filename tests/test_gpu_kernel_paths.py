@@ -261,6 +261,42 @@ def test_dense_called_directly_has_the_bits_of_its_own_call(policy, M, K, N, act
     assert taken is not None and torch.equal(own, taken)
 
 
+def test_direct_calls_at_every_new_batch(monkeypatch):
+    """Sizes that alternate, and one that is new, are called directly throughout; a wrong one raises what the layer's own call raises."""
+    import keras_b200 as keras
+    from keras_b200.models import direct
+
+    keras.config.set_dtype_policy("mixed_bfloat16")
+    try:
+        i = keras.Input((None, 64))
+        model = keras.Model(i, keras.layers.Dense(96)(keras.layers.LayerNormalization()(keras.layers.Dense(128, activation="gelu")(i))))
+        narrow = keras.layers.Dense(64)
+        narrow(torch.zeros(2, 32, device="cuda"))
+    finally:
+        keras.config.set_dtype_policy("float32")
+    taken, plain = [], direct._dense
+
+    def counted(layer, x):
+        out = plain(layer, x)
+        taken.append(out is not None)
+        return out
+
+    monkeypatch.setattr(direct, "_dense", counted)
+    with torch.no_grad():
+        model(torch.randn(2, 5, 64, device="cuda"))
+        for b, t in ((2, 5), (3, 7), (2, 5), (3, 7), (200, 9)):
+            x = torch.randn(b, t, 64, device="cuda")
+            del taken[:]
+            mine = model(x)
+            assert taken == [True, True], (b, t)
+            with monkeypatch.context() as m:
+                m.setattr(direct, "usable", lambda x: False)
+                assert torch.equal(mine, model(x))
+        assert plain(narrow, torch.randn(2, 64, device="cuda").bfloat16()) is None
+    with pytest.raises(ValueError, match="incompatible"):
+        narrow(torch.zeros(2, 64, device="cuda"))
+
+
 def test_direct_calls_see_every_change_of_a_layer(monkeypatch):
     import keras_b200 as keras
     from keras_b200.models import direct
