@@ -425,14 +425,31 @@ def _sub_ordinary(layer):
 
 
 # ------------------------------------------------------------------------------------------------ the graph
-_PLANS = weakref.WeakKeyDictionary()  # beside the graphs, not in them: a copied or pickled graph has other layers
+class _Plan:
+    """What was found in a graph.  It lives in the graph, and so no longer than the layers: one that was kept beside it held their weights until
+    a collection after the one that took the graph.  A copied or pickled graph has other layers, and none."""
+
+    __slots__ = ("nodes", "runs", "pairs", "__weakref__")
+
+    def __init__(self, nodes):
+        self.nodes = nodes
+        self.runs, self.pairs = _build_plan(nodes)
+
+    def __deepcopy__(self, memo):
+        return None
+
+    def __reduce__(self):
+        return type(None), ()
+
+
+_PLANS = weakref.WeakValueDictionary()  # the plans in use, by the graph's identity: clearing it has them made anew
 
 
 def plan_of(function, nodes):
-    plan = _PLANS.get(function)
-    if plan is None or plan[0] is not nodes:
-        plan = _PLANS[function] = (nodes, *_build_plan(nodes))
-    return plan[1:]
+    plan = function.__dict__.get("_direct_plan")
+    if plan is None or plan.nodes is not nodes or _PLANS.get(id(function)) is not plan:
+        plan = function.__dict__["_direct_plan"] = _PLANS[id(function)] = _Plan(nodes)
+    return plan.runs, plan.pairs
 
 
 def _build_plan(nodes):

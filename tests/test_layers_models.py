@@ -200,3 +200,25 @@ def test_recorded_inputs_note_who_reads_the_batch_itself():
 
     assert read("bfloat16") == read("mixed_bfloat16", "bfloat16") == set()
     assert read("bfloat16", "float32") == read("float16", "bfloat16") == read("bfloat16", channels=3) == {0}
+
+
+def test_the_plan_of_a_graph_lives_as_long_as_the_graph():
+    import copy
+    import gc
+    import pickle
+    import weakref
+
+    from keras_b200.models import direct
+
+    i = keras.Input((8,))
+    model = keras.Model(i, layers.Dense(4)(layers.Dense(8)(i)))
+    nodes = model._ordered_nodes()
+    plan = direct.plan_of(model, nodes)
+    assert direct.plan_of(model, nodes)[0] is plan[0] and direct.plan_of(model, list(nodes))[0] is not plan[0]
+    for other in (copy.deepcopy(model), pickle.loads(pickle.dumps(model)), copy.copy(model)):
+        mine = other._ordered_nodes()
+        assert direct.plan_of(other, mine)[0] is not plan[0] and set(direct.plan_of(other, mine)[0]) <= {id(n) for n in mine}
+    kept = [weakref.ref(model), weakref.ref(model.layers[1]), weakref.ref(model.layers[1].kernel._value)]
+    del model, i, nodes, plan, other, mine
+    gc.collect()
+    assert [w() for w in kept] == [None] * 3
