@@ -673,7 +673,11 @@ struct ClusterPlan {
 };
 
 template <int R>
-void fill_plan(ClusterPlan& c, int S, int U) {
+bool allow_plan(const ClusterPlan& c, int U);
+
+// false: the device refuses a kernel
+template <int R>
+bool fill_plan(ClusterPlan& c, int S, int U) {
   const int kw = U <= 64 ? 4 : U <= 128 ? 8 : U <= 192 ? 12 : 16;
   c.rows = R;
   c.threads = cluster_threads<R>();
@@ -682,6 +686,7 @@ void fill_plan(ClusterPlan& c, int S, int U) {
   c.backward = lstm_cluster_backward_kernel<R>;
   c.smem_forward = ((size_t)c.tiles * 2 * R * GEMV_WARPS * kw + 2 * GEMV_WARPS * R * COLS + (size_t)c.tiles * c.threads) * 4;
   c.smem_backward = ((size_t)c.tiles * 2 * S * peer_part(R) + 2 * R * DZ_ROW + (size_t)c.tiles * UNITS * R) * 4;
+  return allow_plan<R>(c, U);
 }
 constexpr int CLUSTER_SMEM = 200 * 1024;  // above the largest of these: four tiles of ten rows, 256 units forward 174 KB, backward 110
 
@@ -691,10 +696,13 @@ bool allow(LstmKernel k) {
   if (!fine) cudaGetLastError();
   return fine;
 }
+// The kernels of a plan, asked for once per device: each one that is named is loaded, so none that the size does not take.
 template <int R>
-bool allow_rows() {
-  return allow(lstm_cluster_forward_kernel<R, 4>) && allow(lstm_cluster_forward_kernel<R, 8>) && allow(lstm_cluster_forward_kernel<R, 12>) &&
-         allow(lstm_cluster_forward_kernel<R, 16>) && allow(lstm_cluster_backward_kernel<R>);
+bool allow_plan(const ClusterPlan& c, int U) {
+  static signed char known[KB_MAX_DEVICES][4] = {{0}};  // by the K width; 0: not asked, 1: fine, -1: refused
+  signed char& slot = known[kb_device_slot()][U <= 64 ? 0 : U <= 128 ? 1 : U <= 192 ? 2 : 3];
+  if (slot == 0) slot = allow(c.forward) && allow(c.backward) ? 1 : -1;
+  return slot > 0;
 }
 
 void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int S) {
@@ -706,13 +714,13 @@ void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int S) {
 }
 
 // Clusters of `S` CTAs, one an SM, that run at once (a GPC has to hold a whole one: 7 of sixteen CTAs, 15 of eight, 33 of four on a B200), or
-// 0 where a kernel is refused.  Asked once per device and size.
+// 0 where the kernel is refused.  Asked once per device and size.
 int active_clusters(int S) {
   static int known[KB_MAX_DEVICES][CLUSTER_MAX + 1] = {{0}};  // 0: not asked; else 1 + answer
   int& slot = known[kb_device_slot()][S];
   if (slot == 0) {
     int n = 0;
-    bool fine = allow_rows<2>() && allow_rows<4>() && allow_rows<8>() && allow_rows<10>();
+    bool fine = allow(lstm_cluster_forward_kernel<10, 16>);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)S * 64);
     cfg.blockDim = dim3(cluster_threads<10>());
@@ -735,11 +743,8 @@ ClusterPlan cluster_plan(int B, int U) {
   const int each = (B + at_once - 1) / at_once;  // rows of a cluster
   const int per = (each + 9) / 10;
   c.tiles = per > TILES_MAX ? TILES_MAX : per;
-  if (each <= 2) fill_plan<2>(c, S, U);
-  else if (each <= 4) fill_plan<4>(c, S, U);
-  else if (each <= 8) fill_plan<8>(c, S, U);
-  else fill_plan<10>(c, S, U);
-  return c;
+  const bool fine = each <= 2 ? fill_plan<2>(c, S, U) : each <= 4 ? fill_plan<4>(c, S, U) : each <= 8 ? fill_plan<8>(c, S, U) : fill_plan<10>(c, S, U);
+  return fine ? c : ClusterPlan{};
 }
 
 size_t lstm_smem(int U, bool backward) {
