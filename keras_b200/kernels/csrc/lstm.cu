@@ -734,16 +734,25 @@ int active_clusters(int S) {
   return slot - 1;
 }
 
-// The smallest tile whose clusters hold all rows at once, or tiles of ten rows, several a cluster, in waves beyond that.
-ClusterPlan cluster_plan(int B, int U) {
+// The smallest tiles whose clusters hold all rows at once, up to four of ten rows a cluster, and in as many even waves as it takes beyond that: four full
+// tiles in each wave but the last leave that one half empty (1024 rows x 96 units, 20 steps: forward 294 us, even 184; the kernels above 257).
+// Clusters of eleven or twelve CTAs hold half of the SMs, one a GPC.  From the second wave on, a forward step of the kernels above, which hold all,
+// is then the shorter one where it has fewer than 10 / 17 of the rows one after the other (512 rows x 176 units: 80 rows 349 us, 40 rows 298; 1024 x 192:
+// 707 and 721); backward, what they send through L2 keeps them behind (866 and 942).
+ClusterPlan cluster_plan(int B, int U, bool backward) {
   ClusterPlan c;
   if (B <= 0 || U <= 0 || U % 4 || U > CLUSTER_UNITS) return c;
   const int S = (U + UNITS - 1) / UNITS, at_once = active_clusters(S);
   if (at_once <= 0) return c;
-  const int each = (B + at_once - 1) / at_once;  // rows of a cluster
-  const int per = (each + 9) / 10;
-  c.tiles = per > TILES_MAX ? TILES_MAX : per;
-  const bool fine = each <= 2 ? fill_plan<2>(c, S, U) : each <= 4 ? fill_plan<4>(c, S, U) : each <= 8 ? fill_plan<8>(c, S, U) : fill_plan<10>(c, S, U);
+  const int waves = (B + at_once * 10 * TILES_MAX - 1) / (at_once * 10 * TILES_MAX);
+  const int each = (B + at_once * waves - 1) / (at_once * waves);  // rows of a cluster
+  c.tiles = (each + 9) / 10;
+  if (!backward && waves > 1 && S > 10 && S <= 12) {
+    const int groups = kb_sm_count() / S, tiles = (B + ROWS - 1) / ROWS;
+    if (waves * c.tiles * 10 * 10 > (tiles + groups - 1) / groups * ROWS * 17) return ClusterPlan{};
+  }
+  const int rows = (each + c.tiles - 1) / c.tiles;
+  const bool fine = rows <= 2 ? fill_plan<2>(c, S, U) : rows <= 4 ? fill_plan<4>(c, S, U) : rows <= 8 ? fill_plan<8>(c, S, U) : fill_plan<10>(c, S, U);
   return fine ? c : ClusterPlan{};
 }
 
@@ -753,8 +762,8 @@ size_t lstm_smem(int U, bool backward) {
 }
 }  // namespace
 
-// Whether the layer runs on clusters, which need no counters.
-KB_API int kb200_lstm_clustered(int B, int U) { return cluster_plan(B, U).rows > 0 ? 1 : 0; }
+// Whether this direction of the layer runs on clusters, which need no counters.
+KB_API int kb200_lstm_clustered(int B, int U, int backward) { return cluster_plan(B, U, backward != 0).rows > 0 ? 1 : 0; }
 
 // Row groups of a launch (the length of `counters`), or 0 when the kernel does not take the layer.
 KB_API int kb200_lstm_groups(int B, int U) {
@@ -776,7 +785,7 @@ KB_API int kb200_lstm(int backward, const float* xz, const float* bias, const fl
   const int tiles = (B + ROWS - 1) / ROWS;
   LstmArgs a{xz, bias, h0, c0, R, hprev, out, hT, cT, gates, cs, dout, dhT, dcT, dz, dh0, dc0, counters, err, B, T, U, reverse,
              (U + UNITS - 1) / UNITS, (tiles + groups - 1) / groups * ROWS};
-  const ClusterPlan plan = cluster_plan(B, U);
+  const ClusterPlan plan = cluster_plan(B, U, backward != 0);
   if (plan.rows > 0) {
     a.rows_per_group = plan.rows * plan.tiles;
     cudaLaunchConfig_t cfg = {};

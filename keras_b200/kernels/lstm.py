@@ -53,7 +53,7 @@ def _composed(xz, bias, h, c, R, reverse):
 
 def _launch(backward, xz, bias, h0, c0, R, hprev, out, hT, cT, gates, cs, dout, dhT, dcT, dz, dh0, dc0, reverse):
     B, T, U = xz.shape[0], xz.shape[1], R.shape[0]
-    counters = None if kops._lib().kb200_lstm_clustered(_i(B), _i(U)) else torch.zeros(_groups(B, U), dtype=torch.int32, device=xz.device)
+    counters = None if kops._lib().kb200_lstm_clustered(_i(B), _i(U), _i(backward)) else torch.zeros(_groups(B, U), dtype=torch.int32, device=xz.device)
     p = kops._p
     code = kops._lib().kb200_lstm(_i(backward), p(xz), p(bias), p(h0), p(c0), p(R), p(hprev), p(out), p(hT), p(cT), p(gates), p(cs), p(dout), p(dhT), p(dcT),
                                   p(dz), p(dh0), p(dc0), p(counters), p(_err_flag(xz.device)), _i(B), _i(T), _i(U), _i(1 if reverse else 0), kops._stream())

@@ -14,7 +14,7 @@ def _rel(a, b):
 # every height of a row tile (2, 4, 8, 10 rows) with its remainders, every K width (64, 128, 192, 256 units), units that end inside a CTA's
 # sixteen, several tiles a cluster (300 rows), more clusters than run at once (2500 rows), the first size beyond the clusters (260)
 @pytest.mark.parametrize("B,T,U", [(1, 1, 4), (7, 2, 256), (28, 3, 256), (50, 3, 248), (64, 12, 256), (71, 3, 256), (300, 3, 256), (2500, 2, 24), (33, 3, 128),
-                                   (40, 6, 176), (64, 4, 48), (5, 6, 68), (9, 3, 260)])
+                                   (40, 6, 176), (64, 4, 48), (5, 6, 68), (9, 3, 260), (85, 3, 252), (512, 2, 176), (768, 2, 192), (1024, 2, 96), (403, 2, 256)])
 @pytest.mark.parametrize("reverse,sequence,states", [(False, True, True), (True, False, False)])
 def test_lstm_on_clusters_against_the_steps_in_64_bits(B, T, U, reverse, sequence, states):
     from keras_b200.kernels import gemm, lstm
