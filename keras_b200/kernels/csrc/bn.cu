@@ -509,16 +509,10 @@ KB_API int kb200_bn_bwd_reduce_mask(const void* dy, const void* x, const unsigne
                     : bn_reduce_launch<float>(1, x, dy, nullptr, bits, mean, invstd, M, C, sums, stream, zeroed != 0);
 }
 
-KB_API int kb200_bn_bwd_apply_mask(const void* dy, const void* x, const unsigned char* bits, const float* mean, const float* invstd,
-                                   const float* gamma, const float* sums, float* /*coef*/, void* dx, void* dres, long long M, int C, int dtype,
-                                   cudaStream_t stream) {
-  return bn_bwd_apply_any(dy, x, nullptr, bits, mean, invstd, gamma, sums, dx, dres, M, C, dtype, stream);
-}
-
-// As kb200_bn_bwd_apply_mask; in addition the gradients of gamma and beta are ADDED into dgamma_acc / dbeta_acc (fp32 [C],
+// As kb200_bn_bwd_apply, with the bit mask; in addition the gradients of gamma and beta are ADDED into dgamma_acc / dbeta_acc (fp32 [C],
 // either may be null): persistent gradient storage, so that no separate accumulation kernel runs.
 KB_API int kb200_bn_bwd_apply_mask_acc(const void* dy, const void* x, const unsigned char* bits, const float* mean, const float* invstd,
-                                       const float* gamma, const float* sums, float* /*coef*/, void* dx, void* dres, float* dgamma_acc,
+                                       const float* gamma, const float* sums, void* dx, void* dres, float* dgamma_acc,
                                        float* dbeta_acc, long long M, int C, int dtype, cudaStream_t stream) {
   return bn_bwd_apply_any(dy, x, nullptr, bits, mean, invstd, gamma, sums, dx, dres, M, C, dtype, stream, dgamma_acc, dbeta_acc);
 }

@@ -211,7 +211,7 @@ int launch(const SgemmParams& p, long long tiles, cudaStream_t stream) {
 // and SM; 77 us with the sums (the library's product 102 and sums 16), 32 x 1024 17 us (51).  The loop runs at 70 % of that rate with 8 x 8
 // sums a thread and 16 warps an SM, as it does with 16 x 8 and 8 warps.
 constexpr int WN = 128, WK = 16, W_STAGES = 3;
-constexpr int w_places(int wm) { return wm == 32 ? 6 : 4; }  // CTAs an SM: shared memory of 31 KB each, and 128 registers a thread
+constexpr int w_places(int wm) { return wm == 32 ? 6 : 4; }  // CTAs an SM: shared memory of 31 or 37 KB each, and 128 registers a thread
 
 struct WgradParams {
   const float* a;

@@ -343,7 +343,7 @@ class FusedBatchNormAct(torch.autograd.Function):
         st = _stream()
         dt = _dt(x)
         _check(lib.kb200_bn_bwd_reduce_mask(_p(dy), _p(x), _p(bits), _p(mean), _p(invstd), _ll(M), _i(C), _i(dt), _p(sums), _i(1 if cleared else 0), st), "bn_bwd_reduce")
-        _check(lib.kb200_bn_bwd_apply_mask_acc(_p(dy), _p(x), _p(bits), _p(mean), _p(invstd), _p(gamma), _p(sums), _vp(0), _p(dx), _p(dres),
+        _check(lib.kb200_bn_bwd_apply_mask_acc(_p(dy), _p(x), _p(bits), _p(mean), _p(invstd), _p(gamma), _p(sums), _p(dx), _p(dres),
                                                _p(slot_g), _p(slot_b), _ll(M), _i(C), _i(dt), st), "bn_bwd_apply")
         dgamma = sums[C:2 * C] if gamma is not None and slot_g is None else None
         dbeta = sums[:C] if slot_b is None else None
