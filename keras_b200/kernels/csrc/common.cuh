@@ -137,7 +137,7 @@ __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { retu
 // log2(Phi(-a) e^(a^2/2) / t) on 0 <= a <= 14 with the least maximum error (a linear program over 6000 Chebyshev points gives its
 // coefficients; 6e-7 relative, in float32 9e-7 for a < 1 and 2.5e-6 for a < 6, where the exponent's rounding is most of it).  For results
 // that are rounded to bf16; those stored as float32 take erff where it is nearer (gemm_sm100.cuh).  Sixteen instructions, two of them on the special-function pipe; 1 + erf(v / sqrt(2))
-// takes twice as many and loses its relative accuracy for negative v.  [16384, 3072, 768] with gelu in the epilogue: 117 -> 94 us.
+// takes twice as many and loses its relative accuracy for negative v.  [16384, 3072, 768] with gelu in the epilogue: 90 us, without 67.
 __device__ __forceinline__ float normal_cdf(float v) {
   const float a = fabsf(v), t = __fdividef(1.f, fmaf(0.35f, a, 1.f)), x = a * 0.8493218002880191f;  // x^2 = a^2 log2(e) / 2
   float p = -0.2692641317844391f;

@@ -126,7 +126,7 @@ def test_lstm_layer_weight_gradients_in_place_and_twice(F, bias):
 @pytest.mark.parametrize("M,K,widths", [(1, 64, (64,)), (7, 72, (72,)), (77, 768, (1001,)), (128, 200, (264,)), (128, 3072, (64, 64, 128)), (33, 256, (1024, 256, 256)),
                                         (129, 64, (64,)), (300, 200, (1001,)), (257, 768, (192, 64, 64)), (130, 512, (4099,))])
 def test_inference_products_read_weights_as_stored(M, K, widths, fp32):
-    """Up to 128 rows straight from the weight, above through one bf16 matrix; any width, one weight or three, every epilogue."""
+    """Few rows straight from the weight, more through one bf16 matrix; any width, one weight or three, every epilogue."""
     from keras_b200.kernels import gemm
     from keras_b200.models import direct
 
@@ -214,7 +214,7 @@ def test_layers_called_directly_agree_with_their_own_calls(policy, batch, monkey
             own = model(ids)
             monkeypatch.undo()
         assert mine.shape == own.shape and mine.dtype == own.dtype
-        # bf16 throughout, some ten roundings deep; the direct calls round parameters of norms and biases less often
+        # bf16 throughout, some ten roundings deep; bit for bit below
         assert _rel(mine.float(), own.double()) < 0.02, name
         a, b = getattr(mine, "_keras_mask", None), getattr(own, "_keras_mask", None)
         assert (a is None) == (b is None) and (a is None or torch.equal(a, b))
