@@ -39,13 +39,19 @@ def weight_gradient(a, b, target=None, bias_target=None, sums=False):
     return c if slot is None else None, db if db_slot is None else None
 
 
+def _tf32():
+    """Whether the caller lets the library round the operands of float32 products.  Asked by the newer of the two settings, which knows of both: once
+    it is used, reading ``allow_tf32`` raises."""
+    return torch.backends.cuda.matmul.fp32_precision not in ("none", "ieee")
+
+
 def takes_weight_gradient(K, M, N, sums):
     """Whether ``weight_gradient`` is the quicker one, against the library's product and, with ``sums``, its column sums (us):
 
     with sums     6400 rows, 256 x 1024 118 -> 77; 128 rows, 256 x 1024 9.1 -> 7.6; beyond, 2000 rows, 512 x 2048 92 -> 107
     without       6400 rows, 32 x 1024 51 -> 17; few rows, 512 of 256 x 1024 11.3 -> 12.9; one column, 102400 of 1 x 400 45 -> 95
     many rows     102400 of 256 x 1024 with sums 1164 -> 1086, without 1066 -> 1086, and 1168 -> 1277 where 250 columns are copied singly"""
-    if not 0 < M <= 256 or N <= 0 or K <= 0 or torch.backends.cuda.matmul.allow_tf32:
+    if not 0 < M <= 256 or N <= 0 or K <= 0 or _tf32():
         return False
     if K > 32768 and M > 128 and (M % 4 or not sums):
         return False
@@ -110,7 +116,7 @@ def dense(x, kernel, bias, activation_name):
     # Few rows and little work: the tiles are few and the split of K is what counts; beyond, the library's larger tiles are as quick or quicker.
     if not _matrix(w) or w.device != x.device or not 0 < M <= 256 or w.shape[0] != x.shape[-1] or w.shape[0] < 16 or w.shape[1] == 0 or M * w.numel() > 1 << 27:
         return None
-    if torch.backends.cuda.matmul.allow_tf32 or torch.is_autocast_enabled("cuda") or (b is not None and (b.dtype != torch.float32 or b.device != x.device or not b.is_contiguous())):
+    if _tf32() or torch.is_autocast_enabled("cuda") or (b is not None and (b.dtype != torch.float32 or b.device != x.device or not b.is_contiguous())):
         return None
     x2 = x.reshape(M, w.shape[0])
     if not _matrix(x2):

@@ -177,3 +177,18 @@ def test_slices_of_tall_weight_gradients_fill_the_chip(monkeypatch):
         assert 0.8 * min(148, K // 256) <= slices * tiles <= 148, (M, N, K, slices)
     for M, N, K in ((512, 512, 2047), (2048, 2560, 5000), (64, 64, 100)):
         assert gemm.split_k_for(M, N, K, None) == 1
+
+
+def test_float32_kernels_ask_for_tf32_by_either_setting():
+    """Code in a process of its own: the settings cannot be unset."""
+    import subprocess
+    import sys
+
+    template = "import torch; {}; from keras_b200.kernels import sgemm; print(sgemm.takes_weight_gradient(6400, 256, 1024, True))"
+    matmul = "torch.backends.cuda.matmul"
+    settings = {"pass": "True", f"{matmul}.allow_tf32 = True": "False", f"{matmul}.fp32_precision = 'tf32'": "False", "torch.backends.fp32_precision = 'tf32'": "False",
+                f"{matmul}.fp32_precision = 'ieee'": "True"}
+    runs = {s: subprocess.Popen([sys.executable, "-c", template.format(s)], stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True) for s in settings}
+    for setting, run in runs.items():
+        out, err = run.communicate(timeout=300)
+        assert out.strip() == settings[setting], (setting, out, err[-400:])
